@@ -365,6 +365,7 @@ int kifmm_plan_create(const kifmm_kernel *kernel, int32_t nequiv, int32_t ncutof
             P->num_sms = sms > 0 ? sms : 148;
             prepare_pool(P->device);
             init_log_table(P->device);
+            log_table(P->device);
             P->hpin = pinned_acquire();
             if (o.stream) {
                 P->stream = (cudaStream_t)o.stream;

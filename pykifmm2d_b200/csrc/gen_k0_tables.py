@@ -1,4 +1,5 @@
-"""Generate k0_tables.h: coefficients for the modified Bessel function K0.
+"""Generate k0_tables.h: coefficients for the modified Bessel function K0 and
+the Hankel function H0.
 
 Method (derived here from the mathematics, evaluated with mpmath at 50 digits):
   0 < x <= 2:  K0(x) = P(t) - log(x/2) * I0(t),  t = x^2, with the power series
@@ -9,6 +10,10 @@ Method (derived here from the mathematics, evaluated with mpmath at 50 digits):
                as a Chebyshev series in u = z/2 - 1 on [-1, 1], coefficients from
                the discrete Chebyshev transform at 64 Chebyshev nodes.
 Terms are kept while they matter at double (FP64) or single (FP32) precision.
+The FP64 pair loops (pair_f64.cuh) take the same series in the forms
+  K0(x)          = P(t) + ln(t/4) I0H(t),  I0H = -I0 / 2,
+  (i/4) H0(x)    = ln(t/4) A(t) + R(t) + i (-pi) A(t),
+  A = -J0 / (4 pi),  R = sum_k (-1)^k p_k t^k / (2 pi)  (p_k those of P; DLMF 10.8.2).
 
 Run:  python pykifmm2d_b200/csrc/gen_k0_tables.py   (rewrites k0_tables.h beside it)
 """
@@ -82,7 +87,12 @@ def main():
     out.append(" * x <= 2: K0 = P(x^2) - log(x/2) I0(x^2) with power series in t = x^2;")
     out.append(" * x >  2: K0 = exp(-x)/sqrt(x) * sum_k c_k T_k(u), u = 4/x - 1 (Chebyshev). */")
     out.append("#pragma once")
-    for name, vals, single in (("K0_I0_D", i0_64, False), ("K0_P_D", p_64, False), ("K0_CHEB_D", ch_64, False),
+    nt = len(i0_64)
+    i0h = [-v / 2 for v in i0_64]
+    h0a = [-(-1) ** k * v / (4 * mp.pi) for k, v in enumerate(i0[:nt])]
+    h0r = [(-1) ** k * v / (2 * mp.pi) for k, v in enumerate(p[:nt])]
+    for name, vals, single in (("K0_I0H_D", i0h, False), ("H0_A_D", h0a, False), ("H0_R_D", h0r, False),
+                               ("K0_I0_D", i0_64, False), ("K0_P_D", p_64, False), ("K0_CHEB_D", ch_64, False),
                                ("K0_I0_F", i0_32, True), ("K0_P_F", p_32, True), ("K0_CHEB_F", ch_32, True)):
         ty = "float" if single else "double"
         out.append(f"#define {name}_N {len(vals)}")

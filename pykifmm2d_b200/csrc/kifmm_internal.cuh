@@ -220,6 +220,7 @@ struct kifmm_plan {
     kifmm::DBuf<unsigned long long> tc_rowmax;  // [L][4Q] largest |value| per M2L operator row
     kifmm::DBuf<double> l2p_taylor;  // Laplace: [L][Q][2p+1] check potential -> Taylor coefficients
     kifmm::DBuf<double> leaf_coef;   // [n_leaf_list][2p+1] Taylor coefficients per apply
+    kifmm::DBuf<double> leaf_den;    // [n_leaf_list][Q] equivalent densities of the leaves (FP64 leaf pass)
     kifmm::DBuf<unsigned char> tc_pre;  // per-apply slices of the source groups
     kifmm::DBuf<int> tc_gexp;
     // planned applies (planned.cu): P2M, L2P and near-field blocks, built on
@@ -338,7 +339,8 @@ constexpr int KIFMM_SCAL_SORT_ERR = 13;  // a radix-sort look-back wait that ran
 constexpr int KIFMM_SCAL_PASS_ERR = 14;
 constexpr int KIFMM_SCAL_TC_ERR = 15;
 constexpr int KIFMM_SCAL_LEAF_SPLIT = 16;  // count of the split leaf list (k_leaf_split_list)
-constexpr int KIFMM_SCAL_WORDS = 17;
+constexpr int KIFMM_SCAL_TICKET = 17;      // item counter of the FP64 leaf pass (zero between launches)
+constexpr int KIFMM_SCAL_WORDS = 18;
 
 // Lanes of the warp holding the same 8-bit digit d (d = 256: no key; such
 // lanes match each other only): nine ballots, one per bit, each lane keeping
@@ -485,6 +487,7 @@ void export_lists(kifmm_plan *P, int64_t *coll, int64_t *m2l, int64_t *n_m2l, in
 void tree_stats(kifmm_plan *P);
 // operators.cu
 void build_operators(kifmm_plan *P);
+const double2 *log_table(int device); // pass_f64.cu: table of the FP64 pair loops' logarithm, once per device
 void init_log_table(int device);     // table of the Laplace P2M logarithm, once per device
 void ensure_side(kifmm_plan *P);      // side stream and its events
 void start_operators(kifmm_plan *P, bool fork_recorded = false);  // build_operators on the side stream

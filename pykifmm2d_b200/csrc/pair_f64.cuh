@@ -1,0 +1,95 @@
+// pair_f64.cuh -- FP64 kernel values for the pair loops (P2M, L2P, P2P).
+//
+// On sm_100a an SM issues 64 FP64 multiply-adds per clock but only 16 FP64
+// conversions, and the CUDA math library's log, sqrt and Bessel functions
+// cost 15 to 50 multiply-adds a call (measured: log 1.27, rsqrt 5.9, sqrt 4.4,
+// int -> double 15.4, fma 60 lane-operations per clock and SM).  The values
+// here take r^2 (no square root), one conflict-free table read and 10
+// multiply-adds for the logarithm, and short power series beside it.
+#pragma once
+#include "kifmm_internal.cuh"
+
+namespace kifmm {
+
+// Natural logarithm of a positive normal number, table-driven (P. T. P. Tang,
+// "Table-driven implementation of the logarithm function in IEEE
+// floating-point arithmetic", ACM TOMS 16, 1990): x = 2^e m with m in [1, 2),
+// c_i = 1 + (i + 1/2)/128 the midpoint of m's subinterval, v_i = 1/c_i
+// rounded to FP64, r = m v_i - 1 (|r| < 2^-8), ln x = e ln2 - ln v_i +
+// log1p(r).  log1p is its series to r^6 with r^6 economised by the Chebyshev
+// polynomial T6 (r^6 = h^6 (T6(r/h) + 48 (r/h)^4 - 18 (r/h)^2 + 1) / 32,
+// h = 2^-8), so five coefficients leave 1.9e-17; the constant it leaves goes
+// into the table.  Max error 1.8 ulp, mean 0.39 (against 60-digit values over
+// 2^-30 .. 2^5).  e comes from the exponent bits by a magic-number add.
+// The table is kept LOGTAB_COPIES times in shared memory, copy c in the 16-byte
+// bank group c: a warp's 32 16-byte reads, eight to a phase, hit eight
+// different groups whatever their entries (one copy measured 2-3 way
+// conflicts, and the reads would then bound the loop instead of the FP64 pipe).
+constexpr int LOGTAB_N = 128, LOGTAB_COPIES = 8;
+constexpr double LOG_LN2 = 0.693147180559945309417232121458176568;
+constexpr double LOG_H2 = 1.0 / 65536.0;  // h^2
+constexpr double LOG_C2 = -0.5 + LOG_H2 * LOG_H2 * 18.0 / 192.0, LOG_C3 = 1.0 / 3.0,
+                 LOG_C4 = -0.25 - LOG_H2 * 48.0 / 192.0, LOG_C5 = 0.2;
+
+// log_table(device) holds [LOGTAB_N] (v_i, -ln v_i - h^6/192); stage its copies into tab[LOGTAB_N * LOGTAB_COPIES] (all threads of the block)
+__device__ __forceinline__ void stage_log_table(double2 *tab, const double2 *__restrict__ g) {
+    for (int i = threadIdx.x; i < LOGTAB_N * LOGTAB_COPIES; i += blockDim.x) tab[i] = g[i / LOGTAB_COPIES];
+}
+
+// ln(2^EADJ x); tl: this lane's copy, tab + (lane & 7).  x positive, normal,
+// finite (pair_ordinary); anything else gives a finite or NaN value and reads
+// inside the table.
+template <int EADJ>
+__device__ __forceinline__ double ln_tab(double x, const double2 *tl) {
+    const int hi = __double2hiint(x), lo = __double2loint(x);
+    const double2 c = tl[((hi >> 13) & (LOGTAB_N - 1)) * LOGTAB_COPIES];
+    const double m = __hiloint2double((hi & 0x000fffff) | 0x3ff00000, lo);
+    const double e = __hiloint2double(0x43300000, (int)((unsigned)hi >> 20)) - (4503599627370496.0 + 1023.0 - EADJ);
+    const double r = fma(m, c.x, -1.0);
+    double q = LOG_C5;
+    q = fma(q, r, LOG_C4);
+    q = fma(q, r, LOG_C3);
+    q = fma(q, r, LOG_C2);
+    return fma(q * r, r, fma(e, LOG_LN2, c.y) + r);
+}
+
+// Number of series terms that reach FP64 precision for t = (k r)^2 below
+// 2^-4, 1 and 4: the terms are at most (H_n - gamma) t^n / (4^n (n!)^2).
+constexpr int SERIES_NARROW = 7, SERIES_MID = 10, SERIES_WIDE = 13;
+// high words of the bounds of t (t < bound iff hiword(t) < these)
+constexpr unsigned SERIES_NARROW_HI = 0x3fb00000u, SERIES_MID_HI = 0x3ff00000u, SERIES_WIDE_HI = 0x40100000u;
+template <int NT>
+__device__ __forceinline__ double series(const double *c, double t) {
+    double a = c[NT - 1];
+#pragma unroll
+    for (int i = NT - 2; i >= 0; i--) a = fma(a, t, c[i]);
+    return a;
+}
+
+// Whether t = r^2 (Laplace) or (k r)^2 is a positive normal number below the
+// bound whose high word is hi_end: those the fast values are for.
+__device__ __forceinline__ bool pair_ordinary(double t, unsigned hi_end) {
+    return (unsigned)(__double2hiint(t) - 0x00100000) < hi_end - 0x00100000u;
+}
+constexpr unsigned LOG_HI_END = 0x7ff00000u;  // every finite number
+
+// Unscaled kernel value of an ordinary pair: ln r^2 (Laplace, times
+// -1/(4 pi)) or K0(k r) = P(t) - ln(t/4) I0(t)/2 (times 1/(2 pi)).
+template <int KIND, int NT>
+__device__ __forceinline__ double pair_value(double t, const double2 *tl) {
+    if (KIND == KIFMM_KERNEL_LAPLACE) return ln_tab<0>(t, tl);
+    return fma(ln_tab<-2>(t, tl), series<NT>(K0_I0H_D, t), series<NT>(K0_P_D, t));
+}
+template <int KIND>
+__device__ __forceinline__ double pair_scale() {
+    return KIND == KIFMM_KERNEL_LAPLACE ? -0.07957747154594767 : 0.15915494309189535;
+}
+// ... of any other pair (coincident points, underflow, k r >= 2) by the math
+// library's functions; kept out of line, so that the pair loops stay small
+template <int KIND>
+__device__ __noinline__ double pair_value_any(double r2, double k) {
+    if (KIND == KIFMM_KERNEL_LAPLACE) return log(r2);
+    return k0_d(k * sqrt(r2));
+}
+
+}  // namespace kifmm

@@ -1,0 +1,312 @@
+// pass_f64.cu -- the FP64 L2P + P2P at the sources (the "plain" form's leaf
+// pass, and the mixed form's with near_fp64): class_fmm.py:73-111.
+#include <algorithm>
+#include <mutex>
+
+#include "pair_f64.cuh"
+#include "passes.cuh"
+
+namespace kifmm {
+
+__device__ double2 g_logtab[LOGTAB_N];
+const double2 *log_table(int device) {
+    static std::mutex mu;
+    static const double2 *tab[64] = {};
+    KIFMM_REQUIRE(device >= 0 && device < 64, KIFMM_ERR_ARG, "device index out of range");
+    std::lock_guard<std::mutex> lock(mu);
+    if (!tab[device]) {
+        double2 t[LOGTAB_N];
+        const long double c0 = (long double)LOG_H2 * LOG_H2 * LOG_H2 / 192.0L;
+        for (int i = 0; i < LOGTAB_N; i++) {
+            t[i].x = (double)(1.0L / (1.0L + ((long double)i + 0.5L) / LOGTAB_N));
+            t[i].y = (double)(-logl((long double)t[i].x) - c0);
+        }
+        void *p = nullptr;
+        KIFMM_CUDA(cudaMemcpyToSymbol(g_logtab, t, sizeof(t)));
+        KIFMM_CUDA(cudaGetSymbolAddress(&p, g_logtab));
+        tab[device] = (const double2 *)p;
+    }
+    return tab[device];
+}
+
+// Equivalent densities of the leaves' local expansions, phi = Inv_l u_down,
+// on the FP64 tensor path: one block per 32 consecutive leaves of one level
+// (leaf_list is level-major), warp w all Q rows for leaves 8w .. 8w + 7.  The
+// level's inverse is read once per block instead of once per leaf.
+// den[leaf_list index][Q].  Reads 4 Q^2 bytes per leaf-block from L2 and
+// 16 Q bytes per leaf: latency-bound (a few microseconds at 65k leaves).
+struct DenArgs {
+    PassArgs A;
+    const int32_t *list;
+    double *den;
+    int lmin, lmax;
+    int64_t loff[MAX_LEVELS + 1];  // leaf_list range of each level
+    int64_t toff[MAX_LEVELS + 1];  // first block of each level
+};
+constexpr int DEN_THREADS = 128, DEN_MT = 8;  // Q <= 8 DEN_MT
+static size_t den_smem(int Q) {
+    const int Kp = (Q + 3) & ~3, Mp = (Q + 7) & ~7;
+    return ((size_t)Kp * pad4mod16(Mp) + 32 * (size_t)pad4mod16(Kp)) * sizeof(double);
+}
+__global__ void __launch_bounds__(DEN_THREADS) k_leaf_density(DenArgs D) {
+    extern __shared__ __align__(16) double sm_den[];
+    const PassArgs &A = D.A;
+    const int Q = A.Q, Kp = (Q + 3) & ~3, Mp = (Q + 7) & ~7, ldm = pad4mod16(Mp), ldx = pad4mod16(Kp);
+    double *mS = sm_den;                  // [Kp][ldm]: Inv[r][c] at c * ldm + r
+    double *xS = mS + (size_t)Kp * ldm;   // [32][ldx]
+    const int tid = threadIdx.x;
+    pdl_trigger();
+    const int64_t b = blockIdx.x;
+    int l = D.lmin;
+    while (l < D.lmax && D.toff[l + 1] <= b) l++;
+    const int64_t w0 = D.loff[l] + (b - D.toff[l]) * 32;
+    const int nt = (int)min((int64_t)32, D.loff[l + 1] - w0);
+    const double *inv = A.ops + (size_t)l * A.stride + A.off_inv;
+    for (int i = tid; i < Kp * Mp; i += DEN_THREADS) {
+        const int r = i / Kp, c = i - r * Kp;
+        mS[c * ldm + r] = r < Q && c < Q ? inv[r * Q + c] : 0.0;
+    }
+    pdl_wait();  // u_down comes from the L2L chain
+    for (int i = tid; i < 32 * Kp; i += DEN_THREADS) {
+        const int n = i / Kp, c = i - n * Kp;
+        xS[n * ldx + c] = n < nt && c < Q ? A.udown[(size_t)D.list[w0 + n] * Q + c] : 0.0;
+    }
+    __syncthreads();
+    const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3, n0 = warp * 8;
+    if (n0 >= nt) return;
+    double acc[DEN_MT][2];
+#pragma unroll
+    for (int i = 0; i < DEN_MT; i++) acc[i][0] = acc[i][1] = 0.0;
+    const double *xb = xS + (size_t)(n0 + g) * ldx + t, *ab = mS + (size_t)t * ldm + g;
+    for (int k0 = 0; k0 < Kp; k0 += 4) {
+        const double bv = xb[k0];
+#pragma unroll
+        for (int i = 0; i < DEN_MT; i++)
+            if (8 * i < Mp) dmma_8x8x4(acc[i][0], acc[i][1], ab[(size_t)k0 * ldm + 8 * i], bv);
+    }
+#pragma unroll
+    for (int i = 0; i < DEN_MT; i++) {
+        const int r = 8 * i + g;
+        if (r >= Q) continue;
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+            if (n0 + 2 * t + j < nt) D.den[(size_t)(w0 + n0 + 2 * t + j) * Q + r] = acc[i][j];
+    }
+}
+
+// L2P + P2P of the leaves, one warp per item: an item is up to ts (<= 32)
+// targets of one leaf.  The warp's targets form ng groups of TB targets; sp =
+// 32 / ng lanes share a group, lane (gi, j) taking sources j, j + sp, ..., so
+// that a leaf of 28 points (the mean on the 1M mixture) keeps 28 lanes busy and
+// each source read from shared memory serves TB pairs.  The leaf's sources
+// (its own points, then its colleagues') are staged in chunks; the L2P is the
+// same loop over the Q equivalent points of the leaf's local expansion, in
+// box-relative coordinates.  Bound by the FP64 pipe: 14 FP64 instructions per
+// Laplace pair, 7 clocks of an SM per 32 pairs (0.23 ms for the 2.8e8 pairs of
+// the 1M mixture).  Warps draw items from a ticket (the leaves differ in work
+// by more than 10x); each warp draws one ticket past the end, so atomicInc's
+// wrap leaves the counter at zero for the next launch.
+constexpr int L64_CHUNK = 64;  // sources staged per pass, two per lane
+struct Leaf64Warp {
+    double2 xy[L64_CHUNK];
+    double z[L64_CHUNK];
+    double red[4][32];
+    int rng[18];
+    int pad[2];
+};
+static_assert(sizeof(Leaf64Warp) % 16 == 0, "Leaf64Warp alignment");
+
+template <int KIND, int NT, int TB>
+__device__ __forceinline__ void pair_loop(const Leaf64Warp &W, const double2 *tl, int j, int sp, int n,
+                                          const double *tx, const double *ty, double k, double k2, unsigned hi_end,
+                                          bool skip_equal, double *acc) {
+#pragma unroll 1
+    for (int u = j; u < n; u += sp) {
+        const double2 s = W.xy[u];
+        const double z = W.z[u];
+#pragma unroll
+        for (int a = 0; a < TB; a++) {
+            const double dx = tx[a] - s.x, dy = ty[a] - s.y;
+            const double r2 = fma(dx, dx, dy * dy);
+            const double t = KIND == KIFMM_KERNEL_LAPLACE ? r2 : r2 * k2;
+            double v = pair_value<KIND, NT>(t, tl), zz = z;
+            if (!pair_ordinary(t, hi_end)) {
+                const bool skip = skip_equal && dx == 0.0 && dy == 0.0;
+                v = 0.0;
+                if (skip) zz = 0.0;
+                else v = pair_value_any<KIND>(r2, k);
+            }
+            acc[a] = fma(v, zz, acc[a]);
+        }
+    }
+}
+// the near sources of the leaf, then the equivalent points of its local expansion
+template <int KIND, int NT, int TB>
+__device__ __forceinline__ double leaf_item(const PassArgs &A, Leaf64Warp &W, const double2 *tl, int t0, int nt, int ns,
+                                            int l, double cx, double cy, const double *den, unsigned hi_end,
+                                            bool check_self, double k2, int lane) {
+    const int ng = (nt + TB - 1) / TB, sp = 32 / ng, j = lane / ng, gi = lane - j * ng;
+    double tx[TB], ty[TB], acc[TB];
+#pragma unroll
+    for (int a = 0; a < TB; a++) {
+        const int i = gi + a * ng < nt ? gi + a * ng : gi;  // unused slots repeat the first
+        tx[a] = A.xs[t0 + i];
+        ty[a] = A.ys[t0 + i];
+        acc[a] = 0.0;
+    }
+    const bool idle = j >= sp;
+    for (int c0 = 0; c0 < ns; c0 += L64_CHUNK) {
+        const int cn = min(L64_CHUNK, ns - c0);
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < L64_CHUNK; h += 32) {
+            const int q = h + lane;
+            if (q < cn) {
+                const int p = range_point(W.rng, c0 + q);
+                W.xy[q] = make_double2(A.xs[p], A.ys[p]);
+                W.z[q] = A.taus[p];
+            }
+        }
+        __syncwarp();
+        pair_loop<KIND, NT, TB>(W, tl, j, sp, idle ? 0 : cn, tx, ty, A.k, k2, hi_end, check_self, acc);
+    }
+    if (l >= 2) {
+        const double *lg = A.ops + (size_t)l * A.stride + A.off_large;
+        __syncwarp();
+        for (int q = lane; q < A.Q; q += 32) {
+            W.xy[q] = make_double2(lg[q], lg[A.Q + q]);
+            W.z[q] = den[q];
+        }
+        __syncwarp();
+#pragma unroll
+        for (int a = 0; a < TB; a++) {
+            tx[a] -= cx;
+            ty[a] -= cy;
+        }
+        pair_loop<KIND, NT, TB>(W, tl, j, sp, idle ? 0 : A.Q, tx, ty, A.k, k2, hi_end, false, acc);
+    }
+#pragma unroll
+    for (int a = 0; a < TB; a++) W.red[a][lane] = acc[a];
+    __syncwarp();
+    double v = 0.0;
+    if (lane < nt) {
+        const int slot = lane / ng, grp = lane - slot * ng;
+        for (int m = 0; m < sp; m++) v += W.red[slot][grp + m * ng];
+    }
+    return v * pair_scale<KIND>();
+}
+template <int KIND, int NT>
+__device__ __forceinline__ double leaf_item_tb(const PassArgs &A, Leaf64Warp &W, const double2 *tl, int t0, int nt,
+                                               int ns, int l, double cx, double cy, const double *den, unsigned hi_end,
+                                               bool check_self, double k2, int lane) {
+    // two targets per lane, or four where that leaves fewer lanes idle
+    // (pair slots per source: TB / (32 / ceil(nt / TB)))
+    const int n2 = (nt + 1) >> 1, n4 = (nt + 3) >> 2;
+    if (4 * (32 / n2) < 2 * (32 / n4))
+        return leaf_item<KIND, NT, 4>(A, W, tl, t0, nt, ns, l, cx, cy, den, hi_end, check_self, k2, lane);
+    return leaf_item<KIND, NT, 2>(A, W, tl, t0, nt, ns, l, cx, cy, den, hi_end, check_self, k2, lane);
+}
+
+constexpr int L64_MAX_WARPS = 8;
+template <int KIND>
+__global__ void __launch_bounds__(32 * L64_MAX_WARPS, 4)
+    k_leaf_eval_d(PassArgs A, const double2 *__restrict__ logtab, const double *__restrict__ den, unsigned nitems,
+                  int ntile, int ts, int check_self, unsigned *__restrict__ ticket) {
+    extern __shared__ __align__(16) unsigned char sm_l64[];
+    double2 *tab = (double2 *)sm_l64;
+    Leaf64Warp &W = ((Leaf64Warp *)(tab + LOGTAB_N * LOGTAB_COPIES))[threadIdx.x >> 5];
+    stage_log_table(tab, logtab);
+    __syncthreads();
+    pdl_trigger();
+    pdl_wait();
+    const int lane = threadIdx.x & 31;
+    const double2 *tl = tab + (lane & (LOGTAB_COPIES - 1));
+    const double k2 = A.k * A.k;
+    const unsigned last = nitems + gridDim.x * (blockDim.x >> 5) - 1;
+    for (;;) {
+        unsigned it = 0;
+        if (lane == 0) it = atomicInc(ticket, last);
+        it = __shfl_sync(0xffffffffu, it, 0);
+        if (it >= nitems) return;
+        const unsigned w = it / ntile;
+        const int rv = A.leaf_rec[(size_t)w * LEAF_REC_WORDS + lane];
+        const int l = __shfl_sync(0xffffffffu, rv, LR_LEVEL), b = __shfl_sync(0xffffffffu, rv, LR_BOT),
+                  e = __shfl_sync(0xffffffffu, rv, LR_TOP), ns = __shfl_sync(0xffffffffu, rv, LR_NSRC);
+        const uint64_t key = (uint64_t)(uint32_t)__shfl_sync(0xffffffffu, rv, LR_KEY_LO) |
+                             ((uint64_t)(uint32_t)__shfl_sync(0xffffffffu, rv, LR_KEY_HI) << 32);
+        __syncwarp();
+        if (lane >= LR_RNG && lane < LR_RNG + 18) W.rng[lane - LR_RNG] = rv;
+        __syncwarp();
+        const double wl = ldexp(A.W, -l);
+        const double cx = A.root + ((double)compact2(key >> 1) + 0.5) * wl;
+        const double cy = A.root + ((double)compact2(key) + 0.5) * wl;
+        // targets and sources lie in 3x3 cells, equivalent points nearer: r^2 <= 8 w^2
+        const double tmax = KIND == KIFMM_KERNEL_LAPLACE ? 0.0 : 8.0 * wl * wl * k2;
+        const double *dn = den + (size_t)w * A.Q;
+        for (int t0 = b + (int)(it - w * ntile) * ts; t0 < e; t0 += ntile * ts) {
+            const int nt = min(ts, e - t0);
+            double v;
+            if (KIND == KIFMM_KERNEL_LAPLACE)
+                v = leaf_item_tb<KIND, 1>(A, W, tl, t0, nt, ns, l, cx, cy, dn, LOG_HI_END, check_self, k2, lane);
+            else if (tmax < 0.0625)
+                v = leaf_item_tb<KIND, SERIES_NARROW>(A, W, tl, t0, nt, ns, l, cx, cy, dn, SERIES_NARROW_HI, check_self,
+                                                      k2, lane);
+            else if (tmax < 1.0)
+                v = leaf_item_tb<KIND, SERIES_MID>(A, W, tl, t0, nt, ns, l, cx, cy, dn, SERIES_MID_HI, check_self, k2,
+                                                   lane);
+            else
+                v = leaf_item_tb<KIND, SERIES_WIDE>(A, W, tl, t0, nt, ns, l, cx, cy, dn, SERIES_WIDE_HI, check_self, k2,
+                                                    lane);
+            if (lane < nt) A.pots[t0 + lane] = v;
+        }
+    }
+}
+
+// the equivalent densities of the leaf list, then the leaf pass
+void launch_leaf_eval_d(kifmm_plan *P, const PassArgs &A, int check_self) {
+    const int64_t nl = P->n_leaf_list;
+    DenArgs D{};
+    D.A = A;
+    D.list = P->leaf_list.p;
+    P->leaf_den.alloc((size_t)nl * P->Q);
+    D.den = P->leaf_den.p;
+    D.lmin = 2;
+    D.lmax = P->L - 1;
+    int64_t tiles = 0;
+    for (int l = 0; l <= MAX_LEVELS; l++) {
+        D.loff[l] = P->leaf_loff[l];
+        D.toff[l] = tiles;
+        if (l >= D.lmin && l <= D.lmax && l < MAX_LEVELS) tiles += (P->leaf_loff[l + 1] - P->leaf_loff[l] + 31) / 32;
+    }
+    if (tiles) {
+        const size_t smem = den_smem(P->Q);
+        ensure_dyn_smem(k_leaf_density, smem);
+        launch_pdl(k_leaf_density, dim3((unsigned)tiles), dim3(DEN_THREADS), smem, P->stream, D);
+    }
+    // Items: whole 32-target tiles once they fill the GPU's resident warps
+    // (32 per SM); smaller tiles for fewer leaves, down to 8 targets, where a
+    // warp's run over its sources is the kernel's length.
+    const int64_t resident = (int64_t)P->num_sms * 4 * L64_MAX_WARPS;
+    int ts = 32;
+    while (ts > 8 && nl * ((P->ppl + ts - 1) / ts) < resident) ts >>= 1;
+    const int ntile = (int)std::min<int64_t>((P->ppl + ts - 1) / ts, 64);
+    const int64_t items = nl * ntile;
+    KIFMM_REQUIRE(items + resident < (1ll << 32), KIFMM_ERR_ARG, "leaf pass: too many leaves");
+    int warps = L64_MAX_WARPS;  // a block's table is shared by its warps; few items: spread them over the SMs
+    while (warps > 1 && items < (int64_t)P->num_sms * warps * 2) warps >>= 1;
+    const unsigned grid = (unsigned)std::min<int64_t>((items + warps - 1) / warps, resident / L64_MAX_WARPS);
+    const size_t smem = LOGTAB_N * LOGTAB_COPIES * sizeof(double2) + (size_t)warps * sizeof(Leaf64Warp);
+    unsigned *ticket = (unsigned *)(P->scal.p + KIFMM_SCAL_TICKET);
+    const double2 *lt = log_table(P->device);
+    if (P->kern.kind == KIFMM_KERNEL_LAPLACE) {
+        ensure_dyn_smem(k_leaf_eval_d<KIFMM_KERNEL_LAPLACE>, smem);
+        launch_pdl(k_leaf_eval_d<KIFMM_KERNEL_LAPLACE>, dim3(grid), dim3(32 * warps), smem, P->stream, A, lt,
+                   (const double *)D.den, (unsigned)items, ntile, ts, check_self, ticket);
+    } else {
+        ensure_dyn_smem(k_leaf_eval_d<KIFMM_KERNEL_MOD_HELMHOLTZ>, smem);
+        launch_pdl(k_leaf_eval_d<KIFMM_KERNEL_MOD_HELMHOLTZ>, dim3(grid), dim3(32 * warps), smem, P->stream, A, lt,
+                   (const double *)D.den, (unsigned)items, ntile, ts, check_self, ticket);
+    }
+}
+
+}  // namespace kifmm

@@ -402,64 +402,6 @@ __global__ void __launch_bounds__(MD_BLOCK, 2) k_m2l_dmma(M2lDmmaArgs M) {
     }
 }
 
-// L2P + P2P for one target leaf per block (class_fmm.py:73-111).
-__global__ void k_leaf_eval_d(PassArgs A, const int32_t *__restrict__ list, int check_self) {
-    extern __shared__ double sm[];
-    const int Q = A.Q;
-    double *qd = sm;                    // [Q] equivalent density of the local expansion
-    double *sx = sm + Q, *sy = sx + blockDim.x, *st = sy + blockDim.x;
-    int g = list[blockIdx.x];
-    int l = A.nlev[g];
-    double cx, cy;
-    node_center(A, g, l, cx, cy);
-    const double *blk = A.ops + (size_t)l * A.stride;
-    if (l >= 2) {
-        const double *inv = blk + A.off_inv;
-        for (int r = threadIdx.x; r < Q; r += blockDim.x) {
-            double s = 0.0;
-            for (int c = 0; c < Q; c++) s = fma(inv[r * Q + c], A.udown[(size_t)g * Q + c], s);
-            qd[r] = s;
-        }
-    } else {
-        for (int r = threadIdx.x; r < Q; r += blockDim.x) qd[r] = 0.0;
-    }
-    __syncthreads();
-    const double *lg = blk + A.off_large;
-    const int b = A.nbot[g], e = A.ntop[g];
-    for (int t0 = b; t0 < e; t0 += blockDim.x) {
-        int t = t0 + threadIdx.x;
-        bool act = t < e;
-        double px = act ? A.xs[t] : 0.0, py = act ? A.ys[t] : 0.0;
-        double acc = 0.0;
-        if (act && l >= 1) {
-            double tx = px - cx, ty = py - cy;
-            for (int q = 0; q < Q; q++) {
-                double dx = tx - lg[q], dy = ty - lg[Q + q];
-                acc += green_d(A.kind, A.k, dx * dx + dy * dy) * qd[q];
-            }
-        }
-        for (int d = 0; d < 9; d++) {
-            int c = A.ncoll[9 * (size_t)g + d];
-            if (c < 0) continue;
-            int cb = A.nbot[c], ce = A.ntop[c];
-            for (int s0 = cb; s0 < ce; s0 += blockDim.x) {
-                __syncthreads();
-                int s = s0 + threadIdx.x;
-                if (s < ce) { sx[threadIdx.x] = A.xs[s]; sy[threadIdx.x] = A.ys[s]; st[threadIdx.x] = A.taus[s]; }
-                __syncthreads();
-                int ns = min((int)blockDim.x, ce - s0);
-                if (act)
-                    for (int u = 0; u < ns; u++) {
-                        double dx = px - sx[u], dy = py - sy[u];
-                        if (check_self && dx == 0.0 && dy == 0.0) continue;
-                        acc += green_d(A.kind, A.k, dx * dx + dy * dy) * st[u];
-                    }
-            }
-        }
-        if (act) A.pots[t] = acc;
-    }
-}
-
 // Evaluation at arbitrary targets: locate by strict '>' descent
 // (numba_locate_points, tree.py:712-727), then L2P and P2P.
 // Targets in Morton order (sort_targets) with the leaves' equivalent densities
@@ -666,13 +608,6 @@ void build_m2l_order(kifmm_plan *P) {
 void launch_p2m_d(kifmm_plan *P, const PassArgs &A) {
 launch_pdl(k_p2m_d, dim3(grid_for(P->n_p2m_list * 32, 32 * P2M_WARPS)), dim3(32 * P2M_WARPS), 0, P->stream, A,
                (const int32_t *)P->p2m_list.p, P->n_p2m_list);
-}
-
-void launch_leaf_eval_d(kifmm_plan *P, const PassArgs &A, int check_self) {
-    int thr = P->ppl <= 64 ? 64 : 128;
-    size_t smem = (size_t)(P->Q + 3 * thr) * sizeof(double);
-    k_leaf_eval_d<<<(unsigned)P->n_leaf_list, thr, smem, P->stream>>>(A, P->leaf_list.p, check_self);
-    KIFMM_LAUNCHED();
 }
 
 void sort_targets(kifmm_plan *P, const double *tx, const double *ty, int64_t n);  // tree.cu

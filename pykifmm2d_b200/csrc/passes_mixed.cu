@@ -841,7 +841,6 @@ void launch_leaf_den(kifmm_plan *P, const PassArgs &A) {
 // m2l_tc.cu / passes.cu
 void run_m2l_tensor(kifmm_plan *P, const PassArgs &A);
 void launch_p2m_d(kifmm_plan *P, const PassArgs &A);
-void launch_leaf_eval_d(kifmm_plan *P, const PassArgs &A, int check_self);
 void launch_eval_targets_d(kifmm_plan *P, const PassArgs &A, const double *tx, const double *ty, int64_t n,
                            int check_self, double *pot);
 void launch_m2m_d(kifmm_plan *P, const PassArgs &A, int l);

@@ -1,0 +1,90 @@
+"""The FP64 pair loops at the edges of their tiles and series.
+
+A point set of at most Ncutoff points is one leaf, whose evaluation is the
+direct sum, so the pair loop stands alone: it is compared with a direct sum in
+extended precision (Laplace) or scipy's Bessel functions.  Bound: each kernel
+value is within a few ulp, each of n additions rounds once, so the error is at
+most (n + 16) eps sum_j (|G_ij| + 1) |tau_j| (+ 1: the logarithm is accurate to
+2^-53 absolutely where it is small).
+"""
+import numpy as np
+import pytest
+
+from conftest import has_gpu
+
+pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not has_gpu(), reason="needs a CUDA GPU")]
+
+EPS = 2.0 ** -52
+
+
+def cloud(n, seed):
+    rng = np.random.default_rng(seed)
+    return rng.uniform(-1, 1, n), rng.uniform(-1, 1, n), rng.standard_normal(n)
+
+
+def direct(kind, k, x, y, tau):
+    """(sum, sum of magnitudes) with pairs of equal coordinates left out"""
+    from scipy import special
+    ld = np.longdouble
+    dx, dy = x[:, None].astype(ld) - x[None, :], y[:, None].astype(ld) - y[None, :]
+    r2 = dx * dx + dy * dy
+    same = r2 == 0
+    r2[same] = 1
+    if kind == "laplace":
+        g = -np.log(r2) / (4 * ld(np.pi))
+    else:
+        g = special.k0(float(k) * np.sqrt(r2).astype(float)).astype(ld) / (2 * ld(np.pi))
+    g[same] = 0
+    return (g @ tau.astype(ld)).astype(float), ((np.abs(g) + 1) @ np.abs(tau)).astype(float)
+
+
+def fmm(kind, k, x, y, cutoff, **kw):
+    import pykifmm2d_b200 as P
+    kern = P.LaplaceKernel() if kind == "laplace" else P.ModifiedHelmholtzKernel(k)
+    f = P.FMM(x, y, P.Get_Kernel_Functions(kern), P.prepare_numba_functions_on_the_fly(kern), 24, cutoff, **kw)
+    f.build_tree()
+    f.precompute()
+    return f
+
+
+# wavenumbers on either side of each series length (t = (k r)^2 up to 8 k^2 W^2,
+# W = 2), and where most pairs are beyond the series
+KERNELS = [("laplace", 0.0), ("k0", 0.04), ("k0", 0.17), ("k0", 0.34), ("k0", 3.0), ("k0", 60.0)]
+
+
+@pytest.mark.parametrize("n", [1, 2, 7, 8, 9, 17, 22, 32, 33, 63, 64, 65, 200])
+@pytest.mark.parametrize("kind,k", KERNELS)
+def test_one_leaf_is_the_direct_sum(kind, k, n):
+    x, y, tau = cloud(n, n)
+    if n > 8:
+        x[5], y[5] = x[2], y[2]  # an exact duplicate
+    for cutoff in (n, 300):
+        f = fmm(kind, k, x, y, cutoff)
+        assert f.tree_info().levels == 1
+        f.build_expansions(tau)
+        ref, mag = direct(kind, k, x, y, tau)
+        for _ in range(2):  # a second evaluation on the same expansions
+            pot = f.evaluate_to_points(x, y, True)
+            assert np.all(np.abs(pot - ref) <= (n + 16) * EPS * mag)
+
+
+@pytest.mark.parametrize("kind,k", KERNELS[:2])
+def test_self_pairs_are_infinite_without_check_self(kind, k):
+    x, y, tau = cloud(40, 3)
+    f = fmm(kind, k, x, y, 64)
+    f.build_expansions(np.abs(tau))
+    assert np.all(np.isposinf(f.evaluate_to_points(x, y, False)))
+
+
+@pytest.mark.parametrize("n,cutoff", [(300, 3), (900, 9), (2500, 31), (2500, 33), (6000, 150)])
+@pytest.mark.parametrize("kind,k", [("laplace", 0.0), ("k0", 0.3), ("k0", 12.0)])
+def test_leaf_tiles_vs_oracle(kind, k, n, cutoff):
+    from oracle import oracle as O
+    x, y, tau = cloud(n, 7)
+    f = fmm(kind, k, x, y, cutoff)
+    f.build_expansions(tau)
+    pot = f.evaluate_to_points(x, y, True)
+    o = O.OracleFMM(x, y, 0 if kind == "laplace" else 1, k, 24, cutoff)
+    o.build_expansions(tau)
+    ref = o.evaluate_to_points(x, y, True)
+    assert np.abs(pot - ref).max() / np.abs(ref).max() <= 1e-9  # the bound of the plain form's other tests
