@@ -1,11 +1,12 @@
 // pair_f64.cuh -- FP64 kernel values for the pair loops (P2M, L2P, P2P).
 //
-// On sm_100a an SM issues 64 FP64 multiply-adds per clock but only 16 FP64
-// conversions, and the CUDA math library's log, sqrt and Bessel functions
-// cost 15 to 50 multiply-adds a call (measured: log 1.27, rsqrt 5.9, sqrt 4.4,
-// int -> double 15.4, fma 60 lane-operations per clock and SM).  The values
-// here take r^2 (no square root), one conflict-free table read and 10
-// multiply-adds for the logarithm, and short power series beside it.
+// On sm_100a an SM issues 64 FP64 multiply-adds per clock (one warp instruction
+// takes two issue slots of its scheduler) but only 16 FP64 conversions, and the
+// CUDA math library's log, sqrt and Bessel functions cost 15 to 50 multiply-adds
+// a call (measured, lane-operations per clock and SM: log 1.27, rsqrt 5.9, sqrt
+// 4.4, int -> double 15.4, fma 60).  The values here take r^2 (no square root),
+// one conflict-free table read and 8 FP64 instructions for the logarithm, and
+// short power series beside it.
 #pragma once
 #include "kifmm_internal.cuh"
 
@@ -19,17 +20,20 @@ namespace kifmm {
 // log1p(r).  log1p is its series to r^6 with r^6 economised by the Chebyshev
 // polynomial T6 (r^6 = h^6 (T6(r/h) + 48 (r/h)^4 - 18 (r/h)^2 + 1) / 32,
 // h = 2^-8), so five coefficients leave 1.9e-17; the constant it leaves goes
-// into the table.  Max error 1.8 ulp, mean 0.39 (against 60-digit values over
-// 2^-30 .. 2^5).  e comes from the exponent bits by a magic-number add.
+// into the table.  Max error 1.6 ulp, mean 0.34 (against 60-digit values over
+// 2^-30 .. 2^5).  e is converted on the XU pipe, beside the FP64 pipe.
 // The table is kept LOGTAB_COPIES times in shared memory, copy c in the 16-byte
 // bank group c: a warp's 32 16-byte reads, eight to a phase, hit eight
 // different groups whatever their entries (one copy measured 2-3 way
 // conflicts, and the reads would then bound the loop instead of the FP64 pipe).
 constexpr int LOGTAB_N = 128, LOGTAB_COPIES = 8;
-constexpr double LOG_LN2 = 0.693147180559945309417232121458176568;
 constexpr double LOG_H2 = 1.0 / 65536.0;  // h^2
-constexpr double LOG_C2 = -0.5 + LOG_H2 * LOG_H2 * 18.0 / 192.0, LOG_C3 = 1.0 / 3.0,
-                 LOG_C4 = -0.25 - LOG_H2 * 48.0 / 192.0, LOG_C5 = 0.2;
+// the polynomial's coefficients r^2 .. r^5 and ln 2, in constant memory, so
+// that they are operands of the multiply-adds
+enum { LOG_C2, LOG_C3, LOG_C4, LOG_C5, LOG_LN2 };
+static __device__ __constant__ double LOG_K[] = {-0.5 + LOG_H2 * LOG_H2 * 18.0 / 192.0, 1.0 / 3.0,
+                                                 -0.25 - LOG_H2 * 48.0 / 192.0, 0.2,
+                                                 0.693147180559945309417232121458176568};
 
 // log_table(device) holds [LOGTAB_N] (v_i, -ln v_i - h^6/192); stage its copies into tab[LOGTAB_N * LOGTAB_COPIES] (all threads of the block)
 __device__ __forceinline__ void stage_log_table(double2 *tab, const double2 *__restrict__ g) {
@@ -37,20 +41,22 @@ __device__ __forceinline__ void stage_log_table(double2 *tab, const double2 *__r
 }
 
 // ln(2^EADJ x); tl: this lane's copy, tab + (lane & 7).  x positive, normal,
-// finite (pair_ordinary); anything else gives a finite or NaN value and reads
-// inside the table.
+// finite; anything else gives a finite or NaN value and reads inside the table.
 template <int EADJ>
 __device__ __forceinline__ double ln_tab(double x, const double2 *tl) {
     const int hi = __double2hiint(x), lo = __double2loint(x);
-    const double2 c = tl[((hi >> 13) & (LOGTAB_N - 1)) * LOGTAB_COPIES];
+    constexpr unsigned ROW = LOGTAB_COPIES * sizeof(double2);  // bytes of an entry's copies
+    static_assert(LOGTAB_N * ROW == 0x4000 && ROW == 0x80, "the shift and mask below");
+    const double2 c = *(const double2 *)((const char *)tl + (((unsigned)hi >> 6) & 0x3f80u));
     const double m = __hiloint2double((hi & 0x000fffff) | 0x3ff00000, lo);
-    const double e = __hiloint2double(0x43300000, (int)((unsigned)hi >> 20)) - (4503599627370496.0 + 1023.0 - EADJ);
+    const double e = (double)((int)((unsigned)hi >> 20) - (1023 - EADJ));
     const double r = fma(m, c.x, -1.0);
-    double q = LOG_C5;
-    q = fma(q, r, LOG_C4);
-    q = fma(q, r, LOG_C3);
-    q = fma(q, r, LOG_C2);
-    return fma(q * r, r, fma(e, LOG_LN2, c.y) + r);
+    double q = LOG_K[LOG_C5];
+    q = fma(q, r, LOG_K[LOG_C4]);
+    q = fma(q, r, LOG_K[LOG_C3]);
+    q = fma(q, r, LOG_K[LOG_C2]);
+    q = fma(q, r, 1.0);
+    return fma(q, r, fma(e, LOG_K[LOG_LN2], c.y));
 }
 
 // Number of series terms that reach FP64 precision for t = (k r)^2 below
@@ -66,11 +72,11 @@ __device__ __forceinline__ double series(const double *c, double t) {
     return a;
 }
 
-// Whether t = r^2 (Laplace) or (k r)^2 is a positive normal number below the
-// bound whose high word is hi_end: those the fast values are for.
-__device__ __forceinline__ bool pair_ordinary(double t, unsigned hi_end) {
-    return (unsigned)(__double2hiint(t) - 0x00100000) < hi_end - 0x00100000u;
-}
+// The fast values are for t = r^2 (Laplace) or (k r)^2 that is a positive
+// normal number below the bound whose high word is hi_end: those whose
+// pair_rank is below hi_end - 2^20.
+__device__ __forceinline__ unsigned pair_rank(double t) { return (unsigned)(__double2hiint(t) - 0x00100000); }
+__device__ __forceinline__ bool pair_ordinary(double t, unsigned hi_end) { return pair_rank(t) < hi_end - 0x00100000u; }
 constexpr unsigned LOG_HI_END = 0x7ff00000u;  // every finite number
 
 // Unscaled kernel value of an ordinary pair: ln r^2 (Laplace, times

@@ -101,11 +101,10 @@ __global__ void __launch_bounds__(DEN_THREADS) k_leaf_density(DenArgs D) {
 // each source read from shared memory serves TB pairs.  The leaf's sources
 // (its own points, then its colleagues') are staged in chunks; the L2P is the
 // same loop over the Q equivalent points of the leaf's local expansion, in
-// box-relative coordinates.  Bound by the FP64 pipe: 14 FP64 instructions per
-// Laplace pair, 7 clocks of an SM per 32 pairs (0.23 ms for the 2.8e8 pairs of
-// the 1M mixture).  Warps draw items from a ticket (the leaves differ in work
-// by more than 10x); each warp draws one ticket past the end, so atomicInc's
-// wrap leaves the counter at zero for the next launch.
+// box-relative coordinates.  Bound by issue: 12 FP64 instructions (two slots
+// each) and about 9 others per Laplace pair.  Warps draw items from a ticket
+// (the leaves differ in work by more than 10x); each warp draws one ticket past
+// the end, so atomicInc's wrap leaves the counter at zero for the next launch.
 constexpr int L64_CHUNK = 64;  // sources staged per pass, two per lane
 struct Leaf64Warp {
     double2 xy[L64_CHUNK];
@@ -116,35 +115,76 @@ struct Leaf64Warp {
 };
 static_assert(sizeof(Leaf64Warp) % 16 == 0, "Leaf64Warp alignment");
 
-template <int KIND, int NT, int TB>
-__device__ __forceinline__ void pair_loop(const Leaf64Warp &W, const double2 *tl, int j, int sp, int n,
+// Sums of the lane's TB targets over sources u, u + sp, ... below n.  CHECKED
+// tests each pair and gives those that the fast value is not for to the math
+// library (coincident pairs are left out with skip_equal); without it the
+// return value tells afterwards whether there was such a pair (one instruction
+// a pair instead of five), and the caller runs the sources again, checked.
+template <int KIND, int NT, int TB, bool CHECKED>
+__device__ __forceinline__ bool pair_loop(const Leaf64Warp &W, const double2 *tl, int &u, int sp, int n,
                                           const double *tx, const double *ty, double k, double k2, unsigned hi_end,
                                           bool skip_equal, double *acc) {
+    unsigned worst = 0;      // largest rank (K0)
+    int least = 0x7fffffff;  // smallest high word (Laplace: r^2 is finite)
 #pragma unroll 1
-    for (int u = j; u < n; u += sp) {
+    for (; u < n; u += sp) {
         const double2 s = W.xy[u];
         const double z = W.z[u];
+        bool all = true;
 #pragma unroll
         for (int a = 0; a < TB; a++) {
             const double dx = tx[a] - s.x, dy = ty[a] - s.y;
             const double r2 = fma(dx, dx, dy * dy);
             const double t = KIND == KIFMM_KERNEL_LAPLACE ? r2 : r2 * k2;
-            double v = pair_value<KIND, NT>(t, tl), zz = z;
-            if (!pair_ordinary(t, hi_end)) {
-                const bool skip = skip_equal && dx == 0.0 && dy == 0.0;
-                v = 0.0;
-                if (skip) zz = 0.0;
-                else v = pair_value_any<KIND>(r2, k);
+            const double v = pair_value<KIND, NT>(t, tl);
+            if (CHECKED) {
+                const bool ok = pair_ordinary(t, hi_end);
+                if (ok) acc[a] = fma(v, z, acc[a]);
+                all = all && ok;
+            } else {
+                acc[a] = fma(v, z, acc[a]);
+                if (KIND == KIFMM_KERNEL_LAPLACE) least = min(least, __double2hiint(t));
+                else worst = max(worst, pair_rank(t));
             }
-            acc[a] = fma(v, zz, acc[a]);
+        }
+        if (CHECKED && !all) {
+#pragma unroll
+            for (int a = 0; a < TB; a++) {
+                const double dx = tx[a] - s.x, dy = ty[a] - s.y;
+                const double r2 = fma(dx, dx, dy * dy);
+                if (!pair_ordinary(KIND == KIFMM_KERNEL_LAPLACE ? r2 : r2 * k2, hi_end) &&
+                    !(skip_equal && dx == 0.0 && dy == 0.0))
+                    acc[a] = fma(pair_value_any<KIND>(r2, k), z, acc[a]);
+            }
         }
     }
+    return KIND == KIFMM_KERNEL_LAPLACE ? least < 0x00100000 : worst >= hi_end - 0x00100000u;
 }
-// the near sources of the leaf, then the equivalent points of its local expansion
-template <int KIND, int NT, int TB>
-__device__ __forceinline__ double leaf_item(const PassArgs &A, Leaf64Warp &W, const double2 *tl, int t0, int nt, int ns,
-                                            int l, double cx, double cy, const double *den, unsigned hi_end,
-                                            bool check_self, double k2, int lane) {
+// the staged sources u, u + sp, ... below n, the first n_own of them checked
+// (the leaf's own points, where the target meets itself; BEYOND: pairs past the
+// series are expected, all are)
+template <int KIND, int NT, int TB, bool BEYOND>
+__device__ __forceinline__ void pair_chunk(Leaf64Warp &W, const double2 *tl, int u, int sp, int n_own, int n,
+                                           const double *tx, const double *ty, double k, double k2, unsigned hi_end,
+                                           bool skip_equal, double *acc) {
+    pair_loop<KIND, NT, TB, true>(W, tl, u, sp, BEYOND ? n : n_own, tx, ty, k, k2, hi_end, skip_equal, acc);
+    if (BEYOND) return;
+    const int lane = threadIdx.x & 31, u0 = u;
+#pragma unroll
+    for (int a = 0; a < TB; a++) W.red[a][lane] = acc[a];
+    if (pair_loop<KIND, NT, TB, false>(W, tl, u, sp, n, tx, ty, k, k2, hi_end, skip_equal, acc)) {
+#pragma unroll
+        for (int a = 0; a < TB; a++) acc[a] = W.red[a][lane];
+        u = u0;
+        pair_loop<KIND, NT, TB, true>(W, tl, u, sp, n, tx, ty, k, k2, hi_end, skip_equal, acc);
+    }
+}
+// the near sources of the leaf (n_own of its own first), then the equivalent
+// points of its local expansion
+template <int KIND, int NT, int TB, bool BEYOND>
+__device__ __forceinline__ double leaf_item(const PassArgs &A, Leaf64Warp &W, const double2 *tl, int t0, int nt,
+                                            int n_own, int ns, int l, double cx, double cy, const double *den,
+                                            unsigned hi_end, bool check_self, double k2, int lane) {
     const int ng = (nt + TB - 1) / TB, sp = 32 / ng, j = lane / ng, gi = lane - j * ng;
     double tx[TB], ty[TB], acc[TB];
 #pragma unroll
@@ -154,7 +194,7 @@ __device__ __forceinline__ double leaf_item(const PassArgs &A, Leaf64Warp &W, co
         ty[a] = A.ys[t0 + i];
         acc[a] = 0.0;
     }
-    const bool idle = j >= sp;
+    const int u0 = j < sp ? j : 1 << 20;  // lanes past the last group idle
     for (int c0 = 0; c0 < ns; c0 += L64_CHUNK) {
         const int cn = min(L64_CHUNK, ns - c0);
         __syncwarp();
@@ -168,7 +208,8 @@ __device__ __forceinline__ double leaf_item(const PassArgs &A, Leaf64Warp &W, co
             }
         }
         __syncwarp();
-        pair_loop<KIND, NT, TB>(W, tl, j, sp, idle ? 0 : cn, tx, ty, A.k, k2, hi_end, check_self, acc);
+        pair_chunk<KIND, NT, TB, BEYOND>(W, tl, u0, sp, min(n_own - c0, cn), cn, tx, ty, A.k, k2, hi_end, check_self,
+                                         acc);
     }
     if (l >= 2) {
         const double *lg = A.ops + (size_t)l * A.stride + A.off_large;
@@ -183,8 +224,9 @@ __device__ __forceinline__ double leaf_item(const PassArgs &A, Leaf64Warp &W, co
             tx[a] -= cx;
             ty[a] -= cy;
         }
-        pair_loop<KIND, NT, TB>(W, tl, j, sp, idle ? 0 : A.Q, tx, ty, A.k, k2, hi_end, false, acc);
+        pair_chunk<KIND, NT, TB, BEYOND>(W, tl, u0, sp, 0, A.Q, tx, ty, A.k, k2, hi_end, false, acc);
     }
+    __syncwarp();
 #pragma unroll
     for (int a = 0; a < TB; a++) W.red[a][lane] = acc[a];
     __syncwarp();
@@ -195,21 +237,25 @@ __device__ __forceinline__ double leaf_item(const PassArgs &A, Leaf64Warp &W, co
     }
     return v * pair_scale<KIND>();
 }
-template <int KIND, int NT>
+template <int KIND, int NT, bool BEYOND = false>
 __device__ __forceinline__ double leaf_item_tb(const PassArgs &A, Leaf64Warp &W, const double2 *tl, int t0, int nt,
-                                               int ns, int l, double cx, double cy, const double *den, unsigned hi_end,
-                                               bool check_self, double k2, int lane) {
-    // two targets per lane, or four where that leaves fewer lanes idle
-    // (pair slots per source: TB / (32 / ceil(nt / TB)))
-    const int n2 = (nt + 1) >> 1, n4 = (nt + 3) >> 2;
-    if (4 * (32 / n2) < 2 * (32 / n4))
-        return leaf_item<KIND, NT, 4>(A, W, tl, t0, nt, ns, l, cx, cy, den, hi_end, check_self, k2, lane);
-    return leaf_item<KIND, NT, 2>(A, W, tl, t0, nt, ns, l, cx, cy, den, hi_end, check_self, k2, lane);
+                                               int n_own, int ns, int l, double cx, double cy, const double *den,
+                                               unsigned hi_end, bool check_self, double k2, int lane) {
+    // the number of targets per lane that leaves the fewest lanes idle: pair
+    // slots per source TB / (32 / ceil(nt / TB)), compared by cross products
+    const int s2 = 32 / ((nt + 1) >> 1), s3 = 32 / ((nt + 2) / 3), s4 = 32 / ((nt + 3) >> 2);
+    if (s4 * 3 >= s3 * 4 && s4 * 2 >= s2 * 4)
+        return leaf_item<KIND, NT, 4, BEYOND>(A, W, tl, t0, nt, n_own, ns, l, cx, cy, den, hi_end, check_self, k2, lane);
+    if (s3 * 2 >= s2 * 3)
+        return leaf_item<KIND, NT, 3, BEYOND>(A, W, tl, t0, nt, n_own, ns, l, cx, cy, den, hi_end, check_self, k2, lane);
+    return leaf_item<KIND, NT, 2, BEYOND>(A, W, tl, t0, nt, n_own, ns, l, cx, cy, den, hi_end, check_self, k2, lane);
 }
 
-constexpr int L64_MAX_WARPS = 8;
+// 16 warps per SM at 128 registers measured 1-5% faster than 24 at 80 (the K0
+// series spill there), and 64-source chunks the same as 96 or 128
+constexpr int L64_MAX_WARPS = 8, L64_BLOCKS_PER_SM = 2;
 template <int KIND>
-__global__ void __launch_bounds__(32 * L64_MAX_WARPS, 4)
+__global__ void __launch_bounds__(32 * L64_MAX_WARPS, L64_BLOCKS_PER_SM)
     k_leaf_eval_d(PassArgs A, const double2 *__restrict__ logtab, const double *__restrict__ den, unsigned nitems,
                   int ntile, int ts, int check_self, unsigned *__restrict__ ticket) {
     extern __shared__ __align__(16) unsigned char sm_l64[];
@@ -246,17 +292,21 @@ __global__ void __launch_bounds__(32 * L64_MAX_WARPS, 4)
         for (int t0 = b + (int)(it - w * ntile) * ts; t0 < e; t0 += ntile * ts) {
             const int nt = min(ts, e - t0);
             double v;
+            const int own = e - b;
             if (KIND == KIFMM_KERNEL_LAPLACE)
-                v = leaf_item_tb<KIND, 1>(A, W, tl, t0, nt, ns, l, cx, cy, dn, LOG_HI_END, check_self, k2, lane);
+                v = leaf_item_tb<KIND, 1>(A, W, tl, t0, nt, own, ns, l, cx, cy, dn, LOG_HI_END, check_self, k2, lane);
             else if (tmax < 0.0625)
-                v = leaf_item_tb<KIND, SERIES_NARROW>(A, W, tl, t0, nt, ns, l, cx, cy, dn, SERIES_NARROW_HI, check_self,
-                                                      k2, lane);
+                v = leaf_item_tb<KIND, SERIES_NARROW>(A, W, tl, t0, nt, own, ns, l, cx, cy, dn, SERIES_NARROW_HI,
+                                                      check_self, k2, lane);
             else if (tmax < 1.0)
-                v = leaf_item_tb<KIND, SERIES_MID>(A, W, tl, t0, nt, ns, l, cx, cy, dn, SERIES_MID_HI, check_self, k2,
-                                                   lane);
+                v = leaf_item_tb<KIND, SERIES_MID>(A, W, tl, t0, nt, own, ns, l, cx, cy, dn, SERIES_MID_HI, check_self,
+                                                   k2, lane);
+            else if (tmax < 4.0)
+                v = leaf_item_tb<KIND, SERIES_WIDE>(A, W, tl, t0, nt, own, ns, l, cx, cy, dn, SERIES_WIDE_HI,
+                                                    check_self, k2, lane);
             else
-                v = leaf_item_tb<KIND, SERIES_WIDE>(A, W, tl, t0, nt, ns, l, cx, cy, dn, SERIES_WIDE_HI, check_self, k2,
-                                                    lane);
+                v = leaf_item_tb<KIND, SERIES_WIDE, true>(A, W, tl, t0, nt, own, ns, l, cx, cy, dn, SERIES_WIDE_HI,
+                                                          check_self, k2, lane);
             if (lane < nt) A.pots[t0 + lane] = v;
         }
     }
@@ -284,17 +334,19 @@ void launch_leaf_eval_d(kifmm_plan *P, const PassArgs &A, int check_self) {
         launch_pdl(k_leaf_density, dim3((unsigned)tiles), dim3(DEN_THREADS), smem, P->stream, D);
     }
     // Items: whole 32-target tiles once they fill the GPU's resident warps
-    // (32 per SM); smaller tiles for fewer leaves, down to 8 targets, where a
+    // (16 per SM); smaller tiles for fewer leaves, down to 8 targets, where a
     // warp's run over its sources is the kernel's length.
-    const int64_t resident = (int64_t)P->num_sms * 4 * L64_MAX_WARPS;
+    const int64_t resident = (int64_t)P->num_sms * L64_BLOCKS_PER_SM * L64_MAX_WARPS;
     int ts = 32;
     while (ts > 8 && nl * ((P->ppl + ts - 1) / ts) < resident) ts >>= 1;
     const int ntile = (int)std::min<int64_t>((P->ppl + ts - 1) / ts, 64);
     const int64_t items = nl * ntile;
     KIFMM_REQUIRE(items + resident < (1ll << 32), KIFMM_ERR_ARG, "leaf pass: too many leaves");
-    int warps = L64_MAX_WARPS;  // a block's table is shared by its warps; few items: spread them over the SMs
-    while (warps > 1 && items < (int64_t)P->num_sms * warps * 2) warps >>= 1;
-    const unsigned grid = (unsigned)std::min<int64_t>((items + warps - 1) / warps, resident / L64_MAX_WARPS);
+    // a block's table is shared by its warps; fewer items than resident warps:
+    // smaller blocks, down to two warps, spread them over the SMs
+    int warps = L64_MAX_WARPS;
+    while (warps > 2 && items < (int64_t)P->num_sms * warps * 2) warps >>= 1;
+    const unsigned grid = (unsigned)std::min<int64_t>((items + warps - 1) / warps, resident / warps);
     const size_t smem = LOGTAB_N * LOGTAB_COPIES * sizeof(double2) + (size_t)warps * sizeof(Leaf64Warp);
     unsigned *ticket = (unsigned *)(P->scal.p + KIFMM_SCAL_TICKET);
     const double2 *lt = log_table(P->device);
