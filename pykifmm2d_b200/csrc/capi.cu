@@ -364,7 +364,6 @@ int kifmm_plan_create(const kifmm_kernel *kernel, int32_t nequiv, int32_t ncutof
             KIFMM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, P->device));
             P->num_sms = sms > 0 ? sms : 148;
             prepare_pool(P->device);
-            init_log_table(P->device);
             log_table(P->device);
             P->hpin = pinned_acquire();
             if (o.stream) {

@@ -488,7 +488,6 @@ void tree_stats(kifmm_plan *P);
 // operators.cu
 void build_operators(kifmm_plan *P);
 const double2 *log_table(int device); // pass_f64.cu: table of the FP64 pair loops' logarithm, once per device
-void init_log_table(int device);     // table of the Laplace P2M logarithm, once per device
 void ensure_side(kifmm_plan *P);      // side stream and its events
 void start_operators(kifmm_plan *P, bool fork_recorded = false);  // build_operators on the side stream
 cudaStream_t device_side_stream(int device);  // one per device, created on first use

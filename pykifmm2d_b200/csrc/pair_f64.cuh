@@ -90,12 +90,23 @@ template <int KIND>
 __device__ __forceinline__ double pair_scale() {
     return KIND == KIFMM_KERNEL_LAPLACE ? -0.07957747154594767 : 0.15915494309189535;
 }
-// ... of any other pair (coincident points, underflow, k r >= 2) by the math
-// library's functions; kept out of line, so that the pair loops stay small
+// K0(sqrt(t)) for t >= 4: exp(-x) / sqrt(x) F(4/x - 1), F as one polynomial
+// (24 multiply-adds; Clenshaw's recurrence on its Chebyshev series takes 50),
+// x = sqrt(t) and 1/x from one reciprocal square root
+__device__ __forceinline__ double k0_far(double t) {
+    const double y = rsqrt(t);
+    double x = t * y;
+    x = fma(0.5 * y, fma(-x, x, t), x);
+    const double u = fma(4.0, y, -1.0);
+    return exp(-x) * rsqrt(x) * series<K0_FAR_D_N>(K0_FAR_D, u);
+}
+// ... of any other pair (coincident points, underflow, k r >= 2); kept out of
+// line, so that the pair loops stay small
 template <int KIND>
 __device__ __noinline__ double pair_value_any(double r2, double k) {
     if (KIND == KIFMM_KERNEL_LAPLACE) return log(r2);
-    return k0_d(k * sqrt(r2));
+    const double t = r2 * (k * k);
+    return t >= 4.0 && t < 1e300 ? k0_far(t) : k0_d(k * sqrt(r2));
 }
 
 }  // namespace kifmm

@@ -84,6 +84,8 @@ __device__ __forceinline__ void dmma_8x8x4(double &c0, double &c1, double a, dou
 // row stride = 4 mod 16 doubles: conflict-free fragment loads
 __host__ __device__ constexpr int pad4mod16(int m) { return m + (20 - m % 16) % 16; }
 // pass_f64.cu
+void launch_p2m_d(kifmm_plan *P, const PassArgs &A);
+void launch_leaf_far_d(kifmm_plan *P, const PassArgs &A);
 void launch_leaf_eval_d(kifmm_plan *P, const PassArgs &A, int check_self);
 // planned.cu
 void launch_planned_p2m(kifmm_plan *P, const PassArgs &A);

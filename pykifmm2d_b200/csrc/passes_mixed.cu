@@ -840,7 +840,6 @@ void launch_leaf_den(kifmm_plan *P, const PassArgs &A) {
 
 // m2l_tc.cu / passes.cu
 void run_m2l_tensor(kifmm_plan *P, const PassArgs &A);
-void launch_p2m_d(kifmm_plan *P, const PassArgs &A);
 void launch_eval_targets_d(kifmm_plan *P, const PassArgs &A, const double *tx, const double *ty, int64_t n,
                            int check_self, double *pot);
 void launch_m2m_d(kifmm_plan *P, const PassArgs &A, int l);
@@ -954,13 +953,7 @@ void run_eval_sources_mixed(kifmm_plan *P, int check_self) {
             if (tiles) launch_pdl(k_leaf_far_taylor, dim3((unsigned)tiles), dim3(FT_THREADS), 0, P->stream, T);
             return;
         }
-        const dim3 grid((unsigned)((P->n_leaf_list + LEAF_WARPS - 1) / LEAF_WARPS)), block(32 * LEAF_WARPS);
-        if (P->kern.kind == KIFMM_KERNEL_LAPLACE)
-            launch_pdl(k_leaf_eval_f<KIFMM_KERNEL_LAPLACE, false, LEAF_FAR>, grid, block, 0, P->stream, A,
-                       P->n_leaf_list, (const int32_t *)nullptr, (const unsigned *)nullptr);
-        else
-            launch_pdl(k_leaf_eval_f<KIFMM_KERNEL_MOD_HELMHOLTZ, false, LEAF_FAR>, grid, block, 0, P->stream, A,
-                       P->n_leaf_list, (const int32_t *)nullptr, (const unsigned *)nullptr);
+        if (P->kern.kind == KIFMM_KERNEL_MOD_HELMHOLTZ) launch_leaf_far_d(P, A);
         return;
     }
     // fewer leaves than one wave of warps: split the big ones over two warps
