@@ -15,7 +15,11 @@ Terms are kept while they matter at double (FP64) or single (FP32) precision.
 The FP64 pair loops (pair_f64.cuh) take the same series in the forms
   K0(x)          = P(t) + ln(t/4) I0H(t),  I0H = -I0 / 2,
   (i/4) H0(x)    = ln(t/4) A(t) + R(t) + i (-pi) A(t),
-  A = -J0 / (4 pi),  R = sum_k (-1)^k p_k t^k / (2 pi)  (p_k those of P; DLMF 10.8.2).
+  A = -J0 / (4 pi),  R = sum_k (-1)^k p_k t^k / (2 pi)  (p_k those of P; DLMF 10.8.2);
+for 4 <= t <= 64 the same A and R (entire functions of t) as polynomials in
+u = (t - 34) / 30, and for t >= 64 Hankel's form (DLMF 10.2.5)
+  H0(x) = sqrt(2 / (pi x)) exp(i (x - pi/4)) (p(v) + i q(v) / x),  v = 128 / t - 1,
+p and q as polynomials in v; coefficients from the Chebyshev transform at 64 nodes.
 
 Run:  python pykifmm2d_b200/csrc/gen_k0_tables.py   (rewrites k0_tables.h beside it)
 """
@@ -87,6 +91,30 @@ def fmt(vals, single):
     return ",\n    ".join("%.17e" % float(v) for v in vals)
 
 
+def cheb_of(f, tol, n=64):
+    """power coefficients of f on [-1, 1], Chebyshev terms kept above tol"""
+    vals = [f(mp.cos(mp.pi * (j + mp.mpf(1) / 2) / n)) for j in range(n)]
+    c = [2 * sum(vals[j] * mp.cos(mp.pi * k * (j + mp.mpf(1) / 2) / n) for j in range(n)) / n for k in range(n)]
+    c[0] /= 2
+    return monomial(c[: max(i for i, v in enumerate(c) if abs(v) > tol) + 1])
+
+
+def hankel():
+    def mid(u):  # (A, R) at t = 34 + 30 u
+        t = 34 + 30 * u
+        x = mp.sqrt(t)
+        a = -mp.besselj(0, x) / (4 * mp.pi)
+        return a, -mp.bessely(0, x) / 4 - mp.log(t / 4) * a
+
+    def far(v):  # p + i q
+        w = (v + 1) / 2
+        x = 8 / mp.sqrt(w)
+        s = (mp.besselj(0, x) + 1j * mp.bessely(0, x)) * mp.sqrt(mp.pi * x / 2) * mp.exp(-1j * (x - mp.pi / 4))
+        return s.real, s.imag * x
+    return (cheb_of(lambda u: mid(u)[0], 3e-18), cheb_of(lambda u: mid(u)[1], 1e-17),
+            cheb_of(lambda v: far(v)[0], 1e-17), cheb_of(lambda v: far(v)[1], 1e-17))
+
+
 def main():
     i0, p = series(40)
     # t <= 4: term k is at most 4^k c_k = 1/(k!)^2 in size; keep while above the precision
@@ -107,7 +135,9 @@ def main():
     i0h = [-v / 2 for v in i0_64]
     h0a = [-(-1) ** k * v / (4 * mp.pi) for k, v in enumerate(i0[:nt])]
     h0r = [(-1) ** k * v / (2 * mp.pi) for k, v in enumerate(p[:nt])]
-    for name, vals, single in (("K0_I0H_D", i0h, False), ("H0_A_D", h0a, False), ("H0_R_D", h0r, False),
+    ma, mr, hp, hq = hankel()
+    for name, vals, single in (("H0_MID_A_D", ma, False), ("H0_MID_R_D", mr, False), ("H0_P_D", hp, False),
+                               ("H0_Q_D", hq, False), ("K0_I0H_D", i0h, False), ("H0_A_D", h0a, False), ("H0_R_D", h0r, False),
                                ("K0_I0_D", i0_64, False), ("K0_P_D", p_64, False), ("K0_CHEB_D", ch_64, False),
                                ("K0_FAR_D", monomial(ch[:24]), False),
                                ("K0_I0_F", i0_32, True), ("K0_P_F", p_32, True), ("K0_CHEB_F", ch_32, True)):

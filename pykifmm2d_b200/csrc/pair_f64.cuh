@@ -79,16 +79,24 @@ __device__ __forceinline__ unsigned pair_rank(double t) { return (unsigned)(__do
 __device__ __forceinline__ bool pair_ordinary(double t, unsigned hi_end) { return pair_rank(t) < hi_end - 0x00100000u; }
 constexpr unsigned LOG_HI_END = 0x7ff00000u;  // every finite number
 
-// Unscaled kernel value of an ordinary pair: ln r^2 (Laplace, times
-// -1/(4 pi)) or K0(k r) = P(t) - ln(t/4) I0(t)/2 (times 1/(2 pi)).
+// Unscaled kernel value: re = ln r^2 (Laplace, times -1/(4 pi)), K0(k r) =
+// P(t) - ln(t/4) I0(t)/2 (times 1/(2 pi)), or the real part of (i/4) H0(k r),
+// ln(t/4) A(t) + R(t), whose imaginary part is -pi a with a = A(t).
+struct PairValue {
+    double re, a;
+};
 template <int KIND, int NT>
-__device__ __forceinline__ double pair_value(double t, const double2 *tl) {
-    if (KIND == KIFMM_KERNEL_LAPLACE) return ln_tab<0>(t, tl);
-    return fma(ln_tab<-2>(t, tl), series<NT>(K0_I0H_D, t), series<NT>(K0_P_D, t));
+__device__ __forceinline__ PairValue pair_value(double t, const double2 *tl) {
+    if (KIND == KIFMM_KERNEL_LAPLACE) return {ln_tab<0>(t, tl), 0.0};
+    const double ln4 = ln_tab<-2>(t, tl);
+    if (KIND == KIFMM_KERNEL_MOD_HELMHOLTZ) return {fma(ln4, series<NT>(K0_I0H_D, t), series<NT>(K0_P_D, t)), 0.0};
+    const double a = series<NT>(H0_A_D, t);
+    return {fma(ln4, a, series<NT>(H0_R_D, t)), a};
 }
 template <int KIND>
 __device__ __forceinline__ double pair_scale() {
-    return KIND == KIFMM_KERNEL_LAPLACE ? -0.07957747154594767 : 0.15915494309189535;
+    return KIND == KIFMM_KERNEL_LAPLACE ? -0.07957747154594767
+                                        : KIND == KIFMM_KERNEL_MOD_HELMHOLTZ ? 0.15915494309189535 : 1.0;
 }
 // K0(sqrt(t)) for t >= 4: exp(-x) / sqrt(x) F(4/x - 1), F as one polynomial
 // (24 multiply-adds; Clenshaw's recurrence on its Chebyshev series takes 50),
@@ -100,13 +108,38 @@ __device__ __forceinline__ double k0_far(double t) {
     const double u = fma(4.0, y, -1.0);
     return exp(-x) * rsqrt(x) * series<K0_FAR_D_N>(K0_FAR_D, u);
 }
+// (i/4) H0(sqrt(t)) for 4 <= t < 64 (A and R as polynomials about t = 34) and
+// for t >= 64 (Hankel's form).  CUDA's j0 and y0 are good to 5e-12 absolutely
+// beyond 8; this is good to a few 1e-17, at about half the instructions of the
+// two calls.
+__device__ __forceinline__ PairValue h0_far(double t) {
+    if (t < 64.0) {
+        const double u = fma(t, 1.0 / 30.0, -34.0 / 30.0), a = series<H0_MID_A_D_N>(H0_MID_A_D, u);
+        return {fma(log(0.25 * t), a, series<H0_MID_R_D_N>(H0_MID_R_D, u)), a};
+    }
+    const double y = rsqrt(t);
+    double x = t * y;
+    x = fma(0.5 * y, fma(-x, x, t), x);
+    const double v = fma(128.0 * y, y, -1.0);
+    const double p = series<H0_P_D_N>(H0_P_D, v), q = series<H0_Q_D_N>(H0_Q_D, v) * y;
+    double s, c;
+    sincos(x, &s, &c);
+    const double m = 0.5641895835477563 * rsqrt(x), cs = c + s, sc = s - c;  // 1 / sqrt(pi x)
+    return {-0.25 * m * fma(p, sc, q * cs), -0.07957747154594767 * m * fma(p, cs, -q * sc)};
+}
 // ... of any other pair (coincident points, underflow, k r >= 2); kept out of
 // line, so that the pair loops stay small
 template <int KIND>
-__device__ __noinline__ double pair_value_any(double r2, double k) {
-    if (KIND == KIFMM_KERNEL_LAPLACE) return log(r2);
+__device__ __noinline__ PairValue pair_value_any(double r2, double k) {
+    if (KIND == KIFMM_KERNEL_LAPLACE) return {log(r2), 0.0};
+    if (KIND == KIFMM_KERNEL_MOD_HELMHOLTZ) {
+        const double t = r2 * (k * k);
+        return {t >= 4.0 && t < 1e300 ? k0_far(t) : k0_d(k * sqrt(r2)), 0.0};
+    }
     const double t = r2 * (k * k);
-    return t >= 4.0 && t < 1e300 ? k0_far(t) : k0_d(k * sqrt(r2));
+    if (t >= 4.0 && t < 1e300) return h0_far(t);
+    const double2 g = green_c(k, r2);
+    return {g.x, -0.3183098861837907 * g.y};
 }
 
 }  // namespace kifmm

@@ -970,8 +970,7 @@ void run_upward_downward(kifmm_plan *P) {
     PassArgs A = make_pass_args(P);
     if (P->n_p2m_list) {
         PhaseScope ph(P, KIFMM_PHASE_P2M);
-        if (P->cplx) launch_p2m_c(P, A);
-        else if (planned_ready(P)) launch_planned_p2m(P, A);
+        if (planned_ready(P)) launch_planned_p2m(P, A);
         else launch_p2m_d(P, A);
     }
     ops_wait_now(P);  // the P2M reads only the check circles

@@ -83,8 +83,10 @@ __device__ __forceinline__ void dmma_8x8x4(double &c0, double &c1, double a, dou
 }
 // row stride = 4 mod 16 doubles: conflict-free fragment loads
 __host__ __device__ constexpr int pad4mod16(int m) { return m + (20 - m % 16) % 16; }
-// pass_f64.cu
+// pass_f64.cu, pass_f64_complex.cu
 void launch_p2m_d(kifmm_plan *P, const PassArgs &A);
+void launch_p2m_dc(kifmm_plan *P, const PassArgs &A);
+void launch_leaf_eval_dc(kifmm_plan *P, const PassArgs &A, int check_self);
 void launch_leaf_far_d(kifmm_plan *P, const PassArgs &A);
 void launch_leaf_eval_d(kifmm_plan *P, const PassArgs &A, int check_self);
 // planned.cu
@@ -92,7 +94,6 @@ void launch_planned_p2m(kifmm_plan *P, const PassArgs &A);
 void launch_planned_leaf(kifmm_plan *P, const PassArgs &A);
 // passes_complex.cu (complex values: FP64 point passes on double2 densities)
 void launch_gather_tau_c(kifmm_plan *P);
-void launch_p2m_c(kifmm_plan *P, const PassArgs &A);
 void run_eval_sources_c(kifmm_plan *P, const PassArgs &A, int check_self);
 void run_eval_targets_c(kifmm_plan *P, const PassArgs &A, const double *tx, const double *ty, int64_t n,
                         int check_self, double *pot);

@@ -5,11 +5,10 @@
 // state is the real image of its complex check potential: Q = 2 Qc doubles,
 // [Re u (Qc), Im u (Qc)], and every translation operator is the real image of
 // the complex one (operators.cu), so M2M, M2L and L2L are the real FP64
-// kernels unchanged.  What touches points is here:
-//   P2M  numba_upwards_pass (class_fmm.py:57-71): check potential on the large
-//        circle from the node's sources;
+// kernels unchanged.  P2M and the L2P + P2P at the sources are in pass_f64.cu;
+// here:
 //   L2P + P2P  numba_target_local_expansion_evaluation / neighbor_evaluation
-//        (class_fmm.py:73-111), at the sources and at separate targets;
+//        (class_fmm.py:73-111) at separate targets;
 //   KF / KA / KAS (class_fmm.py:115-145) for a complex kernel.
 // Densities and potentials are double2 (re, im) in HBM.
 #include "passes.cuh"
@@ -38,114 +37,6 @@ __global__ void k_scatter_pot_c(const double2 *__restrict__ pots, const int32_t 
     pdl_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         pot[perm[i]] = pots[i];
-}
-
-// P2M: one warp per node; lane q (< Qc <= 32) sums over the node's sources,
-// staged 32 at a time in shared memory.
-constexpr int P2MC_WARPS = 8;
-__global__ void __launch_bounds__(32 * P2MC_WARPS) k_p2m_c(PassArgs A, const int32_t *__restrict__ list, int64_t nlist,
-                                                            const double2 *__restrict__ taus) {
-    __shared__ double sx[P2MC_WARPS][32], sy[P2MC_WARPS][32];
-    __shared__ double2 st[P2MC_WARPS][32];
-    pdl_trigger();
-    pdl_wait();
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, Qc = A.Qc;
-    const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    if (w >= nlist) return;
-    const int g = list[w], l = A.nlev[g];
-    double cx, cy;
-    node_center(A, g, l, cx, cy);
-    const double *lg = A.ops + (size_t)l * A.stride + A.off_large;  // x [0, Qc), y [Qc, 2 Qc)
-    const int b = A.nbot[g], e = A.ntop[g];
-    const bool ok = lane < Qc;
-    const double tx = ok ? lg[lane] + cx : 0.0, ty = ok ? lg[Qc + lane] + cy : 0.0;
-    double2 acc = make_double2(0.0, 0.0);
-    for (int s0 = b; s0 < e; s0 += 32) {
-        __syncwarp();
-        if (s0 + lane < e) {
-            sx[wib][lane] = A.xs[s0 + lane];
-            sy[wib][lane] = A.ys[s0 + lane];
-            st[wib][lane] = taus[s0 + lane];
-        }
-        __syncwarp();
-        const int ns = min(32, e - s0);
-        for (int u = 0; u < ns; u++) {
-            const double dx = tx - sx[wib][u], dy = ty - sy[wib][u];
-            cacc(acc, green_z(A.kind, A.k, dx * dx + dy * dy), st[wib][u]);
-        }
-    }
-    if (ok) {
-        A.uup[(size_t)g * A.Q + lane] = acc.x;
-        A.uup[(size_t)g * A.Q + Qc + lane] = acc.y;
-    }
-}
-
-// Local equivalent density of node g (levels >= 2): phi = Inv_l u_down on the
-// real image, as (re, im) pairs phi[q], q < Qc.
-__device__ __forceinline__ void local_density_c(const PassArgs &A, int g, int l, double *phi) {
-    const int Q = A.Q;
-    const double *inv = A.ops + (size_t)l * A.stride + A.off_inv;
-    for (int r = threadIdx.x; r < Q; r += blockDim.x) {
-        double s = 0.0;
-        if (l >= 2)
-            for (int c = 0; c < Q; c++) s = fma(inv[r * Q + c], A.udown[(size_t)g * Q + c], s);
-        phi[r] = s;
-    }
-}
-
-// L2P + P2P for one target leaf per block (class_fmm.py:73-111); the L2P
-// evaluates the local density on the large circle in box-relative coordinates
-// (class_fmm.py:81-87).
-__global__ void k_leaf_eval_c(PassArgs A, const int32_t *__restrict__ list, int check_self,
-                              const double2 *__restrict__ taus, double2 *__restrict__ pots) {
-    extern __shared__ __align__(16) double smc[];
-    const int Q = A.Q, Qc = A.Qc, nb = blockDim.x;
-    double *phi = smc;                       // [Q]: Re at [0, Qc), Im at [Qc, Q)
-    double2 *st = (double2 *)(smc + Q);      // [nb] (Q even: 16-byte aligned)
-    double *sx = (double *)(st + nb), *sy = sx + nb;
-    const int g = list[blockIdx.x], l = A.nlev[g];
-    double cx, cy;
-    node_center(A, g, l, cx, cy);
-    local_density_c(A, g, l, phi);
-    __syncthreads();
-    const double *lg = A.ops + (size_t)l * A.stride + A.off_large;
-    const int b = A.nbot[g], e = A.ntop[g];
-    for (int t0 = b; t0 < e; t0 += nb) {
-        const int t = t0 + threadIdx.x;
-        const bool act = t < e;
-        const double px = act ? A.xs[t] : 0.0, py = act ? A.ys[t] : 0.0;
-        double2 acc = make_double2(0.0, 0.0);
-        if (act && l >= 1) {
-            const double rx = px - cx, ry = py - cy;
-            for (int q = 0; q < Qc; q++) {
-                const double dx = rx - lg[q], dy = ry - lg[Qc + q];
-                cacc(acc, green_z(A.kind, A.k, dx * dx + dy * dy), make_double2(phi[q], phi[Qc + q]));
-            }
-        }
-        for (int d = 0; d < 9; d++) {
-            const int c = A.ncoll[9 * (size_t)g + d];
-            if (c < 0) continue;
-            const int cb = A.nbot[c], ce = A.ntop[c];
-            for (int s0 = cb; s0 < ce; s0 += nb) {
-                __syncthreads();
-                const int s = s0 + threadIdx.x;
-                if (s < ce) {
-                    sx[threadIdx.x] = A.xs[s];
-                    sy[threadIdx.x] = A.ys[s];
-                    st[threadIdx.x] = taus[s];
-                }
-                __syncthreads();
-                const int ns = min(nb, ce - s0);
-                if (act)
-                    for (int u = 0; u < ns; u++) {
-                        const double dx = px - sx[u], dy = py - sy[u];
-                        if (check_self && dx == 0.0 && dy == 0.0) continue;
-                        cacc(acc, green_z(A.kind, A.k, dx * dx + dy * dy), st[u]);
-                    }
-            }
-        }
-        if (act) pots[t] = acc;
-    }
 }
 
 // separate targets: locate by strict '>' descent (tree.py:712-727), L2P, P2P
@@ -254,21 +145,10 @@ void launch_gather_tau_c(kifmm_plan *P) {
                (const double2 *)P->tau.p, (const int32_t *)P->perm.p, P->N, (double2 *)P->taus.p);
 }
 
-void launch_p2m_c(kifmm_plan *P, const PassArgs &A) {
-    KIFMM_REQUIRE(P->Qc <= 32, KIFMM_ERR_ARG, "complex form: Nequiv above 32");
-    launch_pdl(k_p2m_c, dim3(grid_for(P->n_p2m_list * 32, 32 * P2MC_WARPS)), dim3(32 * P2MC_WARPS), 0, P->stream, A,
-               (const int32_t *)P->p2m_list.p, P->n_p2m_list, (const double2 *)P->taus.p);
-}
-
 void run_eval_sources_c(kifmm_plan *P, const PassArgs &A, int check_self) {
     if (P->n_leaf_list) {
         PhaseScope ph(P, KIFMM_PHASE_LEAF);
-        const int thr = P->ppl <= 64 ? 64 : 128;
-        const size_t smem = (size_t)(P->Q + 4 * thr) * sizeof(double);
-        k_leaf_eval_c<<<(unsigned)P->n_leaf_list, thr, smem, P->stream>>>(A, P->leaf_list.p, check_self,
-                                                                           (const double2 *)P->taus.p,
-                                                                           (double2 *)P->pots.p);
-        KIFMM_LAUNCHED();
+        launch_leaf_eval_d(P, A, check_self);
     }
     launch_pdl(k_scatter_pot_c, dim3(grid_for(P->N, 256, P->num_sms * 8)), dim3(256), 0, P->stream,
                (const double2 *)P->pots.p, (const int32_t *)P->perm.p, P->N, (double2 *)P->pot_out.p);

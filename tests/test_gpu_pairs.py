@@ -88,3 +88,40 @@ def test_leaf_tiles_vs_oracle(kind, k, n, cutoff):
     o.build_expansions(tau)
     ref = o.evaluate_to_points(x, y, True)
     assert np.abs(pot - ref).max() / np.abs(ref).max() <= 1e-9  # the bound of the plain form's other tests
+
+
+def direct_complex(kind, k, x, y, tau):
+    from scipy import special
+    dx, dy = x[:, None] - x[None, :], y[:, None] - y[None, :]
+    r = np.sqrt(dx * dx + dy * dy)
+    same = r == 0
+    r[same] = 1
+    if kind == "h0":
+        g = 0.25j * special.hankel1(0, k * r)
+    elif kind == "k0":
+        g = special.k0(k * r) / (2 * np.pi) + 0j
+    else:
+        g = -np.log(r) / (2 * np.pi) + 0j
+    g[same] = 0
+    return g @ tau, (np.abs(g) + 1) @ np.abs(tau)
+
+
+@pytest.mark.parametrize("n", [1, 2, 9, 22, 32, 33, 64, 65, 130])
+@pytest.mark.parametrize("kind,k", [("h0", 0.04), ("h0", 0.17), ("h0", 0.34), ("h0", 4.0), ("h0", 40.0),
+                                    ("laplace", 0.0), ("k0", 0.2), ("k0", 9.0)])
+def test_one_leaf_complex(kind, k, n):
+    """The complex pair loops; scipy's Bessel functions are good to about 1e-15
+    of the function's size near its zeros, hence 64 eps per term."""
+    import pykifmm2d_b200 as P
+    x, y, tau = cloud(n, n)
+    tau = tau + 1j * np.random.default_rng(n + 1).standard_normal(n)
+    if n > 8:
+        x[5], y[5] = x[2], y[2]
+    kern = {"h0": P.HelmholtzKernel, "k0": P.ModifiedHelmholtzKernel}.get(kind, lambda k: P.LaplaceKernel())(k)
+    f = P.FMM(x, y, P.Get_Kernel_Functions(kern), P.prepare_numba_functions_on_the_fly(kern), 24, 200, True)
+    f.build_tree()
+    f.precompute()
+    f.build_expansions(tau)
+    ref, mag = direct_complex(kind, k, x, y, tau)
+    pot = f.evaluate_to_points(x, y, True)
+    assert np.all(np.abs(pot - ref) <= (n + 64) * EPS * mag)
