@@ -55,7 +55,6 @@ __global__ void __launch_bounds__(DEN_THREADS) k_leaf_density(DenArgs D) {
     double *mS = sm_den;                  // [Kp][ldm]: Inv[r][c] at c * ldm + r
     double *xS = mS + (size_t)Kp * ldm;   // [32][ldx]
     const int tid = threadIdx.x;
-    pdl_trigger();
     const int64_t b = blockIdx.x;
     int l = D.lmin;
     while (l < D.lmax && D.toff[l + 1] <= b) l++;
@@ -67,6 +66,9 @@ __global__ void __launch_bounds__(DEN_THREADS) k_leaf_density(DenArgs D) {
         mS[c * ldm + r] = r < Q && c < Q ? inv[r * Q + c] : 0.0;
     }
     pdl_wait();  // u_down comes from the L2L chain
+    // only now: the leaf pass's blocks fill every SM, and waiting there through
+    // the L2L chain they would keep other streams' kernels out
+    pdl_trigger();
     for (int i = tid; i < 32 * Kp; i += DEN_THREADS) {
         const int n = i / Kp, c = i - n * Kp;
         xS[n * ldx + c] = n < nt && c < Q ? A.udown[(size_t)D.list[w0 + n] * Q + c] : 0.0;

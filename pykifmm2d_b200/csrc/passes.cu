@@ -14,8 +14,8 @@ namespace kifmm {
 
 __global__ void k_gather_tau(const double *__restrict__ tau, const int32_t *__restrict__ perm, int64_t n,
                              double *__restrict__ taus) {
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();  // the P2M's blocks fill every SM: not before this kernel runs
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         taus[i] = tau[perm[i]];
 }

@@ -25,8 +25,8 @@ __device__ __forceinline__ void cacc(double2 &acc, double2 a, double2 b) {
 
 __global__ void k_gather_tau_c(const double2 *__restrict__ tau, const int32_t *__restrict__ perm, int64_t n,
                                double2 *__restrict__ taus) {
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         taus[i] = tau[perm[i]];
 }
