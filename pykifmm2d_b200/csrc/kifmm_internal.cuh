@@ -210,7 +210,8 @@ struct kifmm_plan {
 
     // operators
     bool have_ops = false;
-    kifmm::DBuf<double> ops, ops_tmp;
+    kifmm::DBuf<double> ops;
+    kifmm::DBuf<double> ops_tmp;     // [L][49] M2L offset blocks (operators.cu: M2lBlocks)
     kifmm::LevelOps lops[kifmm::MAX_LEVELS + 1]{};
     kifmm::DBuf<float> ops_f;        // FP32 copies for the mixed passes
     kifmm::DBuf<uint16_t> ops_h;     // split half-precision M2L operators
@@ -239,7 +240,6 @@ struct kifmm_plan {
     kifmm::DBuf<int32_t> tperm, tperm2;
     kifmm::DBuf<double> txs, tys, node_den;
     kifmm::DBuf<double> uup, udown;
-    kifmm::DBuf<double> zero4q;      // 4Q zeros: the source of an absent M2L direction
     bool have_expansions = false;
     bool applied = false;  // an apply at the sources ran since the tree / operators were built
 
@@ -535,6 +535,24 @@ void kernel_matrix_device(const kifmm_kernel &k, const double *sx, const double 
 void kernel_apply_device(const kifmm_kernel &k, const double *sx, const double *sy, int64_t ns,
                          const double *tx, const double *ty, int64_t nt, const double *tau, double *out,
                          cudaStream_t s);
+// The 49 M2L offset blocks of a level, P_o = M2LS_o . Inv_l (the 3x3 near ones
+// unused): row-major [Q][Q], or, where k_m2l_dmma reads them (the FP64 form
+// with even Nequiv), column-major with the rows padded to ldq (4 mod 8
+// doubles: conflict-free fragment loads) and the columns to kp (zeros), so
+// that any run of columns is one bulk copy.
+struct M2lBlocks {
+    int qp, kp, ldq;     // rows rounded up to 8, columns to 4, row stride
+    size_t block;        // doubles per offset block
+};
+inline bool m2l_uses_dmma(const kifmm_plan *P) { return P->opt.precision == KIFMM_PREC_FP64 && P->Q % 2 == 0; }
+inline M2lBlocks m2l_blocks(int Q) {
+    M2lBlocks B;
+    B.qp = (Q + 7) & ~7;
+    B.kp = (Q + 3) & ~3;
+    B.ldq = B.qp + 4;
+    B.block = (size_t)B.kp * B.ldq;
+    return B;
+}
 // m2l_tc.cu
 void build_tc_operators(kifmm_plan *P);
 bool uses_tensor_m2l(const kifmm_plan *P);

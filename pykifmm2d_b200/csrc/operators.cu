@@ -30,7 +30,8 @@ struct OpsArgs {
     double rf1, rf2;
     size_t stride;          // doubles per level block
     double *ops;            // level blocks
-    double *poff;           // temp [L][49][Q][Q] = M2LS . Inv (row-major)
+    double *poff;           // [L][49] offset blocks M2LS . Inv: [Q][Q] row-major, or padded (ldq > 0)
+    int kp, ldq;            // padded blocks: columns, row stride (M2lBlocks); ldq = 0: row-major
 };
 
 // level block layout (offsets in doubles)
@@ -227,11 +228,13 @@ __global__ void k_ops_compose(OpsArgs A) {
     }
     __syncthreads();
     if (slot < 49) {
-        double *p = A.poff + ((size_t)l * 49 + slot) * Q * Q;
-        for (int e = threadIdx.x; e < Q * Q; e += blockDim.x) {
-            int r = e / Q, c = e % Q;
+        const int ld = A.ldq;
+        double *p = A.poff + ((size_t)l * 49 + slot) * (ld ? (size_t)A.kp * ld : (size_t)Q * Q);
+        for (int e = threadIdx.x; e < (ld ? A.kp * ld : Q * Q); e += blockDim.x) {
+            const int r = ld ? e % ld : e / Q, c = ld ? e / ld : e % Q;
             double s = 0;
-            for (int t = 0; t < Q; t++) s = fma(mm[r * Q + t], iv[t * Q + c], s);
+            if (r < Q && c < Q)
+                for (int t = 0; t < Q; t++) s = fma(mm[r * Q + t], iv[t * Q + c], s);
             p[e] = s;
         }
     } else if (m2m) {
@@ -344,8 +347,12 @@ void build_operators(kifmm_plan *P) {
     KIFMM_CUDA(cudaMemsetAsync(P->ops.p, 0, A.stride * (size_t)L * sizeof(double), s));
     A.ops = P->ops.p;
     DBuf<double> &tmp = P->ops_tmp;
-    size_t n49 = (size_t)L * 49 * Q * Q;
-    tmp.alloc(n49);
+    // the FP64 M2L reads the offset blocks themselves, the other forms the 4Q x
+    // 4Q blocks per direction that k_ops_assemble makes of them
+    const M2lBlocks MB = m2l_blocks(Q);
+    const bool dmma = m2l_uses_dmma(P);
+    if (dmma) A.kp = MB.kp, A.ldq = MB.ldq;
+    tmp.alloc((size_t)L * 49 * (dmma ? MB.block : (size_t)Q * Q));
     A.poff = tmp.p;
     for (int l = 0; l < L; l++) {
         double *b = P->ops.p + (size_t)l * A.stride;
@@ -379,8 +386,10 @@ void build_operators(kifmm_plan *P) {
         ensure_dyn_smem(k_ops_compose, csm);
         k_ops_compose<<<dim3(L, OPS_COMPOSE_SLOTS), 256, csm, s>>>(A);
         KIFMM_LAUNCHED();
-        k_ops_assemble<<<dim3(L, 9), 256, 0, s>>>(A, rowmax);
-        KIFMM_LAUNCHED();
+        if (!dmma) {
+            k_ops_assemble<<<dim3(L, 9), 256, 0, s>>>(A, rowmax);
+            KIFMM_LAUNCHED();
+        }
     }
     if (mixed) {
         if (P->opt.m2l == KIFMM_M2L_FP32) {  // only the FP32 SIMT M2L reads FP32 operators

@@ -6,6 +6,8 @@
 //   u_down (reference Local_Solutions) -- downward check potential of a node.
 // Nodes of a level are stored sibling-group contiguous, so the four children
 // of an entry (split or X-list cell) form one 4Q vector.
+#include <algorithm>
+
 #include "kifmm_internal.cuh"
 #include "passes.cuh"
 #include "async_copy.cuh"
@@ -102,36 +104,48 @@ __global__ void k_m2l_d(PassArgs A, int l) {
 }
 
 // M2L of every level in one launch on the FP64 tensor path (mma.sync
-// m8n8k4 .f64), class_fmm.py:336-343 recast target-centric:
-//   u_down(children of p) = sum_{d != centre} C_d . u_up(children of p + d),
-// C_d = CM2LS_d . blockdiag(Inv) (4Q x 4Q, column-major).  A block owns 32
-// consecutive split entries of one level (its target groups) and all 4Q rows:
-// D[4Q x 32] = sum over (direction, K chunk of 32) of C_d[:, chunk] .
-// B_d[chunk, 32], B_d's columns the targets' source groups in direction d
-// (a zero vector where a target has none).  Stages run through a ring of two
-// shared-memory slots, warp-specialised: a copy warp fills a slot by bulk
-// copies (the operator chunk as 32 columns of 4Q doubles, the sources as 32
-// rows of 32 doubles, one copy per lane) on the slot's full barrier as soon
-// as the eight compute warps have arrived on its empty barrier, so the
-// copies of stage s + 1 land while stage s computes and no block-wide
-// barrier stands in the loop.  Compute warp w owns row tiles w, w + 8, ...
-// (8 rows each) for all 32 targets.  D is assigned to the
-// children's u_down (the L2L chain adds afterwards).  Needs Q even.
-#ifndef KIFMM_MD_KC
-#define KIFMM_MD_KC 32
-#endif
-#ifndef KIFMM_MD_NBUF
-#define KIFMM_MD_NBUF 2
-#endif
-constexpr int MD_THREADS = 256, MD_TE = 32, MD_KC = KIFMM_MD_KC, MD_MT = 4;  // Q4 <= 8 warps x MD_MT x 8 rows
-constexpr int MD_NBUF = KIFMM_MD_NBUF;  // ring slots: copies run MD_NBUF - 1 stages ahead
-constexpr int MD_BLOCK = MD_THREADS + 32;  // eight compute warps and one copy warp
-static_assert(MD_KC % 4 == 0 && MD_NBUF >= 2 && MD_NBUF <= 8, "DMMA M2L staging shape");
+// m8n8k4 .f64), class_fmm.py:336-343 recast target-centric: for the children
+// ta of a target group and the children sb of its source group in direction d,
+//   u_down(ta) = sum_{d, sb} P_o . u_up(sb),  o = 2 d - ta + sb,
+// P_o one of the level's 40 far offset blocks (Q x Q; near offsets are left
+// out).  A block owns 8 NCT consecutive entries of one level (its target
+// groups) and cp of their four children, 4 / cp of its four compute warps to
+// each, NR row tiles (8 rows) to a warp.  A stage is a pair (d, sb) and a run of
+// kc of the Q columns: the columns of the children's offset blocks, one bulk
+// copy each, and that part of the targets' source vectors (zeros where a
+// target has no source), copied by 16-byte cp.async.  Stages run through a ring
+// of shared-memory slots, warp-specialised: two copy warps fill a slot on its
+// full barriers as soon as the compute warps have arrived on its empty
+// barrier, so the copies of the next stages land while one computes and no
+// block-wide barrier stands in the loop.  A warp whose child has a near offset
+// passes the stage over, and every warp an 8-target column tile without a
+// source.  The result is assigned to the children's u_down (the L2L chain adds
+// afterwards).  Needs Q even.
+//
+// Bound by the FP64 tensor path for large trees (256 multiply-adds in 16 clocks
+// of a scheduler, the vector pipe's rate; 87 us of products in 187 us at 1M
+// points, 234 before) and by the stages' latency for small ones.  What the
+// shape answers to, as measured: two compute warps per scheduler keep the pipe within 2% of its rate from shared memory, one 75-80%;
+// a number of compute warps that is no multiple of four leaves three
+// schedulers waiting for the fourth; one warp issues a bulk copy, or a 512-byte
+// cp.async instruction, about every 86 clocks (64 row copies a stage were 2400
+// of 3300 clocks a stage on a 1k-point tree); a run-time test per column tile
+// took 14 instructions a multiply-add.  Reading the offset blocks instead of
+// assembled 4Q x 4Q ones leaves out the near blocks' products (16% on a full V
+// list) and 1 MB of operator per level.
+constexpr int MD_MAX_NBUF = 8;   // most ring slots
+constexpr int MD_CWARPS = 4;     // compute warps of a block
+constexpr int MD_PWARPS = 2;     // copy warps
+constexpr int MD_BLOCK = 32 * (MD_CWARPS + MD_PWARPS);
 struct M2lDmmaArgs {
     PassArgs A;
-    const double *zero;                 // 4Q zeros
+    const double *blocks;           // [L][49] offset blocks
+    M2lBlocks B;
     int lmin, lmax;
-    int64_t tile_off[MAX_LEVELS + 1];   // first block of each parent level
+    int cp;                         // children per block (1, 2 or 4)
+    int kc;                         // columns of a stage (a multiple of 4)
+    int nbuf;                       // ring slots
+    int64_t tile_off[MAX_LEVELS + 1];  // first tile of each parent level
     long long wait_limit;
     unsigned long long *err;
 };
@@ -140,162 +154,293 @@ struct M2lDmmaArgs {
 __device__ __forceinline__ bool warp_wait_all(uint32_t bar, uint32_t parity, long long limit) {
     return __any_sync(0xffffffffu, mbar_wait(bar, parity, limit));
 }
-static size_t m2l_dmma_smem(int Q4) {
-    const size_t ldo = pad4mod16(Q4), ldx = pad4mod16(MD_KC);
-    const size_t stage = (size_t)MD_KC * ldo + (size_t)MD_TE * ldx;
-    const size_t out = (size_t)MD_TE * (Q4 + 1);
-    return (MD_NBUF * stage > out ? MD_NBUF * stage : out) * sizeof(double) + MD_TE * 8 * sizeof(int) + 64;
+// ... on two mbarriers at the same phase, odd lanes polling the second
+__device__ __forceinline__ bool warp_wait_both(uint32_t bar0, uint32_t bar1, uint32_t parity, long long limit) {
+    return __all_sync(0xffffffffu, mbar_wait(threadIdx.x & 1 ? bar1 : bar0, parity, limit));
 }
-__global__ void __launch_bounds__(MD_BLOCK, 2) k_m2l_dmma(M2lDmmaArgs M) {
+__host__ __device__ __forceinline__ int pad4mod8(int m) { return m + (12 - m % 8) % 8; }
+static size_t m2l_stage_bytes(const M2lBlocks &B, int cp, int te, int kc) {
+    return ((size_t)cp * kc * B.ldq + (size_t)te * pad4mod8(kc)) * sizeof(double);
+}
+static size_t m2l_dmma_smem(const M2lBlocks &B, int cp, int te, int kc, int nbuf) {
+    return std::max(nbuf * m2l_stage_bytes(B, cp, te, kc), (size_t)te * (cp * B.qp + 1) * sizeof(double)) +
+           te * 8 * sizeof(int) + 64;
+}
+// slot of the offset between source child sb in direction dd (0..7, centre
+// left out) and target child ta; -1: near
+__device__ __forceinline__ int m2l_slot(int dd, int ta, int sb) {
+    const int d = dd < 4 ? dd : dd + 1, dx = d / 3 - 1, dy = d - 3 * (dx + 1) - 1;
+    const int ox = 2 * dx - (ta >> 1) + (sb >> 1), oy = 2 * dy - (ta & 1) + (sb & 1);
+    return ox >= -1 && ox <= 1 && oy >= -1 && oy <= 1 ? -1 : (ox + 3) * 7 + oy + 3;
+}
+// a stage's products for the column tiles of mask CM
+template <int NR, int NCT, int CM>
+__device__ __forceinline__ void m2l_ksteps(double (&acc)[NR][NCT][2], const double *o, int ldq, const double *xs,
+                                           int ldx, int kn) {
+#pragma unroll 2
+    for (int k = 0; k < kn; k += 4) {
+        double a[NR], bv[NCT];
+#pragma unroll
+        for (int i = 0; i < NR; i++) a[i] = o[k * ldq + 8 * i];
+#pragma unroll
+        for (int c = 0; c < NCT; c++)
+            if ((CM >> c) & 1) bv[c] = xs[8 * c * ldx + k];
+#pragma unroll
+        for (int c = 0; c < NCT; c++)
+            if ((CM >> c) & 1)
+#pragma unroll
+                for (int i = 0; i < NR; i++) dmma_8x8x4(acc[i][c][0], acc[i][c][1], a[i], bv[c]);
+    }
+}
+template <int NR, int NCT, int CM>
+__device__ __forceinline__ void m2l_masked(int cm, double (&acc)[NR][NCT][2], const double *o, int ldq,
+                                           const double *xs, int ldx, int kn) {
+    if (cm == CM) m2l_ksteps<NR, NCT, CM>(acc, o, ldq, xs, ldx, kn);
+    else if constexpr (CM > 1) m2l_masked<NR, NCT, CM - 1>(cm, acc, o, ldq, xs, ldx, kn);
+}
+template <int NR, int NCT>
+__global__ void __launch_bounds__(MD_BLOCK, NR <= 6 ? 3 : 2) k_m2l_dmma(M2lDmmaArgs M) {
+    constexpr int TE = 8 * NCT;
     extern __shared__ __align__(128) double sm_md[];
     const PassArgs &A = M.A;
-    const int Q = A.Q, Q4 = 4 * Q, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int ldo = pad4mod16(Q4), ldx = pad4mod16(MD_KC);
-    const size_t stage_d = (size_t)MD_KC * ldo + (size_t)MD_TE * ldx;
-    int *ssrc = (int *)(sm_md + (MD_NBUF * stage_d > (size_t)MD_TE * (Q4 + 1) ? MD_NBUF * stage_d
-                                                                              : (size_t)MD_TE * (Q4 + 1)));
-    __shared__ __align__(8) uint64_t bars[MD_NBUF], empty[MD_NBUF];
-    __shared__ int sabort;
-    __shared__ int sact[MD_TE];
-    __shared__ int sdir[8], scm[8], snd;  // active directions, their 8-target column tiles with a source
+    const int Q = A.Q, qp = M.B.qp, kp = M.B.kp, ldq = M.B.ldq, cp = M.cp, kc = M.kc, nbuf = M.nbuf;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int ldx = pad4mod8(kc), RB = cp * qp, oblk = kc * ldq;  // doubles per child of a slot
+    const size_t stage_d = (size_t)cp * oblk + (size_t)TE * ldx;
+    int *ssrc = (int *)(sm_md + (nbuf * stage_d > (size_t)TE * (RB + 1) ? nbuf * stage_d : (size_t)TE * (RB + 1)));
+    __shared__ __align__(8) uint64_t bars[MD_MAX_NBUF], obar[MD_MAX_NBUF], empty[MD_MAX_NBUF];
+    __shared__ int sabort, snst;
+    __shared__ int sact[TE];
+    __shared__ int scm[8], sst[32];  // column tiles with a source; pairs: 4 dd + sb, children mask << 8
     pdl_trigger();
-    const int64_t b = blockIdx.x;
+    const int parts = 4 / cp;
+    const int64_t b = blockIdx.x / parts;
+    const int ta0 = (int)(blockIdx.x - b * parts) * cp;  // this block's children
     int l = M.lmin;
     while (l < M.lmax && M.tile_off[l + 1] <= b) l++;
-    const int64_t e0 = (b - M.tile_off[l]) * MD_TE, ne = A.T.ne[l], eoff = A.T.eoff[l];
-    const double *opl = A.ops + (size_t)(l + 1) * A.stride + A.off_m2l;  // target level's operators
-    pdl_wait();  // u_up comes from the M2M chain
-    if (tid < MD_TE) {  // the tile's targets in M2L target order; sact = 1 + index in the level, 0: none
-        const int64_t e = e0 + tid, ej = e < ne ? (int64_t)A.m2l_perm[eoff + e] : -1;
-        const bool act = ej >= 0 && !(A.ent[ej] & 1);
-        sact[tid] = act ? (int)(ej - eoff) + 1 : 0;
-        for (int dd = 0; dd < 8; dd++) ssrc[tid * 8 + dd] = act ? A.m2l_src8[ej * 8 + dd] : -1;
-    }
+    const int64_t e0 = (b - M.tile_off[l]) * TE, ne = A.T.ne[l], eoff = A.T.eoff[l];
+    const double *opl = M.blocks + (size_t)(l + 1) * 49 * M.B.block;  // target level's operators
     if (tid == 0) {
-        for (int i = 0; i < MD_NBUF; i++) {
-            mbar_init(smem_u32(&bars[i]));              // full: the stage's copies (transaction bytes)
-            mbar_init(smem_u32(&empty[i]), MD_THREADS / 32);  // empty: each compute warp is done with it
+        for (int i = 0; i < nbuf; i++) {
+            mbar_init(smem_u32(&bars[i]), 32 * MD_PWARPS);  // full: every copy lane's copies
+            mbar_init(smem_u32(&obar[i]));                  // ... and the offset blocks (transaction bytes)
+            mbar_init(smem_u32(&empty[i]), MD_CWARPS);      // empty: each compute warp is done with it
         }
         sabort = 0;
     }
-    __syncthreads();
-    // Work skipped: a direction no target of the block has a source in, and
-    // within a direction each 8-target column tile without one (a V-list
-    // group is absent where the colleague is missing, a leaf or empty).
-    if (tid < 8) {
-        int m = 0;
-        for (int n = 0; n < MD_TE; n++) m |= (ssrc[n * 8 + tid] >= 0) << (n >> 3);
-        scm[tid] = m;
-    }
-    __syncthreads();
-    if (tid == 0) {
-        int k = 0;
-        for (int dd = 0; dd < 8; dd++)
-            if (scm[dd]) sdir[k++] = dd;
-        snd = k;
-    }
-    __syncthreads();
-    const int nkc = (Q4 + MD_KC - 1) / MD_KC, nst = snd * nkc;
-    // the lanes of warp 0 issue the copies of stage st into buffer st % 2
-    // (one operator column and one source row each: issued by one thread
-    // they kept warp 0, and the whole block at the next barrier, waiting)
-    auto issue = [&](int st) {
-        const int dd = sdir[st / nkc], d = dd < 4 ? dd : dd + 1, kc = st % nkc, k0 = kc * MD_KC;
-        const int kn = min(MD_KC, Q4 - k0), cm = scm[dd];
-        double *bs = sm_md + (size_t)(st % MD_NBUF) * stage_d;
-        const uint32_t bar = smem_u32(&bars[st % MD_NBUF]);
-        if (lane == 0) mbar_expect_tx(bar, (uint32_t)(kn * Q4 + 8 * __popc(cm) * kn) * 8u);
-        __syncwarp();
-        const double *op = opl + (size_t)d * Q4 * Q4 + (size_t)k0 * Q4;
-        for (int c = lane; c < kn; c += 32)
-            bulk_g2s(smem_u32(bs + (size_t)c * ldo), op + (size_t)c * Q4, (uint32_t)Q4 * 8u, bar);
-        double *xs = bs + (size_t)MD_KC * ldo;
-        for (int n = lane; n < MD_TE; n += 32) {
-            if (!((cm >> (n >> 3)) & 1)) continue;
-            const int je = ssrc[n * 8 + dd];
-            const double *src = je >= 0 ? A.uup + (size_t)(A.T.off[l + 1] + 4 * (je - eoff)) * Q + k0 : M.zero + k0;
-            bulk_g2s(smem_u32(xs + (size_t)n * ldx), src, (uint32_t)kn * 8u, bar);
+    // the source vectors' padding (columns Q .. kp of the last run; kp - Q is 0
+    // or 2) meets zero columns of the operator: it must only be finite to begin
+    // with (later it holds values of the same target's earlier sources)
+    if (kp > Q)
+        for (int i = tid; i < nbuf * TE; i += MD_BLOCK) {
+            const int slot = i / TE, n = i - slot * TE, k = Q - (kp - 1) / kc * kc;
+            double *x = sm_md + slot * stage_d + (size_t)cp * oblk + (size_t)n * ldx;
+            for (int c = k; c < kc; c++) x[c] = 0.0;
         }
-    };
-    const int g = lane >> 2, t = lane & 3, nrt = Q4 / 8;
-    double acc[MD_MT][4][2];
+    pdl_wait();  // u_up comes from the M2M chain
+    for (int i = tid; i < TE * 8; i += MD_BLOCK) {  // the tile's targets in M2L target order
+        const int64_t e = e0 + (i >> 3), ej = e < ne ? (int64_t)A.m2l_perm[eoff + e] : -1;
+        const bool act = ej >= 0 && !(A.ent[ej] & 1);
+        ssrc[i] = act ? A.m2l_src8[ej * 8 + (i & 7)] : -1;
+        if ((i & 7) == 0) sact[i >> 3] = act ? (int)(ej - eoff) + 1 : 0;  // 1 + index in the level, 0: none
+    }
+    __syncthreads();
+    for (int dd = warp; dd < 8; dd += MD_BLOCK / 32) {  // column tiles of direction dd with a source
+        const unsigned m = __ballot_sync(0xffffffffu, lane < TE && ssrc[(lane < TE ? lane : 0) * 8 + dd] >= 0);
+        int cm = 0;
 #pragma unroll
-    for (int i = 0; i < MD_MT; i++)
+        for (int c = 0; c < NCT; c++) cm |= ((m >> (8 * c)) & 0xff) ? 1 << c : 0;
+        if (lane == 0) scm[dd] = cm;
+    }
+    __syncthreads();
+    if (warp == 0) {  // the (direction, source child) pairs with a source and a far child
+        int cm = 0;
+        for (int c = 0; c < cp; c++) cm |= (m2l_slot(lane >> 2, ta0 + c, lane & 3) >= 0) << c;
+        if (!scm[lane >> 2]) cm = 0;
+        const unsigned m = __ballot_sync(0xffffffffu, cm);
+        if (cm) sst[__popc(m & ((1u << lane) - 1))] = lane | cm << 8;
+        if (lane == 0) snst = __popc(m);
+    }
+    __syncthreads();
+    const int npair = snst;
+    const int g = lane >> 2, t = lane & 3, wpc = MD_CWARPS / cp, ch = warp / wpc;  // the warp's child
+    const int row0 = (warp - ch * wpc) * NR * 8;                                   // and its rows there
+    double acc[NR][NCT][2];
 #pragma unroll
-        for (int c = 0; c < 4; c++) acc[i][c][0] = acc[i][c][1] = 0.0;
+    for (int i = 0; i < NR; i++)
+#pragma unroll
+        for (int c = 0; c < NCT; c++) acc[i][c][0] = acc[i][c][1] = 0.0;
     volatile int *abort_flag = &sabort;
-    if (warp == MD_THREADS / 32) {
-        // producer warp: stage st goes into slot st % MD_NBUF once the compute
-        // warps have released the slot's previous stage
-        int issued = 0;
-        for (int st = 0; st < nst; st++) {
-            const int slot = st % MD_NBUF;
-            if (st >= MD_NBUF && !warp_wait_all(smem_u32(&empty[slot]), (uint32_t)(st / MD_NBUF - 1) & 1u, M.wait_limit)) {
-                if (lane == 0) {
-                    *abort_flag = 1;
-                    atomicOr(M.err, 1ull);
+    int slot = 0, round = 0;
+    if (warp >= MD_CWARPS) {
+        // copy warps: a stage goes into the next slot once the compute warps have
+        // released the slot's previous stage.  A lane copies pieces q, q + LQ, ...
+        // of the vectors of targets n0, n0 + rpp, ... (LQ lanes to a vector); the
+        // source groups change with the direction only and are kept in registers.
+        constexpr int LANES = 32 * MD_PWARPS, LQ = 8, RPP = LANES / LQ, MAXI = (TE + RPP - 1) / RPP;
+        const int pl = tid - 32 * MD_CWARPS, n0 = pl / LQ, q0 = pl % LQ;
+        const double *const src0 = A.uup + (int64_t)(A.T.off[l + 1] - 4 * eoff) * Q;
+        int je[MAXI], dir = -1, issued = 0;
+        for (int pr = 0; pr < npair; pr++) {
+            const int sv = sst[pr], dd = (sv >> 2) & 7, sb = sv & 3, ctile = scm[dd];
+            if (dd != dir) {
+                dir = dd;
+#pragma unroll
+                for (int i = 0; i < MAXI; i++) {
+                    const int n = n0 + i * RPP;  // -2: no copy (no such target, or a column tile passed over)
+                    je[i] = n < TE && ((ctile >> (n >> 3)) & 1) ? ssrc[n * 8 + dd] : -2;
                 }
-                break;
             }
-            if (*abort_flag) break;
-            issue(st);
-            issued = st + 1;
-        }
-        // every copy issued lands before the block goes on (consumed stages
-        // have landed already; this matters after an abort)
-        for (int st = issued > MD_NBUF ? issued - MD_NBUF : 0; st < issued; st++)
-            mbar_wait(smem_u32(&bars[st % MD_NBUF]), (uint32_t)(st / MD_NBUF) & 1u, kDrainWaitPolls);
-    } else {
-        for (int st = 0; st < nst; st++) {
-            const int bi = st % MD_NBUF;
-            if (!warp_wait_all(smem_u32(&bars[bi]), (uint32_t)(st / MD_NBUF) & 1u, M.wait_limit)) {
-                if (lane == 0) {
-                    *abort_flag = 1;
-                    atomicOr(M.err, 1ull);
-                }
-                break;
-            }
-            if (*abort_flag) break;
-            const int kn = min(MD_KC, Q4 - (st % nkc) * MD_KC), cm = scm[sdir[st / nkc]];
-            const double *os = sm_md + (size_t)bi * stage_d, *xs = os + (size_t)MD_KC * ldo;
-            for (int k0 = 0; k0 < kn; k0 += 4) {
-                double bv[4];
-#pragma unroll
-                for (int c = 0; c < 4; c++) bv[c] = xs[(size_t)(8 * c + g) * ldx + k0 + t];
-#pragma unroll
-                for (int i = 0; i < MD_MT; i++) {
-                    const int rt = warp + 8 * i;
-                    if (rt < nrt) {
-                        const double av = os[(size_t)(k0 + t) * ldo + 8 * rt + g];
-#pragma unroll
-                        for (int c = 0; c < 4; c++)
-                            if ((cm >> c) & 1) dmma_8x8x4(acc[i][c][0], acc[i][c][1], av, bv[c]);
+            for (int k0 = 0; k0 < kp; k0 += kc) {
+                if (round && !warp_wait_all(smem_u32(&empty[slot]), (uint32_t)(round - 1) & 1u, M.wait_limit)) {
+                    if (lane == 0) {
+                        *abort_flag = 1;
+                        atomicOr(M.err, 1ull);
                     }
+                    break;
                 }
+                if (*abort_flag) break;
+                const int kn = min(kc, kp - k0), kq = min(kc, Q - k0) >> 1;  // columns; 16-byte pieces of a vector
+                const uint32_t ob = smem_u32(&obar[slot]), od = smem_u32(sm_md + slot * stage_d);
+                if (pl == 0) mbar_expect_tx(ob, (uint32_t)(__popc(sv >> 8) * kn * ldq) * 8u);
+                __syncwarp();
+                if (pl < cp && ((sv >> (8 + pl)) & 1))
+                    bulk_g2s(od + (uint32_t)(pl * oblk) * 8u,
+                             opl + (size_t)m2l_slot(dd, ta0 + pl, sb) * M.B.block + (size_t)k0 * ldq,
+                             (uint32_t)(kn * ldq) * 8u, ob);
+                issued++;
+                const uint32_t xd = od + (uint32_t)(cp * oblk + n0 * ldx) * 8u;
+                for (int q = q0; q < kq; q += LQ) {
+#pragma unroll
+                    for (int i = 0; i < MAXI; i++)
+                        if (je[i] != -2)  // -1: zeros
+                            cp_async16(xd + (uint32_t)(i * RPP * ldx + 2 * q) * 8u,
+                                       src0 + (je[i] >= 0 ? (4 * (int64_t)je[i] + sb) * Q + k0 + 2 * q : 0),
+                                       je[i] >= 0 ? 16 : 0);
+                }
+                cp_async_arrive(smem_u32(&bars[slot]));
+                if (++slot == nbuf) slot = 0, round++;
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&empty[bi]));  // this warp is done with the slot
+        }
+        // every copy issued lands before the block goes on (consumed stages have
+        // landed already; this matters after an abort)
+        cp_async_wait_all();
+        if (warp == MD_CWARPS)
+            for (int st = issued > nbuf ? issued - nbuf : 0; st < issued; st++)
+                mbar_wait(smem_u32(&obar[st % nbuf]), (uint32_t)(st / nbuf) & 1u, kDrainWaitPolls);
+    } else {
+        for (int pr = 0; pr < npair; pr++) {
+            const int sv = sst[pr], cm = scm[(sv >> 2) & 7];
+            const bool far = (sv >> (8 + ch)) & 1;
+            for (int k0 = 0; k0 < kp; k0 += kc) {
+                if (!warp_wait_both(smem_u32(&obar[slot]), smem_u32(&bars[slot]), (uint32_t)round & 1u, M.wait_limit)) {
+                    if (lane == 0) {
+                        *abort_flag = 1;
+                        atomicOr(M.err, 1ull);
+                    }
+                    break;
+                }
+                if (*abort_flag) break;
+                if (far) {
+                    const double *os = sm_md + slot * stage_d;
+                    m2l_masked<NR, NCT, (1 << NCT) - 1>(cm, acc, os + (size_t)ch * oblk + t * ldq + row0 + g, ldq,
+                                                        os + (size_t)cp * oblk + (size_t)g * ldx + t, ldx,
+                                                        min(kc, kp - k0));
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&empty[slot]));  // this warp is done with the slot
+                if (++slot == nbuf) slot = 0, round++;
+            }
         }
     }
     __syncthreads();
     if (*abort_flag) return;
     // D through shared memory (the stage buffers are free), then coalesced stores
-    double *cs = sm_md;  // [32 targets][Q4 + 1]
+    double *cs = sm_md;  // [TE targets][RB + 1]
+    if (warp < MD_CWARPS)
 #pragma unroll
-    for (int i = 0; i < MD_MT; i++) {
-        const int rt = warp + 8 * i;
-        if (warp < MD_THREADS / 32 && rt < nrt)
+        for (int i = 0; i < NR; i++)
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-                cs[(size_t)(8 * c + 2 * t) * (Q4 + 1) + 8 * rt + g] = acc[i][c][0];
-                cs[(size_t)(8 * c + 2 * t + 1) * (Q4 + 1) + 8 * rt + g] = acc[i][c][1];
+            for (int c = 0; c < NCT; c++) {
+                const int r = ch * qp + row0 + 8 * i + g;
+                cs[(size_t)(8 * c + 2 * t) * (RB + 1) + r] = acc[i][c][0];
+                cs[(size_t)(8 * c + 2 * t + 1) * (RB + 1) + r] = acc[i][c][1];
             }
-    }
     __syncthreads();
-    for (int n = warp; n < MD_TE; n += MD_BLOCK / 32) {
-        if (!sact[n]) continue;
-        double *dst = A.udown + ((size_t)A.T.off[l + 1] + 4 * (size_t)(sact[n] - 1)) * Q;
-        for (int r = lane; r < Q4; r += 32) dst[r] = cs[(size_t)n * (Q4 + 1) + r];
+    for (int n = warp; n < TE * cp; n += MD_BLOCK / 32) {
+        const int e = n / cp, c = n - e * cp;
+        if (!sact[e]) continue;
+        double *dst = A.udown + ((size_t)A.T.off[l + 1] + 4 * (size_t)(sact[e] - 1) + ta0 + c) * Q;
+        for (int r = lane; r < Q; r += 32) dst[r] = cs[(size_t)e * (RB + 1) + c * qp + r];
+    }
+}
+// Children per block and targets per tile.  Large trees: all four children (a
+// warp each) and 16 targets, three blocks to an SM (32 targets, two blocks to
+// an SM, measured 218 against 187 us at 1M points, 205 against 171 at 500k with
+// Nequiv 40: their last wave costs more than the operator reads saved); while
+// that makes fewer than two blocks per SM, 8 targets, then two children per
+// block (where their row tiles split evenly over two warps): a block's time
+// falls with its products.
+struct M2lShape {
+    int cp, nr, nct;
+};
+static int64_t m2l_tiles(const kifmm_plan *P, int lmin, int lmax, int te) {
+    int64_t t = 0;
+    for (int l = lmin; l <= lmax; l++) t += (P->lt.ne[l] + te - 1) / te;
+    return t;
+}
+static M2lShape m2l_shape(const kifmm_plan *P, const M2lBlocks &B, int lmin, int lmax) {
+    const int tpc = B.qp / 8;
+    M2lShape S{4, tpc, 2};
+    if (m2l_tiles(P, lmin, lmax, 16) < 2 * P->num_sms) S.nct = 1;
+    if (S.nct == 1 && tpc % 2 == 0 && m2l_tiles(P, lmin, lmax, 8) < 2 * P->num_sms) S.cp = 2, S.nr = tpc / 2;
+    return S;
+}
+template <int NR, int NCT>
+static void launch_m2l_dmma(kifmm_plan *P, M2lDmmaArgs &M) {
+    int64_t tiles = 0;
+    for (int l = 0; l <= MAX_LEVELS; l++) {
+        M.tile_off[l] = tiles;
+        if (l >= M.lmin && l <= M.lmax) tiles += m2l_tiles(P, l, l, 8 * NCT);
+    }
+    if (!tiles) return;
+    // A stage has about 24 columns, all of them where an SM gets one block (41 ->
+    // 27 us at 1k points: half as many stages), and the ring as many slots as
+    // leave room for the blocks that an SM gets, three at most.
+    const int64_t blocks = tiles * (4 / M.cp), per_sm = std::min<int64_t>(3, (blocks + P->num_sms - 1) / P->num_sms);
+    const int runs = per_sm == 1 ? 1 : (M.B.kp + 27) / 28;
+    M.kc = ((M.B.kp + runs - 1) / runs + 3) & ~3;
+    const size_t stage = m2l_stage_bytes(M.B, M.cp, 8 * NCT, M.kc);
+    M.nbuf = (int)std::max<int64_t>(2, std::min<int64_t>(MD_MAX_NBUF, (int64_t)(((224 << 10) / per_sm - 4096) / stage)));
+    const size_t smem = m2l_dmma_smem(M.B, M.cp, 8 * NCT, M.kc, M.nbuf);
+    ensure_dyn_smem(k_m2l_dmma<NR, NCT>, smem);
+    launch_pdl(k_m2l_dmma<NR, NCT>, dim3((unsigned)blocks), dim3(MD_BLOCK), smem, P->stream, M);
+}
+template <int NR>
+static void launch_m2l_dmma_nr(kifmm_plan *P, int nct, M2lDmmaArgs &M) {
+    if (nct == 2) launch_m2l_dmma<NR, 2>(P, M);
+    else launch_m2l_dmma<NR, 1>(P, M);
+}
+static void launch_m2l_dmma(kifmm_plan *P, const PassArgs &A, int lmin, int lmax) {
+    M2lDmmaArgs M{};
+    M.A = A;
+    M.blocks = P->ops_tmp.p;
+    M.B = m2l_blocks(P->Q);
+    M.lmin = lmin;
+    M.lmax = lmax;
+    M.wait_limit = plan_wait_polls(P);
+    M.err = P->scal.p + KIFMM_SCAL_PASS_ERR;
+    const M2lShape S = m2l_shape(P, M.B, lmin, lmax);
+    M.cp = S.cp;
+    switch (S.nr) {
+        case 1: return launch_m2l_dmma_nr<1>(P, S.nct, M);
+        case 2: return launch_m2l_dmma_nr<2>(P, S.nct, M);
+        case 3: return launch_m2l_dmma_nr<3>(P, S.nct, M);
+        case 4: return launch_m2l_dmma_nr<4>(P, S.nct, M);
+        case 5: return launch_m2l_dmma_nr<5>(P, S.nct, M);
+        case 6: return launch_m2l_dmma_nr<6>(P, S.nct, M);
+        case 7: return launch_m2l_dmma_nr<7>(P, S.nct, M);
+        default: return launch_m2l_dmma_nr<8>(P, S.nct, M);
     }
 }
 
@@ -978,31 +1123,11 @@ void run_upward_downward(kifmm_plan *P) {
         PhaseScope ph_m2m(P, KIFMM_PHASE_M2M);
         run_m2m_levels(P, A);
     }
-    if (Q % 2 == 0 && 4 * Q <= 8 * MD_MT * 8) {
+    if (m2l_uses_dmma(P)) {
         // FP64 tensor path: all levels' M2L in one launch, then the L2L chain
-        M2lDmmaArgs M{};
-        M.A = A;
-        if (!P->zero4q.p) {
-            P->zero4q.alloc((size_t)4 * Q);
-            KIFMM_CUDA(cudaMemsetAsync(P->zero4q.p, 0, (size_t)4 * Q * sizeof(double), s));
-        }
-        M.zero = P->zero4q.p;
-        M.lmin = 1;
-        M.lmax = L - 2;
-        M.wait_limit = plan_wait_polls(P);
-        M.err = P->scal.p + KIFMM_SCAL_PASS_ERR;
-        int64_t tiles = 0;
-        for (int l = 0; l <= MAX_LEVELS; l++) {
-            M.tile_off[l] = tiles;
-            if (l >= M.lmin && l <= M.lmax) tiles += (P->lt.ne[l] + MD_TE - 1) / MD_TE;
-        }
         {
             PhaseScope ph(P, KIFMM_PHASE_M2L);
-            if (tiles) {
-                const size_t smem = m2l_dmma_smem(4 * Q);
-                ensure_dyn_smem(k_m2l_dmma, smem);
-                launch_pdl(k_m2l_dmma, dim3((unsigned)tiles), dim3(MD_BLOCK), smem, s, M);
-            }
+            launch_m2l_dmma(P, A, 1, L - 2);
         }
         PhaseScope ph(P, KIFMM_PHASE_L2L);
         run_l2l_levels(P, A);

@@ -125,3 +125,28 @@ def test_one_leaf_complex(kind, k, n):
     ref, mag = direct_complex(kind, k, x, y, tau)
     pot = f.evaluate_to_points(x, y, True)
     assert np.all(np.abs(pot - ref) <= (n + 64) * EPS * mag)
+
+
+@pytest.mark.parametrize("nequiv", [4, 6, 8, 10, 12, 16, 18, 20, 24, 28, 30, 32])
+@pytest.mark.parametrize("n,cutoff", [(700, 20), (9000, 9), (60000, 9)])
+def test_fp64_m2l_shapes(n, cutoff, nequiv):
+    """Every number of row tiles, row and column padding, column runs and both
+    tile sizes of the FP64 M2L: the complex form works on states of 2 Nequiv, the
+    real one of Nequiv, and with a real kernel they are the same sums.  Their
+    check-to-equivalent inverses are eliminated differently, so the results
+    differ by rounding times the condition of E2C, about Nequiv / 2 (r2 /
+    r1)^(Nequiv / 2), over at most eight levels."""
+    import pykifmm2d_b200 as P
+    x, y, tau = cloud(n, 11)
+    kern = P.LaplaceKernel()
+    pots = []
+    for cplx in (False, True):
+        f = P.FMM(x, y, P.Get_Kernel_Functions(kern), P.prepare_numba_functions_on_the_fly(kern), nequiv, cutoff, cplx)
+        f.build_tree()
+        f.precompute()
+        f.build_expansions(tau + 0j if cplx else tau)
+        pots.append(f.evaluate_to_points(x, y, True))
+    r21 = (4 - np.sqrt(2) - 0.02) / (np.sqrt(2) + 0.01)
+    tol = 8 * EPS * nequiv / 2 * r21 ** (nequiv / 2)
+    assert np.abs(pots[1].imag).max() <= tol * np.abs(pots[0]).max()
+    assert np.abs(pots[1].real - pots[0]).max() <= tol * np.abs(pots[0]).max()
