@@ -875,135 +875,106 @@ __global__ void __launch_bounds__(LG_THREADS) k_lvl_gemm_b(PassArgs A, int l, in
     }
 }
 
-// The same products on the FP64 tensor path (mma.sync m8n8k4 .f64; the FP64
-// vector pipe sustains a quarter of its rate).  A block takes 32 entries.  It
-// stages by bulk asynchronous copies on one mbarrier: the operator [K][M] row
-// by row into a row stride ldo = 4 mod 16 doubles (conflict-free fragment
-// loads), the entries' columns X into rows of stride ldx, and for L2L the
-// children groups' current u_down (M = 4Q contiguous doubles per entry) into
-// C.  Warp w computes all M rows for entries 8w..8w+7 in chunks of 8*MT rows
-// (MT 8x8 accumulator tiles); results are written (M2M) or added (L2L) into C
-// in shared memory and leave by bulk stores, one row per entry.  Fragments:
+// The same products on the FP64 tensor path (mma.sync m8n8k4 .f64), Q = 4 KS.
+// A block takes 8 entries at a time; warps 2 c and 2 c + 1 take child c of
+// them, half of its row tiles (8 rows) each.  Every operand goes straight from
+// L2 into the fragments' registers: the warp's part of the operator before the
+// wait for the previous level's kernel, then, all loads in flight at once, the
+// entries' vectors (M2M: child c's; L2L: the entry's own, and the child's
+// current values as the accumulators' start).  M2M adds the children's four
+// products in shared memory; L2L stores its fragments.  Fragments:
 // A[row = lane/4][k = lane%4], B[k = lane%4][n = lane/4],
-// C[row = lane/4][n = 2*(lane%4) + {0,1}].  Needs M % 8 == 0, K % 4 == 0 and
-// 16-byte aligned operator rows.  A copy wait that runs out sets *err and the
-// block leaves without writing.
-constexpr int LM_THREADS = 128;
-static size_t lvl_mma_smem(int M, int K) {
-    return ((size_t)K * pad4mod16(M) + 32 * (size_t)pad4mod16(K) + 32 * (size_t)M) * sizeof(double);
-}
-
-template <int MODE, int MT>
-__global__ void __launch_bounds__(LM_THREADS) k_lvl_mma(PassArgs A, int l, int M, int K, long long wait_limit,
-                                                       unsigned long long *err) {
-    extern __shared__ __align__(128) double sm_m[];
-    __shared__ __align__(8) uint64_t bar;
-    __shared__ int snode[32];  // node of the entry (M2M), or of a split entry (L2L); -1 otherwise
-    const int ldo = pad4mod16(M), ldx = pad4mod16(K), Q = A.Q, tid = threadIdx.x;
-    double *opS = sm_m;                  // [K][ldo]
-    double *xS = opS + (size_t)K * ldo;  // [32][ldx]
-    double *cS = xS + (size_t)32 * ldx;  // [32][M]
-    const int64_t ne = A.T.ne[l], eoff = A.T.eoff[l], e0 = (int64_t)blockIdx.x * 32;
-    const int nt = (int)min((int64_t)32, ne - e0);
-    const double *op = A.ops + (size_t)l * A.stride + (MODE == 0 ? A.off_m2m : A.off_l2l);  // [K][M]
-    const size_t child0 = (size_t)A.T.off[l + 1] + 4 * (size_t)e0;  // first child of the block's first entry
-    int has = 0;
-    if (tid < 32) {
+// C[row = lane/4][n = 2*(lane%4) + {0,1}].
+//
+// A level holds 10 to 10,000 entries, and the levels depend on one another: what
+// counts is the time from the previous kernel's end to this one's, here one
+// L2 round trip, KS multiply-adds deep, and the stores.  With the operator and
+// the vectors staged in shared memory by one bulk copy per row (about 86
+// clocks each from one warp) and 32 entries to a warp, a level took 6.8 us
+// (M2M) and 8.3 us (L2L) whatever its size.  Values that the previous kernel
+// wrote are read past L1 (__ldcg).
+constexpr int LD_THREADS = 256, LD_TE = 8;
+template <int MODE, int KS>
+__global__ void __launch_bounds__(LD_THREADS) k_lvl_dmma(PassArgs A, int l) {
+    constexpr int Q = 4 * KS, NR = (Q + 7) / 8, NRW = (NR + 1) / 2;
+    __shared__ double red[MODE == 0 ? 2 : 1][MODE == 0 ? 4 : 1][MODE == 0 ? LD_TE : 1][MODE == 0 ? 8 * NR + 1 : 1];
+    __shared__ int snode[2][LD_TE];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int child = warp >> 1, rt0 = (warp & 1) * NRW;
+    const int64_t ne = A.T.ne[l], eoff = A.T.eoff[l], ntile = (ne + LD_TE - 1) / LD_TE;
+    const double *op = A.ops + (size_t)l * A.stride + (MODE == 0 ? A.off_m2m : A.off_l2l);
+    double a[NRW][KS];
+#pragma unroll
+    for (int i = 0; i < NRW; i++) {
+        const int r = 8 * (rt0 + i) + g;
+#pragma unroll
+        for (int k = 0; k < KS; k++) {
+            const int c = 4 * k + t;  // M2M: [4Q columns][Q rows]; L2L: [Q columns][4Q rows]
+            a[i][k] = r < Q ? (MODE == 0 ? op[(size_t)(child * Q + c) * Q + r] : op[(size_t)c * 4 * Q + child * Q + r]) : 0.0;
+        }
+    }
+    pdl_trigger();
+    int par = 0;
+    for (int64_t tile = blockIdx.x; tile < ntile; tile += gridDim.x, par ^= 1) {
+        const int64_t e0 = tile * LD_TE, en = e0 + g;
+        // nodes of the tile's entries (tree data); L2L passes the X-list cells over
         int node = -1;
-        if (tid < nt) {
-            const int64_t e = eoff + e0 + tid;
-            if (MODE == 0 || !(A.ent[e] & 1)) node = A.ent_node[e];
-        }
-        snode[tid] = node;
-        has = node >= 0;
-    }
-    const uint32_t mb = smem_u32(&bar);
-    if (tid == 0) mbar_init(mb);
-    const int nact = __syncthreads_count(has);
-    if (tid == 0) mbar_expect_tx(mb, (uint32_t)(K * M + nact * K + (MODE == 1 ? nact * M : 0)) * 8u);
-    __syncthreads();
-    // the operator does not depend on the previous level: copy it before waiting
-    for (int c = tid; c < K; c += LM_THREADS)
-        bulk_g2s(smem_u32(opS + (size_t)c * ldo), op + (size_t)c * M, (uint32_t)M * 8u, mb);
-    // launched with programmatic stream serialisation: let the next level's
-    // kernel be scheduled, then wait until the previous kernel has completed
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    for (int c = K + tid; c < K + 64; c += LM_THREADS) {
-        if (c < K + 32) {
-            const int n = c - K;
-            if (n < nt && snode[n] >= 0) {
-                const double *src = MODE == 0 ? A.uup + (child0 + 4 * (size_t)n) * Q : A.udown + (size_t)snode[n] * Q;
-                bulk_g2s(smem_u32(xS + (size_t)n * ldx), src, (uint32_t)K * 8u, mb);
-            }
-        } else if (MODE == 1) {
-            const int n = c - K - 32;
-            if (n < nt && snode[n] >= 0)
-                bulk_g2s(smem_u32(cS + (size_t)n * M), A.udown + (child0 + 4 * (size_t)n) * Q, (uint32_t)M * 8u, mb);
-        }
-    }
-    const bool ok = __syncthreads_and(mbar_wait(mb, 0, wait_limit));
-    if (!ok) {
-        if (tid == 0) atomicOr(err, 1ull);
-        mbar_wait(mb, 0, kDrainWaitPolls);  // let copies in flight land before the block leaves
-        return;
-    }
-    const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-    const int n0 = warp * 8;
-    if (n0 < nt) {
-        const double *xb = xS + (size_t)(n0 + g) * ldx + t;
-        for (int rc = 0; rc < M; rc += 8 * MT) {
-            double acc[MT][2];
+        if (en < ne && (MODE == 0 || !(A.ent[eoff + en] & 1))) node = A.ent_node[eoff + en];
+        if (warp == 0 && t == 0) snode[par][g] = node;
+        if (tile == blockIdx.x) pdl_wait();
+        if (MODE == 1) __syncthreads();
+        double acc[NRW][2], b[KS];
+        const double *src = MODE == 0 ? A.uup + (size_t)(A.T.off[l + 1] + 4 * en + child) * Q : A.udown + (size_t)node * Q;
 #pragma unroll
-            for (int i = 0; i < MT; i++) acc[i][0] = acc[i][1] = 0.0;
-            const double *ab = opS + (size_t)t * ldo + rc + g;
-#pragma unroll 2
-            for (int k0 = 0; k0 < K; k0 += 4) {
-                const double b = xb[k0];
+        for (int k = 0; k < KS; k++) b[k] = node >= 0 ? __ldcg(src + 4 * k + t) : 0.0;
 #pragma unroll
-                for (int i = 0; i < MT; i++)
-                    if (rc + 8 * i < M) dmma_8x8x4(acc[i][0], acc[i][1], ab[(size_t)k0 * ldo + 8 * i], b);
+        for (int i = 0; i < NRW; i++)
+#pragma unroll
+            for (int j = 0; j < 2; j++) {
+                const int r = 8 * (rt0 + i) + g, n = 2 * t + j;
+                acc[i][j] = 0.0;
+                if (MODE == 1 && r < Q && snode[par][n] >= 0)
+                    acc[i][j] = __ldcg(A.udown + (size_t)(A.T.off[l + 1] + 4 * (e0 + n) + child) * Q + r);
             }
 #pragma unroll
-            for (int i = 0; i < MT; i++) {
-                const int r = rc + 8 * i + g;
-                if (r >= M) continue;
+        for (int k = 0; k < KS; k++)
+#pragma unroll
+            for (int i = 0; i < NRW; i++) dmma_8x8x4(acc[i][0], acc[i][1], a[i][k], b[k]);
+        if (MODE == 0) {
+#pragma unroll
+            for (int i = 0; i < NRW; i++)
+                if (rt0 + i < NR) {
+                    red[par][child][2 * t][8 * (rt0 + i) + g] = acc[i][0];
+                    red[par][child][2 * t + 1][8 * (rt0 + i) + g] = acc[i][1];
+                }
+            __syncthreads();
+            for (int i = tid; i < LD_TE * Q; i += LD_THREADS) {
+                const int n = i / Q, r = i - n * Q, nd = snode[par][n];
+                if (nd >= 0)
+                    A.uup[(size_t)nd * Q + r] = (red[par][0][n][r] + red[par][1][n][r]) + (red[par][2][n][r] + red[par][3][n][r]);
+            }
+        } else {
+#pragma unroll
+            for (int i = 0; i < NRW; i++)
 #pragma unroll
                 for (int j = 0; j < 2; j++) {
-                    const int n = n0 + 2 * t + j;
-                    if (n >= nt || snode[n] < 0) continue;
-                    if (MODE == 0) cS[(size_t)n * M + r] = acc[i][j];
-                    else cS[(size_t)n * M + r] += acc[i][j];
+                    const int r = 8 * (rt0 + i) + g, n = 2 * t + j;
+                    if (r < Q && snode[par][n] >= 0)
+                        A.udown[(size_t)(A.T.off[l + 1] + 4 * (e0 + n) + child) * Q + r] = acc[i][j];
                 }
-            }
         }
     }
-    fence_proxy_async();
-    __syncthreads();
-    if (tid < nt && snode[tid] >= 0) {
-        double *dst = MODE == 0 ? A.uup + (size_t)snode[tid] * Q : A.udown + (child0 + 4 * (size_t)tid) * Q;
-        bulk_s2g(dst, smem_u32(cS + (size_t)tid * M), (uint32_t)M * 8u);
-        bulk_commit();
-        bulk_wait_read();
-    }
 }
-
-template <int MODE, int MT>
-static void launch_lvl_mma(kifmm_plan *P, const PassArgs &A, int l, int M, int K, size_t smem) {
-    ensure_dyn_smem(k_lvl_mma<MODE, MT>, smem);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)((P->lt.ne[l] + 31) / 32));
-    cfg.blockDim = dim3(LM_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = P->stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // overlap with the previous level's tail
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    KIFMM_CUDA(cudaLaunchKernelEx(&cfg, k_lvl_mma<MODE, MT>, A, l, M, K, plan_wait_polls(P),
-                                  P->scal.p + KIFMM_SCAL_PASS_ERR));
-    KIFMM_LAUNCHED();
+template <int MODE, int KS>
+static void launch_lvl_dmma(kifmm_plan *P, const PassArgs &A, int l) {
+    if (4 * KS == P->Q) {
+        // past four blocks per SM a block takes several tiles: the operator is read once
+        const int64_t tiles = (P->lt.ne[l] + LD_TE - 1) / LD_TE;
+        launch_pdl(k_lvl_dmma<MODE, KS>, dim3((unsigned)std::min<int64_t>(tiles, (int64_t)P->num_sms * 4)),
+                   dim3(LD_THREADS), 0, P->stream, A, l);
+    } else if constexpr (KS > 1) {
+        launch_lvl_dmma<MODE, KS - 1>(P, A, l);
+    }
 }
 
 // NT columns per block: (ceil(M/4)) x (NT/4) threads <= 256 and at most
@@ -1022,18 +993,7 @@ static void launch_lvl_gemm(kifmm_plan *P, const PassArgs &A, int l) {
     const int Q = P->Q;
     const int M = MODE == 0 ? Q : 4 * Q, K = MODE == 0 ? 4 * Q : Q;
     const int64_t ne = P->lt.ne[l];
-    if (M % 8 == 0 && K % 4 == 0 && A.stride % 2 == 0 && A.off_m2m % 2 == 0 && A.off_l2l % 2 == 0) {
-        // FP64 tensor path with bulk-copy staging (16-byte aligned rows)
-        const size_t smem = lvl_mma_smem(M, K);
-        if (smem <= (size_t)(220 << 10)) {
-            const int mt = M / 8;
-            if (mt <= 2) launch_lvl_mma<MODE, 2>(P, A, l, M, K, smem);
-            else if (mt <= 4) launch_lvl_mma<MODE, 4>(P, A, l, M, K, smem);
-            else if (mt <= 8) launch_lvl_mma<MODE, 8>(P, A, l, M, K, smem);
-            else launch_lvl_mma<MODE, 16>(P, A, l, M, K, smem);
-            return;
-        }
-    }
+    if (Q % 4 == 0) return launch_lvl_dmma<MODE, 16>(P, A, l);  // FP64 tensor path (Nequiv <= 64)
     {  // broadcast form when the operator and the entry tile fit in shared memory
         constexpr int RPT = MODE == 0 ? 8 : 16;
         const int RG = (M + RPT - 1) / RPT, Mp = RG * RPT;
