@@ -230,12 +230,20 @@ __global__ void k_ops_compose(OpsArgs A) {
     if (slot < 49) {
         const int ld = A.ldq;
         double *p = A.poff + ((size_t)l * 49 + slot) * (ld ? (size_t)A.kp * ld : (size_t)Q * Q);
-        for (int e = threadIdx.x; e < (ld ? A.kp * ld : Q * Q); e += blockDim.x) {
-            const int r = ld ? e % ld : e / Q, c = ld ? e / ld : e % Q;
+        double *pad = mm + Q * Q;  // the padded block, [kp][ldq] (smaller than 3 Q^2)
+        if (ld)
+            for (int e = threadIdx.x; e < A.kp * ld; e += blockDim.x) pad[e] = 0.0;
+        if (ld) __syncthreads();
+        for (int e = threadIdx.x; e < Q * Q; e += blockDim.x) {
+            int r = e / Q, c = e % Q;
             double s = 0;
-            if (r < Q && c < Q)
-                for (int t = 0; t < Q; t++) s = fma(mm[r * Q + t], iv[t * Q + c], s);
-            p[e] = s;
+            for (int t = 0; t < Q; t++) s = fma(mm[r * Q + t], iv[t * Q + c], s);
+            if (ld) pad[c * ld + r] = s;
+            else p[e] = s;
+        }
+        if (ld) {
+            __syncthreads();
+            for (int e = threadIdx.x; e < A.kp * ld; e += blockDim.x) p[e] = pad[e];
         }
     } else if (m2m) {
         double *o = b + off_m2m(Q);  // [4Q cols][Q rows]; this child's columns q Q .. q Q + Q - 1
