@@ -234,11 +234,12 @@ struct kifmm_plan {
 
     // workspaces
     kifmm::DBuf<double> tau, taus, pots, pot_out, tx, ty, tpot;
-    // separate targets (evaluate_to_points): Morton-sorted copies, their order, and
-    // the equivalent densities of the leaves' local expansions
-    kifmm::DBuf<uint64_t> tkey, tkey2;
-    kifmm::DBuf<int32_t> tperm, tperm2;
-    kifmm::DBuf<double> txs, tys, node_den;
+    // separate targets (evaluate_to_points, targets.cu): their leaf and rank,
+    // counters and work items, indices in group order, and the nodes' equivalent
+    // densities
+    kifmm::DBuf<int32_t> tleaf, tperm, titems;
+    kifmm::DBuf<unsigned> trank, tcount;
+    kifmm::DBuf<double> node_den;
     kifmm::DBuf<double> uup, udown;
     bool have_expansions = false;
     bool applied = false;  // an apply at the sources ran since the tree / operators were built
@@ -456,6 +457,18 @@ __host__ __device__ __forceinline__ uint64_t compact2(uint64_t v) {
 }
 __host__ __device__ __forceinline__ uint64_t morton(uint64_t ix, uint64_t iy) {
     return (spread2(ix) << 1) | spread2(iy);
+}
+
+// Exact grid cell: j = #{k in [1, 2^D-1] : v > m + k h}.  The gridlines are
+// the midpoints of every level (m + odd * W / 2^(l+1)), exact in FP64 for the
+// coordinate range checked on the host.
+__device__ __forceinline__ uint64_t grid_cell(double v, double m, double h) {
+    const int64_t top = (1ll << KEY_DEPTH) - 1;
+    double t = ceil((v - m) / h) - 1.0;
+    int64_t j = t < 0 ? 0 : (t > (double)top ? top : (int64_t)t);
+    for (int it = 0; it < 8 && j < top && v > m + (double)(j + 1) * h; it++) j++;
+    for (int it = 0; it < 8 && j > 0 && !(v > m + (double)j * h); it++) j--;
+    return (uint64_t)j;
 }
 
 // Source of the M2L from direction d of parent p: the entry (split or X-list

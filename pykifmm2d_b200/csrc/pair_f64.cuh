@@ -127,6 +127,18 @@ __device__ __forceinline__ PairValue h0_far(double t) {
     const double m = 0.5641895835477563 * rsqrt(x), cs = c + s, sc = s - c;  // 1 / sqrt(pi x)
     return {-0.25 * m * fma(p, sc, q * cs), -0.07957747154594767 * m * fma(p, cs, -q * sc)};
 }
+// ... past the series, where the loops evaluate it in line: K0 for 4 <= t <
+// 1e300, H0 for 4 <= t < 64 (h0_far's first form, with the table logarithm)
+template <int KIND>
+__device__ __forceinline__ PairValue pair_value_beyond(double t, const double2 *tl) {
+    if (KIND == KIFMM_KERNEL_MOD_HELMHOLTZ) return {k0_far(t), 0.0};
+    const double u = fma(t, 1.0 / 30.0, -34.0 / 30.0), a = series<H0_MID_A_D_N>(H0_MID_A_D, u);
+    return {fma(ln_tab<-2>(t, tl), a, series<H0_MID_R_D_N>(H0_MID_R_D, u)), a};
+}
+template <int KIND>
+__device__ __forceinline__ bool pair_beyond(double t) {
+    return t >= 4.0 && t < (KIND == KIFMM_KERNEL_MOD_HELMHOLTZ ? 1e300 : 64.0);
+}
 // ... of any other pair (coincident points, underflow, k r >= 2); kept out of
 // line, so that the pair loops stay small
 template <int KIND>

@@ -33,7 +33,8 @@ const double2 *log_table(int device) {
 // on the FP64 tensor path: one block per 32 consecutive leaves of one level
 // (leaf_list is level-major), warp w all Q rows for leaves 8w .. 8w + 7.  The
 // level's inverse is read once per block instead of once per leaf.
-// den[leaf_list index][Q].  Reads 4 Q^2 bytes per leaf-block from L2 and
+// den[leaf_list index][Q]; without a list the level's nodes are taken and den is
+// indexed by node.  Reads 4 Q^2 bytes per leaf-block from L2 and
 // 16 Q bytes per leaf: latency-bound (a few microseconds at 65k leaves).
 struct DenArgs {
     PassArgs A;
@@ -71,7 +72,7 @@ __global__ void __launch_bounds__(DEN_THREADS) k_leaf_density(DenArgs D) {
     pdl_trigger();
     for (int i = tid; i < 32 * Kp; i += DEN_THREADS) {
         const int n = i / Kp, c = i - n * Kp;
-        xS[n * ldx + c] = n < nt && c < Q ? A.udown[(size_t)D.list[w0 + n] * Q + c] : 0.0;
+        xS[n * ldx + c] = n < nt && c < Q ? A.udown[(size_t)(D.list ? D.list[w0 + n] : w0 + n) * Q + c] : 0.0;
     }
     __syncthreads();
     const int warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3, n0 = warp * 8;
@@ -96,20 +97,13 @@ __global__ void __launch_bounds__(DEN_THREADS) k_leaf_density(DenArgs D) {
     }
 }
 
-// the equivalent densities of the leaf list
-const double *launch_leaf_density(kifmm_plan *P, const PassArgs &A) {
-    DenArgs D{};
-    D.A = A;
-    D.list = P->leaf_list.p;
-    P->leaf_den.alloc((size_t)P->n_leaf_list * P->Q);
-    D.den = P->leaf_den.p;
+static const double *launch_density(kifmm_plan *P, DenArgs &D) {
     D.lmin = 2;
     D.lmax = P->L - 1;
     int64_t tiles = 0;
     for (int l = 0; l <= MAX_LEVELS; l++) {
-        D.loff[l] = P->leaf_loff[l];
         D.toff[l] = tiles;
-        if (l >= D.lmin && l <= D.lmax && l < MAX_LEVELS) tiles += (P->leaf_loff[l + 1] - P->leaf_loff[l] + 31) / 32;
+        if (l >= D.lmin && l <= D.lmax && l < MAX_LEVELS) tiles += (D.loff[l + 1] - D.loff[l] + 31) / 32;
     }
     if (tiles) {
         const size_t smem = den_smem(P->Q);
@@ -117,6 +111,25 @@ const double *launch_leaf_density(kifmm_plan *P, const PassArgs &A) {
         launch_pdl(k_leaf_density, dim3((unsigned)tiles), dim3(DEN_THREADS), smem, P->stream, D);
     }
     return D.den;
+}
+// the equivalent densities of the leaf list
+const double *launch_leaf_density(kifmm_plan *P, const PassArgs &A) {
+    DenArgs D{};
+    D.A = A;
+    D.list = P->leaf_list.p;
+    P->leaf_den.alloc((size_t)P->n_leaf_list * P->Q);
+    D.den = P->leaf_den.p;
+    for (int l = 0; l <= MAX_LEVELS; l++) D.loff[l] = P->leaf_loff[l];
+    return launch_density(P, D);
+}
+// ... of every node (targets may lie in leaves without points)
+const double *launch_node_density(kifmm_plan *P, const PassArgs &A) {
+    DenArgs D{};
+    D.A = A;
+    P->node_den.alloc((size_t)P->n_nodes * P->Q);
+    D.den = P->node_den.p;
+    for (int l = 0; l <= MAX_LEVELS; l++) D.loff[l] = l < P->L ? P->lt.off[l] : P->n_nodes;
+    return launch_density(P, D);
 }
 
 void launch_leaf_eval_d(kifmm_plan *P, const PassArgs &A, int check_self) {

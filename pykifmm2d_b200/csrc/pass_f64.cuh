@@ -9,8 +9,9 @@
 
 namespace kifmm {
 
-// equivalent densities of the leaf list (pass_f64.cu)
+// equivalent densities of the leaf list, of every node (pass_f64.cu)
 const double *launch_leaf_density(kifmm_plan *P, const PassArgs &A);
+const double *launch_node_density(kifmm_plan *P, const PassArgs &A);
 
 // L2P + P2P of the leaves, one warp per item: an item is up to ts (<= 32)
 // targets of one leaf.  The warp's targets form ng groups of TB targets; sp =
@@ -108,8 +109,10 @@ __device__ __forceinline__ bool pair_loop(const PairWarp<KIND, CPLX> &W, const d
     }
     return KIND == KIFMM_KERNEL_LAPLACE ? least < 0x00100000 : worst >= hi_end - 0x00100000u;
 }
-// ... where many pairs are past the series (leaves several 1/k wide): either
-// value per pair
+// ... where many pairs are past the series (leaves several 1/k wide): both
+// values for all of the lane's targets where any of them needs it, so that the
+// targets' chains overlap (a call per pair was bound by its latency: 2.5 times
+// its instructions)
 template <int KIND, bool CPLX, int NT, int TB>
 __device__ __forceinline__ void pair_loop_beyond(const PairWarp<KIND, CPLX> &W, const double2 *tl, int u, int sp,
                                                  int n, const double *tx, const double *ty, double k, double k2,
@@ -119,12 +122,38 @@ __device__ __forceinline__ void pair_loop_beyond(const PairWarp<KIND, CPLX> &W, 
         const double2 s = W.xy[u];
         const auto z = W.z[u];
         const double2 pz = W.pz[PairWarp<KIND, CPLX>::H0 ? u : 0];
+        double t[TB];
+        bool some_near = false, some_far = false, some_other = false;
 #pragma unroll
         for (int a = 0; a < TB; a++) {
             const double dx = tx[a] - s.x, dy = ty[a] - s.y;
-            const double r2 = fma(dx, dx, dy * dy), t = r2 * k2;
-            if (pair_ordinary(t, hi_end)) acc[a].add(pair_value<KIND, NT>(t, tl), z, pz);
-            else if (!(skip_equal && dx == 0.0 && dy == 0.0)) acc[a].add(pair_value_any<KIND>(r2, k), z, pz);
+            t[a] = fma(dx, dx, dy * dy) * k2;
+            const bool ok = pair_ordinary(t[a], hi_end), far = pair_beyond<KIND>(t[a]);
+            some_near = some_near || ok;
+            some_far = some_far || far;
+            some_other = some_other || !(ok || far);
+        }
+        if (some_near) {
+#pragma unroll
+            for (int a = 0; a < TB; a++) {
+                const PairValue v = pair_value<KIND, NT>(t[a], tl);
+                if (pair_ordinary(t[a], hi_end)) acc[a].add(v, z, pz);
+            }
+        }
+        if (some_far) {
+#pragma unroll
+            for (int a = 0; a < TB; a++) {
+                const PairValue v = pair_value_beyond<KIND>(t[a], tl);
+                if (pair_beyond<KIND>(t[a])) acc[a].add(v, z, pz);
+            }
+        }
+        if (some_other) {
+#pragma unroll
+            for (int a = 0; a < TB; a++) {
+                const double dx = tx[a] - s.x, dy = ty[a] - s.y;
+                if (!pair_ordinary(t[a], hi_end) && !pair_beyond<KIND>(t[a]) && !(skip_equal && dx == 0.0 && dy == 0.0))
+                    acc[a].add(pair_value_any<KIND>(fma(dx, dx, dy * dy), k), z, pz);
+            }
         }
     }
 }
@@ -160,8 +189,10 @@ __device__ __forceinline__ auto load_value(const double *v, int i) {
     else return v[i];
 }
 
-// The targets and the item of one leaf
+// Up to 32 targets of one leaf
 struct LeafItem {
+    const double *tx, *ty;  // target coordinates, at idx[t0 .. t0 + nt) or, without idx, at t0 ..
+    const int32_t *idx;
     int t0, nt, n_own, ns, l, lane;
     double cx, cy;
     const double *den;
@@ -180,9 +211,10 @@ __device__ __forceinline__ PairSum<KIND, CPLX> leaf_item(const PassArgs &A, Pair
     PairSum<KIND, CPLX> acc[TB];
 #pragma unroll
     for (int a = 0; a < TB; a++) {
-        const int i = gi + a * ng < nt ? gi + a * ng : gi;  // unused slots repeat the first
-        tx[a] = A.xs[I.t0 + i];
-        ty[a] = A.ys[I.t0 + i];
+        int i = I.t0 + (gi + a * ng < nt ? gi + a * ng : gi);  // unused slots repeat the first
+        if (I.idx) i = I.idx[i];
+        tx[a] = I.tx[i];
+        ty[a] = I.ty[i];
 #pragma unroll
         for (int c = 0; c < NC; c++) acc[a].c[c] = 0.0;
     }
@@ -242,10 +274,24 @@ __device__ __forceinline__ PairSum<KIND, CPLX> leaf_item_tb(const PassArgs &A, P
                                                             const double2 *tl, const LeafItem &I, unsigned hi_end) {
     // the number of targets per lane that leaves the fewest lanes idle: pair
     // slots per source TB / (32 / ceil(nt / TB)), compared by cross products
-    const int s2 = 32 / ((I.nt + 1) >> 1), s3 = 32 / ((I.nt + 2) / 3), s4 = 32 / ((I.nt + 3) >> 2);
-    if (s4 * 3 >= s3 * 4 && s4 * 2 >= s2 * 4) return leaf_item<KIND, CPLX, FAR, NT, BEYOND, 4>(A, W, tl, I, hi_end);
-    if (s3 * 2 >= s2 * 3) return leaf_item<KIND, CPLX, FAR, NT, BEYOND, 3>(A, W, tl, I, hi_end);
-    return leaf_item<KIND, CPLX, FAR, NT, BEYOND, 2>(A, W, tl, I, hi_end);
+    if constexpr (BEYOND) return leaf_item<KIND, CPLX, FAR, NT, true, 2>(A, W, tl, I, hi_end);  // (a larger body)
+    else {
+        const int s2 = 32 / ((I.nt + 1) >> 1), s3 = 32 / ((I.nt + 2) / 3), s4 = 32 / ((I.nt + 3) >> 2);
+        if (s4 * 3 >= s3 * 4 && s4 * 2 >= s2 * 4) return leaf_item<KIND, CPLX, FAR, NT, BEYOND, 4>(A, W, tl, I, hi_end);
+        if (s3 * 2 >= s2 * 3) return leaf_item<KIND, CPLX, FAR, NT, BEYOND, 3>(A, W, tl, I, hi_end);
+        return leaf_item<KIND, CPLX, FAR, NT, BEYOND, 2>(A, W, tl, I, hi_end);
+    }
+}
+
+// ... with the series that reaches to tmax, the largest (k r)^2 inside the boxes
+template <int KIND, bool CPLX, bool FAR>
+__device__ __forceinline__ PairSum<KIND, CPLX> leaf_item_series(const PassArgs &A, PairWarp<KIND, CPLX> &W,
+                                                                const double2 *tl, const LeafItem &I, double tmax) {
+    if (KIND == KIFMM_KERNEL_LAPLACE) return leaf_item_tb<KIND, CPLX, FAR, 1>(A, W, tl, I, LOG_HI_END);
+    if (tmax < 0.0625) return leaf_item_tb<KIND, CPLX, FAR, SERIES_NARROW>(A, W, tl, I, SERIES_NARROW_HI);
+    if (tmax < 1.0) return leaf_item_tb<KIND, CPLX, FAR, SERIES_MID>(A, W, tl, I, SERIES_MID_HI);
+    if (tmax < 4.0) return leaf_item_tb<KIND, CPLX, FAR, SERIES_WIDE>(A, W, tl, I, SERIES_WIDE_HI);
+    return leaf_item_tb<KIND, CPLX, FAR, SERIES_WIDE, true>(A, W, tl, I, SERIES_WIDE_HI);
 }
 
 // 16 warps per SM at 128 registers measured 1-5% faster than 24 at 80 (the K0
@@ -266,6 +312,9 @@ __global__ void __launch_bounds__(32 * L64_MAX_WARPS, L64_BLOCKS_PER_SM)
     const int lane = threadIdx.x & 31;
     const double2 *tl = tab + (lane & (LOGTAB_COPIES - 1));
     LeafItem I;
+    I.tx = A.xs;
+    I.ty = A.ys;
+    I.idx = nullptr;
     I.lane = lane;
     I.check_self = check_self;
     I.k2 = A.k * A.k;
@@ -297,13 +346,7 @@ __global__ void __launch_bounds__(32 * L64_MAX_WARPS, L64_BLOCKS_PER_SM)
         for (int t0 = b + (int)(it - w * ntile) * ts; t0 < e; t0 += ntile * ts) {
             I.t0 = t0;
             I.nt = min(ts, e - t0);
-            PairSum<KIND, CPLX> v;
-            if (KIND == KIFMM_KERNEL_LAPLACE) v = leaf_item_tb<KIND, CPLX, FAR, 1>(A, W, tl, I, LOG_HI_END);
-            else if (tmax < 0.0625)
-                v = leaf_item_tb<KIND, CPLX, FAR, SERIES_NARROW>(A, W, tl, I, SERIES_NARROW_HI);
-            else if (tmax < 1.0) v = leaf_item_tb<KIND, CPLX, FAR, SERIES_MID>(A, W, tl, I, SERIES_MID_HI);
-            else if (tmax < 4.0) v = leaf_item_tb<KIND, CPLX, FAR, SERIES_WIDE>(A, W, tl, I, SERIES_WIDE_HI);
-            else v = leaf_item_tb<KIND, CPLX, FAR, SERIES_WIDE, true>(A, W, tl, I, SERIES_WIDE_HI);
+            const PairSum<KIND, CPLX> v = leaf_item_series<KIND, CPLX, FAR>(A, W, tl, I, tmax);
             if (lane >= I.nt) continue;
             if constexpr (CPLX) ((double2 *)A.pots)[t0 + lane] = make_double2(v.c[0], v.c[1]);
             else A.pots[t0 + lane] = FAR ? A.pots[t0 + lane] + v.c[0] : v.c[0];

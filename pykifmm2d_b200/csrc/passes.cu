@@ -444,48 +444,6 @@ static void launch_m2l_dmma(kifmm_plan *P, const PassArgs &A, int lmin, int lmax
     }
 }
 
-// Evaluation at arbitrary targets: locate by strict '>' descent
-// (numba_locate_points, tree.py:712-727), then L2P and P2P.
-// Targets in Morton order (sort_targets) with the leaves' equivalent densities
-// precomputed (k_leaf_den); out[order[i]] is target i's potential.
-__global__ void k_eval_targets_d(PassArgs A, const double *__restrict__ tx, const double *__restrict__ ty, int64_t n,
-                                 int check_self, const int32_t *__restrict__ order, const double *__restrict__ den,
-                                 double *__restrict__ pot) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double px = tx[i], py = ty[i];
-        int g = 0, l = 0;
-        while (A.nflag[g] & NF_SPLIT) {
-            double cx, cy;
-            node_center(A, g, l, cx, cy);
-            g = A.nchild[g] + 2 * (px > cx) + (py > cy);
-            l++;
-        }
-        double cx, cy;
-        node_center(A, g, l, cx, cy);
-        double acc = 0.0;
-        if (l >= 2) {
-            const double *blk = A.ops + (size_t)l * A.stride;
-            const double *lg = blk + A.off_large;
-            double rx = px - cx, ry = py - cy;
-            const double *dg = den + (size_t)g * A.Q;
-            for (int q = 0; q < A.Q; q++) {
-                double dx = rx - lg[q], dy = ry - lg[A.Q + q];
-                acc += green_d(A.kind, A.k, dx * dx + dy * dy) * dg[q];
-            }
-        }
-        for (int d = 0; d < 9; d++) {
-            int c = A.ncoll[9 * (size_t)g + d];
-            if (c < 0) continue;
-            for (int s = A.nbot[c]; s < A.ntop[c]; s++) {
-                double dx = px - A.xs[s], dy = py - A.ys[s];
-                if (check_self && dx == 0.0 && dy == 0.0) continue;
-                acc += green_d(A.kind, A.k, dx * dx + dy * dy) * A.taus[s];
-            }
-        }
-        pot[order[i]] = acc;
-    }
-}
-
 PassArgs make_pass_args(kifmm_plan *P) {
     PassArgs A{};
     A.T = P->lt;
@@ -644,18 +602,6 @@ void build_m2l_order(kifmm_plan *P) {
                P->lt, P->m2l_hist.p);
     launch_pdl(k_m2l_place, dim3(gr), dim3(256), 0, P->stream, (const uint64_t *)P->ent.p,
                (const uint16_t *)P->m2l_key.p, n, P->m2l_hist.p, P->m2l_perm.p);
-    KIFMM_LAUNCHED();
-}
-
-void sort_targets(kifmm_plan *P, const double *tx, const double *ty, int64_t n);  // tree.cu
-void launch_leaf_den(kifmm_plan *P, const PassArgs &A);                          // passes_mixed.cu
-
-void launch_eval_targets_d(kifmm_plan *P, const PassArgs &A, const double *tx, const double *ty, int64_t n,
-                           int check_self, double *pot) {
-    sort_targets(P, tx, ty, n);
-    launch_leaf_den(P, A);
-    k_eval_targets_d<<<grid_for(n, 128, P->num_sms * 16), 128, 0, P->stream>>>(
-        A, P->txs.p, P->tys.p, n, check_self, P->tperm.p, P->node_den.p, pot);
     KIFMM_LAUNCHED();
 }
 
@@ -1134,19 +1080,6 @@ void run_eval_sources(kifmm_plan *P, int check_self) {
         }
     }
     launch_scatter_pot(P);
-}
-
-void run_eval_targets(kifmm_plan *P, const double *tx, const double *ty, int64_t n, int check_self, double *pot) {
-    PassArgs A = make_pass_args(P);
-    if (P->cplx) {
-        run_eval_targets_c(P, A, tx, ty, n, check_self, pot);
-        return;
-    }
-    if (P->opt.precision == KIFMM_PREC_MIXED) {
-        run_eval_targets_mixed(P, tx, ty, n, check_self, pot);
-        return;
-    }
-    launch_eval_targets_d(P, A, tx, ty, n, check_self, pot);
 }
 
 // ------------------------------------------------ kernel-function utilities

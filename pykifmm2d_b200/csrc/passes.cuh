@@ -95,12 +95,8 @@ void launch_planned_leaf(kifmm_plan *P, const PassArgs &A);
 // passes_complex.cu (complex values: FP64 point passes on double2 densities)
 void launch_gather_tau_c(kifmm_plan *P);
 void run_eval_sources_c(kifmm_plan *P, const PassArgs &A, int check_self);
-void run_eval_targets_c(kifmm_plan *P, const PassArgs &A, const double *tx, const double *ty, int64_t n,
-                        int check_self, double *pot);
 // passes_mixed.cu
 void run_passes_mixed(kifmm_plan *P);
 void run_eval_sources_mixed(kifmm_plan *P, int check_self);
-void run_eval_targets_mixed(kifmm_plan *P, const double *tx, const double *ty, int64_t n, int check_self,
-                            double *pot);
 
 }  // namespace kifmm

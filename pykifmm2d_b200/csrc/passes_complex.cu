@@ -5,11 +5,9 @@
 // state is the real image of its complex check potential: Q = 2 Qc doubles,
 // [Re u (Qc), Im u (Qc)], and every translation operator is the real image of
 // the complex one (operators.cu), so M2M, M2L and L2L are the real FP64
-// kernels unchanged.  P2M and the L2P + P2P at the sources are in pass_f64.cu;
-// here:
-//   L2P + P2P  numba_target_local_expansion_evaluation / neighbor_evaluation
-//        (class_fmm.py:73-111) at separate targets;
-//   KF / KA / KAS (class_fmm.py:115-145) for a complex kernel.
+// kernels unchanged.  P2M, L2P and P2P are in pass_f64.cuh and targets.cu; here
+// are the density and potential permutations and KF / KA / KAS
+// (class_fmm.py:115-145) for a complex kernel.
 // Densities and potentials are double2 (re, im) in HBM.
 #include "passes.cuh"
 
@@ -37,50 +35,6 @@ __global__ void k_scatter_pot_c(const double2 *__restrict__ pots, const int32_t 
     pdl_wait();
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         pot[perm[i]] = pots[i];
-}
-
-// separate targets: locate by strict '>' descent (tree.py:712-727), L2P, P2P
-__global__ void k_eval_targets_c(PassArgs A, const double *__restrict__ tx, const double *__restrict__ ty, int64_t n,
-                                 int check_self, const double2 *__restrict__ taus, double2 *__restrict__ pot) {
-    const int Q = A.Q, Qc = A.Qc;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double px = tx[i], py = ty[i];
-        int g = 0, l = 0;
-        while (A.nflag[g] & NF_SPLIT) {
-            double cx, cy;
-            node_center(A, g, l, cx, cy);
-            g = A.nchild[g] + 2 * (px > cx) + (py > cy);
-            l++;
-        }
-        double cx, cy;
-        node_center(A, g, l, cx, cy);
-        double2 acc = make_double2(0.0, 0.0);
-        if (l >= 2) {
-            const double *blk = A.ops + (size_t)l * A.stride;
-            const double *inv = blk + A.off_inv, *lg = blk + A.off_large;
-            const double *u = A.udown + (size_t)g * Q;
-            const double rx = px - cx, ry = py - cy;
-            for (int q = 0; q < Qc; q++) {
-                double pr = 0.0, pi = 0.0;
-                for (int c = 0; c < Q; c++) {
-                    pr = fma(inv[q * Q + c], u[c], pr);
-                    pi = fma(inv[(Qc + q) * Q + c], u[c], pi);
-                }
-                const double dx = rx - lg[q], dy = ry - lg[Qc + q];
-                cacc(acc, green_z(A.kind, A.k, dx * dx + dy * dy), make_double2(pr, pi));
-            }
-        }
-        for (int d = 0; d < 9; d++) {
-            const int c = A.ncoll[9 * (size_t)g + d];
-            if (c < 0) continue;
-            for (int s = A.nbot[c]; s < A.ntop[c]; s++) {
-                const double dx = px - A.xs[s], dy = py - A.ys[s];
-                if (check_self && dx == 0.0 && dy == 0.0) continue;
-                cacc(acc, green_z(A.kind, A.k, dx * dx + dy * dy), taus[s]);
-            }
-        }
-        pot[i] = acc;
-    }
 }
 
 // ------------------------------------------------ kernel-function utilities
@@ -152,13 +106,6 @@ void run_eval_sources_c(kifmm_plan *P, const PassArgs &A, int check_self) {
     }
     launch_pdl(k_scatter_pot_c, dim3(grid_for(P->N, 256, P->num_sms * 8)), dim3(256), 0, P->stream,
                (const double2 *)P->pots.p, (const int32_t *)P->perm.p, P->N, (double2 *)P->pot_out.p);
-}
-
-void run_eval_targets_c(kifmm_plan *P, const PassArgs &A, const double *tx, const double *ty, int64_t n,
-                        int check_self, double *pot) {
-    k_eval_targets_c<<<grid_for(n, 128, P->num_sms * 16), 128, 0, P->stream>>>(
-        A, tx, ty, n, check_self, (const double2 *)P->taus.p, (double2 *)pot);
-    KIFMM_LAUNCHED();
 }
 
 void direct_sum_device_c(const kifmm_kernel &kn, const double *x, const double *y, const double *tau, int64_t n,

@@ -15,6 +15,7 @@
 //     accumulation; or FP32 tiles on the CUDA cores (this file);
 //   * the local expansion's equivalent density Inv_l u_down formed in FP64.
 // Coincident source/target pairs contribute zero, as in the reference.
+#include "leaf_f32.cuh"
 #include "passes.cuh"
 
 namespace kifmm {
@@ -238,11 +239,6 @@ constexpr int LEAF_BLOCKS_PER_SM = KIFMM_LEAF_BLOCKS_PER_SM;  // resident blocks
 constexpr int LEAF_CHUNK = KIFMM_LEAF_CHUNK;                  // sources staged per pass
 static_assert(LEAF_CHUNK + 31 <= 200, "the leaf kernel's quotients (small_div) need cn + sp - 1 <= 200");
 
-__device__ __forceinline__ float lg2_ftz(float x) {
-    float y;
-    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
 __device__ __forceinline__ float pair_r2(float tx, float ty, const float4 &sv) {
     const float dx = tx - sv.x, dy = ty - sv.y;
     return fmaf(dx, dx, dy * dy);
@@ -256,47 +252,12 @@ __device__ __forceinline__ float pair_lg2_floor(float tx, float ty, const float4
     return lg2_ftz(fmaf(dx, dx, fmaf(dy, dy, 1.17549435e-38f)));
 }
 
-// Packed FP32 pairs (sm_100 .f32x2 arithmetic): one 64-bit register holds a
-// value for each of a lane's two targets.  Sources are staged with their
-// coordinates and charge duplicated, (x, x | y, y) and (z, z), so one
-// instruction forms both targets' offsets, squared distances and products:
-// the same IEEE operations as the scalar form, issued half as often.
-typedef unsigned long long f32x2;
 constexpr f32x2 F2_FLOOR = 0x0080000000800000ull;  // (FLT_MIN, FLT_MIN)
-__device__ __forceinline__ f32x2 f2_pack(float a, float b) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void f2_unpack(f32x2 v, float &a, float &b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ f32x2 f2_sub(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f32x2 f2_add(f32x2 a, f32x2 b) {
-    f32x2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f32x2 f2_fma(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
 // r^2 + FLT_MIN of both targets to one source (as pair_lg2_floor)
 __device__ __forceinline__ f32x2 pair2_r2_floor(f32x2 tx, f32x2 ty, const ulonglong2 &s) {
     const f32x2 dx = f2_sub(tx, s.x), dy = f2_sub(ty, s.y);
     return f2_fma(dx, dx, f2_fma(dy, dy, F2_FLOOR));
 }
-__device__ __forceinline__ f32x2 lg2_pair(f32x2 r) {
-    float a, b;
-    f2_unpack(r, a, b);
-    return f2_pack(lg2_ftz(a), lg2_ftz(b));
-}
-
 // Laplace pair sums of one lane holding two targets (tx, ty packed): over its
 // sources at list positions j + k SP, k in [k0, k1), of z log2(r^2 + FLT_MIN),
 // in FP32 blocks of at most 32 sources (two chains per target, alternating
@@ -766,82 +727,8 @@ __global__ void __launch_bounds__(32 * LEAF_WARPS, LEAF_BLOCKS_PER_SM)
     if (w < off[nplan]) leaf_eval_f_leaf<KIND>(args[lo], w - off[lo]);
 }
 
-// Separate targets (class_fmm.py:379-399 with targets other than the
-// sources), one thread per target in Morton order (sort_targets): descent to
-// the target's leaf, L2P from the leaf's equivalent density (k_leaf_den, in
-// FP64), P2P over the leaf's colleagues in FP32 (pairs at distance 0 skipped),
-// result written to the target's own position.  Neighbouring lanes mostly
-// share a leaf, so node tables and near sources are read once per warp.
-__global__ void k_leaf_den(PassArgs A, int64_t nn, double *__restrict__ den) {
-    const int lane = threadIdx.x & 31;
-    const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5, ws = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const int Q = A.Q;
-    for (int64_t g = w0; g < nn; g += ws) {
-        const int l = A.nlev[g];
-        if ((A.nflag[g] & NF_SPLIT) || l < 2) continue;
-        const double *inv = A.ops + (size_t)l * A.stride + A.off_inv;
-        const double *u = A.udown + (size_t)g * Q;
-        for (int q = lane; q < Q; q += 32) {
-            double s = 0.0;
-            for (int c = 0; c < Q; c++) s = fma(inv[q * Q + c], u[c], s);
-            den[(size_t)g * Q + q] = s;
-        }
-    }
-}
-
-template <int KIND>
-__global__ void k_eval_targets_s(PassArgs A, const double *__restrict__ tx, const double *__restrict__ ty,
-                                 const int32_t *__restrict__ order, int64_t n, const double *__restrict__ den,
-                                 double *__restrict__ pot) {
-    const float kk = (float)A.k;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double px = tx[i], py = ty[i];
-        int g = 0, l = 0;
-        while (A.nflag[g] & NF_SPLIT) {
-            double cx, cy;
-            node_center(A, g, l, cx, cy);
-            g = A.nchild[g] + 2 * (px > cx) + (py > cy);
-            l++;
-        }
-        double cx, cy;
-        node_center(A, g, l, cx, cy);
-        const float rx = (float)(px - cx), ry = (float)(py - cy);
-        double far = 0.0;  // L2P in FP64
-        if (l >= 2) {
-            const double *lgd = A.ops + (size_t)l * A.stride + A.off_large;
-            const double *dg = den + (size_t)g * A.Q;
-            for (int q = 0; q < A.Q; q++) {
-                const double dx = (px - cx) - lgd[q], dy = (py - cy) - lgd[A.Q + q];
-                far = fma(green_d(A.kind, A.k, dx * dx + dy * dy), dg[q], far);
-            }
-        }
-        float acc = 0.f;
-        for (int d = 0; d < 9; d++) {
-            const int c = A.ncoll[9 * (size_t)g + d];
-            if (c < 0) continue;
-            for (int s = A.nbot[c]; s < A.ntop[c]; s++) {
-                const float dx = rx - (float)(A.xs[s] - cx), dy = ry - (float)(A.ys[s] - cy);
-                const float r2 = fmaf(dx, dx, dy * dy);
-                if (r2 > 0.f) acc = fmaf((float)A.taus[s], gsum_term<KIND>(r2, kk), acc);
-            }
-        }
-        pot[order[i]] = (double)(acc * gsum_scale<KIND>()) + far;
-    }
-}
-
-void sort_targets(kifmm_plan *P, const double *tx, const double *ty, int64_t n);  // tree.cu
-
-void launch_leaf_den(kifmm_plan *P, const PassArgs &A) {
-    const int64_t nn = P->n_nodes;
-    P->node_den.alloc((size_t)nn * P->Q);
-    k_leaf_den<<<grid_for(nn * 32, 256, P->num_sms * 16), 256, 0, P->stream>>>(A, nn, P->node_den.p);
-    KIFMM_LAUNCHED();
-}
-
 // m2l_tc.cu / passes.cu
 void run_m2l_tensor(kifmm_plan *P, const PassArgs &A);
-void launch_eval_targets_d(kifmm_plan *P, const PassArgs &A, const double *tx, const double *ty, int64_t n,
-                           int check_self, double *pot);
 void launch_m2m_d(kifmm_plan *P, const PassArgs &A, int l);
 void launch_l2l_d(kifmm_plan *P, const PassArgs &A, int l);
 void run_m2m_levels(kifmm_plan *P, const PassArgs &A);
@@ -1071,25 +958,6 @@ void launch_leaf_f_batch(int kind, const PassArgs *dargs, const int64_t *doff, i
     else
         k_leaf_eval_f_batch<KIFMM_KERNEL_MOD_HELMHOLTZ><<<(unsigned)blocks, 32 * LEAF_WARPS, 0, s>>>(dargs, doff,
                                                                                                       nplan);
-    KIFMM_LAUNCHED();
-}
-
-void run_eval_targets_mixed(kifmm_plan *P, const double *tx, const double *ty, int64_t n, int check_self,
-                            double *pot) {
-    PassArgs A = make_pass_args(P);
-    if (P->opt.near_fp64) {
-        launch_eval_targets_d(P, A, tx, ty, n, check_self, pot);
-        return;
-    }
-    sort_targets(P, tx, ty, n);
-    launch_leaf_den(P, A);
-    const unsigned gr = grid_for(n, 128, P->num_sms * 16);
-    if (P->kern.kind == KIFMM_KERNEL_LAPLACE)
-        k_eval_targets_s<KIFMM_KERNEL_LAPLACE><<<gr, 128, 0, P->stream>>>(A, P->txs.p, P->tys.p, P->tperm.p, n,
-                                                                          P->node_den.p, pot);
-    else
-        k_eval_targets_s<KIFMM_KERNEL_MOD_HELMHOLTZ><<<gr, 128, 0, P->stream>>>(A, P->txs.p, P->tys.p, P->tperm.p,
-                                                                                n, P->node_den.p, pot);
     KIFMM_LAUNCHED();
 }
 

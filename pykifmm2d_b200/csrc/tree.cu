@@ -99,18 +99,6 @@ __global__ void k_bbox(const double *__restrict__ x, const double *__restrict__ 
     }
 }
 
-// Exact grid cell: j = #{k in [1, 2^D-1] : v > m + k h}.  The gridlines are
-// the midpoints of every level (m + odd * W / 2^(l+1)), exact in FP64 for the
-// coordinate range checked on the host.
-__device__ __forceinline__ uint64_t grid_cell(double v, double m, double h) {
-    const int64_t top = (1ll << KEY_DEPTH) - 1;
-    double t = ceil((v - m) / h) - 1.0;
-    int64_t j = t < 0 ? 0 : (t > (double)top ? top : (int64_t)t);
-    for (int it = 0; it < 8 && j < top && v > m + (double)(j + 1) * h; it++) j++;
-    for (int it = 0; it < 8 && j > 0 && !(v > m + (double)j * h); it++) j--;
-    return (uint64_t)j;
-}
-
 __global__ void k_keys(const double *__restrict__ x, const double *__restrict__ y, int64_t n, double m, double M,
                        double h, uint64_t *__restrict__ key, int32_t *__restrict__ perm, unsigned long long *outside) {
     unsigned long long out = 0;
@@ -125,35 +113,6 @@ __global__ void k_keys(const double *__restrict__ x, const double *__restrict__ 
     if (!outside) return;
     for (int o = 16; o; o >>= 1) out += __shfl_xor_sync(0xffffffffu, out, o);
     if ((threadIdx.x & 31) == 0 && out) atomicAdd(outside, out);
-}
-
-// Separate targets in the Morton order of the plan's root box, so that the
-// targets of one warp mostly share a leaf (its node tables and near sources
-// are then read once per warp, not once per lane): keys of the coordinates
-// clamped into the box, a sort by the top 32 key bits (16 levels), and the
-// coordinates gathered in that order.  Non-finite coordinates get key 0.
-__global__ void k_target_keys(const double *__restrict__ x, const double *__restrict__ y, int64_t n, double m,
-                              double h, uint64_t *__restrict__ key, int32_t *__restrict__ perm) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double a = x[i], b = y[i];
-        key[i] = (h > 0 && isfinite(a) && isfinite(b)) ? morton(grid_cell(a, m, h), grid_cell(b, m, h)) : 0;
-        perm[i] = (int32_t)i;
-    }
-}
-
-__global__ void k_gather2(const double *__restrict__ x, const double *__restrict__ y, const int32_t *__restrict__ perm,
-                          int64_t n, double *__restrict__ xs, double *__restrict__ ys);
-
-void sort_targets(kifmm_plan *P, const double *tx, const double *ty, int64_t n) {
-    KIFMM_REQUIRE(n < (1ll << 31), KIFMM_ERR_ARG, "evaluate_to_points: more than 2^31 - 1 targets");
-    P->tkey.alloc(n); P->tkey2.alloc(n); P->tperm.alloc(n); P->tperm2.alloc(n);
-    P->txs.alloc(n); P->tys.alloc(n);
-    cudaStream_t s = P->stream;
-    const unsigned gs = grid_for(n, 256, P->num_sms * 8);
-    k_target_keys<<<gs, 256, 0, s>>>(tx, ty, n, P->root_min, std::ldexp(P->W, -KEY_DEPTH), P->tkey.p, P->tperm.p);
-    KIFMM_LAUNCHED();
-    radix_sort_pairs_bits(P->tkey.p, P->tperm.p, P->tkey2.p, P->tperm2.p, n, 2 * KEY_DEPTH - 32, 32, P);
-    launch_pdl(k_gather2, dim3(gs), dim3(256), 0, s, tx, ty, (const int32_t *)P->tperm.p, n, P->txs.p, P->tys.p);
 }
 
 // k_keys with the root box read from the device (no host round trip after

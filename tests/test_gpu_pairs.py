@@ -150,3 +150,72 @@ def test_fp64_m2l_shapes(n, cutoff, nequiv):
     tol = 8 * EPS * nequiv / 2 * r21 ** (nequiv / 2)
     assert np.abs(pots[1].imag).max() <= tol * np.abs(pots[0]).max()
     assert np.abs(pots[1].real - pots[0]).max() <= tol * np.abs(pots[0]).max()
+
+
+def direct_targets(kind, k, x, y, tau, tx, ty):
+    """(sum over sources not at the target, sum of magnitudes, sum of |tau| / distance)"""
+    from scipy import special
+    ld = np.longdouble
+    dx, dy = tx[:, None].astype(ld) - x[None, :], ty[:, None].astype(ld) - y[None, :]
+    r2 = dx * dx + dy * dy
+    same = r2 == 0
+    r2[same] = 1
+    r = np.sqrt(r2)
+    if kind == "laplace":
+        g = -np.log(r2) / (4 * ld(np.pi)) + 0j
+    elif kind == "k0":
+        g = special.k0(k * r.astype(float)) / (2 * np.pi) + 0j
+    else:
+        g = 0.25j * special.hankel1(0, k * r.astype(float))
+    g[same] = 0
+    inv = np.where(same, 0, np.abs(tau)[None, :] / r).sum(1)
+    return (g @ tau).astype(complex), ((np.abs(g) + 1) @ np.abs(tau)).astype(float), inv.astype(float)
+
+
+@pytest.mark.parametrize("m", [1, 31, 32, 33, 63, 64, 65, 129, 2049, 5000])
+@pytest.mark.parametrize("kind,k,precision", [("laplace", 0.0, "fp64"), ("laplace", 0.0, "mixed"), ("k0", 0.3, "fp64"),
+                                              ("k0", 2.0, "mixed"), ("h0", 1.0, "fp64")])
+def test_targets_of_one_leaf(kind, k, precision, m):
+    """Item sizes of the target groups, targets on sources, and targets outside
+    the root box.  FP64 bound as above.  Mixed: offsets are rounded to 2^-24 of the
+    box width W = 8 (targets outside it lie within W), which moves a kernel value
+    by that over the distance, and FP32 sums of n terms round n times."""
+    import pykifmm2d_b200 as P
+    n, w = 50, 8.0
+    x, y, tau = cloud(n, 5)
+    rng = np.random.default_rng(m)
+    tx, ty = rng.uniform(-1.5, 1.5, m), rng.uniform(-1.5, 1.5, m)
+    tx[:3], ty[:3] = x[:3][:m], y[:3][:m]
+    kern = {"h0": P.HelmholtzKernel, "k0": P.ModifiedHelmholtzKernel}.get(kind, lambda k: P.LaplaceKernel())(k)
+    f = P.FMM(x, y, P.Get_Kernel_Functions(kern), P.prepare_numba_functions_on_the_fly(kern), 24, 64, kind == "h0",
+              precision=precision)
+    f.build_tree()
+    f.precompute()
+    f.build_expansions(tau)
+    ref, mag, inv = direct_targets(kind, k, x, y, tau, tx, ty)
+    pot = f.evaluate_to_points(tx, ty, True)
+    tol = (n + 64) * EPS * mag
+    if precision == "mixed":
+        tol = 2.0 ** -23 * ((n + 16) * mag + w * inv)
+    assert np.all(np.abs(pot - ref) <= tol)
+
+
+@pytest.mark.parametrize("kind,k,cplx", [("laplace", 0.0, False), ("k0", 5.0, False), ("h0", 3.0, True)])
+def test_targets_at_the_sources_fp64(kind, k, cplx):
+    """Separate targets that are the source points (reordered) give the values at
+    the sources: the same sums in another order."""
+    import pykifmm2d_b200 as P
+    n = 20000
+    x, y, tau = cloud(n, 9)
+    x[:5000] *= 0.01
+    y[:5000] *= 0.01
+    kern = {"h0": P.HelmholtzKernel, "k0": P.ModifiedHelmholtzKernel}.get(kind, lambda k: P.LaplaceKernel())(k)
+    f = P.FMM(x, y, P.Get_Kernel_Functions(kern), P.prepare_numba_functions_on_the_fly(kern), 24, 40, cplx)
+    f.build_tree()
+    f.precompute()
+    f.build_expansions(tau)
+    at = f.evaluate_to_points(x, y, True)
+    p = np.random.default_rng(1).permutation(n)
+    pot = f.evaluate_to_points(x[p].copy(), y[p].copy(), True)
+    _, mag, _ = direct_targets(kind, k, x, y, tau, x[:64], y[:64])
+    assert np.abs(pot - at[p]).max() <= n * EPS * mag.max()
