@@ -193,6 +193,26 @@ static void copy_in(kifmm_plan *P, DBuf<double> &dst, const double *src, int64_t
                                    P->stream));
 }
 
+// Whether p is memory of the plan's device that its kernels can address in
+// place; anything else a copy takes (another device's memory, managed memory).
+static bool local_device_memory(const kifmm_plan *P, const void *p) {
+    cudaPointerAttributes at{};
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return at.type == cudaMemoryTypeDevice && at.device == P->device;
+}
+// the densities of the next apply: read in place where they are on the device
+static void set_tau(kifmm_plan *P, const double *tau, int64_t n, int mem) {
+    if (mem == KIFMM_MEM_DEVICE && tau && local_device_memory(P, tau)) {
+        P->tau_src = tau;
+        return;
+    }
+    copy_in(P, P->tau, tau, n, mem);
+    P->tau_src = P->tau.p;
+}
+
 // Device-side failures reported through a flag (a tensor-core M2L wait that
 // ran out of its poll budget); read after the stream has drained.
 static void check_device_flags(kifmm_plan *P) {
@@ -249,7 +269,7 @@ void apply_prologue(kifmm_plan *P);
 void mixed_upward(kifmm_plan *P, const PassArgs &A);
 void mixed_l2l(kifmm_plan *P, const PassArgs &A);
 PassArgs mixed_leaf_args(kifmm_plan *P);
-void launch_scatter_pot(kifmm_plan *P);
+void launch_scatter_pot(kifmm_plan *P, double *pot);
 void launch_leaf_f_batch(int kind, const PassArgs *dargs, const int64_t *doff, int nplan, int64_t nleaf,
                          cudaStream_t s);
 bool uses_tensor_m2l(const kifmm_plan *P);
@@ -394,6 +414,7 @@ int kifmm_build_tree(kifmm_plan *P, const double *x, const double *y, int64_t n,
         PhaseScope ph(P, KIFMM_PHASE_TREE);
         P->have_mats = false;
         P->applied = false;
+        P->exp_zeroed = false;
         near_join(P);
         // the tree build's many small launches on the plan's highest-priority
         // stream, ahead of the operator build that it starts on the side stream
@@ -426,7 +447,7 @@ int kifmm_build_expansions(kifmm_plan *P, const double *tau, int32_t mem) {
         KIFMM_REQUIRE(P->have_ops, KIFMM_ERR_STATE, "build_expansions: call precompute first");
         use_device(P);
         P->have_expansions = false;
-        copy_in(P, P->tau, tau, P->cplx ? 2 * P->N : P->N, mem);
+        set_tau(P, tau, P->cplx ? 2 * P->N : P->N, mem);
         run_upward_downward(P);
         P->have_expansions = true;
     });
@@ -438,9 +459,12 @@ int kifmm_evaluate_to_sources(kifmm_plan *P, double *pot, int32_t check_self, in
         KIFMM_REQUIRE(P->have_expansions, KIFMM_ERR_STATE, "evaluate: call build_expansions first");
         KIFMM_REQUIRE(mem == KIFMM_MEM_HOST || mem == KIFMM_MEM_DEVICE, KIFMM_ERR_ARG, "bad mem flag");
         use_device(P);
-        run_eval_sources(P, check_self != 0);
+        const int64_t nv = P->cplx ? 2 * P->N : P->N;
+        const bool direct = mem == KIFMM_MEM_DEVICE && pot && local_device_memory(P, pot);
+        if (!direct) P->pot_out.alloc(nv);
+        run_eval_sources(P, check_self != 0, direct ? pot : P->pot_out.p);
         P->applied = true;
-        copy_out(P, pot, P->pot_out.p, P->cplx ? 2 * P->N : P->N, mem);
+        if (!direct) copy_out(P, pot, P->pot_out.p, nv, mem);
     });
 }
 
@@ -478,11 +502,13 @@ int kifmm_synchronize(kifmm_plan *P) {
 // One apply on device pointers, no host synchronisation: what the graph holds.
 static void apply_device(kifmm_plan *P, const double *tau, double *pot, bool check_self) {
     const int64_t nv = P->cplx ? 2 * P->N : P->N;
-    P->tau.alloc(nv);
-    KIFMM_CUDA(cudaMemcpyAsync(P->tau.p, tau, nv * sizeof(double), cudaMemcpyDeviceToDevice, P->stream));
+    const bool direct = local_device_memory(P, pot);
+    set_tau(P, tau, nv, KIFMM_MEM_DEVICE);
+    if (!direct) P->pot_out.alloc(nv);
     run_upward_downward(P);
-    run_eval_sources(P, check_self);
-    KIFMM_CUDA(cudaMemcpyAsync(pot, P->pot_out.p, nv * sizeof(double), cudaMemcpyDeviceToDevice, P->stream));
+    run_eval_sources(P, check_self, direct ? pot : P->pot_out.p);
+    if (!direct)
+        KIFMM_CUDA(cudaMemcpyAsync(pot, P->pot_out.p, nv * sizeof(double), cudaMemcpyDeviceToDevice, P->stream));
     P->applied = true;
 }
 
@@ -757,7 +783,7 @@ static void batch_record(kifmm_batch *B, const double *const *tau, double *const
     htoff.assign(1, 0);
     for (int r = 0; r < n; r++) {
         kifmm_plan *P = B->plans[r];
-        KIFMM_CUDA(cudaMemcpyAsync(P->tau.p, tau[r], P->N * sizeof(double), cudaMemcpyDeviceToDevice, P->stream));
+        set_tau(P, tau[r], P->N, KIFMM_MEM_DEVICE);
         apply_prologue(P);
         int64_t t = 0;
         if (P->L >= 3) {
@@ -792,9 +818,11 @@ static void batch_record(kifmm_batch *B, const double *const *tau, double *const
     fork_all();
     for (int r = 0; r < n; r++) {
         kifmm_plan *P = B->plans[r];
-        launch_scatter_pot(P);
-        KIFMM_CUDA(cudaMemcpyAsync(pot[r], P->pot_out.p, P->N * sizeof(double), cudaMemcpyDeviceToDevice,
-                                   P->stream));
+        const bool direct = local_device_memory(P, pot[r]);
+        launch_scatter_pot(P, direct ? pot[r] : P->pot_out.p);
+        if (!direct)
+            KIFMM_CUDA(cudaMemcpyAsync(pot[r], P->pot_out.p, P->N * sizeof(double), cudaMemcpyDeviceToDevice,
+                                       P->stream));
     }
     join_all();
     launch_lane_sums(B->d_sumlane, n, B->d_sums, B->stream);

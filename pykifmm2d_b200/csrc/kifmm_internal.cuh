@@ -241,6 +241,8 @@ struct kifmm_plan {
     kifmm::DBuf<unsigned> trank, tcount;
     kifmm::DBuf<double> node_den;
     kifmm::DBuf<double> uup, udown;
+    const double *tau_src = nullptr;  // densities of the apply being issued (tau, or the caller's device array)
+    bool exp_zeroed = false;  // uup, udown cleared since the tree was built
     bool have_expansions = false;
     bool applied = false;  // an apply at the sources ran since the tree / operators were built
 
@@ -539,7 +541,7 @@ bool planned_ready(const kifmm_plan *P);
 void build_plan_matrices(kifmm_plan *P);
 // passes.cu
 void run_upward_downward(kifmm_plan *P);
-void run_eval_sources(kifmm_plan *P, int check_self);
+void run_eval_sources(kifmm_plan *P, int check_self, double *pot);
 void run_eval_targets(kifmm_plan *P, const double *tx, const double *ty, int64_t n, int check_self, double *pot);
 void direct_sum_device(const kifmm_kernel &k, const double *x, const double *y, const double *tau, int64_t n,
                        const int64_t *tg, int64_t nt, double *out, cudaStream_t s);

@@ -348,8 +348,9 @@ __global__ void __launch_bounds__(32 * L64_MAX_WARPS, L64_BLOCKS_PER_SM)
             I.nt = min(ts, e - t0);
             const PairSum<KIND, CPLX> v = leaf_item_series<KIND, CPLX, FAR>(A, W, tl, I, tmax);
             if (lane >= I.nt) continue;
-            if constexpr (CPLX) ((double2 *)A.pots)[t0 + lane] = make_double2(v.c[0], v.c[1]);
-            else A.pots[t0 + lane] = FAR ? A.pots[t0 + lane] + v.c[0] : v.c[0];
+            const int o = A.out ? A.perm[t0 + lane] : t0 + lane;
+            if constexpr (CPLX) ((double2 *)(A.out ? A.out : A.pots))[o] = make_double2(v.c[0], v.c[1]);
+            else (A.out ? A.out : A.pots)[o] = FAR ? A.pots[t0 + lane] + v.c[0] : v.c[0];
         }
     }
 }

@@ -14,10 +14,13 @@
 
 namespace kifmm {
 
+// Densities to tree order.  The apply's first kernel: it also clears the
+// scalars that an apply starts from (error flags, ticket), flags[0 .. nflag).
 __global__ void k_gather_tau(const double *__restrict__ tau, const int32_t *__restrict__ perm, int64_t n,
-                             double *__restrict__ taus) {
+                             double *__restrict__ taus, unsigned long long *__restrict__ flags, int nflag) {
     pdl_wait();
     pdl_trigger();  // the P2M's blocks fill every SM: not before this kernel runs
+    if (blockIdx.x == 0 && threadIdx.x < nflag) flags[threadIdx.x] = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         taus[i] = tau[perm[i]];
 }
@@ -985,13 +988,16 @@ void apply_prologue(kifmm_plan *P) {
     P->pots.alloc(n * vw);
     P->uup.alloc((size_t)NN * Q);
     P->udown.alloc((size_t)NN * Q);
-    // error flags of the level passes and the tensor-core M2L, and the
-    // expansions, cleared first so that the kernels below form one chain of
-    // programmatic dependent launches
-    KIFMM_CUDA(cudaMemsetAsync(P->scal.p + KIFMM_SCAL_PASS_ERR, 0,
-                               (KIFMM_SCAL_WORDS - KIFMM_SCAL_PASS_ERR) * sizeof(unsigned long long), s));
-    KIFMM_CUDA(cudaMemsetAsync(P->uup.p, 0, (size_t)NN * Q * sizeof(double), s));
-    KIFMM_CUDA(cudaMemsetAsync(P->udown.p, 0, (size_t)NN * Q * sizeof(double), s));
+    // Expansions start at zero, once per tree: every apply writes the same nodes'
+    // (P2M the leaves with points, M2M the entries, M2L every child of a split
+    // entry), and the others stay zero.
+    if (!P->exp_zeroed) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        KIFMM_CUDA(cudaStreamIsCapturing(s, &cap));
+        KIFMM_CUDA(cudaMemsetAsync(P->uup.p, 0, (size_t)NN * Q * sizeof(double), s));
+        KIFMM_CUDA(cudaMemsetAsync(P->udown.p, 0, (size_t)NN * Q * sizeof(double), s));
+        P->exp_zeroed = cap == cudaStreamCaptureStatusNone;  // (captured: they run with the graph)
+    }
     if (P->opt.planned) {
         ops_wait_now(P);
         build_plan_matrices(P);  // first apply after build_tree / precompute
@@ -1000,8 +1006,9 @@ void apply_prologue(kifmm_plan *P) {
     if (P->cplx)
         launch_gather_tau_c(P);
     else
-        launch_pdl(k_gather_tau, dim3(grid_for(n, 256, P->num_sms * 8)), dim3(256), 0, s, (const double *)P->tau.p,
-                   (const int32_t *)P->perm.p, n, P->taus.p);
+        launch_pdl(k_gather_tau, dim3(grid_for(n, 256, P->num_sms * 8)), dim3(256), 0, s, P->tau_src,
+                   (const int32_t *)P->perm.p, n, P->taus.p, P->scal.p + KIFMM_SCAL_PASS_ERR,
+                   KIFMM_SCAL_WORDS - KIFMM_SCAL_PASS_ERR);
 }
 
 void run_upward_downward(kifmm_plan *P) {
@@ -1052,34 +1059,27 @@ void run_upward_downward(kifmm_plan *P) {
 }
 
 // potentials from tree order to the caller's order
-void launch_scatter_pot(kifmm_plan *P) {
+void launch_scatter_pot(kifmm_plan *P, double *pot) {
     const int64_t n = P->N;
     launch_pdl(k_scatter_pot, dim3(grid_for(n, 256, P->num_sms * 8)), dim3(256), 0, P->stream,
-               (const double *)P->pots.p, (const int32_t *)P->perm.p, n, P->pot_out.p);
+               (const double *)P->pots.p, (const int32_t *)P->perm.p, n, pot);
 }
 
-void run_eval_sources(kifmm_plan *P, int check_self) {
-    int64_t n = P->N;
-    P->pot_out.alloc(P->cplx ? 2 * n : n);
-    if (P->cplx) {
-        run_eval_sources_c(P, make_pass_args(P), check_self);
+// Potentials at the sources into pot (device, caller's order).  The FP64 and
+// the planned leaf passes write them there themselves.
+void run_eval_sources(kifmm_plan *P, int check_self, double *pot) {
+    PassArgs A = make_pass_args(P);
+    A.out = pot;
+    A.perm = P->perm.p;
+    const bool planned = check_self && planned_ready(P);
+    if (!planned && P->opt.precision == KIFMM_PREC_MIXED) {
+        run_eval_sources_mixed(P, A, check_self);
         return;
     }
-    if (check_self && planned_ready(P)) {
-        if (P->n_leaf_list) {
-            PhaseScope ph(P, KIFMM_PHASE_LEAF);
-            launch_planned_leaf(P, make_pass_args(P));
-        }
-    } else if (P->opt.precision == KIFMM_PREC_MIXED) {
-        run_eval_sources_mixed(P, check_self);
-    } else {
-        PassArgs A = make_pass_args(P);
-        if (P->n_leaf_list) {
-            PhaseScope ph(P, KIFMM_PHASE_LEAF);
-            launch_leaf_eval_d(P, A, check_self);
-        }
-    }
-    launch_scatter_pot(P);
+    if (!P->n_leaf_list) return;
+    PhaseScope ph(P, KIFMM_PHASE_LEAF);
+    if (planned) launch_planned_leaf(P, A);
+    else launch_leaf_eval_d(P, A, check_self);
 }
 
 // ------------------------------------------------ kernel-function utilities

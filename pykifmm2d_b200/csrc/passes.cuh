@@ -21,6 +21,8 @@ struct PassArgs {
     const int32_t *nbot, *ntop, *nchild, *nent, *ncoll;
     const double *xs, *ys, *taus;
     double *pots;
+    double *out;            // potentials in the caller's order (null: pots, tree order)
+    const int32_t *perm;    // tree order -> caller's index
     double *uup, *udown;
     const int32_t *leaf_rec;  // [n_leaf_list][LEAF_REC_WORDS] leaf records (build_leaf_records)
     const int32_t *m2l_perm;  // [n_ent] entries of each level in M2L target order (build_m2l_order)
@@ -94,9 +96,8 @@ void launch_planned_p2m(kifmm_plan *P, const PassArgs &A);
 void launch_planned_leaf(kifmm_plan *P, const PassArgs &A);
 // passes_complex.cu (complex values: FP64 point passes on double2 densities)
 void launch_gather_tau_c(kifmm_plan *P);
-void run_eval_sources_c(kifmm_plan *P, const PassArgs &A, int check_self);
 // passes_mixed.cu
 void run_passes_mixed(kifmm_plan *P);
-void run_eval_sources_mixed(kifmm_plan *P, int check_self);
+void run_eval_sources_mixed(kifmm_plan *P, PassArgs A, int check_self);  // A.out: the caller's potentials
 
 }  // namespace kifmm

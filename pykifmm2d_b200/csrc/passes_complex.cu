@@ -6,7 +6,7 @@
 // [Re u (Qc), Im u (Qc)], and every translation operator is the real image of
 // the complex one (operators.cu), so M2M, M2L and L2L are the real FP64
 // kernels unchanged.  P2M, L2P and P2P are in pass_f64.cuh and targets.cu; here
-// are the density and potential permutations and KF / KA / KAS
+// are the densities' permutation and KF / KA / KAS
 // (class_fmm.py:115-145) for a complex kernel.
 // Densities and potentials are double2 (re, im) in HBM.
 #include "passes.cuh"
@@ -22,19 +22,12 @@ __device__ __forceinline__ void cacc(double2 &acc, double2 a, double2 b) {
 }
 
 __global__ void k_gather_tau_c(const double2 *__restrict__ tau, const int32_t *__restrict__ perm, int64_t n,
-                               double2 *__restrict__ taus) {
+                               double2 *__restrict__ taus, unsigned long long *__restrict__ flags, int nflag) {
     pdl_wait();
     pdl_trigger();
+    if (blockIdx.x == 0 && threadIdx.x < nflag) flags[threadIdx.x] = 0;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         taus[i] = tau[perm[i]];
-}
-
-__global__ void k_scatter_pot_c(const double2 *__restrict__ pots, const int32_t *__restrict__ perm, int64_t n,
-                                double2 *__restrict__ pot) {
-    pdl_trigger();
-    pdl_wait();
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        pot[perm[i]] = pots[i];
 }
 
 // ------------------------------------------------ kernel-function utilities
@@ -96,16 +89,8 @@ __global__ void k_kapply_c(int kind, double k, const double *sx, const double *s
 // ------------------------------------------------------------ host side
 void launch_gather_tau_c(kifmm_plan *P) {
     launch_pdl(k_gather_tau_c, dim3(grid_for(P->N, 256, P->num_sms * 8)), dim3(256), 0, P->stream,
-               (const double2 *)P->tau.p, (const int32_t *)P->perm.p, P->N, (double2 *)P->taus.p);
-}
-
-void run_eval_sources_c(kifmm_plan *P, const PassArgs &A, int check_self) {
-    if (P->n_leaf_list) {
-        PhaseScope ph(P, KIFMM_PHASE_LEAF);
-        launch_leaf_eval_d(P, A, check_self);
-    }
-    launch_pdl(k_scatter_pot_c, dim3(grid_for(P->N, 256, P->num_sms * 8)), dim3(256), 0, P->stream,
-               (const double2 *)P->pots.p, (const int32_t *)P->perm.p, P->N, (double2 *)P->pot_out.p);
+               (const double2 *)P->tau_src, (const int32_t *)P->perm.p, P->N, (double2 *)P->taus.p,
+               P->scal.p + KIFMM_SCAL_PASS_ERR, KIFMM_SCAL_WORDS - KIFMM_SCAL_PASS_ERR);
 }
 
 void direct_sum_device_c(const kifmm_kernel &kn, const double *x, const double *y, const double *tau, int64_t n,

@@ -823,13 +823,21 @@ PassArgs mixed_leaf_args(kifmm_plan *P) {
     return A;
 }
 
-void run_eval_sources_mixed(kifmm_plan *P, int check_self) {
+static void eval_sources_f(kifmm_plan *P, int check_self);
+void launch_scatter_pot(kifmm_plan *P, double *pot);
+void run_eval_sources_mixed(kifmm_plan *P, PassArgs A, int check_self) {
     if (!P->n_leaf_list) return;
-    PhaseScope ph(P, KIFMM_PHASE_LEAF);
     if (P->opt.near_fp64) {
-        launch_leaf_eval_d(P, make_pass_args(P), check_self);
+        PhaseScope ph(P, KIFMM_PHASE_LEAF);
+        launch_leaf_eval_d(P, A, check_self);
         return;
-    }  // FP32 form: coincident pairs always contribute zero
+    }
+    eval_sources_f(P, check_self);
+    launch_scatter_pot(P, A.out);
+}
+static void eval_sources_f(kifmm_plan *P, int check_self) {
+    PhaseScope ph(P, KIFMM_PHASE_LEAF);
+    // FP32 form: coincident pairs always contribute zero
     PassArgs A = mixed_leaf_args(P);
     if (P->near_pending) {  // the near field is in P->pots (near_launch): add the far field
         KIFMM_CUDA(cudaStreamWaitEvent(P->stream, P->near_done, 0));

@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(PL_THREADS) k_planned_leaf(PassArgs A, const i
         }
     }
     __syncthreads();
-    for (int t = tid; t < nt; t += PL_THREADS) A.pots[b + t] = acc[t];
+    for (int t = tid; t < nt; t += PL_THREADS) A.out[A.perm[b + t]] = acc[t];
 }
 
 // ------------------------------------------------------------ host side

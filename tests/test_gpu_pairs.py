@@ -219,3 +219,28 @@ def test_targets_at_the_sources_fp64(kind, k, cplx):
     pot = f.evaluate_to_points(x[p].copy(), y[p].copy(), True)
     _, mag, _ = direct_targets(kind, k, x, y, tau, x[:64], y[:64])
     assert np.abs(pot - at[p]).max() <= n * EPS * mag.max()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_expansions_of_a_rebuilt_tree(precision):
+    """The expansions are cleared once per tree: an object whose points move to
+    other trees (more and fewer nodes, empty leaves in other places), with
+    several applies on each, gives what a new object gives."""
+    import pykifmm2d_b200 as P
+    kern = P.LaplaceKernel()
+    make = lambda x, y: P.FMM(x, y, P.Get_Kernel_Functions(kern), P.prepare_numba_functions_on_the_fly(kern), 24, 20,
+                              precision=precision)
+    x, y, tau = cloud(6000, 2)
+    f = make(x, y)
+    for seed, squeeze in ((2, 1.0), (3, 0.02), (4, 1.0), (5, 0.3)):
+        nx, ny, _ = cloud(6000, seed)
+        nx[:4000] *= squeeze
+        x[:], y[:] = nx, ny
+        f.build_tree()
+        f.precompute()
+        for t in (tau * 3, tau):
+            f.build_expansions(t)
+            pot = f.evaluate_to_points(x, y, True).copy()
+        g = make(x.copy(), y.copy())
+        g.build_expansions(tau)
+        np.testing.assert_array_equal(pot, g.evaluate_to_points(g.x, g.y, True))
