@@ -844,15 +844,18 @@ __global__ void __launch_bounds__(LG_THREADS) k_lvl_gemm_b(PassArgs A, int l, in
 // wrote are read past L1 (__ldcg).
 constexpr int LD_THREADS = 256, LD_TE = 8;
 template <int MODE, int KS>
-__global__ void __launch_bounds__(LD_THREADS) k_lvl_dmma(PassArgs A, int l) {
-    constexpr int Q = 4 * KS, NR = (Q + 7) / 8, NRW = (NR + 1) / 2;
-    __shared__ double red[MODE == 0 ? 2 : 1][MODE == 0 ? 4 : 1][MODE == 0 ? LD_TE : 1][MODE == 0 ? 8 * NR + 1 : 1];
-    __shared__ int snode[2][LD_TE];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+struct LvlTile {
+    static constexpr int Q = 4 * KS, NR = (Q + 7) / 8, NRW = (NR + 1) / 2;
+    double red[MODE == 0 ? 2 : 1][MODE == 0 ? 4 : 1][MODE == 0 ? LD_TE : 1][MODE == 0 ? 8 * NR + 1 : 1];
+    int snode[2][LD_TE];
+};
+// the warp's part of level l's operator
+template <int MODE, int KS>
+__device__ __forceinline__ void lvl_operator(const PassArgs &A, int l, double (&a)[LvlTile<MODE, KS>::NRW][KS]) {
+    constexpr int Q = 4 * KS, NRW = LvlTile<MODE, KS>::NRW;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int child = warp >> 1, rt0 = (warp & 1) * NRW;
-    const int64_t ne = A.T.ne[l], eoff = A.T.eoff[l], ntile = (ne + LD_TE - 1) / LD_TE;
     const double *op = A.ops + (size_t)l * A.stride + (MODE == 0 ? A.off_m2m : A.off_l2l);
-    double a[NRW][KS];
 #pragma unroll
     for (int i = 0; i < NRW; i++) {
         const int r = 8 * (rt0 + i) + g;
@@ -862,68 +865,132 @@ __global__ void __launch_bounds__(LD_THREADS) k_lvl_dmma(PassArgs A, int l) {
             a[i][k] = r < Q ? (MODE == 0 ? op[(size_t)(child * Q + c) * Q + r] : op[(size_t)c * 4 * Q + child * Q + r]) : 0.0;
         }
     }
-    pdl_trigger();
-    int par = 0;
-    for (int64_t tile = blockIdx.x; tile < ntile; tile += gridDim.x, par ^= 1) {
-        const int64_t e0 = tile * LD_TE, en = e0 + g;
-        // nodes of the tile's entries (tree data); L2L passes the X-list cells over
-        int node = -1;
-        if (en < ne && (MODE == 0 || !(A.ent[eoff + en] & 1))) node = A.ent_node[eoff + en];
-        if (warp == 0 && t == 0) snode[par][g] = node;
-        if (tile == blockIdx.x) pdl_wait();
-        if (MODE == 1) __syncthreads();
-        double acc[NRW][2], b[KS];
-        const double *src = MODE == 0 ? A.uup + (size_t)(A.T.off[l + 1] + 4 * en + child) * Q : A.udown + (size_t)node * Q;
+}
+// one tile (LD_TE entries) of level l by the whole block; wait: the previous
+// kernel's results have not been waited for
+template <int MODE, int KS>
+__device__ __forceinline__ void lvl_tile(const PassArgs &A, int l, int64_t tile, int par, bool wait,
+                                         const double (&a)[LvlTile<MODE, KS>::NRW][KS], LvlTile<MODE, KS> &S) {
+    constexpr int Q = 4 * KS, NR = LvlTile<MODE, KS>::NR, NRW = LvlTile<MODE, KS>::NRW;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+    const int child = warp >> 1, rt0 = (warp & 1) * NRW;
+    const int64_t ne = A.T.ne[l], eoff = A.T.eoff[l], e0 = tile * LD_TE, en = e0 + g;
+    // nodes of the tile's entries (tree data); L2L passes the X-list cells over
+    int node = -1;
+    if (en < ne && (MODE == 0 || !(A.ent[eoff + en] & 1))) node = A.ent_node[eoff + en];
+    if (warp == 0 && t == 0) S.snode[par][g] = node;
+    if (wait) pdl_wait();
+    if (MODE == 1) __syncthreads();
+    double acc[NRW][2], b[KS];
+    const double *src = MODE == 0 ? A.uup + (size_t)(A.T.off[l + 1] + 4 * en + child) * Q : A.udown + (size_t)node * Q;
 #pragma unroll
-        for (int k = 0; k < KS; k++) b[k] = node >= 0 ? __ldcg(src + 4 * k + t) : 0.0;
+    for (int k = 0; k < KS; k++) b[k] = node >= 0 ? __ldcg(src + 4 * k + t) : 0.0;
+#pragma unroll
+    for (int i = 0; i < NRW; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int r = 8 * (rt0 + i) + g, n = 2 * t + j;
+            acc[i][j] = 0.0;
+            if (MODE == 1 && r < Q && S.snode[par][n] >= 0)
+                acc[i][j] = __ldcg(A.udown + (size_t)(A.T.off[l + 1] + 4 * (e0 + n) + child) * Q + r);
+        }
+#pragma unroll
+    for (int k = 0; k < KS; k++)
+#pragma unroll
+        for (int i = 0; i < NRW; i++) dmma_8x8x4(acc[i][0], acc[i][1], a[i][k], b[k]);
+    if (MODE == 0) {
+#pragma unroll
+        for (int i = 0; i < NRW; i++)
+            if (rt0 + i < NR) {
+                S.red[par][child][2 * t][8 * (rt0 + i) + g] = acc[i][0];
+                S.red[par][child][2 * t + 1][8 * (rt0 + i) + g] = acc[i][1];
+            }
+        __syncthreads();
+        for (int i = tid; i < LD_TE * Q; i += LD_THREADS) {
+            const int n = i / Q, r = i - n * Q, nd = S.snode[par][n];
+            if (nd >= 0)
+                A.uup[(size_t)nd * Q + r] =
+                    (S.red[par][0][n][r] + S.red[par][1][n][r]) + (S.red[par][2][n][r] + S.red[par][3][n][r]);
+        }
+    } else {
 #pragma unroll
         for (int i = 0; i < NRW; i++)
 #pragma unroll
             for (int j = 0; j < 2; j++) {
                 const int r = 8 * (rt0 + i) + g, n = 2 * t + j;
-                acc[i][j] = 0.0;
-                if (MODE == 1 && r < Q && snode[par][n] >= 0)
-                    acc[i][j] = __ldcg(A.udown + (size_t)(A.T.off[l + 1] + 4 * (e0 + n) + child) * Q + r);
+                if (r < Q && S.snode[par][n] >= 0)
+                    A.udown[(size_t)(A.T.off[l + 1] + 4 * (e0 + n) + child) * Q + r] = acc[i][j];
             }
-#pragma unroll
-        for (int k = 0; k < KS; k++)
-#pragma unroll
-            for (int i = 0; i < NRW; i++) dmma_8x8x4(acc[i][0], acc[i][1], a[i][k], b[k]);
-        if (MODE == 0) {
-#pragma unroll
-            for (int i = 0; i < NRW; i++)
-                if (rt0 + i < NR) {
-                    red[par][child][2 * t][8 * (rt0 + i) + g] = acc[i][0];
-                    red[par][child][2 * t + 1][8 * (rt0 + i) + g] = acc[i][1];
-                }
-            __syncthreads();
-            for (int i = tid; i < LD_TE * Q; i += LD_THREADS) {
-                const int n = i / Q, r = i - n * Q, nd = snode[par][n];
-                if (nd >= 0)
-                    A.uup[(size_t)nd * Q + r] = (red[par][0][n][r] + red[par][1][n][r]) + (red[par][2][n][r] + red[par][3][n][r]);
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < NRW; i++)
-#pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    const int r = 8 * (rt0 + i) + g, n = 2 * t + j;
-                    if (r < Q && snode[par][n] >= 0)
-                        A.udown[(size_t)(A.T.off[l + 1] + 4 * (e0 + n) + child) * Q + r] = acc[i][j];
-                }
-        }
+    }
+}
+template <int MODE, int KS>
+__global__ void __launch_bounds__(LD_THREADS) k_lvl_dmma(PassArgs A, int l) {
+    __shared__ LvlTile<MODE, KS> S;
+    const int64_t ntile = (A.T.ne[l] + LD_TE - 1) / LD_TE;
+    double a[LvlTile<MODE, KS>::NRW][KS];
+    lvl_operator<MODE, KS>(A, l, a);
+    pdl_trigger();
+    int par = 0;
+    for (int64_t tile = blockIdx.x; tile < ntile; tile += gridDim.x, par ^= 1)
+        lvl_tile<MODE, KS>(A, l, tile, par, tile == blockIdx.x, a, S);
+}
+// M2M of a run of consecutive small levels l0, l0 - 1, ... (count of them, at
+// most LC_TILES tiles each) by one cluster: a barrier of the cluster takes the
+// place of a launch between levels (2.9 us a level against 5.8 for five levels
+// of 1k points, and one launch to issue).  The blocks exchange the levels'
+// vectors through L2: stores before the barrier's release, reads past L1 after
+// its acquire.  L2L levels, without the sum over children, take 2.6-3.0 us as
+// launches of their own, the same as in a cluster.
+constexpr int LC_BLOCKS = 8, LC_TILES = 16;
+template <int KS>
+__global__ void __launch_bounds__(LD_THREADS) k_m2m_chain(PassArgs A, int l0, int count) {
+    constexpr int MODE = 0, NRW = LvlTile<MODE, KS>::NRW;
+    constexpr bool AHEAD = NRW * KS <= 40;  // the next level's operator is loaded before the barrier (registers)
+    __shared__ LvlTile<MODE, KS> S;
+    int par = 0;
+    double a[NRW][KS];
+    lvl_operator<MODE, KS>(A, l0, a);
+    pdl_trigger();
+    for (int i = 0; i < count; i++) {
+        const int l = l0 - i;
+        const int64_t ntile = (A.T.ne[l] + LD_TE - 1) / LD_TE;
+        for (int64_t tile = blockIdx.x; tile < ntile; tile += LC_BLOCKS, par ^= 1)
+            lvl_tile<MODE, KS>(A, l, tile, par, i == 0 && tile == blockIdx.x, a, S);
+        if (i == 0 && blockIdx.x >= ntile) pdl_wait();
+        if (i + 1 == count) break;
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        if (AHEAD) lvl_operator<MODE, KS>(A, l - 1, a);
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (!AHEAD) lvl_operator<MODE, KS>(A, l - 1, a);
     }
 }
 template <int MODE, int KS>
 static void launch_lvl_dmma(kifmm_plan *P, const PassArgs &A, int l) {
-    if (4 * KS == P->Q) {
-        // past four blocks per SM a block takes several tiles: the operator is read once
-        const int64_t tiles = (P->lt.ne[l] + LD_TE - 1) / LD_TE;
-        launch_pdl(k_lvl_dmma<MODE, KS>, dim3((unsigned)std::min<int64_t>(tiles, (int64_t)P->num_sms * 4)),
-                   dim3(LD_THREADS), 0, P->stream, A, l);
-    } else if constexpr (KS > 1) {
-        launch_lvl_dmma<MODE, KS - 1>(P, A, l);
-    }
+    if constexpr (KS > 1)
+        if (4 * KS != P->Q) return launch_lvl_dmma<MODE, KS - 1>(P, A, l);
+    // past four blocks per SM a block takes several tiles: the operator is read once
+    const int64_t tiles = (P->lt.ne[l] + LD_TE - 1) / LD_TE;
+    launch_pdl(k_lvl_dmma<MODE, KS>, dim3((unsigned)std::min<int64_t>(tiles, (int64_t)P->num_sms * 4)), dim3(LD_THREADS),
+               0, P->stream, A, l);
+}
+template <int KS>
+static void launch_m2m_chain(kifmm_plan *P, const PassArgs &A, int l, int count) {
+    if constexpr (KS > 1)
+        if (4 * KS != P->Q) return launch_m2m_chain<KS - 1>(P, A, l, count);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(LC_BLOCKS);
+    cfg.blockDim = dim3(LD_THREADS);
+    cfg.stream = P->stream;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = LC_BLOCKS;
+    at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    KIFMM_CUDA(cudaLaunchKernelEx(&cfg, k_m2m_chain<KS>, A, l, count));
+    KIFMM_LAUNCHED();
 }
 
 // NT columns per block: (ceil(M/4)) x (NT/4) threads <= 256 and at most
@@ -942,7 +1009,6 @@ static void launch_lvl_gemm(kifmm_plan *P, const PassArgs &A, int l) {
     const int Q = P->Q;
     const int M = MODE == 0 ? Q : 4 * Q, K = MODE == 0 ? 4 * Q : Q;
     const int64_t ne = P->lt.ne[l];
-    if (Q % 4 == 0) return launch_lvl_dmma<MODE, 16>(P, A, l);  // FP64 tensor path (Nequiv <= 64)
     {  // broadcast form when the operator and the entry tile fit in shared memory
         constexpr int RPT = MODE == 0 ? 8 : 16;
         const int RG = (M + RPT - 1) / RPT, Mp = RG * RPT;
@@ -964,17 +1030,29 @@ static void launch_lvl_gemm(kifmm_plan *P, const PassArgs &A, int l) {
     KIFMM_LAUNCHED();
 }
 
-void launch_m2m_d(kifmm_plan *P, const PassArgs &A, int l) { launch_lvl_gemm<0>(P, A, l); }
-void launch_l2l_d(kifmm_plan *P, const PassArgs &A, int l) { launch_lvl_gemm<1>(P, A, l); }
-
-// the upward M2M over levels L-2 .. 2 and the downward L2L over 2 .. L-2
+// The upward M2M over levels L-2 .. 2 and the downward L2L over 2 .. L-2: on the
+// FP64 tensor path for Nequiv a multiple of four (up to 64), with runs of small
+// M2M levels in one launch.
 void run_m2m_levels(kifmm_plan *P, const PassArgs &A) {
-    for (int l = P->L - 2; l >= 2; l--)
-        if (P->lt.ne[l]) launch_m2m_d(P, A, l);
+    for (int l = P->L - 2, count; l >= 2; l -= count) {
+        count = 0;
+        while (l - count >= 2 && P->lt.ne[l - count] > 0 && P->lt.ne[l - count] <= LC_TILES * LD_TE) count++;
+        if (P->Q % 4 == 0 && count > 1) {
+            launch_m2m_chain<16>(P, A, l, count);
+            continue;
+        }
+        count = 1;
+        if (!P->lt.ne[l]) continue;
+        if (P->Q % 4 == 0) launch_lvl_dmma<0, 16>(P, A, l);
+        else launch_lvl_gemm<0>(P, A, l);
+    }
 }
 void run_l2l_levels(kifmm_plan *P, const PassArgs &A) {
-    for (int l = 2; l <= P->L - 2; l++)
-        if (P->lt.ne[l]) launch_l2l_d(P, A, l);
+    for (int l = 2; l <= P->L - 2; l++) {
+        if (!P->lt.ne[l]) continue;
+        if (P->Q % 4 == 0) launch_lvl_dmma<1, 16>(P, A, l);
+        else launch_lvl_gemm<1>(P, A, l);
+    }
 }
 
 // Buffers of an apply, its cleared flags and expansions, and the densities in

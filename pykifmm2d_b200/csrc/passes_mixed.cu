@@ -729,8 +729,6 @@ __global__ void __launch_bounds__(32 * LEAF_WARPS, LEAF_BLOCKS_PER_SM)
 
 // m2l_tc.cu / passes.cu
 void run_m2l_tensor(kifmm_plan *P, const PassArgs &A);
-void launch_m2m_d(kifmm_plan *P, const PassArgs &A, int l);
-void launch_l2l_d(kifmm_plan *P, const PassArgs &A, int l);
 void run_m2m_levels(kifmm_plan *P, const PassArgs &A);
 void run_l2l_levels(kifmm_plan *P, const PassArgs &A);
 
