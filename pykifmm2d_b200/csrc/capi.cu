@@ -268,8 +268,7 @@ struct TempCtx {
 void apply_prologue(kifmm_plan *P);
 void mixed_upward(kifmm_plan *P, const PassArgs &A);
 void mixed_l2l(kifmm_plan *P, const PassArgs &A);
-PassArgs mixed_leaf_args(kifmm_plan *P);
-void launch_scatter_pot(kifmm_plan *P, double *pot);
+void mixed_far(kifmm_plan *P, PassArgs A, cudaEvent_t near_done);
 void launch_leaf_f_batch(int kind, const PassArgs *dargs, const int64_t *doff, int nplan, int64_t nleaf,
                          cudaStream_t s);
 bool uses_tensor_m2l(const kifmm_plan *P);
@@ -526,7 +525,10 @@ int kifmm_graph_capture(kifmm_plan *P, const double *tau, double *pot, int32_t c
         struct Restore {
             kifmm_plan *P;
             bool prof;
-            ~Restore() { P->profiling = prof; }
+            ~Restore() {
+                P->profiling = prof;
+                P->own_capture = false;
+            }
         } restore{P, prof};
         apply_device(P, tau, pot, check_self != 0);  // allocates; sets kernel attributes
         P->have_expansions = true;
@@ -534,6 +536,7 @@ int kifmm_graph_capture(kifmm_plan *P, const double *tau, double *pot, int32_t c
         check_device_flags(P);
         KIFMM_CUDA(cudaStreamBeginCapture(P->stream, cudaStreamCaptureModeThreadLocal));
         cudaGraph_t g = nullptr;
+        P->own_capture = true;
         try {
             apply_device(P, tau, pot, check_self != 0);
         } catch (...) {
@@ -759,8 +762,8 @@ static void check_batch_plan(kifmm_plan *P, int device, int form) {
 }
 
 // Every plan's first phase (densities in, P2M, M2M, M2L slices) in its branch,
-// the packed M2L, the L2L and leaf arguments in the branches, the packed leaf
-// passes, then the scatters: fork and join through events, so that the capture
+// the packed M2L, the L2L in the branches, the packed near fields, then the far
+// fields: fork and join through events, so that the capture
 // holds the branches as parallel paths of one graph.
 static void batch_record(kifmm_batch *B, const double *const *tau, double *const *pot,
                          std::vector<unsigned char> &htc, std::vector<int64_t> &htoff,
@@ -803,7 +806,7 @@ static void batch_record(kifmm_batch *B, const double *const *tau, double *const
         if (P->L >= 3) mixed_l2l(P, make_pass_args(P));
         if (!P->n_leaf_list) continue;
         const int k = P->kern.kind == KIFMM_KERNEL_LAPLACE ? 0 : 1;
-        hleaf[k].push_back(mixed_leaf_args(P));
+        hleaf[k].push_back(make_pass_args(P));
         hloff[k].push_back(hloff[k].back() + P->n_leaf_list);
     }
     join_all();
@@ -819,7 +822,10 @@ static void batch_record(kifmm_batch *B, const double *const *tau, double *const
     for (int r = 0; r < n; r++) {
         kifmm_plan *P = B->plans[r];
         const bool direct = local_device_memory(P, pot[r]);
-        launch_scatter_pot(P, direct ? pot[r] : P->pot_out.p);
+        PassArgs A = make_pass_args(P);
+        A.out = direct ? pot[r] : P->pot_out.p;
+        A.perm = P->perm.p;
+        if (P->n_leaf_list) mixed_far(P, A, nullptr);
         if (!direct)
             KIFMM_CUDA(cudaMemcpyAsync(pot[r], P->pot_out.p, P->N * sizeof(double), cudaMemcpyDeviceToDevice,
                                        P->stream));

@@ -158,6 +158,7 @@ struct kifmm_plan {
     // so that its small launches are scheduled ahead of the near pass's blocks
     cudaStream_t far_stream = nullptr;
     cudaEvent_t far_fork = nullptr, far_done = nullptr;
+    bool own_capture = false;  // kifmm_graph_capture is recording (both halves of an apply: streams forked are joined)
     bool near_pending = false;  // P->pots holds the near field of the last apply, far field not added yet
     cudaEvent_t ops_fork = nullptr, ops_done = nullptr;
     cudaEvent_t ops_circ = nullptr;  // side stream: the check circles are written (the P2M's only operator input)
@@ -197,7 +198,6 @@ struct kifmm_plan {
     kifmm::DBuf<int32_t> leaf_list, p2m_list;
     kifmm::DBuf<int32_t> leaf_rec;   // [n_leaf_list][32] leaf records (passes.cuh, LeafRec)
     kifmm::DBuf<int32_t> m2l_perm;   // [n_ent] M2L target order of the entries (build_m2l_order)
-    kifmm::DBuf<int32_t> leaf_split; // leaves of more than 32 points (split leaf pass)
     kifmm::DBuf<uint16_t> m2l_key;   // [n_ent] direction mask of each entry (256: not split)
     kifmm::DBuf<int32_t> m2l_src8;   // [n_ent][8] source entry per direction (-1: none)
     kifmm::DBuf<unsigned> m2l_hist;  // [MAX_LEVELS + 1][257] counts, then cursors
@@ -341,9 +341,8 @@ inline long long plan_wait_polls(const kifmm_plan *P) {
 constexpr int KIFMM_SCAL_SORT_ERR = 13;  // a radix-sort look-back wait that ran out
 constexpr int KIFMM_SCAL_PASS_ERR = 14;
 constexpr int KIFMM_SCAL_TC_ERR = 15;
-constexpr int KIFMM_SCAL_LEAF_SPLIT = 16;  // count of the split leaf list (k_leaf_split_list)
-constexpr int KIFMM_SCAL_TICKET = 17;      // item counter of the FP64 leaf pass (zero between launches)
-constexpr int KIFMM_SCAL_WORDS = 18;
+constexpr int KIFMM_SCAL_TICKET = 16;      // item counter of the FP64 leaf pass (zero between launches)
+constexpr int KIFMM_SCAL_WORDS = 17;
 
 // Lanes of the warp holding the same 8-bit digit d (d = 256: no key; such
 // lanes match each other only): nine ballots, one per bit, each lane keeping

@@ -138,9 +138,9 @@ void launch_leaf_eval_d(kifmm_plan *P, const PassArgs &A, int check_self) {
         launch_leaf_eval<KIFMM_KERNEL_LAPLACE, false, false>(P, A, check_self);
     else launch_leaf_eval<KIFMM_KERNEL_MOD_HELMHOLTZ, false, false>(P, A, check_self);
 }
-// the K0 far field, added to the near field in pots
-void launch_leaf_far_d(kifmm_plan *P, const PassArgs &A) {
-    launch_leaf_eval<KIFMM_KERNEL_MOD_HELMHOLTZ, false, true>(P, A, 0);
+// the K0 far field, added to the near field in pots (there after near_done)
+void launch_leaf_far_d(kifmm_plan *P, const PassArgs &A, cudaEvent_t near_done) {
+    launch_leaf_eval<KIFMM_KERNEL_MOD_HELMHOLTZ, false, true>(P, A, 0, near_done);
 }
 void launch_p2m_d(kifmm_plan *P, const PassArgs &A) {
     if (P->cplx) launch_p2m_dc(P, A);

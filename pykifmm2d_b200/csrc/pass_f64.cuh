@@ -9,8 +9,7 @@
 
 namespace kifmm {
 
-// equivalent densities of the leaf list, of every node (pass_f64.cu)
-const double *launch_leaf_density(kifmm_plan *P, const PassArgs &A);
+// equivalent densities of every node (pass_f64.cu)
 const double *launch_node_density(kifmm_plan *P, const PassArgs &A);
 
 // L2P + P2P of the leaves, one warp per item: an item is up to ts (<= 32)
@@ -368,10 +367,12 @@ static void pair_grid(const kifmm_plan *P, int64_t items, size_t warp_bytes, int
     *smem = LOGTAB_N * LOGTAB_COPIES * sizeof(double2) + (size_t)w * warp_bytes;
 }
 
+// (near_done: an event that the leaf pass, but not the densities, comes after)
 template <int KIND, bool CPLX, bool FAR>
-static void launch_leaf_eval(kifmm_plan *P, const PassArgs &A, int check_self) {
+static void launch_leaf_eval(kifmm_plan *P, const PassArgs &A, int check_self, cudaEvent_t near_done = nullptr) {
     const int64_t nl = P->n_leaf_list;
     const double *den = launch_leaf_density(P, A);
+    if (near_done) KIFMM_CUDA(cudaStreamWaitEvent(P->stream, near_done, 0));
     // Items: whole 32-target tiles once they fill the GPU's resident warps (16
     // per SM); smaller tiles for fewer leaves, down to 8 targets, where a
     // warp's run over its sources is the kernel's length.

@@ -89,7 +89,8 @@ __host__ __device__ constexpr int pad4mod16(int m) { return m + (20 - m % 16) % 
 void launch_p2m_d(kifmm_plan *P, const PassArgs &A);
 void launch_p2m_dc(kifmm_plan *P, const PassArgs &A);
 void launch_leaf_eval_dc(kifmm_plan *P, const PassArgs &A, int check_self);
-void launch_leaf_far_d(kifmm_plan *P, const PassArgs &A);
+void launch_leaf_far_d(kifmm_plan *P, const PassArgs &A, cudaEvent_t near_done);
+const double *launch_leaf_density(kifmm_plan *P, const PassArgs &A);
 void launch_leaf_eval_d(kifmm_plan *P, const PassArgs &A, int check_self);
 // planned.cu
 void launch_planned_p2m(kifmm_plan *P, const PassArgs &A);

@@ -127,6 +127,7 @@ struct TaylorArgs {
     PassArgs A;
     const int32_t *list;
     double *coef;
+    const double *den;  // [leaf_list index][Q] densities, null where no point lies outside the root box
     int lmin, lmax;
     int64_t loff[MAX_LEVELS + 1];  // leaf_list range of each level
     int64_t toff[MAX_LEVELS + 1];  // first block of each level
@@ -354,19 +355,13 @@ __constant__ unsigned c_recip16[33] = {
     3856, 3641,  3450,  3277,  3121,  2979,  2850,  2731, 2622, 2521, 2428, 2341, 2260, 2185, 2115, 2048};
 __device__ __forceinline__ int small_div(int x, int d) { return (int)(((unsigned)x * c_recip16[d]) >> 16); }
 
-// the L2P + P2P of leaf w of A's leaf list, by one warp: its 32-target tiles
-// [tile0, tile1) (all of them by default).  PART: LEAF_BOTH writes near + far
-// field, LEAF_NEAR the near field alone (P2P, run under the far-field chain),
-// LEAF_FAR adds the far field (L2P) to what LEAF_NEAR wrote.
-enum LeafPart { LEAF_BOTH = 0, LEAF_NEAR = 1, LEAF_FAR = 2 };
-template <int KIND, int PART = LEAF_BOTH>
-__device__ __forceinline__ void leaf_eval_f_leaf(const PassArgs &A, int64_t w, int tile0 = 0, int tile1 = 1 << 20) {
-    constexpr int R = 2 * KIFMM_TAYLOR_P + 1;
+// the P2P of leaf w of A's leaf list, by one warp: its 32-target tiles [tile0,
+// tile1) (all of them by default), into pots
+template <int KIND>
+__device__ __forceinline__ void leaf_near_f(const PassArgs &A, int64_t w, int tile0 = 0, int tile1 = 1 << 20) {
     constexpr float CLAMP = 1.17549435e-38f;  // FLT_MIN
     __shared__ ulonglong2 sxys[LEAF_WARPS][LEAF_CHUNK + 32];  // (x, x | y, y) per staged source
     __shared__ f32x2 szs[LEAF_WARPS][LEAF_CHUNK + 32];        // (z, z)
-    __shared__ double qds[LEAF_WARPS][R > 64 ? R : 64];
-    __shared__ float qfs[LEAF_WARPS][R > 64 ? R : 64];
     __shared__ double red[LEAF_WARPS][2][32];
     __shared__ float redf[LEAF_WARPS][2][32];
     __shared__ int rngs[LEAF_WARPS][18];
@@ -375,7 +370,6 @@ __device__ __forceinline__ void leaf_eval_f_leaf(const PassArgs &A, int64_t w, i
         // the leaf record: node, level, point range, cell key and source ranges
         // in one coalesced load (list[w] is the record's node)
         const int rv = A.leaf_rec[w * LEAF_REC_WORDS + lane];
-        const int g = __shfl_sync(0xffffffffu, rv, LR_NODE);
         const int l = __shfl_sync(0xffffffffu, rv, LR_LEVEL);
         const uint64_t key = (uint64_t)(uint32_t)__shfl_sync(0xffffffffu, rv, LR_KEY_LO) |
                              ((uint64_t)(uint32_t)__shfl_sync(0xffffffffu, rv, LR_KEY_HI) << 32);
@@ -386,24 +380,11 @@ __device__ __forceinline__ void leaf_eval_f_leaf(const PassArgs &A, int64_t w, i
             cy = A.root + ((double)compact2(key) + 0.5) * wl;
         }
         const bool lap = KIND == KIFMM_KERNEL_LAPLACE;
-        const bool taylor = lap && A.taylor != nullptr && l >= 2 && PART != LEAF_NEAR;
-        double *qd = qds[wib];
-        float *qf = qfs[wib];
         ulonglong2 *sxy = sxys[wib];
         f32x2 *sz = szs[wib];
         const double width = ldexp(A.W, -l);
         const double sc = lap ? 1.0 / width : 1.0;     // coordinate scale
         const double lw = lap ? -2.0 * log2(sc) : 0.0; // log2 of the squared length unit
-        if (taylor) {  // Taylor coefficients of the local expansion (k_leaf_taylor, FP64)
-            const double *cf = A.leaf_coef + (size_t)w * R;
-            for (int r = lane; r < R; r += 32) {
-                const double v = cf[r];
-                qd[r] = v;
-                qf[r] = (float)v;
-            }
-        } else if (PART != LEAF_NEAR) {
-            local_density(A, g, l, qd, lane);
-        }
         const float kk = (float)A.k;
         const float lclamp = lg2_ftz(CLAMP);
         const int b = __shfl_sync(0xffffffffu, rv, LR_BOT), e = __shfl_sync(0xffffffffu, rv, LR_TOP);
@@ -473,7 +454,7 @@ __device__ __forceinline__ void leaf_eval_f_leaf(const PassArgs &A, int64_t w, i
             const f32x2 tx2 = f2_pack(txa, txb), ty2 = f2_pack(tya, tyb);
             double neara = 0.0, nearb = 0.0;
             float exa = 0.f, exb = 0.f;  // charges of the leaf's own points met at the floor
-            for (int c0 = 0; PART != LEAF_FAR && c0 < ns; c0 += LEAF_CHUNK) {
+            for (int c0 = 0; c0 < ns; c0 += LEAF_CHUNK) {
                 const int cn = min(LEAF_CHUNK, ns - c0);
                 if (t0 == tfirst || ns > LEAF_CHUNK) gather(c0, cn, lap && t0 == tfirst);
                 // lane (gi, j) takes sources j, j + sp, ...; j + (it - 1) sp < cn + 32
@@ -517,103 +498,56 @@ __device__ __forceinline__ void leaf_eval_f_leaf(const PassArgs &A, int64_t w, i
                 const int slot = lane < ng ? 0 : 1, grp = lane - slot * ng;
                 double v = 0.0;
                 float ex = 0.f;
-                for (int m = 0; PART != LEAF_FAR && m < sp; m++) {
+                for (int m = 0; m < sp; m++) {
                     v += red[wib][slot][grp + m * ng];
                     ex += redf[wib][slot][grp + m * ng];
                 }
-                if (lap && PART != LEAF_FAR) {
+                if (lap) {
                     // the skipped charges leave log2(w^2) * sum(tau); the one skipped
                     // pair is almost always the target itself: take its FP64 charge
                     const double tau_t = A.taus[t];
                     const double exd = ex == (float)tau_t ? tau_t : (double)ex;
                     v += lw * (tsum - exd);
                 }
-                const double pxd = A.xs[t] - cx, pyd = A.ys[t] - cy;
-                // far field (L2P) in FP64
-                double far = 0.0;
-                if (l >= 2 && PART != LEAF_NEAR) {
-                    const double zx = pxd * sc, zy = pyd * sc;
-                    if (taylor && zx * zx + zy * zy <= 0.5625) {
-                        // Horner: orders P..9 in FP32 (weighted by |z/rho|^9 < 0.008 where
-                        // used), then 8..1 in FP64
-                        const float zxf = (float)zx, zyf = (float)zy;
-                        float fr = qf[R - 2], fi = qf[R - 1];
-                        for (int jj = KIFMM_TAYLOR_P - 1; jj >= 9; jj--) {
-                            const float nr = fmaf(fr, zxf, fmaf(-fi, zyf, qf[2 * jj - 1]));
-                            const float ni = fmaf(fr, zyf, fmaf(fi, zxf, qf[2 * jj]));
-                            fr = nr;
-                            fi = ni;
-                        }
-                        double sr = fr, si = fi;
-                        for (int jj = 8; jj >= 1; jj--) {
-                            double nr = fma(sr, zx, fma(-si, zy, qd[2 * jj - 1]));
-                            double ni = fma(sr, zy, fma(si, zx, qd[2 * jj]));
-                            sr = nr;
-                            si = ni;
-                        }
-                        far = qd[0] + (sr * zx - si * zy);
-                    } else {
-                        // direct FP64 sum over the equivalent points (out-of-box targets, K0)
-                        const double *lgd = A.ops + (size_t)l * A.stride + A.off_large;
-                        const double *inv = A.ops + (size_t)l * A.stride + A.off_inv;
-                        const double *u = A.udown + (size_t)g * A.Q;
-                        for (int q = 0; q < A.Q; q++) {
-                            double qq = taylor ? 0.0 : qd[q];
-                            if (taylor)
-                                for (int c = 0; c < A.Q; c++) qq = fma(inv[q * A.Q + c], u[c], qq);
-                            double dx = pxd - lgd[q], dy = pyd - lgd[A.Q + q];
-                            far = fma(green_d(A.kind, A.k, dx * dx + dy * dy), qq, far);
-                        }
-                    }
-                }
-                if (PART == LEAF_BOTH) A.pots[t] = v * (double)gsum_scale<KIND>() + far;
-                else if (PART == LEAF_NEAR) A.pots[t] = v * (double)gsum_scale<KIND>();
-                else A.pots[t] += far;
+                A.pots[t] = v * (double)gsum_scale<KIND>();
             }
             __syncwarp();
         }
     }
 }
 
-// One warp per leaf.  With `split` (a leaf list smaller than one wave of the
-// GPU, where the kernel lasts as long as its heaviest leaf) warps nlist ..
-// nlist + *nsplit - 1 take the tiles after the first of the leaves in
-// split_list, so a leaf of more than 32 points runs on two warps.
-template <int KIND, bool SPLIT, int PART = LEAF_BOTH>
-__global__ void __launch_bounds__(32 * LEAF_WARPS, LEAF_BLOCKS_PER_SM)
-    k_leaf_eval_f(PassArgs A, int64_t nlist, const int32_t *__restrict__ split_list,
-                  const unsigned *__restrict__ nsplit) {
+// One warp per leaf, or with SPLIT (a leaf list smaller than half a wave of the
+// GPU, where the kernel lasts as long as its heaviest leaf) two: the second takes
+// the tiles after the leaf's first 32 points and leaves at once where there are
+// none.
+template <int KIND, bool SPLIT>
+__global__ void __launch_bounds__(32 * LEAF_WARPS, LEAF_BLOCKS_PER_SM) k_leaf_near_f(PassArgs A, int64_t nlist) {
     pdl_trigger();
     pdl_wait();
-    const int64_t wstride = (int64_t)gridDim.x * LEAF_WARPS;
+    const int64_t w = (int64_t)blockIdx.x * LEAF_WARPS + (threadIdx.x >> 5);
     if (!SPLIT) {
-        for (int64_t w = (int64_t)blockIdx.x * LEAF_WARPS + (threadIdx.x >> 5); w < nlist; w += wstride)
-            leaf_eval_f_leaf<KIND, PART>(A, w);
-        return;
-    }
-    const int64_t total = nlist + *nsplit;
-    for (int64_t w = (int64_t)blockIdx.x * LEAF_WARPS + (threadIdx.x >> 5); w < total; w += wstride) {
-        const bool first = w < nlist;
-        leaf_eval_f_leaf<KIND>(A, first ? w : (int64_t)split_list[w - nlist], first ? 0 : 1, first ? 1 : 1 << 20);
+        if (w < nlist) leaf_near_f<KIND>(A, w);
+    } else if (w < 2 * nlist) {
+        leaf_near_f<KIND>(A, w >> 1, w & 1, w & 1 ? 1 << 20 : 1);
     }
 }
 
-// The far field of the Laplace leaves after a near-only pass (LEAF_NEAR), with
-// every lane busy: one block per 32 consecutive leaves of one level (the
+// The far field of the Laplace leaves, added to the near field that pots holds,
+// with every lane busy: one block per 32 consecutive leaves of one level (the
 // k_leaf_taylor tiling), each thread a target of those leaves.  The leaves'
 // Taylor coefficients (written by k_leaf_taylor) are staged in shared memory,
-// orders >= 9 as FP32 and orders <= 8 as FP64, and the Horner L2P is the
-// one of leaf_eval_f_leaf step for step, so the sum added to the near field
-// in pots is the same; targets beyond the series radius take the direct sum
-// over the equivalent points.  Replaces the far-only warp-per-leaf pass,
-// whose Horner ran on about half the lanes.
+// orders >= 9 as FP32 and orders <= 8 as FP64.  Targets beyond the series radius
+// (points outside the root box; no others) take the direct sum over the
+// equivalent points with the leaves' densities (k_leaf_density): formed per
+// target from the inverse, a dozen such points in a million made this kernel
+// 149 us long where it takes 21.
 constexpr int FT_THREADS = 128;
 __global__ void __launch_bounds__(FT_THREADS) k_leaf_far_taylor(TaylorArgs T) {
     constexpr int R = 2 * KIFMM_TAYLOR_P + 1;
     __shared__ float qf[32][R + 1];
     __shared__ double qd[32][17];  // orders 0..8
     __shared__ double scx[32], scy[32], ssc[32];
-    __shared__ int sbot[32], spre[33], snode[32], slev[32];
+    __shared__ int sbot[32], spre[33], slev[32];
     const PassArgs &A = T.A;
     pdl_trigger();
     const int64_t b = blockIdx.x;
@@ -634,7 +568,6 @@ __global__ void __launch_bounds__(FT_THREADS) k_leaf_far_taylor(TaylorArgs T) {
             scy[tid] = A.root + ((double)compact2(key) + 0.5) * wl;
             ssc[tid] = 1.0 / wl;
             sbot[tid] = rec[LR_BOT];
-            snode[tid] = rec[LR_NODE];
             slev[tid] = lv;
             cnt = rec[LR_TOP] - rec[LR_BOT];
         }
@@ -662,7 +595,7 @@ __global__ void __launch_bounds__(FT_THREADS) k_leaf_far_taylor(TaylorArgs T) {
         const double pxd = A.xs[t] - scx[n], pyd = A.ys[t] - scy[n];
         const double zx = pxd * ssc[n], zy = pyd * ssc[n];
         double far;
-        if (zx * zx + zy * zy <= 0.5625) {
+        if (!T.den || zx * zx + zy * zy <= 0.5625) {
             const float zxf = (float)zx, zyf = (float)zy;
             float fr = qf[n][R - 2], fi = qf[n][R - 1];
             for (int jj = KIFMM_TAYLOR_P - 1; jj >= 9; jj--) {
@@ -680,41 +613,23 @@ __global__ void __launch_bounds__(FT_THREADS) k_leaf_far_taylor(TaylorArgs T) {
             }
             far = qd[n][0] + (sr * zx - si * zy);
         } else {
-            // direct FP64 sum over the equivalent points (targets outside the series radius)
-            const int lv = slev[n], g = snode[n];
-            const double *lgd = A.ops + (size_t)lv * A.stride + A.off_large;
-            const double *inv = A.ops + (size_t)lv * A.stride + A.off_inv;
-            const double *u = A.udown + (size_t)g * A.Q;
+            const double *lgd = A.ops + (size_t)slev[n] * A.stride + A.off_large, *den = T.den + (size_t)(w0 + n) * A.Q;
             far = 0.0;
             for (int q = 0; q < A.Q; q++) {
-                double qq = 0.0;
-                for (int c = 0; c < A.Q; c++) qq = fma(inv[q * A.Q + c], u[c], qq);
-                double dx = pxd - lgd[q], dy = pyd - lgd[A.Q + q];
-                far = fma(green_d(A.kind, A.k, dx * dx + dy * dy), qq, far);
+                const double dx = pxd - lgd[q], dy = pyd - lgd[A.Q + q];
+                far = fma(green_d(A.kind, A.k, dx * dx + dy * dy), den[q], far);
             }
         }
-        A.pots[t] += far;
+        if (A.out) A.out[A.perm[t]] = A.pots[t] + far;
+        else         A.pots[t] += far;
     }
 }
 
-// the leaves of more than 32 points (their tiles after the first), for the
-// split form of k_leaf_eval_f
-__global__ void k_leaf_split_list(const int32_t *__restrict__ rec, int64_t nlist, int32_t *__restrict__ out,
-                                  unsigned *__restrict__ count) {
-    const int64_t w = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const bool big = w < nlist && rec[w * LEAF_REC_WORDS + LR_TOP] - rec[w * LEAF_REC_WORDS + LR_BOT] > 32;
-    const unsigned peers = __ballot_sync(0xffffffffu, big);
-    unsigned base = 0;
-    if ((threadIdx.x & 31) == 0 && peers) base = atomicAdd(count, (unsigned)__popc(peers));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (big) out[base + __popc(peers & ((1u << (threadIdx.x & 31)) - 1))] = (int32_t)w;
-}
-
-// The leaf pass of several plans in one launch (serving batches): warp w of
+// The near field of several plans in one launch (serving batches): warp w of
 // the grid takes leaf w - off[r] of plan r, off[r] <= w < off[r + 1].
 template <int KIND>
 __global__ void __launch_bounds__(32 * LEAF_WARPS, LEAF_BLOCKS_PER_SM)
-    k_leaf_eval_f_batch(const PassArgs *__restrict__ args, const int64_t *__restrict__ off, int nplan) {
+    k_leaf_near_f_batch(const PassArgs *__restrict__ args, const int64_t *__restrict__ off, int nplan) {
     pdl_trigger();
     pdl_wait();
     const int64_t w = (int64_t)blockIdx.x * LEAF_WARPS + (threadIdx.x >> 5);
@@ -724,7 +639,7 @@ __global__ void __launch_bounds__(32 * LEAF_WARPS, LEAF_BLOCKS_PER_SM)
         if (off[mid] <= w) lo = mid;
         else hi = mid;
     }
-    if (w < off[nplan]) leaf_eval_f_leaf<KIND>(args[lo], w - off[lo]);
+    if (w < off[nplan]) leaf_near_f<KIND>(args[lo], w - off[lo]);
 }
 
 // m2l_tc.cu / passes.cu
@@ -732,8 +647,10 @@ void run_m2l_tensor(kifmm_plan *P, const PassArgs &A);
 void run_m2m_levels(kifmm_plan *P, const PassArgs &A);
 void run_l2l_levels(kifmm_plan *P, const PassArgs &A);
 
+bool near_split(const kifmm_plan *P);
+void near_launch(kifmm_plan *P, cudaStream_t s);
+void near_fork(kifmm_plan *P);
 // P2M and M2M of the mixed apply
-void near_launch(kifmm_plan *P);
 void mixed_upward(kifmm_plan *P, const PassArgs &A) {
     if (P->n_p2m_list) {
         PhaseScope ph(P, KIFMM_PHASE_P2M);
@@ -754,14 +671,17 @@ void mixed_l2l(kifmm_plan *P, const PassArgs &A) {
 void run_passes_mixed(kifmm_plan *P) {
     const int Q = P->Q, L = P->L;
     if (L < 3) return;  // expansions cleared by run_upward_downward
-    // the near field at the sources on a low-priority stream, the far-field
-    // chain below on a high-priority one (launches and allocations swapped
-    // there, joined back into the plan's stream at the end)
-    const bool near = near_possible(P);
-    HighPriorityFork fork(P, near);
+    // The near field at the sources on a low-priority stream.  A leaf list of
+    // less than half a wave starts with the apply and runs beside the chain; a
+    // larger one starts after the M2M chain, under a far-field chain on a
+    // high-priority stream (launches and allocations swapped there, joined back
+    // into the plan's stream at the end).
+    const bool near = near_possible(P), early = near && near_split(P);
+    if (early) near_fork(P);
+    HighPriorityFork fork(P, near && !early);
     PassArgs A = make_pass_args(P);
     mixed_upward(P, A);
-    if (near) near_launch(P);  // after the M2M chain, under the M2L and L2L
+    if (near && !early) near_fork(P);  // after the M2M chain, under the M2L and L2L
     if (P->opt.m2l == KIFMM_M2L_FP32) {
         PhaseScope ph(P, KIFMM_PHASE_M2L);
         const int thr = ((4 * Q + 31) / 32) * 32;
@@ -782,8 +702,6 @@ void run_passes_mixed(kifmm_plan *P) {
     mixed_l2l(P, A);
 }
 
-// The arguments of the FP32 leaf kernel; for the Laplace kernel this first
-// launches the Taylor coefficients of the leaves' local expansions.
 // the 32-leaf tiles of the leaves at levels >= 2 (k_leaf_taylor, k_leaf_far_taylor)
 static TaylorArgs taylor_tiling(kifmm_plan *P, const PassArgs &A, int64_t *ntiles) {
     TaylorArgs T{};
@@ -802,9 +720,18 @@ static TaylorArgs taylor_tiling(kifmm_plan *P, const PassArgs &A, int64_t *ntile
     return T;
 }
 
-PassArgs mixed_leaf_args(kifmm_plan *P) {
-    PassArgs A = make_pass_args(P);
-    if (P->kern.kind == KIFMM_KERNEL_LAPLACE && P->l2p_taylor.p && P->L >= 3) {
+// The far field at the sources, added to the near field in pots, to A.out.
+// near_done (or null): the event after which pots holds the near field; the
+// Taylor coefficients and densities do not wait for it.
+void launch_scatter_pot(kifmm_plan *P, double *pot);  // passes.cu
+void mixed_far(kifmm_plan *P, PassArgs A, cudaEvent_t near_done) {
+    // leaves above level 2 have no far field: their potentials go out by the scatter
+    const bool all = P->leaf_loff[2] == 0;
+    double *pot = A.out;
+    if (!all) A.out = nullptr;
+    if (P->kern.kind == KIFMM_KERNEL_MOD_HELMHOLTZ) {
+        if (P->L >= 3) launch_leaf_far_d(P, A, near_done), near_done = nullptr;
+    } else if (P->l2p_taylor.p && P->L >= 3) {
         constexpr int R = 2 * KIFMM_TAYLOR_P + 1;
         KIFMM_REQUIRE(P->Q % 4 == 0, KIFMM_ERR_ARG, "mixed Laplace form: Nequiv must be a multiple of 4");
         P->leaf_coef.alloc((size_t)P->n_leaf_list * R);
@@ -812,90 +739,51 @@ PassArgs mixed_leaf_args(kifmm_plan *P) {
         int64_t tiles = 0;
         TaylorArgs T = taylor_tiling(P, A, &tiles);
         if (tiles) {
+            if (P->n_outside) T.den = launch_leaf_density(P, A);
             const size_t smem = ((size_t)P->Q * pad4mod16(8 * TY_MTR) + 32 * (size_t)pad4mod16(P->Q) + 32 * (size_t)R) *
                                 sizeof(double);
             ensure_dyn_smem(k_leaf_taylor, smem);
             launch_pdl(k_leaf_taylor, dim3((unsigned)tiles), dim3(TY_THREADS), smem, P->stream, T);
+            if (near_done) KIFMM_CUDA(cudaStreamWaitEvent(P->stream, near_done, 0));
+            near_done = nullptr;
+            launch_pdl(k_leaf_far_taylor, dim3((unsigned)tiles), dim3(FT_THREADS), 0, P->stream, T);
         }
     }
-    return A;
+    if (near_done) KIFMM_CUDA(cudaStreamWaitEvent(P->stream, near_done, 0));
+    if (!all) launch_scatter_pot(P, pot);
 }
 
-static void eval_sources_f(kifmm_plan *P, int check_self);
-void launch_scatter_pot(kifmm_plan *P, double *pot);
 void run_eval_sources_mixed(kifmm_plan *P, PassArgs A, int check_self) {
     if (!P->n_leaf_list) return;
+    PhaseScope ph(P, KIFMM_PHASE_LEAF);
     if (P->opt.near_fp64) {
-        PhaseScope ph(P, KIFMM_PHASE_LEAF);
         launch_leaf_eval_d(P, A, check_self);
         return;
     }
-    eval_sources_f(P, check_self);
-    launch_scatter_pot(P, A.out);
-}
-static void eval_sources_f(kifmm_plan *P, int check_self) {
-    PhaseScope ph(P, KIFMM_PHASE_LEAF);
     // FP32 form: coincident pairs always contribute zero
-    PassArgs A = mixed_leaf_args(P);
-    if (P->near_pending) {  // the near field is in P->pots (near_launch): add the far field
-        KIFMM_CUDA(cudaStreamWaitEvent(P->stream, P->near_done, 0));
-        P->near_pending = false;
-        if (A.leaf_coef) {  // Laplace: every leaf of level >= 2 has its Taylor coefficients
-            int64_t tiles = 0;
-            TaylorArgs T = taylor_tiling(P, A, &tiles);
-            if (tiles) launch_pdl(k_leaf_far_taylor, dim3((unsigned)tiles), dim3(FT_THREADS), 0, P->stream, T);
-            return;
-        }
-        if (P->kern.kind == KIFMM_KERNEL_MOD_HELMHOLTZ) launch_leaf_far_d(P, A);
-        return;
-    }
-    // fewer leaves than one wave of warps: split the big ones over two warps
-    const int64_t nl = P->n_leaf_list;
-    const bool split = nl < (int64_t)P->num_sms * LEAF_BLOCKS_PER_SM * LEAF_WARPS / 2;
-    const int32_t *slist = nullptr;
-    const unsigned *scount = nullptr;
-    if (split) {
-        P->leaf_split.alloc((size_t)nl);
-        unsigned *cnt = (unsigned *)(P->scal.p + KIFMM_SCAL_LEAF_SPLIT);
-        KIFMM_CUDA(cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), P->stream));
-        k_leaf_split_list<<<(unsigned)((nl + 255) / 256), 256, 0, P->stream>>>(P->leaf_rec.p, nl, P->leaf_split.p,
-                                                                                cnt);
-        KIFMM_LAUNCHED();
-        slist = P->leaf_split.p;
-        scount = cnt;
-    }
-    const int64_t warps = split ? 2 * nl : nl;
-    unsigned gr = (unsigned)std::min<int64_t>((warps + LEAF_WARPS - 1) / LEAF_WARPS, 1ll << 30);
-    const dim3 grid(gr), block(32 * LEAF_WARPS);
-    if (P->kern.kind == KIFMM_KERNEL_LAPLACE) {
-        if (split) launch_pdl(k_leaf_eval_f<KIFMM_KERNEL_LAPLACE, true>, grid, block, 0, P->stream, A, nl, slist, scount);
-        else launch_pdl(k_leaf_eval_f<KIFMM_KERNEL_LAPLACE, false>, grid, block, 0, P->stream, A, nl, slist, scount);
-    } else {
-        if (split)
-            launch_pdl(k_leaf_eval_f<KIFMM_KERNEL_MOD_HELMHOLTZ, true>, grid, block, 0, P->stream, A, nl, slist, scount);
-        else
-            launch_pdl(k_leaf_eval_f<KIFMM_KERNEL_MOD_HELMHOLTZ, false>, grid, block, 0, P->stream, A, nl, slist,
-                       scount);
-    }
+    const bool pending = P->near_pending;  // the near field is on its way into P->pots
+    P->near_pending = false;
+    if (!pending) near_launch(P, P->stream);
+    mixed_far(P, A, pending ? P->near_done : nullptr);
 }
 
 // The near field at the sources (P2P of every leaf over its colleagues) needs
 // only the sorted points and charges, none of the expansions, so the apply
 // runs it on a stream of its own while the far-field chain leaves SMs idle,
-// and the evaluation at the sources adds only the far field (LEAF_FAR).
+// and the evaluation at the sources adds only the far field (mixed_far).
 // Mixed FP32 near field, where the near sum does not depend on check_self
-// (coincident pairs contribute zero); not inside a stream capture and not for
-// leaf lists smaller than one wave (those split big leaves over two warps
-// instead).  A later evaluation at other targets leaves the pass unused.
-// The near pass runs on a stream of the lowest priority and the far-field
-// chain on one of the highest, and the pass starts after the M2M chain, under
-// the source slicing, M2L and L2L: started with the apply its blocks, filling
-// every SM, held off the M2M chain's small level launches even with the
-// priorities (M2M 0.086 -> 0.18 ms at 1M points).  Measured per step against
-// the single leaf pass after the chain: 1M mixture 1.005 -> 0.953 ms (0.971-
-// 0.994 when started with the apply), 4M uniform 2.446 -> 2.444 ms, 2M K0
+// (coincident pairs contribute zero).  A later evaluation at other targets
+// leaves the pass unused; a second one at the sources runs it again.
+// The near pass runs on a stream of the lowest priority.  For large leaf lists
+// the far-field chain runs on one of the highest, and the pass starts after the
+// M2M chain, under the source slicing, M2L and L2L: started with the apply its
+// blocks, filling every SM, held off the M2M chain's small level launches even
+// with the priorities (M2M 0.086 -> 0.18 ms at 1M points).  Measured per step
+// against the single leaf pass after the chain: 1M mixture 1.005 -> 0.953 ms
+// (0.971-0.994 when started with the apply), 4M uniform 2.446 -> 2.444 ms, 2M K0
 // annulus 6.02 -> 5.20 ms (the K0 near field is several times longer than the
-// chain, which runs under it).
+// chain, which runs under it).  Lists of less than half a wave start with the
+// apply.
 
 // the plan's near stream (lowest priority) and far stream (highest), once,
 // from the per-device pool
@@ -912,21 +800,39 @@ bool near_possible(kifmm_plan *P) {
     if (P->opt.precision != KIFMM_PREC_MIXED || P->opt.near_fp64 || P->opt.planned || P->cplx || nl <= 0)
         return false;
     if (P->kern.kind != KIFMM_KERNEL_LAPLACE && P->kern.kind != KIFMM_KERNEL_MOD_HELMHOLTZ) return false;
-    if (nl < (int64_t)P->num_sms * LEAF_BLOCKS_PER_SM * LEAF_WARPS / 2) return false;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    KIFMM_CUDA(cudaStreamIsCapturing(P->stream, &cap));
-    if (cap != cudaStreamCaptureStatusNone) return false;
+    if (!P->own_capture) {  // a caller's capture may end between the apply and the evaluation that joins
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        KIFMM_CUDA(cudaStreamIsCapturing(P->stream, &cap));
+        if (cap != cudaStreamCaptureStatusNone) return false;
+    }
     ensure_aux_streams(P);
     return true;
 }
+// fewer leaves than half a wave of warps: the big ones are split over two warps
+bool near_split(const kifmm_plan *P) {
+    return P->n_leaf_list < (int64_t)P->num_sms * LEAF_BLOCKS_PER_SM * LEAF_WARPS / 2;
+}
 
-// the near pass, forked from the plan's stream at this point
-void near_launch(kifmm_plan *P) {
+// the near pass on stream s
+void near_launch(kifmm_plan *P, cudaStream_t s) {
     const int64_t nl = P->n_leaf_list;
+    const PassArgs A = make_pass_args(P);
+    const bool split = near_split(P);
+    const dim3 grid((unsigned)(((split ? 2 * nl : nl) + LEAF_WARPS - 1) / LEAF_WARPS)), block(32 * LEAF_WARPS);
+    constexpr int LAP = KIFMM_KERNEL_LAPLACE, K0 = KIFMM_KERNEL_MOD_HELMHOLTZ;
+    if (P->kern.kind == LAP) {
+        if (split) launch_pdl(k_leaf_near_f<LAP, true>, grid, block, 0, s, A, nl);
+        else launch_pdl(k_leaf_near_f<LAP, false>, grid, block, 0, s, A, nl);
+    } else {
+        if (split) launch_pdl(k_leaf_near_f<K0, true>, grid, block, 0, s, A, nl);
+        else launch_pdl(k_leaf_near_f<K0, false>, grid, block, 0, s, A, nl);
+    }
+}
+
+// ... on the near stream, forked from the plan's stream at this point
+void near_fork(kifmm_plan *P) {
     KIFMM_CUDA(cudaEventRecord(P->near_fork, P->stream));
     KIFMM_CUDA(cudaStreamWaitEvent(P->near_stream, P->near_fork, 0));
-    PassArgs A = make_pass_args(P);
-    const dim3 grid((unsigned)((nl + LEAF_WARPS - 1) / LEAF_WARPS)), block(32 * LEAF_WARPS);
     {
         struct Swap {  // the phase timer's events go to the near stream
             kifmm_plan *P;
@@ -935,12 +841,7 @@ void near_launch(kifmm_plan *P) {
             ~Swap() { P->stream = main; }
         } sw(P);
         PhaseScope ph(P, KIFMM_PHASE_LEAF);
-        if (P->kern.kind == KIFMM_KERNEL_LAPLACE)
-            launch_pdl(k_leaf_eval_f<KIFMM_KERNEL_LAPLACE, false, LEAF_NEAR>, grid, block, 0, P->near_stream, A, nl,
-                       (const int32_t *)nullptr, (const unsigned *)nullptr);
-        else
-            launch_pdl(k_leaf_eval_f<KIFMM_KERNEL_MOD_HELMHOLTZ, false, LEAF_NEAR>, grid, block, 0, P->near_stream, A,
-                       nl, (const int32_t *)nullptr, (const unsigned *)nullptr);
+        near_launch(P, P->near_stream);
     }
     KIFMM_CUDA(cudaEventRecord(P->near_done, P->near_stream));
     P->near_pending = true;
@@ -954,15 +855,15 @@ void near_join(kifmm_plan *P) {
     P->near_pending = false;
 }
 
-// the FP32 leaf pass of several plans of one kernel kind in one launch
+// the FP32 near field of several plans of one kernel kind in one launch
 void launch_leaf_f_batch(int kind, const PassArgs *dargs, const int64_t *doff, int nplan, int64_t nleaf,
                          cudaStream_t s) {
     const int64_t blocks = (nleaf + LEAF_WARPS - 1) / LEAF_WARPS;
     KIFMM_REQUIRE(blocks > 0 && blocks < (1ll << 31), KIFMM_ERR_ARG, "batch leaf pass: bad leaf count");
     if (kind == KIFMM_KERNEL_LAPLACE)
-        k_leaf_eval_f_batch<KIFMM_KERNEL_LAPLACE><<<(unsigned)blocks, 32 * LEAF_WARPS, 0, s>>>(dargs, doff, nplan);
+        k_leaf_near_f_batch<KIFMM_KERNEL_LAPLACE><<<(unsigned)blocks, 32 * LEAF_WARPS, 0, s>>>(dargs, doff, nplan);
     else
-        k_leaf_eval_f_batch<KIFMM_KERNEL_MOD_HELMHOLTZ><<<(unsigned)blocks, 32 * LEAF_WARPS, 0, s>>>(dargs, doff,
+        k_leaf_near_f_batch<KIFMM_KERNEL_MOD_HELMHOLTZ><<<(unsigned)blocks, 32 * LEAF_WARPS, 0, s>>>(dargs, doff,
                                                                                                       nplan);
     KIFMM_LAUNCHED();
 }
