@@ -346,6 +346,66 @@ __device__ __forceinline__ void leaf_pairs2_sp(int sp, const ulonglong2 *sxy, co
 #undef KIFMM_LEAF_SP
 }
 
+// K0 of two pairs of one target in packed FP32, for 0 < x <= 2 on both sides: the
+// operations of k0_f, in its order, so that the values are the same to the bit.
+// The square root of r^2 is one Newton step on the reciprocal square root
+// (s = r^2 y, s + (r^2 - s^2) y / 2), equal to sqrtf for every FP32 mantissa
+// (checked over all 2^24 of [1, 4); r^2 is held above 2^-80 so that nothing
+// underflows).  The logarithms stay the math library's.
+__device__ __forceinline__ f32x2 f2_dup(float a) { return f2_pack(a, a); }
+__device__ __forceinline__ f32x2 k0_pair_x(f32x2 r2, f32x2 kk) {
+    float ra, rb, ya, yb;
+    f2_unpack(r2, ra, rb);
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(ya) : "f"(ra));
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(yb) : "f"(rb));
+    const f32x2 y = f2_pack(ya, yb), s = f2_mul(r2, y), e = f2_fma(s ^ 0x8000000080000000ull, s, r2);
+    return f2_mul(kk, f2_fma(e, f2_mul(y, f2_dup(0.5f)), s));
+}
+__device__ __forceinline__ f32x2 k0_pair(f32x2 x) {
+    const f32x2 t = f2_mul(x, x);
+    f32x2 a = f2_dup(K0_I0_F[K0_I0_F_N - 1]), b = f2_dup(K0_P_F[K0_P_F_N - 1]);
+#pragma unroll
+    for (int i = K0_I0_F_N - 2; i >= 0; i--) a = f2_fma(a, t, f2_dup(K0_I0_F[i]));
+#pragma unroll
+    for (int i = K0_P_F_N - 2; i >= 0; i--) b = f2_fma(b, t, f2_dup(K0_P_F[i]));
+    float ha, hb;
+    f2_unpack(f2_mul(x, f2_dup(0.5f)), ha, hb);
+    return f2_fma(f2_pack(-logf(ha), -logf(hb)), a, b);
+}
+// K0 pair sums of one lane's target over its sources at list positions j + k
+// sp, k in [0, it), in FP32 blocks of 32 added to `near` in FP64.  Two sources
+// at a time: every value a packed instruction's half, the sum still one after
+// the other.  Position it (past the end) is an uncharged pad.
+__device__ __forceinline__ void leaf_pairs_k0(const float *__restrict__ sx, const float *__restrict__ sy,
+                                              const float *__restrict__ sz, int j, int sp, int it, float tx, float ty,
+                                              float kk, double &near) {
+    const f32x2 tx2 = f2_dup(tx), ty2 = f2_dup(ty), kk2 = f2_dup(kk);
+    for (int kb = 0; kb < it; kb += 32) {
+        const int ke = min(it, kb + 32);
+        float acc = 0.f;
+#pragma unroll 1
+        for (int k = kb; k < ke; k += 2) {
+            const int u = j + k * sp, v = u + sp;
+            const f32x2 dx = f2_sub(tx2, f2_pack(sx[u], sx[v])), dy = f2_sub(ty2, f2_pack(sy[u], sy[v]));
+            const f32x2 r2 = f2_fma(dx, dx, f2_mul(dy, dy)), x = k0_pair_x(r2, kk2);
+            const float za = sz[u], zb = sz[v];
+            float ra, rb, xa, xb;
+            f2_unpack(r2, ra, rb);
+            f2_unpack(x, xa, xb);
+            if (ra >= 0x1p-80f && rb >= 0x1p-80f && xa <= 2.f && xb <= 2.f) {
+                float ga, gb;
+                f2_unpack(k0_pair(x), ga, gb);
+                acc = fmaf(za, ga, acc);
+                acc = fmaf(zb, gb, acc);
+            } else {  // the target itself, far pairs, not-a-number
+                if (ra > 0.f) acc = fmaf(za, k0_f(kk * sqrtf(ra)), acc);
+                if (rb > 0.f) acc = fmaf(zb, k0_f(kk * sqrtf(rb)), acc);
+            }
+        }
+        near += (double)acc;
+    }
+}
+
 // x / d for 0 <= x <= 200 and 1 <= d <= 32 as a multiply and a shift (the
 // lane-layout quotients of the leaf kernel; a division by a run-time value
 // costs a reciprocal and a dozen fix-up instructions): c = ceil(2^16 / d)
@@ -360,8 +420,11 @@ __device__ __forceinline__ int small_div(int x, int d) { return (int)(((unsigned
 template <int KIND>
 __device__ __forceinline__ void leaf_near_f(const PassArgs &A, int64_t w, int tile0 = 0, int tile1 = 1 << 20) {
     constexpr float CLAMP = 1.17549435e-38f;  // FLT_MIN
-    __shared__ ulonglong2 sxys[LEAF_WARPS][LEAF_CHUNK + 32];  // (x, x | y, y) per staged source
-    __shared__ f32x2 szs[LEAF_WARPS][LEAF_CHUNK + 32];        // (z, z)
+    constexpr bool LAP = KIND == KIFMM_KERNEL_LAPLACE;
+    // Laplace: (x, x | y, y) and (z, z) per staged source; K0: x, y, z apart
+    __shared__ ulonglong2 sxys[LAP ? LEAF_WARPS : 1][LAP ? LEAF_CHUNK + 32 : 1];
+    __shared__ f32x2 szs[LAP ? LEAF_WARPS : 1][LAP ? LEAF_CHUNK + 32 : 1];
+    __shared__ float sks[LAP ? 1 : LEAF_WARPS][3][LAP ? 1 : LEAF_CHUNK + 64];
     __shared__ double red[LEAF_WARPS][2][32];
     __shared__ float redf[LEAF_WARPS][2][32];
     __shared__ int rngs[LEAF_WARPS][18];
@@ -380,8 +443,9 @@ __device__ __forceinline__ void leaf_near_f(const PassArgs &A, int64_t w, int ti
             cy = A.root + ((double)compact2(key) + 0.5) * wl;
         }
         const bool lap = KIND == KIFMM_KERNEL_LAPLACE;
-        ulonglong2 *sxy = sxys[wib];
-        f32x2 *sz = szs[wib];
+        ulonglong2 *sxy = sxys[LAP ? wib : 0];
+        f32x2 *sz = szs[LAP ? wib : 0];
+        float(*sk)[LAP ? 1 : LEAF_CHUNK + 64] = sks[LAP ? 0 : wib];
         const double width = ldexp(A.W, -l);
         const double sc = lap ? 1.0 / width : 1.0;     // coordinate scale
         const double lw = lap ? -2.0 * log2(sc) : 0.0; // log2 of the squared length unit
@@ -396,7 +460,7 @@ __device__ __forceinline__ void leaf_near_f(const PassArgs &A, int64_t w, int ti
         if (lane >= LR_RNG && lane < LR_RNG + 18) rng[lane - LR_RNG] = rv;
         double tsum = 0.0;  // FP64 sum of the near sources' charges (Laplace)
         // stage sources [c0, c0 + cn) of the list, padded with 32 far, uncharged
-        // ones; four elements per lane per pass, loads issued before any is used
+        // ones (K0: 64 uncharged ones at the centre); four elements per lane per pass, loads issued before any is used
         auto gather = [&](int c0, int cn, bool sum) {
             __syncwarp();
             int pre[9], off[9];
@@ -428,13 +492,25 @@ __device__ __forceinline__ void leaf_near_f(const PassArgs &A, int64_t w, int ti
                     if (si[k] >= 0) {
                         const float fx = (float)((vx[k] - cx) * sc), fy = (float)((vy[k] - cy) * sc);
                         const float fz = (float)vt[k];
-                        sxy[q0 + lane + 32 * k] = make_ulonglong2(f2_pack(fx, fx), f2_pack(fy, fy));
-                        sz[q0 + lane + 32 * k] = f2_pack(fz, fz);
+                        const int o = q0 + lane + 32 * k;
+                        if (LAP) {
+                            sxy[o] = make_ulonglong2(f2_pack(fx, fx), f2_pack(fy, fy));
+                            sz[o] = f2_pack(fz, fz);
+                        } else {
+                            sk[0][o] = fx;
+                            sk[1][o] = fy;
+                            sk[2][o] = fz;
+                        }
                         if (sum) tsum += vt[k];
                     }
             }
-            sxy[cn + lane] = make_ulonglong2(f2_pack(1e18f, 1e18f), f2_pack(1e18f, 1e18f));
-            sz[cn + lane] = 0ull;
+            if (LAP) {
+                sxy[cn + lane] = make_ulonglong2(f2_pack(1e18f, 1e18f), f2_pack(1e18f, 1e18f));
+                sz[cn + lane] = 0ull;
+            } else {
+#pragma unroll
+                for (int h = 0; h < 64; h += 32) sk[0][cn + h + lane] = sk[1][cn + h + lane] = sk[2][cn + h + lane] = 0.f;
+            }
             __syncwarp();
         };
         __syncwarp();
@@ -467,22 +543,7 @@ __device__ __forceinline__ void leaf_near_f(const PassArgs &A, int64_t w, int ti
                     leaf_pairs2_sp<true>(sp, sxy, sz, j, 0, kown, tx2, ty2, en, neara, nearb, exa, exb);
                     leaf_pairs2_sp<false>(sp, sxy, sz, j, kown, it, tx2, ty2, en, neara, nearb, exa, exb);
                 } else {
-                    for (int k0 = 0; k0 < it; k0 += 32) {
-                        const int k1 = min(it, k0 + 32);
-                        float acc = 0.f;
-    #pragma unroll 1
-                        for (int k = k0; k < k1; k++) {
-                            const int u = j + k * sp;
-                            float sx, sy, sw, unused;
-                            f2_unpack(sxy[u].x, sx, unused);
-                            f2_unpack(sxy[u].y, sy, unused);
-                            f2_unpack(sz[u], sw, unused);
-                            const float4 sv = make_float4(sx, sy, sw, 0.f);
-                            const float r2 = pair_r2(txa, tya, sv);
-                            if (r2 > 0.f) acc = fmaf(sv.z, gsum_term<KIND>(r2, kk), acc);
-                        }
-                        neara += (double)acc;
-                    }
+                    leaf_pairs_k0(sk[0], sk[1], sk[2], j, sp, it, txa, tya, kk, neara);
                 }
             }
             if (lap && t0 == tfirst)

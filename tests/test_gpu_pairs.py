@@ -244,3 +244,23 @@ def test_expansions_of_a_rebuilt_tree(precision):
         g = make(x.copy(), y.copy())
         g.build_expansions(tau)
         np.testing.assert_array_equal(pot, g.evaluate_to_points(g.x, g.y, True))
+
+
+@pytest.mark.parametrize("n", [1, 2, 7, 22, 31, 33, 63, 64, 65, 130, 200])
+@pytest.mark.parametrize("k", [0.3, 2.0, 12.0])
+def test_one_leaf_k0_mixed(k, n):
+    """The FP32 near pass alone, with pairs on both sides of k r = 2 (where the
+    packed series ends).  Bound with u = 2^-23: a block adds at most 32 values,
+    a value is within 16 u (|G| + 1), and coordinates rounded relative to the box
+    move r by at most 2 u, the value by 2 u / (2 pi r) < u / r."""
+    x, y, tau = cloud(n, 100 + n)
+    if n > 8:
+        x[5], y[5] = x[2], y[2]
+    f = fmm("k0", k, x, y, 300, precision="mixed")
+    assert f.tree_info().levels == 1
+    f.build_expansions(tau)
+    pot = f.evaluate_to_points(x, y, True)
+    ref, mag = direct("k0", k, x, y, tau)
+    r = np.hypot(x[:, None] - x[None, :], y[:, None] - y[None, :])
+    r[r == 0] = 1
+    assert np.all(np.abs(pot - ref) <= 50 * 2.0 ** -23 * (mag + (1 / r) @ np.abs(tau)))
