@@ -252,7 +252,7 @@ struct kifmm_plan {
     kifmm::DBuf<int32_t> hash_idx;    // [hash_cap] sorted entry index of the entry in each slot
     kifmm::DBuf<int32_t> perm2;
     kifmm::DBuf<uint32_t> sort_hist;
-    kifmm::DBuf<unsigned long long> sort_status;  // radix sort look-back words
+    kifmm::DBuf<uint32_t> sort_status;  // radix sort look-back words
     kifmm::DBuf<unsigned long long> scal;  // small device scalars
     kifmm::DBuf<int64_t> misc;
     // pinned host words (kifmm::HP_*): read-backs land here by asynchronous
@@ -344,15 +344,16 @@ constexpr int KIFMM_SCAL_TC_ERR = 15;
 constexpr int KIFMM_SCAL_TICKET = 16;      // item counter of the FP64 leaf pass (zero between launches)
 constexpr int KIFMM_SCAL_WORDS = 17;
 
-// Lanes of the warp holding the same 8-bit digit d (d = 256: no key; such
-// lanes match each other only): nine ballots, one per bit, each lane keeping
-// the lanes that agree with it on every bit.  All 32 lanes must call it.
+// Lanes of the warp holding the same BITS-bit number d: one ballot per bit, each
+// lane keeping the lanes that agree with it on every bit.  All 32 lanes must call
+// it.  (A digit of 8 bits with d = 256 for "no key" takes nine.)
 // __match_any_sync gives the same mask, but its throughput falls with the
 // number of distinct values in the warp, which for radix digits is high.
-__device__ __forceinline__ unsigned warp_match_digit(uint32_t d) {
+template <int BITS>
+__device__ __forceinline__ unsigned warp_match_bits(uint32_t d) {
     unsigned m = 0xffffffffu;
 #pragma unroll
-    for (int b = 0; b < 9; b++) {
+    for (int b = 0; b < BITS; b++) {
         const bool bit = (d >> b) & 1u;
         const unsigned bb = __ballot_sync(0xffffffffu, bit);
         m &= bit ? bb : ~bb;
@@ -573,10 +574,8 @@ bool uses_tensor_m2l(const kifmm_plan *P);
 // radix_sort.cu
 void radix_sort_pairs(uint64_t *key, int32_t *val, uint64_t *key_tmp, int32_t *val_tmp, int64_t n, int bits,
                       kifmm_plan *P);
-void radix_sort_keys(uint64_t *key, uint64_t *key_tmp, int64_t n, int bits, kifmm_plan *P);
+void radix_sort_words(uint64_t *key, int32_t *val, uint64_t *key_tmp, int64_t n, int up, kifmm_plan *P);
 void radix_sort_keys_shifts(uint64_t *key, uint64_t *key_tmp, int64_t n, const int *shifts, int npass,
                             kifmm_plan *P);
-void radix_sort_pairs_bits(uint64_t *key, int32_t *val, uint64_t *key_tmp, int32_t *val_tmp, int64_t n, int lo_bit,
-                           int bits, kifmm_plan *P);
 
 }  // namespace kifmm

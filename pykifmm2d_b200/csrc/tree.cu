@@ -37,6 +37,7 @@ void build_m2l_order(kifmm_plan *P);     // passes.cu
 namespace kifmm {
 
 constexpr uint64_t KEY56 = (1ull << 56) - 1;
+constexpr int KEY_LOW = 2 * KEY_DEPTH - 32;  // key bits below the 32 that the first sort orders
 
 __device__ __forceinline__ uint64_t ordered_bits(double v) {
     uint64_t u = (uint64_t)__double_as_longlong(v);
@@ -118,6 +119,8 @@ __global__ void k_keys(const double *__restrict__ x, const double *__restrict__ 
 // k_keys with the root box read from the device (no host round trip after
 // k_bbox).  Inputs that the host will reject (non-finite coordinates, |m| or
 // |M| >= 2^23) get key 0 here; the host reports them at its next read-back.
+// WORDS: a point is one word, its key's top 32 bits above its index
+template <bool WORDS>
 __global__ void k_keys_dev(const double *__restrict__ x, const double *__restrict__ y, int64_t n, int fix_bbox,
                            const unsigned long long *__restrict__ scal, uint64_t *__restrict__ key,
                            int32_t *__restrict__ perm, unsigned long long *outside) {
@@ -132,8 +135,12 @@ __global__ void k_keys_dev(const double *__restrict__ x, const double *__restric
         double a = x[i], b = y[i];
         uint64_t k = 0;
         if (h > 0 && isfinite(a) && isfinite(b)) k = morton(grid_cell(a, m, h), grid_cell(b, m, h));
-        key[i] = k;
-        perm[i] = (int32_t)i;
+        if (WORDS) {
+            key[i] = (k >> KEY_LOW) << 32 | (uint64_t)i;
+        } else {
+            key[i] = k;
+            perm[i] = (int32_t)i;
+        }
         out += (a < m || a > M || b < m || b > M);
     }
     for (int o = 16; o; o >>= 1) out += __shfl_xor_sync(0xffffffffu, out, o);
@@ -625,7 +632,7 @@ __global__ void __launch_bounds__(LT_THREADS) k_lists_write(int64_t n_nodes, con
 // fits in shared memory: block l picks the level-l entries out of the
 // collected list, sorts them by the 2l key bits with an LSD radix sort in
 // shared memory (8-bit digits; warp w ranks its contiguous chunk in order with
-// warp_match_digit, so the sort is stable and the warps' chunks keep their
+// warp_match_bits, so the sort is stable and the warps' chunks keep their
 // order), and writes them at the level's offset (the counts of the levels
 // above).  Keys are distinct within a level: a cell is either split or X-list.
 constexpr int ES_THREADS = 1024, ES_WARPS = ES_THREADS / 32, ES_CAP = 12288;
@@ -736,7 +743,7 @@ __global__ void __launch_bounds__(ES_THREADS) k_ent_sort(const uint64_t *__restr
         for (int i = c0 + lane; i - lane < c1; i += 32) {
             const bool ok = i < c1;
             const uint32_t d = ok ? (uint32_t)((A[i] >> sh) & 255) : 256u;
-            const unsigned peers = warp_match_digit(d);
+            const unsigned peers = warp_match_bits<9>(d);
             if (ok && lane == __ffs(peers) - 1) wcnt[w][d] += __popc(peers);
             __syncwarp();
         }
@@ -758,7 +765,7 @@ __global__ void __launch_bounds__(ES_THREADS) k_ent_sort(const uint64_t *__restr
             const bool ok = i < c1;
             const uint64_t k = ok ? A[i] : 0;
             const uint32_t d = ok ? (uint32_t)((k >> sh) & 255) : 256u;
-            const unsigned peers = warp_match_digit(d);
+            const unsigned peers = warp_match_bits<9>(d);
             if (ok) {
                 const uint32_t b = wcnt[w][d];
                 B[b + __popc(peers & lt)] = k;
@@ -890,17 +897,19 @@ static void build_tree_impl(kifmm_plan *P, const double *x, const double *y, int
     unsigned gs = grid_for(n, TB, P->num_sms * 8);
     k_bbox<<<gs, TB, 0, s>>>(xd, yd, n, P->scal.p);
     KIFMM_LAUNCHED();
-    P->pkey.alloc(n); P->perm.alloc(n); P->key2.alloc(n); P->perm2.alloc(n);
+    P->pkey.alloc(n); P->perm.alloc(n); P->key2.alloc(n);
     // the root box stays on the device until the counts below come back
-    launch_pdl(k_keys_dev, dim3(gs), dim3(TB), 0, s, xd, yd, n,
+    launch_pdl(k_keys_dev<true>, dim3(gs), dim3(TB), 0, s, xd, yd, n,
                (int)P->opt.fix_bbox, (const unsigned long long *)P->scal.p, P->pkey.p, P->perm.p, P->scal.p + 8);
     // Sort by the top 32 key bits first (levels 1..16, four 8-bit passes): that
     // orders every cell of level <= 16, enough whenever no split lies deeper
-    // than level 15.  Otherwise sort all 58 bits and count again.
-    constexpr int FAST_BITS = 32, FAST_LEVELS = FAST_BITS / 2;
+    // than level 15.  A point is then one word, those bits above its index, and the
+    // sorted keys have zeros for the low bits.  Otherwise make the whole keys, sort
+    // all 58 bits and count again.
+    constexpr int FAST_LEVELS = 16;
     {
         PhaseScope ph(P, KIFMM_PHASE_SORT);
-        radix_sort_pairs_bits(P->pkey.p, P->perm.p, P->key2.p, P->perm2.p, n, 2 * KEY_DEPTH - FAST_BITS, FAST_BITS, P);
+        radix_sort_words(P->pkey.p, P->perm.p, P->key2.p, n, KEY_LOW, P);
     }
     HashSet H{};
     H.count = P->scal.p + 9;
@@ -979,6 +988,10 @@ static void build_tree_impl(kifmm_plan *P, const double *x, const double *y, int
         if (full || (st[1] <= (unsigned long long)FAST_LEVELS && st[2] == 0)) break;
         spec = false;  // the queued set used the partial order: rebuilt below
         PhaseScope ph(P, KIFMM_PHASE_SORT);
+        P->perm2.alloc(n);
+        // (its count of points outside the box goes to a counter cleared next)
+        launch_pdl(k_keys_dev<false>, dim3(gs), dim3(TB), 0, s, xd, yd, n, (int)P->opt.fix_bbox,
+                   (const unsigned long long *)P->scal.p, P->pkey.p, P->perm.p, P->scal.p + 5);
         radix_sort_pairs(P->pkey.p, P->perm.p, P->key2.p, P->perm2.p, n, 2 * KEY_DEPTH, P);
     }
     P->xs.alloc(n); P->ys.alloc(n);
