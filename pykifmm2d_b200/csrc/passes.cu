@@ -1090,7 +1090,6 @@ void apply_prologue(kifmm_plan *P) {
 }
 
 void run_upward_downward(kifmm_plan *P) {
-    cudaStream_t s = P->stream;
     const int Q = P->Q, L = P->L;
     near_join(P);  // the previous apply's near-field pass, if never evaluated
     apply_prologue(P);
@@ -1103,6 +1102,10 @@ void run_upward_downward(kifmm_plan *P) {
         ops_wait_now(P);
         return;
     }
+    // a planned near field (bound by HBM) beside the chain, as the mixed apply's
+    const bool near = planned_ready(P) && near_possible(P), early = near && near_split(P);
+    if (early) near_fork(P);
+    HighPriorityFork fork(P, near && !early);
     PassArgs A = make_pass_args(P);
     if (P->n_p2m_list) {
         PhaseScope ph(P, KIFMM_PHASE_P2M);
@@ -1114,6 +1117,7 @@ void run_upward_downward(kifmm_plan *P) {
         PhaseScope ph_m2m(P, KIFMM_PHASE_M2M);
         run_m2m_levels(P, A);
     }
+    if (near && !early) near_fork(P);
     if (m2l_uses_dmma(P)) {
         // FP64 tensor path: all levels' M2L in one launch, then the L2L chain
         {
@@ -1131,7 +1135,7 @@ void run_upward_downward(kifmm_plan *P) {
     for (int l = 1; l <= L - 2; l++) {
         int64_t ne = P->lt.ne[l];
         if (!ne) continue;
-        k_m2l_d<<<(unsigned)((ne + M2L_TE - 1) / M2L_TE), thr, smem, s>>>(A, l);
+        k_m2l_d<<<(unsigned)((ne + M2L_TE - 1) / M2L_TE), thr, smem, P->stream>>>(A, l);  // (maybe the far stream)
         KIFMM_LAUNCHED();
     }
 }
@@ -1150,13 +1154,14 @@ void run_eval_sources(kifmm_plan *P, int check_self, double *pot) {
     A.out = pot;
     A.perm = P->perm.p;
     const bool planned = check_self && planned_ready(P);
+    if (!planned && planned_ready(P)) near_join(P);  // (a planned near field is not the one asked for)
     if (!planned && P->opt.precision == KIFMM_PREC_MIXED) {
         run_eval_sources_mixed(P, A, check_self);
         return;
     }
     if (!P->n_leaf_list) return;
     PhaseScope ph(P, KIFMM_PHASE_LEAF);
-    if (planned) launch_planned_leaf(P, A);
+    if (planned) run_planned_leaf(P, A);
     else launch_leaf_eval_d(P, A, check_self);
 }
 

@@ -94,7 +94,8 @@ const double *launch_leaf_density(kifmm_plan *P, const PassArgs &A);
 void launch_leaf_eval_d(kifmm_plan *P, const PassArgs &A, int check_self);
 // planned.cu
 void launch_planned_p2m(kifmm_plan *P, const PassArgs &A);
-void launch_planned_leaf(kifmm_plan *P, const PassArgs &A);
+void launch_planned_near(kifmm_plan *P, cudaStream_t s);
+void run_planned_leaf(kifmm_plan *P, const PassArgs &A);
 // passes_complex.cu (complex values: FP64 point passes on double2 densities)
 void launch_gather_tau_c(kifmm_plan *P);
 // passes_mixed.cu

@@ -708,9 +708,7 @@ void run_m2l_tensor(kifmm_plan *P, const PassArgs &A);
 void run_m2m_levels(kifmm_plan *P, const PassArgs &A);
 void run_l2l_levels(kifmm_plan *P, const PassArgs &A);
 
-bool near_split(const kifmm_plan *P);
 void near_launch(kifmm_plan *P, cudaStream_t s);
-void near_fork(kifmm_plan *P);
 // P2M and M2M of the mixed apply
 void mixed_upward(kifmm_plan *P, const PassArgs &A) {
     if (P->n_p2m_list) {
@@ -858,9 +856,11 @@ void ensure_aux_streams(kifmm_plan *P) {
 
 bool near_possible(kifmm_plan *P) {
     const int64_t nl = P->n_leaf_list;
-    if (P->opt.precision != KIFMM_PREC_MIXED || P->opt.near_fp64 || P->opt.planned || P->cplx || nl <= 0)
-        return false;
-    if (P->kern.kind != KIFMM_KERNEL_LAPLACE && P->kern.kind != KIFMM_KERNEL_MOD_HELMHOLTZ) return false;
+    if (P->cplx || nl <= 0 || (P->opt.planned != 0) != planned_ready(P)) return false;
+    if (!P->opt.planned) {
+        if (P->opt.precision != KIFMM_PREC_MIXED || P->opt.near_fp64) return false;
+        if (P->kern.kind != KIFMM_KERNEL_LAPLACE && P->kern.kind != KIFMM_KERNEL_MOD_HELMHOLTZ) return false;
+    }
     if (!P->own_capture) {  // a caller's capture may end between the apply and the evaluation that joins
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         KIFMM_CUDA(cudaStreamIsCapturing(P->stream, &cap));
@@ -902,7 +902,8 @@ void near_fork(kifmm_plan *P) {
             ~Swap() { P->stream = main; }
         } sw(P);
         PhaseScope ph(P, KIFMM_PHASE_LEAF);
-        near_launch(P, P->near_stream);
+        if (planned_ready(P)) launch_planned_near(P, P->near_stream);
+        else near_launch(P, P->near_stream);
     }
     KIFMM_CUDA(cudaEventRecord(P->near_done, P->near_stream));
     P->near_pending = true;

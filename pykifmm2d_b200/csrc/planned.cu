@@ -17,9 +17,11 @@
 //         colleagues (rows padded with zeros to 16 bytes):
 //         near_t = sum_s N[t][s] tau_s, pairs with equal coordinates zero
 //         (evaluate_to_points(..., check_self=True), class_fmm.py:105-108).
-// Each apply then streams the blocks once: one CTA per leaf stages the leaf's
-// concatenated charges in shared memory and each warp reduces whole target
-// rows with 16-byte loads (HBM-bound matrix-vector products).  Values are
+// Each apply then streams the blocks once (HBM-bound matrix-vector products).
+// The near pass depends on no expansion and runs on a stream of its own beside
+// the M2L and L2L; the L2P is added to it at the end.  500k points, K0 FP64: an
+// apply 588 us with one leaf kernel after the chain, 546 as two kernels, 511 with
+// the near pass beside it, 454 with the blocks and loads as they are now.  Values are
 // computed in FP64; the near blocks are stored in FP32 for the mixed
 // precision (no FP32 coordinate differences are involved), in FP64 otherwise.
 #include "passes.cuh"
@@ -135,96 +137,146 @@ __global__ void k_plan_fill_p2m(PassArgs A, const int32_t *__restrict__ p2m, int
     }
 }
 
-// planned P2M: one warp per node, lanes over the Q check points
+// planned P2M: one warp per node, eight lanes over the Q check points (PM_Q each)
+// and four over the sources
 __global__ void k_planned_p2m(PassArgs A, const int32_t *__restrict__ p2m, int64_t np2m,
                               const int64_t *__restrict__ p2m_off, const double *__restrict__ mat) {
+    constexpr int PM_Q = 5;
     pdl_trigger();
     pdl_wait();
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, j = lane & 7, s0 = lane >> 3;
     const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     if (w >= np2m) return;
-    const int g = p2m[w], b = A.nbot[g], n = A.ntop[g] - b, Q = A.Q;
+    const int g = p2m[w];
     const double *m = mat + p2m_off[w];
-    for (int q0 = 0; q0 < Q; q0 += 32) {
-        const int q = q0 + lane;
-        double acc0 = 0.0, acc1 = 0.0;
-        if (q < Q) {
-            int s = 0;
-            for (; s + 1 < n; s += 2) {
-                acc0 = fma(m[(size_t)s * Q + q], A.taus[b + s], acc0);
-                acc1 = fma(m[(size_t)(s + 1) * Q + q], A.taus[b + s + 1], acc1);
-            }
-            if (s < n) acc0 = fma(m[(size_t)s * Q + q], A.taus[b + s], acc0);
-            A.uup[(size_t)g * Q + q] = acc0 + acc1;
+    const int b = A.nbot[g], n = A.ntop[g] - b, Q = A.Q;
+    for (int q0 = 0; q0 < Q; q0 += 8 * PM_Q) {
+        double acc[PM_Q] = {};
+#pragma unroll 2
+        for (int s = s0; s < n; s += 4) {
+            const double v = A.taus[b + s];
+            const double *row = m + (size_t)s * Q + q0 + j;
+#pragma unroll
+            for (int r = 0; r < PM_Q; r++)
+                if (q0 + j + 8 * r < Q) acc[r] = fma(__ldcs(row + 8 * r), v, acc[r]);
+        }
+#pragma unroll
+        for (int r = 0; r < PM_Q; r++) {
+            acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], 8);
+            acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], 16);
+            if (s0 == 0 && q0 + j + 8 * r < Q) A.uup[(size_t)g * Q + q0 + j + 8 * r] = acc[r];
         }
     }
 }
 
-// planned L2P + near field: one CTA per leaf.  The leaf's concatenated
-// charges are staged in shared memory (PL_CHUNK at a time), its u_down too;
-// each warp takes whole target rows, lanes over the row with 16-byte loads
-// (FP32 rows: products summed in FP32 per lane, then in FP64 across lanes).
-constexpr int PL_THREADS = 128, PL_CHUNK = 1024;
-template <typename T>
-__global__ void __launch_bounds__(PL_THREADS) k_planned_leaf(PassArgs A, const int32_t *__restrict__ leaves,
-                                                             int64_t nleaf, const int64_t *__restrict__ near_off,
-                                                             const int64_t *__restrict__ l2p_off,
-                                                             const T *__restrict__ near,
-                                                             const double *__restrict__ l2p) {
+constexpr int PL_ROWS = 4;
+constexpr int PL_STAGE = 4096;      // bytes of staged charges
+
+// asks for `bytes` (a multiple of 16, from a 16-byte boundary) to be brought into L2
+__device__ __forceinline__ void l2_prefetch(const void *p, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+
+// planned near field: one CTA per leaf, into pots.  The leaf's concatenated
+// charges are staged in shared memory (PL_STAGE bytes at a time); each warp takes
+// PL_ROWS target rows at a time, lanes over a row with 16-byte loads (FP32 rows:
+// products summed in FP32 per lane, then in FP64 across lanes).
+template <typename T, int THREADS>
+__global__ void __launch_bounds__(THREADS) k_planned_near(PassArgs A, const int64_t *__restrict__ near_off,
+                                                             const T *__restrict__ near) {
     constexpr int VW = 16 / sizeof(T);  // values per 16-byte load
+    constexpr int CHUNK = PL_STAGE / sizeof(T);
     extern __shared__ __align__(16) double pl_sm[];
-    T *tch = (T *)pl_sm;                                   // [PL_CHUNK] charges of the chunk
-    double *us = pl_sm + PL_CHUNK;                         // [Q] u_down of the leaf
-    double *acc = us + A.Q;                                // [n_t] per-target sums
-    __shared__ int rng[18];
-    __shared__ int s_ns;
+    T *tch = (T *)pl_sm;                                   // [CHUNK] charges of the chunk
+    double *acc = pl_sm + PL_STAGE / sizeof(double);       // [n_t] per-target sums
+    __shared__ int rec[LEAF_REC_WORDS];
     pdl_trigger();
     pdl_wait();
     const int64_t i = blockIdx.x;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = PL_THREADS / 32;
-    const int g = leaves[i], l = A.nlev[g], b = A.nbot[g], nt = A.ntop[g] - b, Q = A.Q;
-    if (tid == 0) s_ns = leaf_ranges(A, g, rng);
-    for (int q = tid; q < Q; q += PL_THREADS) us[q] = l >= 2 ? A.udown[(size_t)g * Q + q] : 0.0;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid < LEAF_REC_WORDS) rec[tid] = A.leaf_rec[i * LEAF_REC_WORDS + tid];
+    const int64_t n0 = near_off[i];
+    const int64_t sz = near_off[i + 1] - n0;
+    if (sizeof(T) == 4 && tid == 0 && sz > 0) l2_prefetch(near + n0, (uint32_t)(sz * sizeof(T)));
     __syncthreads();
-    const int ns = s_ns, nsp = (int)((near_off[i + 1] - near_off[i]) / max(nt, 1));
-    // far field: L2P rows
-    const double *lb = l2p + l2p_off[i];
-    for (int t = warp; t < nt; t += nw) {
-        double f = 0.0;
-        if (l >= 2)
-            for (int q = lane; q < Q; q += 32) f = fma(lb[(size_t)t * Q + q], us[q], f);
-        for (int o = 16; o; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
-        if (lane == 0) acc[t] = f;
-    }
-    const T *nb = near + near_off[i];
-    for (int c0 = 0; c0 < nsp; c0 += PL_CHUNK) {
-        const int cn = min(PL_CHUNK, nsp - c0);  // a multiple of VW
+    const int b = rec[LR_BOT], nt = rec[LR_TOP] - b, ns = rec[LR_NSRC];
+    const int nsp = (int)pad_row(ns, VW);
+    const T *nb = near + n0;
+    if (sz <= 0) return;  // no points
+    for (int c0 = 0; c0 < nsp; c0 += CHUNK) {
+        const int cn = min(CHUNK, nsp - c0);  // a multiple of VW
         __syncthreads();
-        for (int s = tid; s < cn; s += PL_THREADS)
-            tch[s] = c0 + s < ns ? (T)A.taus[range_point(rng, c0 + s)] : (T)0;
+        for (int s = tid; s < cn; s += THREADS)
+            tch[s] = c0 + s < ns ? (T)A.taus[range_point(rec + LR_RNG, c0 + s)] : (T)0;
         __syncthreads();
-        for (int t = warp; t < nt; t += nw) {
-            const T *row = nb + (size_t)t * nsp + c0;
-            T part = 0;
-#pragma unroll 2
+        for (int t0 = warp * PL_ROWS; t0 < nt; t0 += THREADS / 32 * PL_ROWS) {
+            const T *row[PL_ROWS];
+            T part[PL_ROWS];
+#pragma unroll
+            for (int r = 0; r < PL_ROWS; r++) {
+                row[r] = nb + (size_t)min(t0 + r, nt - 1) * nsp + c0;
+                part[r] = 0;
+            }
+#pragma unroll 1
             for (int s = lane * VW; s < cn; s += 32 * VW) {
                 if (VW == 4) {
-                    const float4 m = *(const float4 *)(row + s);
                     const float4 v = *(const float4 *)(tch + s);
-                    part = fmaf(m.x, v.x, fmaf(m.y, v.y, fmaf(m.z, v.z, fmaf(m.w, v.w, part))));
+#pragma unroll
+                    for (int r = 0; r < PL_ROWS; r++) {
+                        const float4 m = __ldcs((const float4 *)(row[r] + s));
+                        part[r] = fmaf(m.x, v.x, fmaf(m.y, v.y, fmaf(m.z, v.z, fmaf(m.w, v.w, part[r]))));
+                    }
                 } else {
-                    const double2 m = *(const double2 *)(row + s);
                     const double2 v = *(const double2 *)(tch + s);
-                    part = fma(m.x, v.x, fma(m.y, v.y, part));
+#pragma unroll
+                    for (int r = 0; r < PL_ROWS; r++) {
+                        const double2 m = __ldcs((const double2 *)(row[r] + s));
+                        part[r] = fma(m.x, v.x, fma(m.y, v.y, part[r]));
+                    }
                 }
             }
-            double d = (double)part;
-            for (int o = 16; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-            if (lane == 0) acc[t] += d;
+            double d[PL_ROWS];
+#pragma unroll
+            for (int r = 0; r < PL_ROWS; r++) d[r] = (double)part[r];
+            for (int o = 16; o; o >>= 1)
+#pragma unroll
+                for (int r = 0; r < PL_ROWS; r++) d[r] += __shfl_xor_sync(0xffffffffu, d[r], o);
+#pragma unroll
+            for (int r = 0; r < PL_ROWS; r++)
+                if (lane == r && t0 + r < nt) acc[t0 + r] = (c0 ? acc[t0 + r] : 0.0) + d[r];
         }
     }
     __syncthreads();
-    for (int t = tid; t < nt; t += PL_THREADS) A.out[A.perm[b + t]] = acc[t];
+    for (int t = tid; t < nt; t += THREADS) A.pots[b + t] = acc[t];
+}
+
+// planned L2P: one CTA per leaf, eight lanes per row; adds the near field in pots
+// and writes the potentials in the caller's order
+template <int THREADS>
+__global__ void __launch_bounds__(THREADS) k_planned_far(PassArgs A, const int64_t *__restrict__ l2p_off,
+                                                            const double *__restrict__ l2p) {
+    pdl_trigger();
+    pdl_wait();
+    const int64_t i = blockIdx.x;
+    const int j = threadIdx.x & 7, Q = A.Q;
+    const int32_t *rec = A.leaf_rec + i * LEAF_REC_WORDS;
+    const double *lb = l2p + l2p_off[i];
+    const int g = rec[LR_NODE], l = rec[LR_LEVEL], b = rec[LR_BOT], nt = rec[LR_TOP] - b;
+    const double *u = A.udown + (size_t)g * Q;
+    for (int t0 = 0; t0 < nt; t0 += THREADS / 8) {
+        const int t = t0 + (threadIdx.x >> 3);
+        const bool in = t < nt, wr = in && j == 0;
+        const double near = wr ? A.pots[b + t] : 0.0;
+        const int32_t to = wr ? A.perm[b + t] : 0;
+        double f = 0.0;
+        if (l >= 2 && in) {
+            const double *row = lb + (size_t)t * Q;
+#pragma unroll 3
+            for (int q = j; q < Q; q += 8) f = fma(__ldcs(row + q), u[q], f);
+        }
+        for (int o = 4; o; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
+        if (wr) A.out[to] = near + f;
+    }
 }
 
 // ------------------------------------------------------------ host side
@@ -286,20 +338,40 @@ void launch_planned_p2m(kifmm_plan *P, const PassArgs &A) {
                (const double *)P->pm_p2m.p);
 }
 
-void launch_planned_leaf(kifmm_plan *P, const PassArgs &A) {
-    const dim3 grid((unsigned)P->n_leaf_list), block(PL_THREADS);
-    const size_t smem = (size_t)(PL_CHUNK + P->Q + P->ppl) * sizeof(double);  // leaves hold <= Ncutoff points
-    if (P->opt.precision == KIFMM_PREC_MIXED) {
-        ensure_dyn_smem(k_planned_leaf<float>, smem);
-        launch_pdl(k_planned_leaf<float>, grid, block, smem, P->stream, A, (const int32_t *)P->leaf_list.p,
-                   P->n_leaf_list, (const int64_t *)P->pm_near_off.p, (const int64_t *)P->pm_l2p_off.p,
-                   (const float *)P->pm_near32.p, (const double *)P->pm_l2p.p);
-    } else {
-        ensure_dyn_smem(k_planned_leaf<double>, smem);
-        launch_pdl(k_planned_leaf<double>, grid, block, smem, P->stream, A, (const int32_t *)P->leaf_list.p,
-                   P->n_leaf_list, (const int64_t *)P->pm_near_off.p, (const int64_t *)P->pm_l2p_off.p,
-                   (const double *)P->pm_near64.p, (const double *)P->pm_l2p.p);
-    }
+// Threads of a leaf's block: 64, so that many small blocks keep loads in flight
+// while others stage their charges or reduce (500k points, lists of 250: the near
+// pass 157 us, 175 with 128 threads); 256 where there are too few leaves to fill
+// the GPU and a leaf's own time counts (10k points: an apply 52 us, 90 with 64).
+template <typename T, int THREADS>
+static void launch_near(kifmm_plan *P, cudaStream_t s, const T *mat) {
+    const size_t smem = PL_STAGE + (size_t)P->ppl * sizeof(double);  // leaves hold <= Ncutoff points
+    ensure_dyn_smem(k_planned_near<T, THREADS>, smem);
+    launch_pdl(k_planned_near<T, THREADS>, dim3((unsigned)P->n_leaf_list), dim3(THREADS), smem, s, make_pass_args(P),
+               (const int64_t *)P->pm_near_off.p, mat);
+}
+template <int THREADS>
+static void launch_near(kifmm_plan *P, cudaStream_t s) {
+    if (P->opt.precision == KIFMM_PREC_MIXED) launch_near<float, THREADS>(P, s, P->pm_near32.p);
+    else launch_near<double, THREADS>(P, s, P->pm_near64.p);
+}
+
+// the near field into pots, on stream s
+void launch_planned_near(kifmm_plan *P, cudaStream_t s) {
+    if (near_split(P)) launch_near<256>(P, s);
+    else launch_near<64>(P, s);
+}
+
+// the potentials at the sources: the near field, unless it is under way on its own
+// stream, then the far field added to it
+void run_planned_leaf(kifmm_plan *P, const PassArgs &A) {
+    if (P->near_pending) near_join(P);
+    else launch_planned_near(P, P->stream);
+    auto far = [&](auto kern, int threads) {
+        launch_pdl(kern, dim3((unsigned)P->n_leaf_list), dim3(threads), 0, P->stream, A,
+                   (const int64_t *)P->pm_l2p_off.p, (const double *)P->pm_l2p.p);
+    };
+    if (near_split(P)) far(k_planned_far<256>, 256);
+    else far(k_planned_far<64>, 64);
 }
 
 }  // namespace kifmm

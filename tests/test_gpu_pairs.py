@@ -264,3 +264,40 @@ def test_one_leaf_k0_mixed(k, n):
     r = np.hypot(x[:, None] - x[None, :], y[:, None] - y[None, :])
     r[r == 0] = 1
     assert np.all(np.abs(pot - ref) <= 50 * 2.0 ** -23 * (mag + (1 / r) @ np.abs(tau)))
+
+
+@pytest.mark.parametrize("n,cutoff", [(1, 5), (2, 5), (33, 64), (300, 300), (511, 512), (2000, 700), (1500, 1025)])
+@pytest.mark.parametrize("kind,k", [("laplace", 0.0), ("k0", 3.0)])
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_planned_near_field(precision, kind, k, n, cutoff):
+    """Trees of one or two levels have no far field: the planned apply is the near
+    matrices alone, with rows on both sides of the staged charges' length.  FP32
+    rows: charge and matrix value rounded once each, at most 65 products a lane."""
+    x, y, tau = cloud(n, n + 1)
+    f = fmm(kind, k, x, y, cutoff, precision=precision, planned=True)
+    assert f.tree_info().levels <= 2
+    f.build_expansions(tau)
+    ref, mag = direct(kind, k, x, y, tau)
+    bound = (n + 16) * EPS * mag if precision == "fp64" else 70 * 2.0 ** -23 * mag
+    for _ in range(2):
+        assert np.all(np.abs(f.evaluate_to_points(x, y, True) - ref) <= bound)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("n,cutoff", [(900, 9), (90000, 20)])
+def test_planned_near_field_under_way(precision, n, cutoff):
+    """The planned near pass starts with the apply: evaluations that use it, that do
+    not (self pairs kept, or other targets), and applies never evaluated."""
+    x, y, tau = cloud(n, 5)
+    f = fmm("laplace", 0.0, x, y, cutoff, precision=precision, planned=True)
+    f.build_expansions(tau)
+    a = f.evaluate_to_points(x, y, True)
+    f.build_expansions(-tau)
+    f.build_expansions(tau)
+    other = f.evaluate_to_points(x[:50] + 1e-3, y[:50], False)
+    self_pairs = f.evaluate_to_points(x, y, False)
+    assert np.all(np.isfinite(other)) and (precision == "mixed" or np.all(np.isinf(self_pairs)))
+    b = f.evaluate_to_points(x, y, True)
+    f.build_expansions(tau)
+    np.testing.assert_array_equal(a, b)
+    np.testing.assert_array_equal(a, f.evaluate_to_points(x, y, True))
