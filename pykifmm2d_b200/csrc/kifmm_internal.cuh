@@ -509,6 +509,7 @@ cudaStream_t device_side_stream(int device);  // one per device, created on firs
 void join_operators(kifmm_plan *P);   // main stream waits for it
 void ops_wait_now(kifmm_plan *P);     // issue a deferred join's stream wait (before any operator is read)
 void ops_wait_circles(kifmm_plan *P); // ... for the check circles only (before the P2M)
+bool near_under_way(kifmm_plan *P);   // passes_mixed.cu: an evaluation may wait for a near-field pass in flight
 void near_join(kifmm_plan *P);        // main stream waits for a near-field pass in flight, which is dropped
 bool near_possible(kifmm_plan *P);    // passes_mixed.cu: whether the apply runs the near field on its own stream
 bool near_split(const kifmm_plan *P); // passes_mixed.cu: ... and does so from the start of the apply (few leaves)

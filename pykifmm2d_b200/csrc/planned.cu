@@ -364,7 +364,7 @@ void launch_planned_near(kifmm_plan *P, cudaStream_t s) {
 // the potentials at the sources: the near field, unless it is under way on its own
 // stream, then the far field added to it
 void run_planned_leaf(kifmm_plan *P, const PassArgs &A) {
-    if (P->near_pending) near_join(P);
+    if (near_under_way(P)) near_join(P);
     else launch_planned_near(P, P->stream);
     auto far = [&](auto kern, int threads) {
         launch_pdl(kern, dim3((unsigned)P->n_leaf_list), dim3(threads), 0, P->stream, A,

@@ -301,3 +301,33 @@ def test_planned_near_field_under_way(precision, n, cutoff):
     f.build_expansions(tau)
     np.testing.assert_array_equal(a, b)
     np.testing.assert_array_equal(a, f.evaluate_to_points(x, y, True))
+
+
+@pytest.mark.parametrize("n,cutoff", [(900, 9), (90000, 20)])
+@pytest.mark.parametrize("precision,planned", [("fp64", True), ("mixed", True), ("mixed", False)])
+def test_evaluation_in_a_callers_capture(precision, planned, n, cutoff):
+    """A capture that the caller begins after the apply holds the evaluation alone: it
+    cannot wait for a near pass that is under way, and replays on later densities."""
+    import torch
+    x, y, tau = (torch.as_tensor(v, device="cuda") for v in cloud(n, 8))
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    f = fmm("laplace", 0.0, x, y, cutoff, precision=precision, planned=planned, stream=stream.cuda_stream)
+    pot, ref = torch.zeros_like(tau), torch.zeros_like(tau)
+    f.build_expansions(tau)
+    f.evaluate_to_points(x, y, True, out=ref)
+    f.synchronize()
+    f.build_expansions(tau)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=stream):
+        f.evaluate_to_points(x, y, True, out=pot)
+    with torch.cuda.stream(stream):
+        g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(pot, ref)
+    f.build_expansions(tau.flip(0).contiguous())
+    f.evaluate_to_points(x, y, True, out=ref)
+    with torch.cuda.stream(stream):
+        g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(pot, ref)
