@@ -189,8 +189,8 @@ def time_full_steps(torch, cfg, xd, yd, td, precision, steps, warmup, flush, pro
 
 
 def leaf_alone_ms(torch, f, xd, yd, flush, reps=3):
-    """Event-timed leaf phase (Taylor coefficients + the single-pass L2P + P2P
-    kernel) of evaluations at the sources on the plan's current expansions."""
+    """Event-timed leaf phase (near pass, Taylor coefficients, far pass, one after
+    the other) of evaluations at the sources on the plan's current expansions."""
     from pykifmm2d_b200 import _lib as B
     lib = B.load()
     out = torch.empty_like(xd)
@@ -283,7 +283,7 @@ def measured_traffic():
 
 
 def build_rooflines(cfg, info, phase, precision, pk, pk_src, n):
-    """Rooflines of the dominant kernel (the leaf L2P+P2P kernel), of the
+    """Rooflines of the dominant kernels (the leaf L2P and P2P), of the
     tensor-core M2L and of the Morton radix sort, from the phase timers
     (CUDA events on the plan's stream, averaged over the timed steps)."""
     from pykifmm2d_b200 import _lib as B
@@ -299,9 +299,9 @@ def build_rooflines(cfg, info, phase, precision, pk, pk_src, n):
     if t > 0:
         peak = fp32_peak if precision == "mixed" else fp64_peak
         ach = fl / t / 1e12
-        name = "k_leaf_eval_f" if precision == "mixed" else "k_leaf_eval_d"
+        name = "k_leaf_near_f" if precision == "mixed" else "k_leaf_eval_d"
         out["dominant"] = {
-            "kernel": name + " (P2P + L2P, one launch per step)", "bound": "fp32" if precision == "mixed" else "fp64",
+            "kernel": "k_leaf_near_f (P2P) + k_leaf_far_taylor (L2P)" if precision == "mixed" else name + " (P2P + L2P)", "bound": "fp32" if precision == "mixed" else "fp64",
             "achieved": ach, "peak": peak, "unit": "TFLOP/s", "frac": ach / peak,
             "traffic": traffic.get(name),
             "work": f"{pairs:.4g} P2P pairs x {p2p_flops_per_pair(cfg['kernel']):.0f} flops per launch",
@@ -329,7 +329,7 @@ def build_rooflines(cfg, info, phase, precision, pk, pk_src, n):
                        "frac": ach / pk["hbm_gbs"], "traffic": traffic.get("k_os_pass"),
                        "work": "52 B per point: the algorithmic minimum of sorting the points (read x, y, tau; "
                                "write them sorted with an int32 index)",
-                       "executed_bytes": 4 * 36.0 * n,
+                       "executed_bytes": (24.0 + 8 + 4 * 16 + 4) * n,
                        "peak_source": pk_src}
     out["composite"] = composite_roofline(cfg, info, ph, precision, pk, pk_src, n)
     return out
@@ -405,8 +405,8 @@ def run_ours(args, cfg, rank, world, dist):
     _, _, phase, _, _ = time_full_steps(torch, cfg, xd, yd, td, precision, 3, 1, flush, profile=True)
     # In a step the near field at the sources runs under the far-field chain,
     # sharing the SMs, so its phase time is not the kernel's own: the leaf
-    # kernel alone (near + far field in one pass, a second evaluation on the
-    # same expansions) is timed for the roofline.
+    # kernels alone (near, then far field, a second evaluation on the same
+    # expansions) are timed for the roofline.
     leaf_alone = leaf_alone_ms(torch, f, xd, yd, flush)
     tot = float(sum(times))
     if dist is not None:
@@ -464,7 +464,7 @@ def run_ours(args, cfg, rank, world, dist):
     rooflines = build_rooflines(cfg, info, ph_roof, precision, pk, pk_src, n)
     if "dominant" in rooflines:
         rooflines["dominant"]["timing"] = (
-            "leaf kernel alone: event-timed single-pass evaluation at the sources on the step's expansions "
+            "leaf kernels alone: event-timed second evaluation at the sources on the step's expansions "
             f"({leaf_alone:.4f} ms, Taylor coefficients included); in the timed steps its near-field part runs "
             "on a low-priority stream under the far-field chain (phases_ms.leaf counts it there)")
     line = {
@@ -583,7 +583,7 @@ def run_c4(torch, flush):
             t = line["phases_ms"]["leaf"] * 1e-3
             ach = float(info.n_p2p_pairs) * 40.0 / t / 1e12 if t > 0 else None
             out["roofline_k0_p2p"] = {
-                "kernel": "k_leaf_eval_f<K0> (P2P + L2P)", "bound": "fp32", "achieved": ach, "peak": peak,
+                "kernel": "k_leaf_near_f<K0> (P2P) + k_leaf_eval_d<K0> (L2P)", "bound": "fp32", "achieved": ach, "peak": peak,
                 "unit": "TFLOP/s", "frac": ach / peak if ach else None,
                 "work": f"{info.n_p2p_pairs} P2P pairs x 40 flops (K0 series) per launch",
                 "peak_source": f"SIMT peak at sm_max_mhz ({pk_src})"}
@@ -645,7 +645,7 @@ def run_planned(torch, flush, steps=5):
                     leaf_bytes = float(info.n_p2p_pairs) * nb + 8.0 * cfg["neq"] * x.size + 24.0 * x.size
                     ach = leaf_bytes / (ph["leaf"] * 1e-3) / 1e9 if ph["leaf"] > 0 else None
                     line[key].update({"matrix_bytes": int(info.planned_bytes),
-                                      "roofline_leaf": {"kernel": "k_planned_leaf (L2P + near field as matrices)",
+                                      "roofline_leaf": {"kernel": "k_planned_near + k_planned_far (near field and L2P as matrices)",
                                                         "bound": "hbm", "achieved": ach, "peak": pk["hbm_gbs"],
                                                         "unit": "GB/s", "frac": ach / pk["hbm_gbs"] if ach else None,
                                                         "work": f"{nb} B per near-field pair + 8 Q B per point "

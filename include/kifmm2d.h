@@ -63,7 +63,7 @@ typedef struct kifmm_kernel {
 /* Arithmetic of the evaluation passes. */
 enum {
     KIFMM_PREC_FP64 = 0,  /* every pass in FP64 ("plain") */
-    KIFMM_PREC_MIXED = 1  /* FP32 near field and P2M/L2P, compensated M2L */
+    KIFMM_PREC_MIXED = 1  /* FP32 near field, FP64 P2M, M2M, L2L, sliced M2L, L2P FP64 with FP32 high orders */
 };
 /* M2L form used with KIFMM_PREC_MIXED. */
 enum {
@@ -187,8 +187,8 @@ int kifmm_graph_launch(kifmm_plan *plan);
 
 /* Packed applies of several plans (a serving batch): the same pair as
  * kifmm_graph_capture for plans[0..nplan), with the M2L of all plans in ONE
- * tensor-core launch and the near field + L2P of all plans in one launch per
- * kernel kind; the per-plan passes (P2M, M2M, L2L, gathers) run as parallel
+ * tensor-core launch and the near field of all plans in one launch per kernel
+ * kind; the per-plan passes (P2M, M2M, L2L, L2P, gathers) run as parallel
  * branches of the graph.  Each plan's result is the same as its own apply
  * (the packed kernels run the same per-tile / per-leaf code on that plan's
  * data).  kifmm_batch_capture first runs one normal apply
