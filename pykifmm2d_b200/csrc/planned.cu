@@ -341,7 +341,7 @@ void launch_planned_p2m(kifmm_plan *P, const PassArgs &A) {
 // Threads of a leaf's block: 64, so that many small blocks keep loads in flight
 // while others stage their charges or reduce (500k points, lists of 250: the near
 // pass 157 us, 175 with 128 threads); 256 where there are too few leaves to fill
-// the GPU and a leaf's own time counts (10k points: an apply 52 us, 90 with 64).
+// the GPU and a leaf's own time counts (10k points: an apply 55 us, 90 with 64).
 template <typename T, int THREADS>
 static void launch_near(kifmm_plan *P, cudaStream_t s, const T *mat) {
     const size_t smem = PL_STAGE + (size_t)P->ppl * sizeof(double);  // leaves hold <= Ncutoff points

@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_os_hist(const uint64_t *__restri
 // What bounds it: the ranking's ballots (8 per key and warp; the ALU pipe is busy
 // 67% of a 4M-key pass), then latency.  Two blocks of 16 warps per SM: with 8 warps
 // of twice the keys each the chain of a warp's ranking steps was exposed (4M keys
-// and values: 73 us a pass, now 44 for words; 1M 23 -> 17.5, 300k 18.7 -> 9.2).
+// and values: 73 us a pass, now 44 for words; 1M 23 -> 17.5, 300k 18.7 -> 10.6).
 // Look-back words are 32 bits, and a block reads them with all its threads.
 constexpr int OS_THREADS = 512;
 constexpr int OS_WARPS = OS_THREADS / 32;
@@ -399,12 +399,11 @@ static void os_run(uint64_t *key, int32_t *val, uint64_t *key_tmp, int32_t *val_
     KIFMM_REQUIRE(n < (1ll << 31), KIFMM_ERR_ARG, "radix sort: more than 2^31 keys");
     KIFMM_REQUIRE(npass <= OS_MAX_PASSES, KIFMM_ERR_ARG, "radix sort: too many passes");
     cudaStream_t s = P->stream;
-    // keys per thread: 4 while a tile per SM holds them all (300k: a pass 9.2 us, 12.5
-    // with 8), 8 while two do (1M: the tree 22 us shorter than with 16, as with 4),
-    // then 16 (4M: 18 us shorter than with 8, 52 than with 4).  Pairs, which need
-    // more registers, stay at 8.
-    const int64_t wave = (int64_t)P->num_sms * OS_THREADS;
-    const int items = n <= 4 * wave ? 4 : n <= 16 * wave || mode == OS_PAIRS ? 8 : 16;
+    // keys per thread: 8 while two tiles per SM hold them all (1M: the tree 21 us
+    // shorter than with 16), then 16 (4M: 18 us shorter than with 8).  4 keys make a
+    // pass of 300k 9.2 instead of 10.6 us and no call shorter; at 4M they cost 52 us.
+    // Pairs, which need more registers, stay at 8.
+    const int items = n <= 16 * (int64_t)P->num_sms * OS_THREADS || mode == OS_PAIRS ? 8 : 16;
     const int64_t tile = OS_THREADS * items, ntiles = (n + tile - 1) / tile;
     OsShifts sh{};
     sh.n = npass;
@@ -437,9 +436,9 @@ static void os_run(uint64_t *key, int32_t *val, uint64_t *key_tmp, int32_t *val_
                                                                sh.s[p], unpack, hist + 256 * p, stat, ctr + p);
         };
         auto size = [&](auto m) {
-            if (items == 4) go(m, std::integral_constant<int, 4>{});
-            else if (items == 8 || decltype(m)::value == OS_PAIRS) go(m, std::integral_constant<int, 8>{});
-            else go(m, std::integral_constant<int, decltype(m)::value == OS_PAIRS ? 8 : 16>{});
+            constexpr int WIDE = decltype(m)::value == OS_PAIRS ? 8 : 16;
+            if (items == 8) go(m, std::integral_constant<int, 8>{});
+            else go(m, std::integral_constant<int, WIDE>{});
         };
         if (mode == OS_PAIRS) size(std::integral_constant<int, OS_PAIRS>{});
         else if (mode == OS_UNPACK && last) size(std::integral_constant<int, OS_UNPACK>{});

@@ -1,4 +1,4 @@
-"""The tree's point sort at the edges of its tiles (2048, 4096 and 8192 words), of a
+"""The tree's point sort at the edges of its tiles (4096 and 8192 words), of a
 look-back group (32 tiles) and of the point counts where the tile size changes: each
 point must come out in the leaf whose cell holds it, and each leaf hold its count."""
 import numpy as np
