@@ -62,6 +62,16 @@ struct PairSum {
     }
 };
 
+// Whether a target's r^2 to a source may be infinite or not a number.  The
+// unchecked Laplace loop, which looks for small r^2 only, would take such a pair
+// for an ordinary one.  Sources are checked when the tree is built; separate
+// targets are anything.
+template <int KIND>
+__device__ __forceinline__ bool out_of_reach(double x, double y) {
+    constexpr double REACH = 0x1p500;  // r^2 stays below 2^1002
+    return KIND == KIFMM_KERNEL_LAPLACE && !(fabs(x) < REACH && fabs(y) < REACH);
+}
+
 // Sums of the lane's TB targets over sources u, u + sp, ... below n.  CHECKED
 // tests each pair and gives those that the fast value is not for to the math
 // library (coincident pairs are left out with skip_equal); without it the
@@ -72,7 +82,7 @@ __device__ __forceinline__ bool pair_loop(const PairWarp<KIND, CPLX> &W, const d
                                           const double *tx, const double *ty, double k, double k2, unsigned hi_end,
                                           bool skip_equal, PairSum<KIND, CPLX> *acc) {
     unsigned worst = 0;      // largest rank (K0, H0)
-    int least = 0x7fffffff;  // smallest high word (Laplace: r^2 is finite)
+    int least = 0x7fffffff;  // smallest high word (Laplace: r^2 is finite, see out_of_reach)
 #pragma unroll 1
     for (; u < n; u += sp) {
         const double2 s = W.xy[u];
@@ -208,15 +218,19 @@ __device__ __forceinline__ PairSum<KIND, CPLX> leaf_item(const PassArgs &A, Pair
     const int ng = (nt + TB - 1) / TB, sp = 32 / ng, j = lane / ng, gi = lane - j * ng;
     double tx[TB], ty[TB];
     PairSum<KIND, CPLX> acc[TB];
+    bool wild = false;  // a separate target out of the unchecked loop's reach
 #pragma unroll
     for (int a = 0; a < TB; a++) {
         int i = I.t0 + (gi + a * ng < nt ? gi + a * ng : gi);  // unused slots repeat the first
         if (I.idx) i = I.idx[i];
         tx[a] = I.tx[i];
         ty[a] = I.ty[i];
+        if (I.idx) wild = wild || out_of_reach<KIND>(tx[a], ty[a]);
 #pragma unroll
         for (int c = 0; c < NC; c++) acc[a].c[c] = 0.0;
     }
+    if (I.idx) wild = __any_sync(0xffffffffu, wild);
+    const int n_own = wild ? I.ns : I.n_own;
     const int u0 = j < sp ? j : 1 << 20;  // lanes past the last group idle
     for (int c0 = 0; !FAR && c0 < I.ns; c0 += L64_CHUNK) {
         const int cn = min(L64_CHUNK, I.ns - c0);
@@ -230,7 +244,7 @@ __device__ __forceinline__ PairSum<KIND, CPLX> leaf_item(const PassArgs &A, Pair
             }
         }
         __syncwarp();
-        pair_chunk<KIND, CPLX, NT, TB, BEYOND>(W, tl, u0, sp, min(I.n_own - c0, cn), cn, tx, ty, A.k, I.k2, hi_end,
+        pair_chunk<KIND, CPLX, NT, TB, BEYOND>(W, tl, u0, sp, min(n_own - c0, cn), cn, tx, ty, A.k, I.k2, hi_end,
                                                I.check_self, acc);
     }
     if (I.l >= 2) {
@@ -247,7 +261,7 @@ __device__ __forceinline__ PairSum<KIND, CPLX> leaf_item(const PassArgs &A, Pair
             tx[a] -= I.cx;
             ty[a] -= I.cy;
         }
-        pair_chunk<KIND, CPLX, NT, TB, BEYOND>(W, tl, u0, sp, 0, Qc, tx, ty, A.k, I.k2, hi_end, false, acc);
+        pair_chunk<KIND, CPLX, NT, TB, BEYOND>(W, tl, u0, sp, wild ? Qc : 0, Qc, tx, ty, A.k, I.k2, hi_end, false, acc);
     }
     __syncwarp();
 #pragma unroll

@@ -299,11 +299,13 @@ __device__ __forceinline__ void target_item_f(const PassArgs &A, const TargetArg
     const int ns = warp_ranges(A, J.g, false, W.rng, lane);
     double tx[TB], ty[TB];
     float rx[TB], ry[TB], acc[TB];
+    bool wild = false;
 #pragma unroll
     for (int a = 0; a < TB; a++) {
         const int i = T.order[J.start + min(lane + 32 * a, J.n - 1)];  // lanes past the end repeat the last target
         tx[a] = T.tx[i] - cx;
         ty[a] = T.ty[i] - cy;
+        wild = wild || out_of_reach<KIND>(tx[a], ty[a]);
         rx[a] = (float)tx[a];
         ry[a] = (float)ty[a];
         acc[a] = 0.f;
@@ -319,7 +321,8 @@ __device__ __forceinline__ void target_item_f(const PassArgs &A, const TargetArg
         __syncwarp();
         const double wl = ldexp(A.W, -J.level), k2 = A.k * A.k, tmax = 4.0 * wl * wl * k2;  // r < 2 w inside the box
         if (KIND == KIFMM_KERNEL_LAPLACE)
-            pair_chunk<KIND, false, 1, TB, false>(W, tl, 0, 1, 0, A.Q, tx, ty, A.k, k2, LOG_HI_END, false, far);
+            pair_chunk<KIND, false, 1, TB, false>(W, tl, 0, 1, wild ? A.Q : 0, A.Q, tx, ty, A.k, k2, LOG_HI_END, false,
+                                                  far);
         else if (tmax < 0.0625)
             pair_chunk<KIND, false, SERIES_NARROW, TB, false>(W, tl, 0, 1, 0, A.Q, tx, ty, A.k, k2, SERIES_NARROW_HI,
                                                               false, far);
