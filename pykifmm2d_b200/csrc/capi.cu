@@ -559,6 +559,7 @@ int kifmm_graph_launch(kifmm_plan *P) {
         KIFMM_REQUIRE(P, KIFMM_ERR_ARG, "null plan");
         KIFMM_REQUIRE(P->graph, KIFMM_ERR_STATE, "graph launch: call kifmm_graph_capture first");
         use_device(P);
+        near_join(P);  // an apply never evaluated: its near pass reads and writes what the graph does
         KIFMM_CUDA(cudaGraphLaunch(P->graph, P->stream));
     });
 }
@@ -985,6 +986,11 @@ int kifmm_batch_launch(kifmm_batch *B) {
     return guarded([&] {
         KIFMM_REQUIRE(B && B->graph, KIFMM_ERR_ARG, "batch launch: no captured batch");
         KIFMM_CUDA(cudaSetDevice(B->device));
+        for (auto *P : B->plans)  // near passes of applies never evaluated, as in kifmm_graph_launch
+            if (P->near_pending) {
+                KIFMM_CUDA(cudaStreamWaitEvent(B->stream, P->near_done, 0));
+                P->near_pending = false;
+            }
         KIFMM_CUDA(cudaGraphLaunch(B->graph, B->stream));
     });
 }

@@ -51,3 +51,86 @@ def test_targets_anywhere(kind, k, iscomplex, precision):
     n_pairs = 9 * 40 + 24
     scale = np.abs(ref).max() + np.abs(tau).sum()
     assert np.abs(pot[12:] - ref).max() <= n_pairs * EPS * scale
+
+
+# (points, Ncutoff): a tree whose near pass starts with the apply, one whose near
+# pass starts after the M2M chain, and one with leaves above level 2
+TREES = [(900, 9), (90000, 20), (-52, 20)]
+
+
+def lopsided(n, seed):
+    """n < 0: a few points in three quadrants (leaves of level 1), the others in the
+    fourth (leaves of level 2, the only ones with a far field)"""
+    x, y, tau = cloud(abs(n), seed)
+    if n < 0:
+        x[12:], y[12:] = np.abs(x[12:]), np.abs(y[12:])
+        x[:4], y[:4] = -np.abs(x[:4]), -np.abs(y[:4])
+        x[4:8], y[4:8] = -np.abs(x[4:8]), np.abs(y[4:8])
+        x[8:12], y[8:12] = np.abs(x[8:12]), -np.abs(y[8:12])
+    return x, y, tau
+
+
+def on_device(*arrays):
+    import torch
+    return [torch.as_tensor(v, device="cuda") for v in arrays]
+
+
+@pytest.mark.parametrize("n,cutoff", TREES)
+@pytest.mark.parametrize("kind,precision,planned", [("laplace", "mixed", False), ("k0", "mixed", False),
+                                                    ("laplace", "fp64", True), ("laplace", "mixed", True)])
+def test_replay_after_an_apply_never_evaluated(kind, precision, planned, n, cutoff):
+    """The near pass of an apply may still be under way when a graph of the same plan
+    is launched; the evaluation that follows is of the graph's densities."""
+    import torch
+    x, y, tau, other = on_device(*lopsided(n, 8), np.random.default_rng(9).standard_normal(abs(n)))
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    f = fmm(kind, 2.0, x, y, cutoff, precision=precision, planned=planned, stream=stream.cuda_stream)
+    if n < 0:
+        nodes, _ = f.export_tree()
+        assert np.any((nodes[:, 0] == 1) & (nodes[:, 3] == 1) & (nodes[:, 6] > 0))
+    pot, at = torch.zeros_like(tau), torch.zeros_like(tau)
+    f.capture_apply(tau, pot, True)
+    f.replay()
+    f.synchronize()
+    ref = pot.clone()
+    elsewhere = x[:5] + 1e-3, y[:5].clone()
+    for look in (False, True):
+        pot.zero_()
+        torch.cuda.synchronize()
+        f.build_expansions(other)
+        if look:
+            f.evaluate_to_points(*elsewhere, False)
+        f.replay()
+        f.evaluate_to_points(x, y, True, out=at)
+        f.synchronize()
+        assert torch.equal(pot, ref) and torch.equal(at, ref)
+
+
+@pytest.mark.parametrize("n,cutoff", TREES)
+@pytest.mark.parametrize("kind", ["laplace", "k0"])
+def test_batch_after_an_apply_never_evaluated(kind, n, cutoff):
+    import torch
+    from pykifmm2d_b200.serving import PackedBatch
+    x, y, tau, other = on_device(*lopsided(n, 8), np.random.default_rng(9).standard_normal(abs(n)))
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    # every plan on the batch's stream, so that only the near passes run beside it
+    fs = [fmm(kind, 2.0, x, y, cutoff, precision="mixed", stream=stream.cuda_stream) for _ in range(2)]
+    taus, pots = [tau, other.clone()], [torch.zeros_like(tau) for _ in range(2)]
+    batch = PackedBatch(fs, taus, pots, stream)
+    batch.launch()
+    batch.synchronize()
+    refs = [p.clone() for p in pots]
+    at = torch.zeros_like(tau)
+    for p in pots:
+        p.zero_()
+    torch.cuda.synchronize()
+    for f in fs:
+        f.build_expansions(other)
+    batch.launch()
+    fs[0].evaluate_to_points(x, y, True, out=at)
+    batch.synchronize()
+    fs[0].synchronize()
+    assert all(torch.equal(p, r) for p, r in zip(pots, refs)) and torch.equal(at, refs[0])
+    batch.close()
