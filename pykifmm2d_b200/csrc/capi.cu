@@ -448,6 +448,8 @@ int kifmm_build_expansions(kifmm_plan *P, const double *tau, int32_t mem) {
         P->have_expansions = false;
         set_tau(P, tau, P->cplx ? 2 * P->N : P->N, mem);
         run_upward_downward(P);
+        if (P->callers_graph && P->near_pending)  // joined here (kept pending): a caller's graph may be replayed next
+            KIFMM_CUDA(cudaStreamWaitEvent(P->stream, P->near_done, 0));
         P->have_expansions = true;
     });
 }

@@ -159,6 +159,7 @@ struct kifmm_plan {
     cudaStream_t far_stream = nullptr;
     cudaEvent_t far_fork = nullptr, far_done = nullptr;
     bool own_capture = false;  // kifmm_graph_capture is recording (both halves of an apply: streams forked are joined)
+    bool callers_graph = false;  // a caller's graph may hold work of this plan (passes_mixed.cu: callers_capture)
     bool near_pending = false;  // P->pots holds the near field of the last apply, far field not added yet
     cudaEvent_t ops_fork = nullptr, ops_done = nullptr;
     cudaEvent_t ops_circ = nullptr;  // side stream: the check circles are written (the P2M's only operator input)
@@ -511,6 +512,7 @@ void ops_wait_now(kifmm_plan *P);     // issue a deferred join's stream wait (be
 void ops_wait_circles(kifmm_plan *P); // ... for the check circles only (before the P2M)
 bool near_under_way(kifmm_plan *P);   // passes_mixed.cu: an evaluation may wait for a near-field pass in flight
 void near_join(kifmm_plan *P);        // main stream waits for a near-field pass in flight, which is dropped
+bool callers_capture(kifmm_plan *P);  // passes_mixed.cu: the plan's stream is in a capture of the caller's
 bool near_possible(kifmm_plan *P);    // passes_mixed.cu: whether the apply runs the near field on its own stream
 bool near_split(const kifmm_plan *P); // passes_mixed.cu: ... and does so from the start of the apply (few leaves)
 void near_fork(kifmm_plan *P);        // passes_mixed.cu: starts it there

@@ -857,18 +857,25 @@ void ensure_aux_streams(kifmm_plan *P) {
         KIFMM_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
 }
 
+// Whether the plan's stream is in a capture of the caller's.  A plan that was in one
+// is marked: the caller may replay that graph at any time, without a call into this
+// library that could join a near pass, so the plan's later applies join theirs.
+bool callers_capture(kifmm_plan *P) {
+    if (P->own_capture) return false;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    KIFMM_CUDA(cudaStreamIsCapturing(P->stream, &cap));
+    if (cap == cudaStreamCaptureStatusNone) return false;
+    P->callers_graph = true;
+    return true;
+}
+
+// options with a near pass apart from the leaf pass
+static bool near_form(const kifmm_plan *P) {
+    return !P->cplx && (P->opt.planned || (P->opt.precision == KIFMM_PREC_MIXED && !P->opt.near_fp64));
+}
 bool near_possible(kifmm_plan *P) {
-    const int64_t nl = P->n_leaf_list;
-    if (P->cplx || nl <= 0 || (P->opt.planned != 0) != planned_ready(P)) return false;
-    if (!P->opt.planned) {
-        if (P->opt.precision != KIFMM_PREC_MIXED || P->opt.near_fp64) return false;
-        if (P->kern.kind != KIFMM_KERNEL_LAPLACE && P->kern.kind != KIFMM_KERNEL_MOD_HELMHOLTZ) return false;
-    }
-    if (!P->own_capture) {  // a caller's capture may end between the apply and the evaluation that joins
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        KIFMM_CUDA(cudaStreamIsCapturing(P->stream, &cap));
-        if (cap != cudaStreamCaptureStatusNone) return false;
-    }
+    if (!near_form(P) || P->n_leaf_list <= 0 || (P->opt.planned != 0) != planned_ready(P)) return false;
+    if (callers_capture(P)) return false;  // it may end between the apply and the evaluation that joins
     ensure_aux_streams(P);
     return true;
 }
@@ -916,10 +923,7 @@ void near_fork(kifmm_plan *P) {
 // A capture of the caller's that began after the apply cannot depend on it: there
 // the host waits for it, and it is dropped.
 bool near_under_way(kifmm_plan *P) {
-    if (!P->near_pending || P->own_capture) return P->near_pending;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    KIFMM_CUDA(cudaStreamIsCapturing(P->stream, &cap));
-    if (cap == cudaStreamCaptureStatusNone) return true;
+    if (!near_form(P) || !callers_capture(P) || !P->near_pending) return P->near_pending;
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     KIFMM_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
     const cudaError_t rc = cudaEventSynchronize(P->near_done);

@@ -134,3 +134,33 @@ def test_batch_after_an_apply_never_evaluated(kind, n, cutoff):
     fs[0].synchronize()
     assert all(torch.equal(p, r) for p, r in zip(pots, refs)) and torch.equal(at, refs[0])
     batch.close()
+
+
+@pytest.mark.parametrize("n,cutoff", TREES)
+@pytest.mark.parametrize("kind,precision,planned", [("laplace", "mixed", False), ("k0", "mixed", False),
+                                                    ("laplace", "fp64", True)])
+@pytest.mark.parametrize("whole", [False, True])
+def test_callers_graph_after_an_apply_never_evaluated(kind, precision, planned, n, cutoff, whole):
+    """A graph of the caller's holding an evaluation, or a whole apply, replayed
+    straight after a build_expansions."""
+    import torch
+    x, y, tau, other = on_device(*lopsided(n, 8), np.random.default_rng(9).standard_normal(abs(n)))
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    f = fmm(kind, 2.0, x, y, cutoff, precision=precision, planned=planned, stream=stream.cuda_stream)
+    pot, ref = torch.zeros_like(tau), torch.zeros_like(tau)
+    f.build_expansions(tau if whole else other)
+    f.evaluate_to_points(x, y, True, out=ref)
+    f.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=stream):
+        if whole:
+            f.build_expansions(tau)
+        f.evaluate_to_points(x, y, True, out=pot)
+    for _ in range(3):
+        f.build_expansions(other)
+        with torch.cuda.stream(stream):
+            pot.zero_()
+            g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(pot, ref)
