@@ -194,8 +194,10 @@ static void copy_in(kifmm_plan *P, DBuf<double> &dst, const double *src, int64_t
 }
 
 // Whether p is memory of the plan's device that its kernels can address in
-// place; anything else a copy takes (another device's memory, managed memory).
-static bool local_device_memory(const kifmm_plan *P, const void *p) {
+// place; anything else a copy takes (another device's memory, managed memory, an
+// array that is not aligned to the kernels' loads: complex values are double2).
+static bool usable_in_place(const kifmm_plan *P, const void *p) {
+    if ((uintptr_t)p % (P->cplx ? sizeof(double2) : sizeof(double))) return false;
     cudaPointerAttributes at{};
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
         cudaGetLastError();
@@ -205,7 +207,7 @@ static bool local_device_memory(const kifmm_plan *P, const void *p) {
 }
 // the densities of the next apply: read in place where they are on the device
 static void set_tau(kifmm_plan *P, const double *tau, int64_t n, int mem) {
-    if (mem == KIFMM_MEM_DEVICE && tau && local_device_memory(P, tau)) {
+    if (mem == KIFMM_MEM_DEVICE && tau && usable_in_place(P, tau)) {
         P->tau_src = tau;
         return;
     }
@@ -461,7 +463,7 @@ int kifmm_evaluate_to_sources(kifmm_plan *P, double *pot, int32_t check_self, in
         KIFMM_REQUIRE(mem == KIFMM_MEM_HOST || mem == KIFMM_MEM_DEVICE, KIFMM_ERR_ARG, "bad mem flag");
         use_device(P);
         const int64_t nv = P->cplx ? 2 * P->N : P->N;
-        const bool direct = mem == KIFMM_MEM_DEVICE && pot && local_device_memory(P, pot);
+        const bool direct = mem == KIFMM_MEM_DEVICE && pot && usable_in_place(P, pot);
         if (!direct) P->pot_out.alloc(nv);
         run_eval_sources(P, check_self != 0, direct ? pot : P->pot_out.p);
         P->applied = true;
@@ -503,7 +505,7 @@ int kifmm_synchronize(kifmm_plan *P) {
 // One apply on device pointers, no host synchronisation: what the graph holds.
 static void apply_device(kifmm_plan *P, const double *tau, double *pot, bool check_self) {
     const int64_t nv = P->cplx ? 2 * P->N : P->N;
-    const bool direct = local_device_memory(P, pot);
+    const bool direct = usable_in_place(P, pot);
     set_tau(P, tau, nv, KIFMM_MEM_DEVICE);
     if (!direct) P->pot_out.alloc(nv);
     run_upward_downward(P);
@@ -824,7 +826,7 @@ static void batch_record(kifmm_batch *B, const double *const *tau, double *const
     fork_all();
     for (int r = 0; r < n; r++) {
         kifmm_plan *P = B->plans[r];
-        const bool direct = local_device_memory(P, pot[r]);
+        const bool direct = usable_in_place(P, pot[r]);
         PassArgs A = make_pass_args(P);
         A.out = direct ? pot[r] : P->pot_out.p;
         A.perm = P->perm.p;

@@ -164,3 +164,36 @@ def test_callers_graph_after_an_apply_never_evaluated(kind, precision, planned, 
             g.replay()
         torch.cuda.synchronize()
         assert torch.equal(pot, ref)
+
+
+@pytest.mark.parametrize("kind,iscomplex,precision", [("h0", True, "fp64"), ("laplace", True, "fp64"),
+                                                      ("laplace", False, "fp64"), ("laplace", False, "mixed")])
+def test_device_arrays_of_any_alignment(kind, iscomplex, precision):
+    """Densities and potentials one double past a 16-byte boundary, through the C ABI
+    (whose arrays are doubles): the values of aligned ones, eagerly and replayed."""
+    import torch
+    from pykifmm2d_b200 import _lib as B
+    x, y, tau = on_device(*cloud(3000, 6))
+    width = 2 if iscomplex else 1
+    t = torch.stack([tau, tau.flip(0)], 1).reshape(-1) if iscomplex else tau
+    stream = torch.cuda.Stream()
+    f = fmm(kind, 2.0, x, y, 40, iscomplex, precision=precision, stream=stream.cuda_stream)
+    buf = {off: [torch.zeros(3000 * width + 2, dtype=torch.float64, device="cuda") for _ in range(2)] for off in (0, 1)}
+    pots = []
+    for off, (bt, bp) in buf.items():
+        at, ap = bt[off:off + t.numel()], bp[off:off + t.numel()]
+        assert ap.data_ptr() % 16 == 8 * off
+        at.copy_(t)
+        torch.cuda.synchronize()
+        lib = B.load()
+        B.check(lib.kifmm_build_expansions(f._plan, at.data_ptr(), B.MEM_DEVICE))
+        B.check(lib.kifmm_evaluate_to_sources(f._plan, ap.data_ptr(), 1, B.MEM_DEVICE))
+        f.synchronize()
+        pots.append(ap.clone())
+        ap.zero_()
+        torch.cuda.synchronize()
+        B.check(lib.kifmm_graph_capture(f._plan, at.data_ptr(), ap.data_ptr(), 1))
+        B.check(lib.kifmm_graph_launch(f._plan))
+        f.synchronize()
+        pots.append(ap.clone())
+    assert all(torch.equal(p, pots[0]) for p in pots[1:]) and pots[0].abs().max() > 0
