@@ -899,6 +899,10 @@ int kifmm_batch_capture(kifmm_plan *const *plans, int32_t nplan, const double *c
         for (int r = 0; r < nplan; r++) {
             kifmm_plan *P = plans[r];
             use_device(P);
+            // copies of arrays that are not used in place (earlier applies may have
+            // used theirs in place): no allocation during the capture
+            if (!usable_in_place(P, tau[r])) P->tau.alloc(P->N);
+            if (!usable_in_place(P, pot[r])) P->pot_out.alloc(P->N);
             if (P->applied) continue;
             drop_graph(P);
             KIFMM_CUDA(cudaStreamWaitEvent(P->stream, B->ev[nplan], 0));

@@ -197,3 +197,58 @@ def test_device_arrays_of_any_alignment(kind, iscomplex, precision):
         f.synchronize()
         pots.append(ap.clone())
     assert all(torch.equal(p, pots[0]) for p in pots[1:]) and pots[0].abs().max() > 0
+
+
+@pytest.mark.parametrize("rebuilt", [False, True])
+def test_batch_with_managed_memory(rebuilt):
+    """A packed batch whose densities and results are managed memory, of plans whose
+    earlier applies used device arrays in place."""
+    import ctypes
+
+    from cuda.bindings import runtime
+    from pykifmm2d_b200 import _lib as B
+    import torch
+    lib = B.load()
+    stream = torch.cuda.Stream()
+    sizes = [3000, 5000]
+    fs, arrays, refs, managed = [], [], [], []
+    for r, n in enumerate(sizes):
+        x, y, tau = on_device(*cloud(n, r))
+        torch.cuda.synchronize()
+        m = n // 2 if rebuilt else n
+        f = fmm("laplace", 0.0, x[:m].contiguous(), y[:m].contiguous(), 40, precision="mixed", stream=stream.cuda_stream)
+        f.build_expansions(tau[:m].contiguous())
+        f.evaluate_to_points(f.x, f.y, True)
+        if rebuilt:
+            f.x, f.y = x, y
+            f.build_tree()
+            f.precompute()
+        f.synchronize()
+        fs.append(f)
+        g = fmm("laplace", 0.0, x, y, 40, precision="mixed", stream=stream.cuda_stream)
+        g.build_expansions(tau)
+        refs.append(g.evaluate_to_points(x, y, True).cpu().numpy())
+        g.synchronize()
+        pair = []
+        for _ in range(2):
+            err, p = runtime.cudaMallocManaged(8 * n, runtime.cudaMemAttachGlobal)
+            assert int(err) == 0
+            managed.append(p)
+            pair.append((int(p), np.ctypeslib.as_array((ctypes.c_double * n).from_address(int(p)))))
+        pair[0][1][:] = tau.cpu().numpy()
+        pair[1][1][:] = 0
+        arrays.append(pair)
+    ptrs = [(ctypes.c_void_p * 2)(*[a[k][0] for a in arrays]) for k in (0, 1)]
+    plans = (ctypes.c_void_p * 2)(*[f._plan.value for f in fs])
+    h = ctypes.c_void_p()
+    B.check(lib.kifmm_batch_capture(plans, 2, ptrs[0], ptrs[1], 1, ctypes.c_void_p(stream.cuda_stream), ctypes.byref(h)))
+    for _ in range(2):
+        for a in arrays:
+            a[1][1][:] = 0
+        B.check(lib.kifmm_batch_launch(h))
+        B.check(lib.kifmm_batch_synchronize(h))
+        for a, ref in zip(arrays, refs):
+            np.testing.assert_array_equal(a[1][1], ref)
+    B.check(lib.kifmm_batch_destroy(h))
+    for p in managed:
+        runtime.cudaFree(p)
