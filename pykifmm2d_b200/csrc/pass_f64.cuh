@@ -203,6 +203,7 @@ struct LeafItem {
     const double *tx, *ty;  // target coordinates, at idx[t0 .. t0 + nt) or, without idx, at t0 ..
     const int32_t *idx;
     int t0, nt, n_own, ns, l, lane;
+    int lanes;              // targets that the lanes are laid out for (>= nt): a sum's order depends on this
     double cx, cy;
     const double *den;
     bool check_self;
@@ -215,13 +216,13 @@ __device__ __forceinline__ PairSum<KIND, CPLX> leaf_item(const PassArgs &A, Pair
                                                          const LeafItem &I, unsigned hi_end) {
     constexpr int NC = PairWarp<KIND, CPLX>::NC;
     const int nt = I.nt, lane = I.lane;
-    const int ng = (nt + TB - 1) / TB, sp = 32 / ng, j = lane / ng, gi = lane - j * ng;
+    const int ng = (I.lanes + TB - 1) / TB, sp = 32 / ng, j = lane / ng, gi = lane - j * ng;
     double tx[TB], ty[TB];
     PairSum<KIND, CPLX> acc[TB];
     bool wild = false;  // a separate target out of the unchecked loop's reach
 #pragma unroll
     for (int a = 0; a < TB; a++) {
-        int i = I.t0 + (gi + a * ng < nt ? gi + a * ng : gi);  // unused slots repeat the first
+        int i = I.t0 + (gi + a * ng < nt ? gi + a * ng : min(gi, nt - 1));  // unused slots repeat another
         if (I.idx) i = I.idx[i];
         tx[a] = I.tx[i];
         ty[a] = I.ty[i];
@@ -289,7 +290,7 @@ __device__ __forceinline__ PairSum<KIND, CPLX> leaf_item_tb(const PassArgs &A, P
     // slots per source TB / (32 / ceil(nt / TB)), compared by cross products
     if constexpr (BEYOND) return leaf_item<KIND, CPLX, FAR, NT, true, 2>(A, W, tl, I, hi_end);  // (a larger body)
     else {
-        const int s2 = 32 / ((I.nt + 1) >> 1), s3 = 32 / ((I.nt + 2) / 3), s4 = 32 / ((I.nt + 3) >> 2);
+        const int s2 = 32 / ((I.lanes + 1) >> 1), s3 = 32 / ((I.lanes + 2) / 3), s4 = 32 / ((I.lanes + 3) >> 2);
         if (s4 * 3 >= s3 * 4 && s4 * 2 >= s2 * 4) return leaf_item<KIND, CPLX, FAR, NT, BEYOND, 4>(A, W, tl, I, hi_end);
         if (s3 * 2 >= s2 * 3) return leaf_item<KIND, CPLX, FAR, NT, BEYOND, 3>(A, W, tl, I, hi_end);
         return leaf_item<KIND, CPLX, FAR, NT, BEYOND, 2>(A, W, tl, I, hi_end);
@@ -358,7 +359,7 @@ __global__ void __launch_bounds__(32 * L64_MAX_WARPS, L64_BLOCKS_PER_SM)
         const double tmax = KIND == KIFMM_KERNEL_LAPLACE ? 0.0 : (FAR ? 4.0 : 8.0) * wl * wl * I.k2;
         for (int t0 = b + (int)(it - w * ntile) * ts; t0 < e; t0 += ntile * ts) {
             I.t0 = t0;
-            I.nt = min(ts, e - t0);
+            I.lanes = I.nt = min(ts, e - t0);
             const PairSum<KIND, CPLX> v = leaf_item_series<KIND, CPLX, FAR>(A, W, tl, I, tmax);
             if (lane >= I.nt) continue;
             const int o = A.out ? A.perm[t0 + lane] : t0 + lane;

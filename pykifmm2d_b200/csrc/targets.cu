@@ -18,9 +18,11 @@
 namespace kifmm {
 
 struct TargetItem {
-    int g, start, n, level;  // leaf, first grouped target, targets (<= TI_MAX)
+    int g, start;    // leaf, first grouped target
+    short n, lanes;  // targets (<= TI_MAX), the largest n of the leaf's items
+    int level;
 };
-constexpr int TI_MAX = 64;  // targets of an item: two per lane in the packed FP32 loop
+constexpr int TI_MAX = 64;  // most targets of an item: two per lane in the packed FP32 loop
 
 // counters of a call (P->tcount): [0] targets laid out, [1] items, [2] ticket
 enum { TC_TARGETS, TC_ITEMS, TC_TICKET, TC_WORDS };
@@ -99,8 +101,10 @@ __global__ void __launch_bounds__(TL_THREADS) k_target_leaf(PassArgs A, const do
     }
 }
 
-// first position of each node's targets, and the work items of `per` targets
-__global__ void k_target_items(PassArgs A, int64_t nn, int per, const unsigned *__restrict__ cnt,
+// first position of each node's targets, and the work items of at most `per`
+// targets: as many whole ones as there are and the rest, or (even) all of a leaf's
+// within one target of each other, so that they can share a lane layout
+__global__ void k_target_items(PassArgs A, int64_t nn, int per, bool even, const unsigned *__restrict__ cnt,
                                unsigned *__restrict__ off, TargetItem *__restrict__ items,
                                unsigned *__restrict__ tcount) {
     const int lane = threadIdx.x & 31;
@@ -126,8 +130,11 @@ __global__ void k_target_items(PassArgs A, int64_t nn, int per, const unsigned *
         const unsigned cj = __shfl_sync(0xffffffffu, c, j), oj = __shfl_sync(0xffffffffu, bc, j),
                        fj = __shfl_sync(0xffffffffu, bi, j), nj = __shfl_sync(0xffffffffu, it, j);
         const int lv = A.nlev[g0 + j];
-        for (unsigned q = lane; q < nj; q += 32)
-            items[fj + q] = TargetItem{(int)(g0 + j), (int)(oj + q * per), (int)min((unsigned)per, cj - q * per), lv};
+        const unsigned w = even ? cj / nj : per, rest = even ? cj - w * nj : 0;
+        for (unsigned q = lane; q < nj; q += 32) {
+            const unsigned b = q * w + min(q, rest), n = min(w + (q < rest), cj - b);
+            items[fj + q] = TargetItem{(int)(g0 + j), (int)(oj + b), (short)n, (short)(w + (rest != 0)), lv};
+        }
     }
 }
 
@@ -205,15 +212,14 @@ __global__ void __launch_bounds__(32 * L64_MAX_WARPS, L64_BLOCKS_PER_SM)
         node_center(A, J.g, J.level, I.cx, I.cy);
         I.den = T.den + (size_t)J.g * A.Q;
         const double wl = ldexp(A.W, -J.level);
-        for (int t0 = 0; t0 < J.n; t0 += 32) {
-            I.t0 = J.start + t0;
-            I.nt = min(32, J.n - t0);
-            const PairSum<KIND, CPLX> v = leaf_item_series<KIND, CPLX, false>(A, W, tl, I, 8.0 * wl * wl * I.k2);
-            if (lane >= I.nt) continue;
-            const int o = T.order[I.t0 + lane];
-            if constexpr (CPLX) ((double2 *)T.pot)[o] = make_double2(v.c[0], v.c[1]);
-            else T.pot[o] = v.c[0];
-        }
+        I.t0 = J.start;
+        I.nt = J.n;
+        I.lanes = J.lanes;
+        const PairSum<KIND, CPLX> v = leaf_item_series<KIND, CPLX, false>(A, W, tl, I, 8.0 * wl * wl * I.k2);
+        if (lane >= I.nt) continue;
+        const int o = T.order[I.t0 + lane];
+        if constexpr (CPLX) ((double2 *)T.pot)[o] = make_double2(v.c[0], v.c[1]);
+        else T.pot[o] = v.c[0];
     }
 }
 
@@ -365,11 +371,11 @@ static TargetArgs group_targets(kifmm_plan *P, const PassArgs &A, const double *
                                 int check_self, bool fp32, double *pot) {
     KIFMM_REQUIRE(n < (1ll << 31), KIFMM_ERR_ARG, "evaluate_to_points: more than 2^31 - 1 targets");
     cudaStream_t s = P->stream;
-    // Targets per item: 64, fewer where that leaves the resident warps less than
-    // four items each (a launch of 1.3 rounds of items lasts two); down to 32 for
-    // the FP32 form, which keeps a target on one lane, and to 8 for the others.
+    // Targets per item: 64 in the FP32 form, which keeps a target on one lane, 32 in
+    // the others; fewer where that leaves the resident warps less than four items
+    // each (a launch of 1.3 rounds of items lasts two), down to 32 and 8.
     const int64_t nn = P->n_nodes, want = 4 * (int64_t)P->num_sms * L64_BLOCKS_PER_SM * L64_MAX_WARPS;
-    int per = TI_MAX;
+    int per = fp32 ? TI_MAX : 32;
     while (per > (fp32 ? 32 : 8) && n / per < want) per >>= 1;
     const int64_t max_items = (n + per - 1) / per + std::min(n, nn);
     P->tleaf.alloc(n);
@@ -382,7 +388,7 @@ static TargetArgs group_targets(kifmm_plan *P, const PassArgs &A, const double *
     k_target_leaf<<<(unsigned)((n + TL_TILE - 1) / TL_TILE), TL_THREADS, 0, s>>>(
         A, tx, ty, n, std::ldexp(P->W, -KEY_DEPTH), cnt, P->tleaf.p, P->trank.p);
     KIFMM_LAUNCHED();
-    k_target_items<<<(unsigned)((nn + 255) / 256), 256, 0, s>>>(A, nn, per, cnt, off, (TargetItem *)P->titems.p,
+    k_target_items<<<(unsigned)((nn + 255) / 256), 256, 0, s>>>(A, nn, per, !fp32, cnt, off, (TargetItem *)P->titems.p,
                                                                 P->tcount.p);
     KIFMM_LAUNCHED();
     k_target_place<<<grid_for(n, 256, P->num_sms * 16), 256, 0, s>>>(n, P->tleaf.p, P->trank.p, off, P->tperm.p);

@@ -252,3 +252,19 @@ def test_batch_with_managed_memory(rebuilt):
     B.check(lib.kifmm_batch_destroy(h))
     for p in managed:
         runtime.cudaFree(p)
+
+
+@pytest.mark.parametrize("kind,k,iscomplex,precision", [
+    ("laplace", 0.0, False, "fp64"), ("laplace", 0.0, True, "fp64"), ("laplace", 0.0, False, "mixed"),
+    ("k0", 2.0, False, "fp64"), ("k0", 60.0, False, "fp64"), ("k0", 2.0, False, "mixed"), ("h0", 2.0, True, "fp64")])
+@pytest.mark.parametrize("m", [700, 20000, 300000])
+def test_equal_calls_at_targets_give_equal_bits(kind, k, iscomplex, precision, m):
+    """The order in which targets are grouped by leaf is not fixed; their sums are.
+    Leaves with fewer targets than an item holds, a few items each, and many."""
+    x, y, tau = cloud(2000, 3)
+    f = fmm(kind, k, x, y, 40, iscomplex, precision=precision)
+    f.build_expansions(tau + 0j if iscomplex else tau)
+    tx, ty, _ = cloud(m, 4)
+    ref = f.evaluate_to_points(tx, ty, False)
+    for _ in range(4):
+        np.testing.assert_array_equal(f.evaluate_to_points(tx, ty, False), ref)
