@@ -14,28 +14,34 @@ namespace kifmm {
 
 // Natural logarithm of a positive normal number, table-driven (P. T. P. Tang,
 // "Table-driven implementation of the logarithm function in IEEE
-// floating-point arithmetic", ACM TOMS 16, 1990): x = 2^e m with m in [1, 2),
-// c_i = 1 + (i + 1/2)/128 the midpoint of m's subinterval, v_i = 1/c_i
-// rounded to FP64, r = m v_i - 1 (|r| < 2^-8), ln x = e ln2 - ln v_i +
-// log1p(r).  log1p is its series to r^6 with r^6 economised by the Chebyshev
-// polynomial T6 (r^6 = h^6 (T6(r/h) + 48 (r/h)^4 - 18 (r/h)^2 + 1) / 32,
-// h = 2^-8), so five coefficients leave 1.9e-17; the constant it leaves goes
-// into the table.  Max error 1.6 ulp, mean 0.34 (against 60-digit values over
-// 2^-30 .. 2^5).  e is converted on the XU pipe, beside the FP64 pipe.
+// floating-point arithmetic", ACM TOMS 16, 1990): x = 2^e m with m in
+// [0.699, 1.398), so that e = 0 around 1 and nothing cancels there; v_i = 1/c_i
+// rounded to FP64, c_i the midpoint of m's subinterval, r = m v_i - 1 (|r| <
+// 2^-9), ln x = e ln2 - ln v_i + log1p(r).  The subinterval that holds 1 has v = 1,
+// so its values are log1p(r) alone.  log1p(r) / r is its series to r^4 with the
+// next term economised by the Chebyshev polynomial T5 (r^5 = h^5 (T5(r/h) + 20
+// (r/h)^3 - 5 r/h) / 16, h = 2^-9).  Error against 113-bit values, 400,000
+// samples a range: at most 4.0 ulp within 0.4% of 1 (mean 0.9), 1.6 elsewhere
+// (mean 0.26 over 2^-30 .. 2^5).  With m in [1, 2) and half as many subintervals,
+// at the same number of instructions but one, the error was 1e-16 absolutely, of
+// any relative size beside 1.
+// e is converted on the XU pipe, beside the FP64 pipe.
 // The table is kept LOGTAB_COPIES times in shared memory, copy c in the 16-byte
 // bank group c: a warp's 32 16-byte reads, eight to a phase, hit eight
 // different groups whatever their entries (one copy measured 2-3 way
 // conflicts, and the reads would then bound the loop instead of the FP64 pipe).
-constexpr int LOGTAB_N = 128, LOGTAB_COPIES = 8;
-constexpr double LOG_H2 = 1.0 / 65536.0;  // h^2
-// the polynomial's coefficients r^2 .. r^5 and ln 2, in constant memory, so
+constexpr int LOGTAB_N = 256, LOGTAB_COPIES = 8;
+constexpr double LOG_H2 = 1.0 / 262144.0;     // h^2
+constexpr unsigned LOG_M_HI = 0x3fe65800u;    // high word of the least m: 1.0 lies in the middle of subinterval 154
+constexpr unsigned LOG_STEP_HI = 0x00100000u / LOGTAB_N;  // high words of a subinterval
+// the polynomial's coefficients r .. r^4 and ln 2, in constant memory, so
 // that they are operands of the multiply-adds
 enum { LOG_C2, LOG_C3, LOG_C4, LOG_C5, LOG_LN2 };
-static __device__ __constant__ double LOG_K[] = {-0.5 + LOG_H2 * LOG_H2 * 18.0 / 192.0, 1.0 / 3.0,
-                                                 -0.25 - LOG_H2 * 48.0 / 192.0, 0.2,
+static __device__ __constant__ double LOG_K[] = {-0.5 + LOG_H2 * LOG_H2 * 5.0 / 96.0, 1.0 / 3.0,
+                                                 -0.25 - LOG_H2 * 20.0 / 96.0, 0.2,
                                                  0.693147180559945309417232121458176568};
 
-// log_table(device) holds [LOGTAB_N] (v_i, -ln v_i - h^6/192); stage its copies into tab[LOGTAB_N * LOGTAB_COPIES] (all threads of the block)
+// log_table(device) holds [LOGTAB_N] (v_i, -ln v_i); stage its copies into tab[LOGTAB_N * LOGTAB_COPIES] (all threads of the block)
 __device__ __forceinline__ void stage_log_table(double2 *tab, const double2 *__restrict__ g) {
     for (int i = threadIdx.x; i < LOGTAB_N * LOGTAB_COPIES; i += blockDim.x) tab[i] = g[i / LOGTAB_COPIES];
 }
@@ -44,12 +50,13 @@ __device__ __forceinline__ void stage_log_table(double2 *tab, const double2 *__r
 // finite; anything else gives a finite or NaN value and reads inside the table.
 template <int EADJ>
 __device__ __forceinline__ double ln_tab(double x, const double2 *tl) {
-    const int hi = __double2hiint(x), lo = __double2loint(x);
+    // t: e + EADJ above 20 bits of the distance from the least m
+    const unsigned t = (unsigned)__double2hiint(x) - (LOG_M_HI - ((unsigned)EADJ << 20));
     constexpr unsigned ROW = LOGTAB_COPIES * sizeof(double2);  // bytes of an entry's copies
-    static_assert(LOGTAB_N * ROW == 0x4000 && ROW == 0x80, "the shift and mask below");
-    const double2 c = *(const double2 *)((const char *)tl + (((unsigned)hi >> 6) & 0x3f80u));
-    const double m = __hiloint2double((hi & 0x000fffff) | 0x3ff00000, lo);
-    const double e = (double)((int)((unsigned)hi >> 20) - (1023 - EADJ));
+    static_assert(LOGTAB_N * ROW == 0x8000 && ROW == 0x80 && LOG_STEP_HI == 0x1000, "the shift and mask below");
+    const double2 c = *(const double2 *)((const char *)tl + ((t >> 5) & 0x7f80u));
+    const double m = __hiloint2double((int)((t & 0x000fffffu) + LOG_M_HI), __double2loint(x));
+    const double e = (double)((int)t >> 20);
     const double r = fma(m, c.x, -1.0);
     double q = LOG_K[LOG_C5];
     q = fma(q, r, LOG_K[LOG_C4]);

@@ -2,6 +2,7 @@
 // and the L2P + P2P at the sources (class_fmm.py:73-111), for real densities
 // (the "plain" form; the mixed form takes its P2M from here, its K0 far field,
 // and with near_fp64 its leaf pass) and for complex ones.
+#include <cstring>
 #include <mutex>
 
 #include "pass_f64.cuh"
@@ -16,10 +17,17 @@ const double2 *log_table(int device) {
     std::lock_guard<std::mutex> lock(mu);
     if (!tab[device]) {
         double2 t[LOGTAB_N];
-        const long double c0 = (long double)LOG_H2 * LOG_H2 * LOG_H2 / 192.0L;
-        for (int i = 0; i < LOGTAB_N; i++) {
-            t[i].x = (double)(1.0L / (1.0L + ((long double)i + 0.5L) / LOGTAB_N));
-            t[i].y = (double)(-logl((long double)t[i].x) - c0);
+        for (int i = 0; i < LOGTAB_N; i++) {  // subintervals [a, b) of m
+            const auto value = [](uint64_t hi) {
+                double d;
+                hi <<= 32;
+                memcpy(&d, &hi, sizeof(d));
+                return d;
+            };
+            const double a = value(LOG_M_HI + i * LOG_STEP_HI), b = value(LOG_M_HI + (i + 1) * LOG_STEP_HI);
+            const bool one = a <= 1.0 && 1.0 < b;
+            t[i].x = one ? 1.0 : (double)(1.0L / (((long double)a + b) * 0.5L));
+            t[i].y = one ? 0.0 : (double)-logl((long double)t[i].x);
         }
         void *p = nullptr;
         KIFMM_CUDA(cudaMemcpyToSymbol(g_logtab, t, sizeof(t)));

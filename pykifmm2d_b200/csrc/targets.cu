@@ -230,7 +230,10 @@ __global__ void __launch_bounds__(32 * L64_MAX_WARPS, L64_BLOCKS_PER_SM)
 // offsets, squared distances and products of both in one instruction, the same
 // operations as the single form.  Bound by the 16/clk/SM lg2 unit (Laplace):
 // 3M targets, 8e8 pairs, 0.17 ms.
-constexpr int TF_BLOCKS_PER_SM = 3;
+// Two blocks of twelve warps to an SM: the logarithm table takes 32 KB a block, and
+// three blocks of eight warps left the gathers 28 KB of L1 (3M targets: 509 us, now
+// 479).
+constexpr int TF_WARPS = 12, TF_BLOCKS_PER_SM = 2;
 struct NearWarp {
     ulonglong2 xy[L64_CHUNK];  // (x, x | y, y)
     f32x2 z[L64_CHUNK];        // (z, z)
@@ -348,7 +351,7 @@ __device__ __forceinline__ void target_item_f(const PassArgs &A, const TargetArg
             T.pot[T.order[J.start + lane + 32 * a]] = (double)(acc[a] * SCALE) + far[a].c[0] * pair_scale<KIND>();
 }
 template <int KIND>
-__global__ void __launch_bounds__(32 * L64_MAX_WARPS, TF_BLOCKS_PER_SM)
+__global__ void __launch_bounds__(32 * TF_WARPS, TF_BLOCKS_PER_SM)
     k_eval_targets_f(PassArgs A, const double2 *__restrict__ logtab, TargetArgs T) {
     extern __shared__ __align__(16) unsigned char sm_tgf[];
     double2 *tab = (double2 *)sm_tgf;
@@ -405,24 +408,24 @@ static TargetArgs group_targets(kifmm_plan *P, const PassArgs &A, const double *
     return T;
 }
 // at most one warp per item; the items are counted on the device
-static unsigned target_grid(const kifmm_plan *P, int64_t n, int blocks_per_sm) {
+static unsigned target_grid(const kifmm_plan *P, int64_t n, int warps, int blocks_per_sm) {
     const int64_t items = std::min<int64_t>(n, n / 8 + P->n_nodes);
-    return (unsigned)std::min<int64_t>((items + L64_MAX_WARPS - 1) / L64_MAX_WARPS,
-                                       (int64_t)P->num_sms * blocks_per_sm);
+    return (unsigned)std::min<int64_t>((items + warps - 1) / warps, (int64_t)P->num_sms * blocks_per_sm);
 }
 template <int KIND, bool CPLX>
 static void eval_targets_d(kifmm_plan *P, const PassArgs &A, const TargetArgs &T, int64_t n) {
     const size_t smem = LOGTAB_N * LOGTAB_COPIES * sizeof(double2) + L64_MAX_WARPS * sizeof(PairWarp<KIND, CPLX>);
     ensure_dyn_smem(k_eval_targets_d<KIND, CPLX>, smem);
-    k_eval_targets_d<KIND, CPLX><<<target_grid(P, n, L64_BLOCKS_PER_SM), 32 * L64_MAX_WARPS, smem, P->stream>>>(A, log_table(P->device), T);
+    k_eval_targets_d<KIND, CPLX><<<target_grid(P, n, L64_MAX_WARPS, L64_BLOCKS_PER_SM), 32 * L64_MAX_WARPS, smem,
+                                   P->stream>>>(A, log_table(P->device), T);
     KIFMM_LAUNCHED();
 }
 template <int KIND>
 static void eval_targets_f(kifmm_plan *P, const PassArgs &A, const TargetArgs &T, int64_t n) {
     const size_t smem = LOGTAB_N * LOGTAB_COPIES * sizeof(double2) +
-                        L64_MAX_WARPS * (sizeof(PairWarp<KIND, false>) + sizeof(NearWarp));
+                        TF_WARPS * (sizeof(PairWarp<KIND, false>) + sizeof(NearWarp));
     ensure_dyn_smem(k_eval_targets_f<KIND>, smem);
-    k_eval_targets_f<KIND><<<target_grid(P, n, TF_BLOCKS_PER_SM), 32 * L64_MAX_WARPS, smem, P->stream>>>(
+    k_eval_targets_f<KIND><<<target_grid(P, n, TF_WARPS, TF_BLOCKS_PER_SM), 32 * TF_WARPS, smem, P->stream>>>(
         A, log_table(P->device), T);
     KIFMM_LAUNCHED();
 }

@@ -268,3 +268,40 @@ def test_equal_calls_at_targets_give_equal_bits(kind, k, iscomplex, precision, m
     ref = f.evaluate_to_points(tx, ty, False)
     for _ in range(4):
         np.testing.assert_array_equal(f.evaluate_to_points(tx, ty, False), ref)
+
+
+def log_targets():
+    """distances r with exact squares: beside 1, and of 26 random bits over 2^-30 .. 2^20"""
+    k = np.arange(3, 27)
+    beside = np.concatenate([[1.0], 1 + 2.0 ** -k, 1 - 2.0 ** -k])
+    rng = np.random.default_rng(2)
+    wide = np.ldexp(np.floor(rng.uniform(0.5, 1, 4000) * 2 ** 26) / 2 ** 26, rng.integers(-29, 21, 4000))
+    close = 1 + np.floor(rng.uniform(-0.4, 0.4, 4000) * 2 ** 25) / 2 ** 25
+    return np.concatenate([beside, wide, close])
+
+
+@pytest.mark.parametrize("iscomplex", [False, True])
+@pytest.mark.parametrize("at_sources", [False, True])
+def test_logarithm_is_relatively_accurate(at_sources, iscomplex):
+    """One charge at the origin: the potential is the logarithm of r^2 times its
+    scale, to its last bits also where it is small, and zero at r = 1.  Bound: 4.0 ulp
+    (an ulp is at most 2^-52 of the value) for the logarithm, one for its scale and
+    one for the product with it."""
+    r = log_targets()
+    r2 = r.astype(np.longdouble) ** 2
+    ref = np.where(np.abs(r2 - 1) < 0.5, np.log1p(np.maximum(r2, 0.25) - 1), np.log(r2)) / (-16 * np.arctan(np.longdouble(1)))
+    if at_sources:
+        x = np.concatenate([[0.0], r])
+        y = np.zeros_like(x)
+        tau = np.zeros_like(x)
+        tau[0] = 1
+        f = fmm("laplace", 0.0, x, y, len(x), iscomplex)
+        f.build_expansions(tau + 0j if iscomplex else tau)
+        pot = f.evaluate_to_points(x, y, True)[1:]
+    else:
+        f = fmm("laplace", 0.0, np.array([0.0, 1.0]), np.array([0.0, 1.0]), 4, iscomplex)
+        f.build_expansions(np.array([1.0, 0.0]) + (0j if iscomplex else 0))
+        pot = f.evaluate_to_points(r, 0 * r, True)
+        np.testing.assert_array_equal(pot, f.evaluate_to_points(0 * r, r, True))
+    assert np.all(np.abs(pot - ref.astype(float)) <= 6.0 * EPS * np.abs(ref).astype(float))
+    assert r[0] == 1 and pot[0] == 0
