@@ -176,7 +176,8 @@ struct HashSet {
     unsigned long long *tab;
     uint64_t mask;
     uint64_t *list;
-    unsigned long long *count;  // entries appended to list
+    unsigned long long *count;  // split cells appended to list
+    unsigned long long *xcount; // X-list cells appended behind them
     unsigned long long *ovf;
     uint64_t cap;               // list capacity
     unsigned long long *lcount; // [32] entries per level, counted as they are appended
@@ -331,20 +332,18 @@ __global__ void __launch_bounds__(256) k_closure(const uint64_t *__restrict__ ke
     }
 }
 
-__device__ __forceinline__ unsigned long long hs_count(const HashSet &H) {
-    unsigned long long n = *((volatile unsigned long long *)H.count);
-    return n > H.cap ? H.cap : n;
-}
-
 // X-list (tree.py:546-576, numba_get_Xlist :446-458): for levels 1..L-2, a
 // real leaf (cell not split, parent split) next to a split cell becomes an
 // X-list cell (every split cell lies on a level <= L-2, so the level range
 // follows from the split cells themselves).  One item per (split cell, neighbour); the warp's new cells are
-// appended together (one count atomic per warp, one level atomic per level).
+// appended together (one count atomic per warp, one level atomic per level),
+// behind the split cells and counted apart from them: a block that starts late
+// must not take cells that another block is appending, whose list words may still
+// be those of an earlier tree.
 __global__ void __launch_bounds__(256) k_xlist(HashSet H) {
     pdl_trigger();
     pdl_wait();
-    const unsigned long long n = hs_count(H);
+    const unsigned long long n_split = *H.count, n = min(n_split, (unsigned long long)H.cap);
     const int lane = threadIdx.x & 31;
     const int64_t total = 9 * (int64_t)n, stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t base = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) & ~(int64_t)31; base < total;
@@ -358,7 +357,7 @@ __global__ void __launch_bounds__(256) k_xlist(HashSet H) {
             const int d = (int)(j - 9 * i);
             const uint64_t s = H.list[i];
             l = (int)(s >> ENT_LEVEL_SHIFT);
-            if (d != 4 && !(s & 1) && l >= 1) {  // split cells lie on levels <= L-2
+            if (d != 4 && l >= 1) {  // split cells lie on levels <= L-2
                 const uint64_t k = (s >> 1) & KEY56;
                 const int64_t cx = (int64_t)compact2(k >> 1) + d / 3 - 1, cy = (int64_t)compact2(k) + d % 3 - 1;
                 const int64_t side = 1ll << l;
@@ -375,7 +374,7 @@ __global__ void __launch_bounds__(256) k_xlist(HashSet H) {
         if (!fm) continue;
         const int lead = __ffs(fm) - 1;
         unsigned long long b0 = 0;
-        if (lane == lead) b0 = atomicAdd(H.count, (unsigned long long)__popc(fm));
+        if (lane == lead) b0 = n_split + atomicAdd(H.xcount, (unsigned long long)__popc(fm));
         b0 = __shfl_sync(0xffffffffu, b0, lead);
         if (fresh) {
             const unsigned peers = __match_any_sync(fm, l);
@@ -914,6 +913,7 @@ static void build_tree_impl(kifmm_plan *P, const double *x, const double *y, int
     HashSet H{};
     H.count = P->scal.p + 9;
     H.ovf = P->scal.p + 10;
+    H.xcount = P->scal.p + 11;
     P->misc.alloc(128);
     P->m2l_hist.alloc((size_t)(MAX_LEVELS + 1) * M2L_KEYS);
     unsigned long long *lc = (unsigned long long *)P->misc.p;  // [32] entries per level
@@ -931,11 +931,11 @@ static void build_tree_impl(kifmm_plan *P, const double *x, const double *y, int
         P->hash.alloc(hcap);
         P->hash_cap = hcap;
         P->list.alloc(cap);
-        // one launch clears the table (all ones), the set's count and overflow
+        // one launch clears the table (all ones), the set's counts and overflow
         // flag, the per-level entry counts and the later list counters (misc),
         // and the M2L target order's histogram
         launch_fill(P, {{P->hash.p, 2 * hcap, 0xFFFFFFFFu},
-                        {P->scal.p + 9, 4, 0u},
+                        {P->scal.p + 9, 6, 0u},
                         {P->misc.p, 2 * 128, 0u},
                         {P->m2l_hist.p, (size_t)(MAX_LEVELS + 1) * M2L_KEYS, 0u}});
         H.tab = (unsigned long long *)P->hash.p;
@@ -946,7 +946,7 @@ static void build_tree_impl(kifmm_plan *P, const double *x, const double *y, int
         launch_pdl(k_closure, dim3(cgrid), dim3(TB), 0, s, (const uint64_t *)P->pkey.p, n, (int64_t)P->ppl, H);
         // the X-list reads the complete split set: nine items per entry, grid-stride
         launch_pdl(k_xlist, dim3(grid_for(9 * (int64_t)cap, TB, P->num_sms * 8)), dim3(TB), 0, s, H);
-        KIFMM_CUDA(cudaMemcpyAsync(P->hpin + HP_SCAL + 9, P->scal.p + 9, 2 * sizeof(unsigned long long),
+        KIFMM_CUDA(cudaMemcpyAsync(P->hpin + HP_SCAL + 9, P->scal.p + 9, 3 * sizeof(unsigned long long),
                                    cudaMemcpyDeviceToHost, s));
         KIFMM_CUDA(cudaMemcpyAsync(P->hpin + HP_MISC, lc, sizeof(lcount), cudaMemcpyDeviceToHost, s));
         KIFMM_CUDA(cudaEventRecord(P->tree_ev, s));
@@ -1020,11 +1020,11 @@ static void build_tree_impl(kifmm_plan *P, const double *x, const double *y, int
                 queue_closure(cap);
             }
             KIFMM_CUDA(cudaEventSynchronize(P->tree_ev));
-            unsigned long long cv[2];
+            unsigned long long cv[3];  // split cells, overflow, X-list cells
             memcpy(cv, P->hpin + HP_SCAL + 9, sizeof(cv));
             memcpy(lcount, P->hpin + HP_MISC, sizeof(lcount));
-            if (cv[1] == 0 && cv[0] <= cap) {
-                n_ent = (int64_t)cv[0];
+            if (cv[1] == 0 && cv[0] + cv[2] <= cap) {
+                n_ent = (int64_t)(cv[0] + cv[2]);
                 break;
             }
             KIFMM_REQUIRE(attempt < 5, KIFMM_ERR_NOMEM, "build_tree: split-cell set overflow");

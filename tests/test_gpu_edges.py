@@ -305,3 +305,39 @@ def test_logarithm_is_relatively_accurate(at_sources, iscomplex):
         np.testing.assert_array_equal(pot, f.evaluate_to_points(0 * r, r, True))
     assert np.all(np.abs(pot - ref.astype(float)) <= 6.0 * EPS * np.abs(ref).astype(float))
     assert r[0] == 1 and pot[0] == 0
+
+
+def test_trees_of_moving_points_vs_oracle():
+    """Two objects whose points move between clouds of other depths (all with points
+    on one circle, so that their deep cells lie side by side), built in turn with
+    other work under way: the words of an earlier tree that a build finds in its
+    buffers are in none of its cells."""
+    import pykifmm2d_b200 as P
+    from oracle import oracle as O
+    n, cutoff = 40000, 12
+    clouds, want = [], []
+    for seed, sigma in enumerate((1e-1, 1e-3, 1e-2, 3e-4)):
+        rng = np.random.default_rng(seed)
+        th = rng.uniform(0, 2 * np.pi, n // 2)
+        th[:n // 4] *= sigma
+        c = rng.uniform(-0.9, 0.9, (2, 8))[:, rng.integers(0, 8, n - n // 2)]
+        z = c + sigma * rng.standard_normal(c.shape)
+        clouds.append(np.concatenate([[np.cos(th), np.sin(th)], z], 1))
+        want.append(O.OracleTree(clouds[-1][0], clouds[-1][1], cutoff).export()[0])
+    clouds = [on_device(*c) for c in clouds]
+    kern = P.LaplaceKernel()
+    fs = []
+    for _ in range(2):
+        x, y = (v.clone() for v in clouds[0])
+        fs.append(P.FMM(x, y, P.Get_Kernel_Functions(kern), P.prepare_numba_functions_on_the_fly(kern), 32, cutoff,
+                        precision="mixed"))
+    for i in range(200):
+        k, f = (i * 7 // 5) % 4, fs[i % 2]
+        f.x.copy_(clouds[k][0])
+        f.y.copy_(clouds[k][1])
+        f.build_tree()
+        f.precompute()
+        f.build_expansions(f.x)
+        f.evaluate_to_points(f.x, f.y, True)
+        if i % 23 < 2:
+            np.testing.assert_array_equal(f.export_tree()[0], want[k])
