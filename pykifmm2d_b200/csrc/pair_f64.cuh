@@ -86,6 +86,13 @@ __device__ __forceinline__ unsigned pair_rank(double t) { return (unsigned)(__do
 __device__ __forceinline__ bool pair_ordinary(double t, unsigned hi_end) { return pair_rank(t) < hi_end - 0x00100000u; }
 constexpr unsigned LOG_HI_END = 0x7ff00000u;  // every finite number
 
+// k^2 for (k r)^2.  Where it would lose bits (k below 1.5e-154) it is 0, which makes
+// no pair ordinary: pair_value_any takes k r.
+__device__ __forceinline__ double pair_k2(double k) {
+    const double k2 = k * k;
+    return k2 < 2.2250738585072014e-308 ? 0.0 : k2;
+}
+
 // Unscaled kernel value: re = ln r^2 (Laplace, times -1/(4 pi)), K0(k r) =
 // P(t) - ln(t/4) I0(t)/2 (times 1/(2 pi)), or the real part of (i/4) H0(k r),
 // ln(t/4) A(t) + R(t), whose imaginary part is -pi a with a = A(t).

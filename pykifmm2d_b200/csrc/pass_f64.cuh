@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(32 * L64_MAX_WARPS, L64_BLOCKS_PER_SM)
     I.idx = nullptr;
     I.lane = lane;
     I.check_self = check_self;
-    I.k2 = A.k * A.k;
+    I.k2 = pair_k2(A.k);
     const unsigned last = nitems + gridDim.x * (blockDim.x >> 5) - 1;
     for (;;) {
         unsigned it = 0;
@@ -459,7 +459,7 @@ __global__ void __launch_bounds__(32 * L64_MAX_WARPS, L64_BLOCKS_PER_SM)
     pdl_wait();
     const int lane = threadIdx.x & 31;
     const double2 *tl = tab + (lane & (LOGTAB_COPIES - 1));
-    const double k2 = A.k * A.k;
+    const double k2 = pair_k2(A.k);
     const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
     for (int64_t w = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); w < nlist; w += nw) {
         const int g = list[w], l = A.nlev[g], b = A.nbot[g], e = A.ntop[g];

@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(32 * L64_MAX_WARPS, L64_BLOCKS_PER_SM)
     I.idx = T.order;
     I.lane = lane;
     I.check_self = T.check_self;
-    I.k2 = A.k * A.k;
+    I.k2 = pair_k2(A.k);
     I.n_own = 0;  // a coincidence with a source is the exception here
     const unsigned nitems = T.tcount[TC_ITEMS];
     for (unsigned it = next_item(T, lane); it < nitems; it = next_item(T, lane)) {
@@ -328,7 +328,7 @@ __device__ __forceinline__ void target_item_f(const PassArgs &A, const TargetArg
         __syncwarp();
         for (int q = lane; q < A.Q; q += 32) W.stage(q, lg[q], lg[A.Q + q], den[q]);
         __syncwarp();
-        const double wl = ldexp(A.W, -J.level), k2 = A.k * A.k, tmax = 4.0 * wl * wl * k2;  // r < 2 w inside the box
+        const double wl = ldexp(A.W, -J.level), k2 = pair_k2(A.k), tmax = 4.0 * wl * wl * k2;  // r < 2 w inside the box
         if (KIND == KIFMM_KERNEL_LAPLACE)
             pair_chunk<KIND, false, 1, TB, false>(W, tl, 0, 1, wild ? A.Q : 0, A.Q, tx, ty, A.k, k2, LOG_HI_END, false,
                                                   far);

@@ -341,3 +341,25 @@ def test_trees_of_moving_points_vs_oracle():
         f.evaluate_to_points(f.x, f.y, True)
         if i % 23 < 2:
             np.testing.assert_array_equal(f.export_tree()[0], want[k])
+
+
+@pytest.mark.parametrize("kind", ["k0", "h0"])
+@pytest.mark.parametrize("k", [1e-152, 1e-158, 1e-161, 1e-170])
+def test_wavenumbers_whose_square_underflows(kind, k):
+    """K0(z) and H0(z) of tiny z are -ln(z / 2) - gamma and its like to the last bit;
+    one leaf, so the potential is the direct sum: the rounding of n additions of values
+    within a few ulp."""
+    n = 30
+    x, y, tau = cloud(n, 1)
+    x, y = 4e6 * x, 4e6 * y  # (k r)^2 is a normal number again for most k here
+    f = fmm(kind, k, x, y, 64, kind == "h0")
+    f.build_expansions(tau + 0j if kind == "h0" else tau)
+    ld = np.longdouble
+    r2 = (x[:, None].astype(ld) - x) ** 2 + (y[:, None].astype(ld) - y) ** 2
+    off = ~np.eye(n, dtype=bool)
+    g = np.zeros((n, n), dtype=np.clongdouble)
+    ln = np.log(ld(k)) + np.log(r2[off]) / 2 - np.log(ld(2)) + ld("0.57721566490153286060651209008240243")
+    g[off] = -ln / (8 * np.arctan(ld(1))) + (0.25j if kind == "h0" else 0)
+    ref, mag = g @ tau, np.abs(g).astype(float) @ np.abs(tau)
+    for pot in (f.evaluate_to_points(x, y, True), f.evaluate_to_points(x.copy(), y.copy(), True)):
+        assert np.all(np.abs(pot - ref) <= (n + 16) * EPS * mag)
