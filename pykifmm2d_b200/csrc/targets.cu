@@ -372,7 +372,6 @@ __global__ void __launch_bounds__(32 * TF_WARPS, TF_BLOCKS_PER_SM)
 // groups the targets and evaluates the leaves' equivalent densities
 static TargetArgs group_targets(kifmm_plan *P, const PassArgs &A, const double *tx, const double *ty, int64_t n,
                                 int check_self, bool fp32, double *pot) {
-    KIFMM_REQUIRE(n < (1ll << 31), KIFMM_ERR_ARG, "evaluate_to_points: more than 2^31 - 1 targets");
     cudaStream_t s = P->stream;
     // Targets per item: 64 in the FP32 form, which keeps a target on one lane, 32 in
     // the others; fewer where that leaves the resident warps less than four items
@@ -430,7 +429,8 @@ static void eval_targets_f(kifmm_plan *P, const PassArgs &A, const TargetArgs &T
     KIFMM_LAUNCHED();
 }
 
-void run_eval_targets(kifmm_plan *P, const double *tx, const double *ty, int64_t n, int check_self, double *pot) {
+// the targets of one grouping: their indices are 32-bit
+static void eval_targets(kifmm_plan *P, const double *tx, const double *ty, int64_t n, int check_self, double *pot) {
     constexpr int LAP = KIFMM_KERNEL_LAPLACE, K0 = KIFMM_KERNEL_MOD_HELMHOLTZ, H0 = KIFMM_KERNEL_HELMHOLTZ;
     const PassArgs A = make_pass_args(P);
     const bool fp32 = P->opt.precision == KIFMM_PREC_MIXED && !P->opt.near_fp64 && !P->cplx;
@@ -445,6 +445,15 @@ void run_eval_targets(kifmm_plan *P, const double *tx, const double *ty, int64_t
         else eval_targets_f<K0>(P, A, T, n);
     } else if (kind == LAP) eval_targets_d<LAP, false>(P, A, T, n);
     else eval_targets_d<K0, false>(P, A, T, n);
+}
+
+// The real forms refuse more than 2^31 - 1 targets; the complex one takes any number,
+// in runs.
+void run_eval_targets(kifmm_plan *P, const double *tx, const double *ty, int64_t n, int check_self, double *pot) {
+    constexpr int64_t RUN = 1ll << 27;
+    KIFMM_REQUIRE(P->cplx || n < (1ll << 31), KIFMM_ERR_ARG, "evaluate_to_points: more than 2^31 - 1 targets");
+    if (!P->cplx) return eval_targets(P, tx, ty, n, check_self, pot);
+    for (int64_t i = 0; i < n; i += RUN) eval_targets(P, tx + i, ty + i, std::min(RUN, n - i), check_self, pot + 2 * i);
 }
 
 }  // namespace kifmm

@@ -363,3 +363,20 @@ def test_wavenumbers_whose_square_underflows(kind, k):
     ref, mag = g @ tau, np.abs(g).astype(float) @ np.abs(tau)
     for pot in (f.evaluate_to_points(x, y, True), f.evaluate_to_points(x.copy(), y.copy(), True)):
         assert np.all(np.abs(pot - ref) <= (n + 16) * EPS * mag)
+
+
+def test_complex_targets_in_runs():
+    """More complex targets than one grouping takes (2^27): the same potentials on
+    either side of the boundary as in a call of their own, up to the rounding of 50
+    additions."""
+    import torch
+    n, m, cut = 50, (1 << 27) + 700, 1 << 27
+    x, y, tau = on_device(*cloud(n, 2))
+    f = fmm("laplace", 0.0, x, y, 64, True)
+    f.build_expansions(tau + 0j)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    tx, ty = (torch.rand(m, generator=g, device="cuda", dtype=torch.float64) for _ in range(2))
+    pot = f.evaluate_to_points(tx, ty, False)
+    for a, b in ((0, 300), (cut - 300, cut + 300), (m - 300, m)):
+        ref = f.evaluate_to_points(tx[a:b].contiguous(), ty[a:b].contiguous(), False)
+        assert (pot[a:b] - ref).abs().max() <= (n + 16) * EPS * tau.abs().sum()
