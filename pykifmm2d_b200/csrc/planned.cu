@@ -137,11 +137,11 @@ __global__ void k_plan_fill_p2m(PassArgs A, const int32_t *__restrict__ p2m, int
     }
 }
 
-// planned P2M: one warp per node, eight lanes over the Q check points (PM_Q each)
-// and four over the sources
+// planned P2M: one warp per node, eight lanes over the Q <= 8 PM_Q check points (PM_Q
+// each) and four over the sources
+template <int PM_Q>
 __global__ void k_planned_p2m(PassArgs A, const int32_t *__restrict__ p2m, int64_t np2m,
                               const int64_t *__restrict__ p2m_off, const double *__restrict__ mat) {
-    constexpr int PM_Q = 5;
     pdl_trigger();
     pdl_wait();
     const int lane = threadIdx.x & 31, j = lane & 7, s0 = lane >> 3;
@@ -150,22 +150,20 @@ __global__ void k_planned_p2m(PassArgs A, const int32_t *__restrict__ p2m, int64
     const int g = p2m[w];
     const double *m = mat + p2m_off[w];
     const int b = A.nbot[g], n = A.ntop[g] - b, Q = A.Q;
-    for (int q0 = 0; q0 < Q; q0 += 8 * PM_Q) {
-        double acc[PM_Q] = {};
+    double acc[PM_Q] = {};
 #pragma unroll 2
-        for (int s = s0; s < n; s += 4) {
-            const double v = A.taus[b + s];
-            const double *row = m + (size_t)s * Q + q0 + j;
+    for (int s = s0; s < n; s += 4) {
+        const double v = A.taus[b + s];
+        const double *row = m + (size_t)s * Q + j;
 #pragma unroll
-            for (int r = 0; r < PM_Q; r++)
-                if (q0 + j + 8 * r < Q) acc[r] = fma(__ldcs(row + 8 * r), v, acc[r]);
-        }
+        for (int r = 0; r < PM_Q; r++)
+            if (j + 8 * r < Q) acc[r] = fma(__ldcs(row + 8 * r), v, acc[r]);
+    }
 #pragma unroll
-        for (int r = 0; r < PM_Q; r++) {
-            acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], 8);
-            acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], 16);
-            if (s0 == 0 && q0 + j + 8 * r < Q) A.uup[(size_t)g * Q + q0 + j + 8 * r] = acc[r];
-        }
+    for (int r = 0; r < PM_Q; r++) {
+        acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], 8);
+        acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], 16);
+        if (s0 == 0 && j + 8 * r < Q) A.uup[(size_t)g * Q + j + 8 * r] = acc[r];
     }
 }
 
@@ -332,11 +330,16 @@ void build_plan_matrices(kifmm_plan *P) {
     P->have_mats = true;
 }
 
-void launch_planned_p2m(kifmm_plan *P, const PassArgs &A) {
-    launch_pdl(k_planned_p2m, dim3(grid_for(P->n_p2m_list * 32, 256)), dim3(256), 0, P->stream, A,
+// the check points per lane that Nequiv takes (at most 64 points, eight lanes)
+template <int PM_Q = 1>
+static void launch_planned_p2m_q(kifmm_plan *P, const PassArgs &A) {
+    if constexpr (PM_Q < 8)
+        if (P->Q > 8 * PM_Q) return launch_planned_p2m_q<PM_Q + 1>(P, A);
+    launch_pdl(k_planned_p2m<PM_Q>, dim3(grid_for(P->n_p2m_list * 32, 256)), dim3(256), 0, P->stream, A,
                (const int32_t *)P->p2m_list.p, P->n_p2m_list, (const int64_t *)P->pm_p2m_off.p,
                (const double *)P->pm_p2m.p);
 }
+void launch_planned_p2m(kifmm_plan *P, const PassArgs &A) { launch_planned_p2m_q(P, A); }
 
 // Threads of a leaf's block: 64, so that many small blocks keep loads in flight
 // while others stage their charges or reduce (500k points, lists of 250: the near

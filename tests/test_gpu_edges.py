@@ -380,3 +380,21 @@ def test_complex_targets_in_runs():
     for a, b in ((0, 300), (cut - 300, cut + 300), (m - 300, m)):
         ref = f.evaluate_to_points(tx[a:b].contiguous(), ty[a:b].contiguous(), False)
         assert (pot[a:b] - ref).abs().max() <= (n + 16) * EPS * tau.abs().sum()
+
+
+@pytest.mark.parametrize("nequiv", [4, 7, 8, 9, 16, 17, 24, 25, 32, 33, 40, 41, 48, 49, 56, 57, 64])
+def test_planned_p2m_of_every_number_of_check_points(nequiv):
+    """Planned expansions, seen at separate targets (which use no planned matrix), are
+    those of the kernels: a check potential is the same sum in another order, carried
+    by the condition of the check-to-equivalent solve, about Nequiv / 2 (r2 /
+    r1)^(Nequiv / 2), over at most eight levels."""
+    x, y, tau = cloud(3000, 5)
+    tx, ty, _ = cloud(200, 6)
+    pots = []
+    for planned in (False, True):
+        f = fmm("laplace", 0.0, x, y, 30, nequiv=nequiv, planned=planned)
+        f.build_expansions(tau)
+        pots.append(f.evaluate_to_points(tx, ty, False))
+    r21 = (4 - np.sqrt(2) - 0.02) / (np.sqrt(2) + 0.01)
+    tol = 8 * EPS * nequiv / 2 * r21 ** (nequiv / 2)
+    assert np.abs(pots[1] - pots[0]).max() <= max(tol, 64 * EPS) * np.abs(pots[0]).max()
