@@ -284,47 +284,50 @@ __global__ void __launch_bounds__(MD_BLOCK, NR <= 6 ? 3 : 2) k_m2l_dmma(M2lDmmaA
         const int pl = tid - 32 * MD_CWARPS, n0 = pl / LQ, q0 = pl % LQ;
         const double *const src0 = A.uup + (int64_t)(A.T.off[l + 1] - 4 * eoff) * Q;
         int je[MAXI], dir = -1, issued = 0;
-        for (int pr = 0; pr < npair; pr++) {
-            const int sv = sst[pr], dd = (sv >> 2) & 7, sb = sv & 3, ctile = scm[dd];
-            if (dd != dir) {
-                dir = dd;
+        auto copy_stages = [&] {  // ends at a wait that runs out, here or in another warp
+            for (int pr = 0; pr < npair; pr++) {
+                const int sv = sst[pr], dd = (sv >> 2) & 7, sb = sv & 3, ctile = scm[dd];
+                if (dd != dir) {
+                    dir = dd;
 #pragma unroll
-                for (int i = 0; i < MAXI; i++) {
-                    const int n = n0 + i * RPP;  // -2: no copy (no such target, or a column tile passed over)
-                    je[i] = n < TE && ((ctile >> (n >> 3)) & 1) ? ssrc[n * 8 + dd] : -2;
-                }
-            }
-            for (int k0 = 0; k0 < kp; k0 += kc) {
-                if (round && !warp_wait_all(smem_u32(&empty[slot]), (uint32_t)(round - 1) & 1u, M.wait_limit)) {
-                    if (lane == 0) {
-                        *abort_flag = 1;
-                        atomicOr(M.err, 1ull);
+                    for (int i = 0; i < MAXI; i++) {
+                        const int n = n0 + i * RPP;  // -2: no copy (no such target, or a column tile passed over)
+                        je[i] = n < TE && ((ctile >> (n >> 3)) & 1) ? ssrc[n * 8 + dd] : -2;
                     }
-                    break;
                 }
-                if (*abort_flag) break;
-                const int kn = min(kc, kp - k0), kq = min(kc, Q - k0) >> 1;  // columns; 16-byte pieces of a vector
-                const uint32_t ob = smem_u32(&obar[slot]), od = smem_u32(sm_md + slot * stage_d);
-                if (pl == 0) mbar_expect_tx(ob, (uint32_t)(__popc(sv >> 8) * kn * ldq) * 8u);
-                __syncwarp();
-                if (pl < cp && ((sv >> (8 + pl)) & 1))
-                    bulk_g2s(od + (uint32_t)(pl * oblk) * 8u,
-                             opl + (size_t)m2l_slot(dd, ta0 + pl, sb) * M.B.block + (size_t)k0 * ldq,
-                             (uint32_t)(kn * ldq) * 8u, ob);
-                issued++;
-                const uint32_t xd = od + (uint32_t)(cp * oblk + n0 * ldx) * 8u;
-                for (int q = q0; q < kq; q += LQ) {
+                for (int k0 = 0; k0 < kp; k0 += kc) {
+                    if (round && !warp_wait_all(smem_u32(&empty[slot]), (uint32_t)(round - 1) & 1u, M.wait_limit)) {
+                        if (lane == 0) {
+                            *abort_flag = 1;
+                            atomicOr(M.err, 1ull);
+                        }
+                        return;
+                    }
+                    if (*abort_flag) return;
+                    const int kn = min(kc, kp - k0), kq = min(kc, Q - k0) >> 1;  // columns; 16-byte pieces of a vector
+                    const uint32_t ob = smem_u32(&obar[slot]), od = smem_u32(sm_md + slot * stage_d);
+                    if (pl == 0) mbar_expect_tx(ob, (uint32_t)(__popc(sv >> 8) * kn * ldq) * 8u);
+                    __syncwarp();
+                    if (pl < cp && ((sv >> (8 + pl)) & 1))
+                        bulk_g2s(od + (uint32_t)(pl * oblk) * 8u,
+                                 opl + (size_t)m2l_slot(dd, ta0 + pl, sb) * M.B.block + (size_t)k0 * ldq,
+                                 (uint32_t)(kn * ldq) * 8u, ob);
+                    issued++;
+                    const uint32_t xd = od + (uint32_t)(cp * oblk + n0 * ldx) * 8u;
+                    for (int q = q0; q < kq; q += LQ) {
 #pragma unroll
-                    for (int i = 0; i < MAXI; i++)
-                        if (je[i] != -2)  // -1: zeros
-                            cp_async16(xd + (uint32_t)(i * RPP * ldx + 2 * q) * 8u,
-                                       src0 + (je[i] >= 0 ? (4 * (int64_t)je[i] + sb) * Q + k0 + 2 * q : 0),
-                                       je[i] >= 0 ? 16 : 0);
+                        for (int i = 0; i < MAXI; i++)
+                            if (je[i] != -2)  // -1: zeros
+                                cp_async16(xd + (uint32_t)(i * RPP * ldx + 2 * q) * 8u,
+                                           src0 + (je[i] >= 0 ? (4 * (int64_t)je[i] + sb) * Q + k0 + 2 * q : 0),
+                                           je[i] >= 0 ? 16 : 0);
+                    }
+                    cp_async_arrive(smem_u32(&bars[slot]));
+                    if (++slot == nbuf) slot = 0, round++;
                 }
-                cp_async_arrive(smem_u32(&bars[slot]));
-                if (++slot == nbuf) slot = 0, round++;
             }
-        }
+        };
+        copy_stages();
         // every copy issued lands before the block goes on (consumed stages have
         // landed already; this matters after an abort)
         cp_async_wait_all();
@@ -332,29 +335,32 @@ __global__ void __launch_bounds__(MD_BLOCK, NR <= 6 ? 3 : 2) k_m2l_dmma(M2lDmmaA
             for (int st = issued > nbuf ? issued - nbuf : 0; st < issued; st++)
                 mbar_wait(smem_u32(&obar[st % nbuf]), (uint32_t)(st / nbuf) & 1u, kDrainWaitPolls);
     } else {
-        for (int pr = 0; pr < npair; pr++) {
-            const int sv = sst[pr], cm = scm[(sv >> 2) & 7];
-            const bool far = (sv >> (8 + ch)) & 1;
-            for (int k0 = 0; k0 < kp; k0 += kc) {
-                if (!warp_wait_both(smem_u32(&obar[slot]), smem_u32(&bars[slot]), (uint32_t)round & 1u, M.wait_limit)) {
-                    if (lane == 0) {
-                        *abort_flag = 1;
-                        atomicOr(M.err, 1ull);
+        auto compute_stages = [&] {
+            for (int pr = 0; pr < npair; pr++) {
+                const int sv = sst[pr], cm = scm[(sv >> 2) & 7];
+                const bool far = (sv >> (8 + ch)) & 1;
+                for (int k0 = 0; k0 < kp; k0 += kc) {
+                    if (!warp_wait_both(smem_u32(&obar[slot]), smem_u32(&bars[slot]), (uint32_t)round & 1u, M.wait_limit)) {
+                        if (lane == 0) {
+                            *abort_flag = 1;
+                            atomicOr(M.err, 1ull);
+                        }
+                        return;
                     }
-                    break;
+                    if (*abort_flag) return;
+                    if (far) {
+                        const double *os = sm_md + slot * stage_d;
+                        m2l_masked<NR, NCT, (1 << NCT) - 1>(cm, acc, os + (size_t)ch * oblk + t * ldq + row0 + g, ldq,
+                                                            os + (size_t)cp * oblk + (size_t)g * ldx + t, ldx,
+                                                            min(kc, kp - k0));
+                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&empty[slot]));  // this warp is done with the slot
+                    if (++slot == nbuf) slot = 0, round++;
                 }
-                if (*abort_flag) break;
-                if (far) {
-                    const double *os = sm_md + slot * stage_d;
-                    m2l_masked<NR, NCT, (1 << NCT) - 1>(cm, acc, os + (size_t)ch * oblk + t * ldq + row0 + g, ldq,
-                                                        os + (size_t)cp * oblk + (size_t)g * ldx + t, ldx,
-                                                        min(kc, kp - k0));
-                }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&empty[slot]));  // this warp is done with the slot
-                if (++slot == nbuf) slot = 0, round++;
             }
-        }
+        };
+        compute_stages();
     }
     __syncthreads();
     if (*abort_flag) return;
