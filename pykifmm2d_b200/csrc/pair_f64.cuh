@@ -41,9 +41,15 @@ static __device__ __constant__ double LOG_K[] = {-0.5 + LOG_H2 * LOG_H2 * 5.0 / 
                                                  -0.25 - LOG_H2 * 20.0 / 96.0, 0.2,
                                                  0.693147180559945309417232121458176568};
 
-// log_table(device) holds [LOGTAB_N] (v_i, -ln v_i); stage its copies into tab[LOGTAB_N * LOGTAB_COPIES] (all threads of the block)
+// log_table(device) holds [LOGTAB_N] (v_i, -ln v_i); stage its copies into
+// tab[LOGTAB_N * LOGTAB_COPIES] (all threads of the block; the lanes of a warp write
+// their copies in different bank groups)
 __device__ __forceinline__ void stage_log_table(double2 *tab, const double2 *__restrict__ g) {
-    for (int i = threadIdx.x; i < LOGTAB_N * LOGTAB_COPIES; i += blockDim.x) tab[i] = g[i / LOGTAB_COPIES];
+    for (int i = threadIdx.x; i < LOGTAB_N; i += blockDim.x) {
+        const double2 v = g[i];
+#pragma unroll
+        for (int c = 0; c < LOGTAB_COPIES; c++) tab[i * LOGTAB_COPIES + ((c + i) & (LOGTAB_COPIES - 1))] = v;
+    }
 }
 
 // ln(2^EADJ x); tl: this lane's copy, tab + (lane & 7).  x positive, normal,
