@@ -215,7 +215,6 @@ struct kifmm_plan {
     kifmm::DBuf<double> ops_tmp;     // [L][49] M2L offset blocks (operators.cu: M2lBlocks)
     kifmm::LevelOps lops[kifmm::MAX_LEVELS + 1]{};
     kifmm::DBuf<float> ops_f;        // FP32 copies for the mixed passes
-    kifmm::DBuf<uint16_t> ops_h;     // split half-precision M2L operators
     size_t ops_stride = 0;           // doubles per level block
     kifmm::DBuf<unsigned char> tc_a; // tensor-core M2L operator slices
     kifmm::DBuf<double> tc_rowscale;
@@ -433,10 +432,6 @@ __device__ __forceinline__ double2 green_c(double k, double r2) {
 __device__ __forceinline__ double2 green_z(int kind, double k, double r2) {
     if (kind == KIFMM_KERNEL_HELMHOLTZ) return green_c(k, r2);
     return make_double2(green_d(kind, k, r2), 0.0);
-}
-__device__ __forceinline__ float green_f(int kind, float k, float r2) {
-    if (kind == KIFMM_KERNEL_LAPLACE) return -0.0795774715f * __logf(r2);
-    return 0.159154943f * k0_f(k * sqrtf(r2));
 }
 
 // Morton helpers (interleave with the x bit above the y bit)

@@ -13,9 +13,6 @@
 
 namespace kifmm {
 
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-    return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
-}
 __device__ __forceinline__ void cacc(double2 &acc, double2 a, double2 b) {
     acc.x = fma(a.x, b.x, fma(-a.y, b.y, acc.x));
     acc.y = fma(a.x, b.y, fma(a.y, b.x, acc.y));

@@ -23,13 +23,7 @@ namespace kifmm {
 constexpr float LN2_OVER_4PI = 0.05515890934390497f;   // ln 2 / (4 pi)
 constexpr float INV_2PI_F = 0.15915494309189535f;
 
-// Kernel value in FP32 for relative offsets; Laplace returns log2(r^2)
-// (scaled by -ln2/(4pi) once at the end of each sum).
-template <int KIND>
-__device__ __forceinline__ float gsum_term(float r2, float k) {
-    if (KIND == KIFMM_KERNEL_LAPLACE) return __log2f(r2);
-    return k0_f(k * sqrtf(r2));
-}
+// scale of the near sums: Laplace sums log2(r^2)
 template <int KIND>
 __device__ __forceinline__ float gsum_scale() {
     return KIND == KIFMM_KERNEL_LAPLACE ? -LN2_OVER_4PI : INV_2PI_F;
@@ -104,18 +98,6 @@ __global__ void k_m2l_f(PassArgs A, int l) {
 #pragma unroll
         for (int t = 0; t < M2LF_TE; t++)
             if (schild[t] >= 0) A.udown[(size_t)schild[t] * Q + r] = (double)acc[t];
-}
-
-// Equivalent density of the local expansion (FP64), for the leaves a warp
-// evaluates.
-__device__ __forceinline__ void local_density(const PassArgs &A, int g, int l, double *qd, int lane) {
-    const double *inv = A.ops + (size_t)l * A.stride + A.off_inv;
-    for (int r = lane; r < A.Q; r += 32) {
-        double s = 0.0;
-        if (l >= 2)
-            for (int c = 0; c < A.Q; c++) s = fma(inv[r * A.Q + c], A.udown[(size_t)g * A.Q + c], s);
-        qd[r] = s;
-    }
 }
 
 // Taylor coefficients of every leaf's local expansion (Laplace, levels >= 2),
@@ -240,21 +222,11 @@ constexpr int LEAF_BLOCKS_PER_SM = KIFMM_LEAF_BLOCKS_PER_SM;  // resident blocks
 constexpr int LEAF_CHUNK = KIFMM_LEAF_CHUNK;                  // sources staged per pass
 static_assert(LEAF_CHUNK + 31 <= 200, "the leaf kernel's quotients (small_div) need cn + sp - 1 <= 200");
 
-__device__ __forceinline__ float pair_r2(float tx, float ty, const float4 &sv) {
-    const float dx = tx - sv.x, dy = ty - sv.y;
-    return fmaf(dx, dx, dy * dy);
-}
-// log2 of r^2 + FLT_MIN: the floor rides in the r^2 multiply-add instead of
-// a separate clamp.  Every pair of distinct points has r^2 >= 2^-48 (scaled
-// FP32 offsets of O(1)), where adding 2^-126 changes nothing; coincident
-// points give log2(FLT_MIN) exactly, as the clamp does.
-__device__ __forceinline__ float pair_lg2_floor(float tx, float ty, const float4 &sv) {
-    const float dx = tx - sv.x, dy = ty - sv.y;
-    return lg2_ftz(fmaf(dx, dx, fmaf(dy, dy, 1.17549435e-38f)));
-}
-
 constexpr f32x2 F2_FLOOR = 0x0080000000800000ull;  // (FLT_MIN, FLT_MIN)
-// r^2 + FLT_MIN of both targets to one source (as pair_lg2_floor)
+// r^2 + FLT_MIN of both targets to one source: the floor rides in the multiply-add
+// instead of a separate clamp.  Every pair of distinct points has r^2 >= 2^-48
+// (scaled FP32 offsets of O(1)), where adding 2^-126 changes nothing; coincident
+// points give FLT_MIN exactly, as a clamp does.
 __device__ __forceinline__ f32x2 pair2_r2_floor(f32x2 tx, f32x2 ty, const ulonglong2 &s) {
     const f32x2 dx = f2_sub(tx, s.x), dy = f2_sub(ty, s.y);
     return f2_fma(dx, dx, f2_fma(dy, dy, F2_FLOOR));
