@@ -235,7 +235,7 @@ class FMM(object):
                  svd_fmm.py:239-242, :281-290);
       device, stream   CUDA device ordinal and stream handle.
     Unlike the reference, repeated ``build_expansions`` calls on one object
-    are exact (workspaces are zeroed on every apply).
+    are exact (every apply writes the same expansions anew).
     """
 
     def __init__(self, x, y, kernel_functions, numba_functions, Nequiv=48, Ncutoff=50, iscomplex=False,

@@ -65,11 +65,10 @@ struct PairSum {
 // Whether a target's r^2 to a source may be infinite or not a number.  The
 // unchecked Laplace loop, which looks for small r^2 only, would take such a pair
 // for an ordinary one.  Sources are checked when the tree is built; separate
-// targets are anything.
-template <int KIND>
+// targets are anything (targets.cu).
 __device__ __forceinline__ bool out_of_reach(double x, double y) {
     constexpr double REACH = 0x1p500;  // r^2 stays below 2^1002
-    return KIND == KIFMM_KERNEL_LAPLACE && !(fabs(x) < REACH && fabs(y) < REACH);
+    return !(fabs(x) < REACH && fabs(y) < REACH);
 }
 
 // Sums of the lane's TB targets over sources u, u + sp, ... below n.  CHECKED
@@ -203,7 +202,7 @@ struct LeafItem {
     const double *tx, *ty;  // target coordinates, at idx[t0 .. t0 + nt) or, without idx, at t0 ..
     const int32_t *idx;
     int t0, nt, n_own, ns, l, lane;
-    int lanes;              // targets that the lanes are laid out for (>= nt): a sum's order depends on this
+    int lanes;              // targets that set the lanes' stride over the sources (>= nt): a sum's order depends on it
     double cx, cy;
     const double *den;
     bool check_self;
@@ -213,25 +212,22 @@ struct LeafItem {
 // points of its local expansion; the sums are returned to lanes < nt
 template <int KIND, bool CPLX, bool FAR, int NT, bool BEYOND, int TB>
 __device__ __forceinline__ PairSum<KIND, CPLX> leaf_item(const PassArgs &A, PairWarp<KIND, CPLX> &W, const double2 *tl,
-                                                         const LeafItem &I, unsigned hi_end) {
+                                                         const LeafItem &I, unsigned hi_end,
+                                                         int ng) {
     constexpr int NC = PairWarp<KIND, CPLX>::NC;
     const int nt = I.nt, lane = I.lane;
-    const int ng = (I.lanes + TB - 1) / TB, sp = 32 / ng, j = lane / ng, gi = lane - j * ng;
+    const int sp = 32 / ng, j = lane / ng, gi = lane - j * ng;
     double tx[TB], ty[TB];
     PairSum<KIND, CPLX> acc[TB];
-    bool wild = false;  // a separate target out of the unchecked loop's reach
 #pragma unroll
     for (int a = 0; a < TB; a++) {
         int i = I.t0 + (gi + a * ng < nt ? gi + a * ng : min(gi, nt - 1));  // unused slots repeat another
         if (I.idx) i = I.idx[i];
         tx[a] = I.tx[i];
         ty[a] = I.ty[i];
-        if (I.idx) wild = wild || out_of_reach<KIND>(tx[a], ty[a]);
 #pragma unroll
         for (int c = 0; c < NC; c++) acc[a].c[c] = 0.0;
     }
-    if (I.idx) wild = __any_sync(0xffffffffu, wild);
-    const int n_own = wild ? I.ns : I.n_own;
     const int u0 = j < sp ? j : 1 << 20;  // lanes past the last group idle
     for (int c0 = 0; !FAR && c0 < I.ns; c0 += L64_CHUNK) {
         const int cn = min(L64_CHUNK, I.ns - c0);
@@ -245,7 +241,7 @@ __device__ __forceinline__ PairSum<KIND, CPLX> leaf_item(const PassArgs &A, Pair
             }
         }
         __syncwarp();
-        pair_chunk<KIND, CPLX, NT, TB, BEYOND>(W, tl, u0, sp, min(n_own - c0, cn), cn, tx, ty, A.k, I.k2, hi_end,
+        pair_chunk<KIND, CPLX, NT, TB, BEYOND>(W, tl, u0, sp, min(I.n_own - c0, cn), cn, tx, ty, A.k, I.k2, hi_end,
                                                I.check_self, acc);
     }
     if (I.l >= 2) {
@@ -262,7 +258,7 @@ __device__ __forceinline__ PairSum<KIND, CPLX> leaf_item(const PassArgs &A, Pair
             tx[a] -= I.cx;
             ty[a] -= I.cy;
         }
-        pair_chunk<KIND, CPLX, NT, TB, BEYOND>(W, tl, u0, sp, wild ? Qc : 0, Qc, tx, ty, A.k, I.k2, hi_end, false, acc);
+        pair_chunk<KIND, CPLX, NT, TB, BEYOND>(W, tl, u0, sp, 0, Qc, tx, ty, A.k, I.k2, hi_end, false, acc);
     }
     __syncwarp();
 #pragma unroll
@@ -283,29 +279,40 @@ __device__ __forceinline__ PairSum<KIND, CPLX> leaf_item(const PassArgs &A, Pair
     for (int c = 0; c < NC; c++) v.c[c] *= pair_scale<KIND>();
     return v;
 }
-template <int KIND, bool CPLX, bool FAR, int NT, bool BEYOND = false>
+// REST: a tile may hold fewer targets than its layout is for (separate targets)
+template <int KIND, bool CPLX, bool FAR, bool REST, int NT, bool BEYOND = false>
 __device__ __forceinline__ PairSum<KIND, CPLX> leaf_item_tb(const PassArgs &A, PairWarp<KIND, CPLX> &W,
                                                             const double2 *tl, const LeafItem &I, unsigned hi_end) {
     // the number of targets per lane that leaves the fewest lanes idle: pair
-    // slots per source TB / (32 / ceil(nt / TB)), compared by cross products
-    if constexpr (BEYOND) return leaf_item<KIND, CPLX, FAR, NT, true, 2>(A, W, tl, I, hi_end);  // (a larger body)
+    // slots per source TB / (32 / ceil(lanes / TB)), compared by cross products
+    const int g2 = (I.lanes + 1) >> 1;
+    if constexpr (BEYOND) return leaf_item<KIND, CPLX, FAR, NT, true, 2>(A, W, tl, I, hi_end, g2);  // (a larger body)
     else {
-        const int s2 = 32 / ((I.lanes + 1) >> 1), s3 = 32 / ((I.lanes + 2) / 3), s4 = 32 / ((I.lanes + 3) >> 2);
-        if (s4 * 3 >= s3 * 4 && s4 * 2 >= s2 * 4) return leaf_item<KIND, CPLX, FAR, NT, BEYOND, 4>(A, W, tl, I, hi_end);
-        if (s3 * 2 >= s2 * 3) return leaf_item<KIND, CPLX, FAR, NT, BEYOND, 3>(A, W, tl, I, hi_end);
-        return leaf_item<KIND, CPLX, FAR, NT, BEYOND, 2>(A, W, tl, I, hi_end);
+        const int g3 = (I.lanes + 2) / 3, g4 = (I.lanes + 3) >> 2, s2 = 32 / g2, s3 = 32 / g3, s4 = 32 / g4;
+        const bool four = s4 * 3 >= s3 * 4 && s4 * 2 >= s2 * 4, three = s3 * 2 >= s2 * 3;
+        if constexpr (!REST) {
+            if (four) return leaf_item<KIND, CPLX, FAR, NT, BEYOND, 4>(A, W, tl, I, hi_end, g4);
+            if (three) return leaf_item<KIND, CPLX, FAR, NT, BEYOND, 3>(A, W, tl, I, hi_end, g3);
+            return leaf_item<KIND, CPLX, FAR, NT, BEYOND, 2>(A, W, tl, I, hi_end, g2);
+        }
+        // fewer targets than the layout is for: as many per lane as they need
+        const int ng = four ? g4 : three ? g3 : g2;
+        if (I.nt > 3 * ng) return leaf_item<KIND, CPLX, FAR, NT, BEYOND, 4>(A, W, tl, I, hi_end, ng);
+        if (I.nt > 2 * ng) return leaf_item<KIND, CPLX, FAR, NT, BEYOND, 3>(A, W, tl, I, hi_end, ng);
+        if (I.nt <= ng) return leaf_item<KIND, CPLX, FAR, NT, BEYOND, 1>(A, W, tl, I, hi_end, ng);
+        return leaf_item<KIND, CPLX, FAR, NT, BEYOND, 2>(A, W, tl, I, hi_end, ng);
     }
 }
 
 // ... with the series that reaches to tmax, the largest (k r)^2 inside the boxes
-template <int KIND, bool CPLX, bool FAR>
+template <int KIND, bool CPLX, bool FAR, bool REST = false>
 __device__ __forceinline__ PairSum<KIND, CPLX> leaf_item_series(const PassArgs &A, PairWarp<KIND, CPLX> &W,
                                                                 const double2 *tl, const LeafItem &I, double tmax) {
-    if (KIND == KIFMM_KERNEL_LAPLACE) return leaf_item_tb<KIND, CPLX, FAR, 1>(A, W, tl, I, LOG_HI_END);
-    if (tmax < 0.0625) return leaf_item_tb<KIND, CPLX, FAR, SERIES_NARROW>(A, W, tl, I, SERIES_NARROW_HI);
-    if (tmax < 1.0) return leaf_item_tb<KIND, CPLX, FAR, SERIES_MID>(A, W, tl, I, SERIES_MID_HI);
-    if (tmax < 4.0) return leaf_item_tb<KIND, CPLX, FAR, SERIES_WIDE>(A, W, tl, I, SERIES_WIDE_HI);
-    return leaf_item_tb<KIND, CPLX, FAR, SERIES_WIDE, true>(A, W, tl, I, SERIES_WIDE_HI);
+    if (KIND == KIFMM_KERNEL_LAPLACE) return leaf_item_tb<KIND, CPLX, FAR, REST, 1>(A, W, tl, I, LOG_HI_END);
+    if (tmax < 0.0625) return leaf_item_tb<KIND, CPLX, FAR, REST, SERIES_NARROW>(A, W, tl, I, SERIES_NARROW_HI);
+    if (tmax < 1.0) return leaf_item_tb<KIND, CPLX, FAR, REST, SERIES_MID>(A, W, tl, I, SERIES_MID_HI);
+    if (tmax < 4.0) return leaf_item_tb<KIND, CPLX, FAR, REST, SERIES_WIDE>(A, W, tl, I, SERIES_WIDE_HI);
+    return leaf_item_tb<KIND, CPLX, FAR, REST, SERIES_WIDE, true>(A, W, tl, I, SERIES_WIDE_HI);
 }
 
 // 16 warps per SM at 128 registers measured 1-5% faster than 24 at 80 (the K0

@@ -11,7 +11,10 @@
 // over the nodes that lays out the groups and their work items, and one pass
 // that writes the targets' indices in group order; a Morton sort of the targets
 // took ten passes over them (0.32 of 1.26 ms at 3M targets).  The order within a
-// group is whatever the atomics give: no target's sum depends on it.
+// group is whatever the atomics give, and with it the targets that share an item;
+// no target's sum depends on it, so that equal calls give equal bits: the FP32 form
+// sums a target on one lane, the others split the sources over lanes in the same
+// way for all of a leaf's targets (TargetItem::lanes).
 #include "leaf_f32.cuh"
 #include "pass_f64.cuh"
 
@@ -19,23 +22,27 @@ namespace kifmm {
 
 struct TargetItem {
     int g, start;    // leaf, first grouped target
-    short n, lanes;  // targets (<= TI_MAX), the largest n of the leaf's items
+    short n, lanes;  // targets (<= TI_MAX); those of the leaf's largest 32-target tile
     int level;
 };
 constexpr int TI_MAX = 64;  // most targets of an item: two per lane in the packed FP32 loop
 
-// counters of a call (P->tcount): [0] targets laid out, [1] items, [2] ticket
-enum { TC_TARGETS, TC_ITEMS, TC_TICKET, TC_WORDS };
+// counters of a call (P->tcount): targets laid out, items, ticket; targets left out of
+// the groups
+enum { TC_TARGETS, TC_ITEMS, TC_TICKET, TC_APART, TC_WORDS };
 
 constexpr int TL_THREADS = 256, TL_PER = 8, TL_TILE = TL_THREADS * TL_PER, TL_SLOTS = 2 * TL_TILE;
 // the leaf of every target and its rank among the leaf's targets; cnt[node]:
 // targets of the node.  The strict '>' descent takes, level by level, the bits of
 // the target's cell on the key grid (whose lines are the cells' midlines at
-// every level): the coordinates clamped into the box, NaN in cell 0.
+// every level): the coordinates clamped into the box, NaN in cell 0.  order (or
+// null): targets out of reach are left out of the groups, leaf ~g, and listed from its
+// end.
 __global__ void __launch_bounds__(TL_THREADS) k_target_leaf(PassArgs A, const double *__restrict__ tx,
                                                             const double *__restrict__ ty, int64_t n, double h,
                                                             unsigned *__restrict__ cnt, int32_t *__restrict__ leaf,
-                                                            unsigned *__restrict__ rank) {
+                                                            unsigned *__restrict__ rank, unsigned *__restrict__ tcount,
+                                                            int32_t *__restrict__ order) {
     __shared__ int key[TL_SLOTS];
     __shared__ unsigned num[TL_SLOTS];
     for (int i = threadIdx.x; i < TL_SLOTS; i += TL_THREADS) {
@@ -45,13 +52,14 @@ __global__ void __launch_bounds__(TL_THREADS) k_target_leaf(PassArgs A, const do
     __syncthreads();
     const int64_t i0 = (int64_t)blockIdx.x * TL_TILE;
     int slot[TL_PER], lf[TL_PER];
-    unsigned rk[TL_PER], cx[TL_PER], cy[TL_PER];
+    unsigned rk[TL_PER], cx[TL_PER], cy[TL_PER], apart = 0;
     // the thread's descents side by side, a level of all of them per pass: their
     // node loads overlap
 #pragma unroll
     for (int k = 0; k < TL_PER; k++) {
         const int64_t i = i0 + k * TL_THREADS + threadIdx.x;
         const double px = i < n ? tx[i] : 0.0, py = i < n ? ty[i] : 0.0;
+        if (order && out_of_reach(px, py)) apart |= 1u << k;
         cx[k] = h > 0 && px == px ? (unsigned)grid_cell(px, A.root, h) << (32 - KEY_DEPTH) : 0u;
         cy[k] = h > 0 && py == py ? (unsigned)grid_cell(py, A.root, h) << (32 - KEY_DEPTH) : 0u;
         lf[k] = 0;
@@ -79,6 +87,11 @@ __global__ void __launch_bounds__(TL_THREADS) k_target_leaf(PassArgs A, const do
         const int64_t i = i0 + k * TL_THREADS + threadIdx.x;
         slot[k] = -1;
         if (i >= n) continue;
+        if ((apart >> k) & 1u) {
+            leaf[i] = ~lf[k];
+            order[n - 1 - atomicAdd(&tcount[TC_APART], 1u)] = (int32_t)i;
+            continue;
+        }
         int s = (int)((unsigned)lf[k] * 2654435761u >> 20) & (TL_SLOTS - 1);
         for (;;) {  // at most TL_TILE distinct leaves in twice as many slots
             const int was = atomicCAS(&key[s], -1, lf[k]);
@@ -101,10 +114,8 @@ __global__ void __launch_bounds__(TL_THREADS) k_target_leaf(PassArgs A, const do
     }
 }
 
-// first position of each node's targets, and the work items of at most `per`
-// targets: as many whole ones as there are and the rest, or (even) all of a leaf's
-// within one target of each other, so that they can share a lane layout
-__global__ void k_target_items(PassArgs A, int64_t nn, int per, bool even, const unsigned *__restrict__ cnt,
+// first position of each node's targets, and the work items of `per` targets
+__global__ void k_target_items(PassArgs A, int64_t nn, int per, const unsigned *__restrict__ cnt,
                                unsigned *__restrict__ off, TargetItem *__restrict__ items,
                                unsigned *__restrict__ tcount) {
     const int lane = threadIdx.x & 31;
@@ -130,23 +141,24 @@ __global__ void k_target_items(PassArgs A, int64_t nn, int per, bool even, const
         const unsigned cj = __shfl_sync(0xffffffffu, c, j), oj = __shfl_sync(0xffffffffu, bc, j),
                        fj = __shfl_sync(0xffffffffu, bi, j), nj = __shfl_sync(0xffffffffu, it, j);
         const int lv = A.nlev[g0 + j];
-        const unsigned w = even ? cj / nj : per, rest = even ? cj - w * nj : 0;
-        for (unsigned q = lane; q < nj; q += 32) {
-            const unsigned b = q * w + min(q, rest), n = min(w + (q < rest), cj - b);
-            items[fj + q] = TargetItem{(int)(g0 + j), (int)(oj + b), (short)n, (short)(w + (rest != 0)), lv};
-        }
+        const short lanes = (short)min(min(cj, (unsigned)per), 32u);
+        for (unsigned q = lane; q < nj; q += 32)
+            items[fj + q] =
+                TargetItem{(int)(g0 + j), (int)(oj + q * per), (short)min((unsigned)per, cj - q * per), lanes, lv};
     }
 }
 
 __global__ void k_target_place(int64_t n, const int32_t *__restrict__ leaf, const unsigned *__restrict__ rank,
                                const unsigned *__restrict__ off, int32_t *__restrict__ order) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        order[off[leaf[i]] + rank[i]] = (int32_t)i;
+        if (leaf[i] >= 0) order[off[leaf[i]] + rank[i]] = (int32_t)i;
 }
 
 struct TargetArgs {
     const double *tx, *ty;     // targets in the caller's order
-    const int32_t *order;      // their indices in group order
+    int64_t n;
+    const int32_t *leaf;       // their leaves (~leaf: not in a group)
+    const int32_t *order;      // their indices in group order, then those not in a group
     const double *den;         // [n_nodes][Q] equivalent densities
     const TargetItem *items;
     unsigned *tcount;
@@ -185,10 +197,50 @@ __device__ __forceinline__ unsigned next_item(const TargetArgs &T, int lane) {
     return __shfl_sync(0xffffffffu, it, 0);
 }
 
+// Laplace sum of a target out of reach over n equivalent points at x[q], x[n + q]:
+// whatever log() gives
+template <bool CPLX>
+__device__ __noinline__ PairSum<KIFMM_KERNEL_LAPLACE, CPLX> far_apart(const double *x, const double *den, int n,
+                                                                      double px, double py) {
+    constexpr int LAP = KIFMM_KERNEL_LAPLACE;
+    PairSum<LAP, CPLX> v{};
+    for (int q = 0; q < n; q++) {
+        const double dx = px - x[q], dy = py - x[n + q];
+        const PairValue g = pair_value_any<LAP>(fma(dx, dx, dy * dy), 0.0);
+        if constexpr (CPLX) v.add(g, make_double2(den[q], den[n + q]), double2{});
+        else v.add(g, den[q], double2{});
+    }
+    return v;
+}
+// ... its potential at leaf g, near sources first
+template <bool CPLX>
+__device__ __noinline__ void target_apart(const PassArgs &A, const TargetArgs &T, int64_t i) {
+    constexpr int LAP = KIFMM_KERNEL_LAPLACE;
+    const int g = ~T.leaf[i];
+    const double px = T.tx[i], py = T.ty[i];
+    PairSum<LAP, CPLX> v{}, far{};
+    for (int d = 0; d < 9; d++) {
+        const int c = A.ncoll[9 * (size_t)g + d];
+        for (int s = c >= 0 ? A.nbot[c] : 0, e = c >= 0 ? A.ntop[c] : 0; s < e; s++) {
+            const double dx = px - A.xs[s], dy = py - A.ys[s];
+            v.add(pair_value_any<LAP>(fma(dx, dx, dy * dy), 0.0), load_value<CPLX>(A.taus, s), double2{});
+        }
+    }
+    const int l = A.nlev[g];
+    if (l >= 2) {
+        double cx, cy;
+        node_center(A, g, l, cx, cy);
+        far = far_apart<CPLX>(A.ops + (size_t)l * A.stride + A.off_large, T.den + (size_t)g * A.Q, A.Qc, px - cx, py - cy);
+    }
+    for (int c = 0; c < PairWarp<LAP, CPLX>::NC; c++)
+        T.pot[PairWarp<LAP, CPLX>::NC * i + c] = (v.c[c] + far.c[c]) * pair_scale<LAP>();
+}
+
 // FP64, real or complex: the leaf pass's pair loops on the item's targets
 template <int KIND, bool CPLX>
 __global__ void __launch_bounds__(32 * L64_MAX_WARPS, L64_BLOCKS_PER_SM)
-    k_eval_targets_d(PassArgs A, const double2 *__restrict__ logtab, TargetArgs T) {
+    k_eval_targets_d(const __grid_constant__ PassArgs A, const double2 *__restrict__ logtab,
+                     const __grid_constant__ TargetArgs T) {
     extern __shared__ __align__(16) unsigned char sm_tgd[];
     double2 *tab = (double2 *)sm_tgd;
     auto &W = ((PairWarp<KIND, CPLX> *)(tab + LOGTAB_N * LOGTAB_COPIES))[threadIdx.x >> 5];
@@ -212,14 +264,21 @@ __global__ void __launch_bounds__(32 * L64_MAX_WARPS, L64_BLOCKS_PER_SM)
         node_center(A, J.g, J.level, I.cx, I.cy);
         I.den = T.den + (size_t)J.g * A.Q;
         const double wl = ldexp(A.W, -J.level);
-        I.t0 = J.start;
-        I.nt = J.n;
         I.lanes = J.lanes;
-        const PairSum<KIND, CPLX> v = leaf_item_series<KIND, CPLX, false>(A, W, tl, I, 8.0 * wl * wl * I.k2);
-        if (lane >= I.nt) continue;
-        const int o = T.order[I.t0 + lane];
-        if constexpr (CPLX) ((double2 *)T.pot)[o] = make_double2(v.c[0], v.c[1]);
-        else T.pot[o] = v.c[0];
+        for (int t0 = 0; t0 < J.n; t0 += 32) {
+            I.t0 = J.start + t0;
+            I.nt = min(32, J.n - t0);
+            const PairSum<KIND, CPLX> v = leaf_item_series<KIND, CPLX, false, true>(A, W, tl, I, 8.0 * wl * wl * I.k2);
+            if (lane >= I.nt) continue;
+            const int o = T.order[I.t0 + lane];
+            if constexpr (CPLX) ((double2 *)T.pot)[o] = make_double2(v.c[0], v.c[1]);
+            else T.pot[o] = v.c[0];
+        }
+    }
+    if constexpr (KIND == KIFMM_KERNEL_LAPLACE) {
+        const unsigned na = T.tcount[TC_APART];
+        for (unsigned w = blockIdx.x * blockDim.x + threadIdx.x; w < na; w += gridDim.x * blockDim.x)
+            target_apart<CPLX>(A, T, T.order[T.n - 1 - w]);
     }
 }
 
@@ -308,13 +367,11 @@ __device__ __forceinline__ void target_item_f(const PassArgs &A, const TargetArg
     const int ns = warp_ranges(A, J.g, false, W.rng, lane);
     double tx[TB], ty[TB];
     float rx[TB], ry[TB], acc[TB];
-    bool wild = false;
 #pragma unroll
     for (int a = 0; a < TB; a++) {
         const int i = T.order[J.start + min(lane + 32 * a, J.n - 1)];  // lanes past the end repeat the last target
         tx[a] = T.tx[i] - cx;
         ty[a] = T.ty[i] - cy;
-        wild = wild || out_of_reach<KIND>(tx[a], ty[a]);
         rx[a] = (float)tx[a];
         ry[a] = (float)ty[a];
         acc[a] = 0.f;
@@ -330,8 +387,7 @@ __device__ __forceinline__ void target_item_f(const PassArgs &A, const TargetArg
         __syncwarp();
         const double wl = ldexp(A.W, -J.level), k2 = pair_k2(A.k), tmax = 4.0 * wl * wl * k2;  // r < 2 w inside the box
         if (KIND == KIFMM_KERNEL_LAPLACE)
-            pair_chunk<KIND, false, 1, TB, false>(W, tl, 0, 1, wild ? A.Q : 0, A.Q, tx, ty, A.k, k2, LOG_HI_END, false,
-                                                  far);
+            pair_chunk<KIND, false, 1, TB, false>(W, tl, 0, 1, 0, A.Q, tx, ty, A.k, k2, LOG_HI_END, false, far);
         else if (tmax < 0.0625)
             pair_chunk<KIND, false, SERIES_NARROW, TB, false>(W, tl, 0, 1, 0, A.Q, tx, ty, A.k, k2, SERIES_NARROW_HI,
                                                               false, far);
@@ -344,6 +400,11 @@ __device__ __forceinline__ void target_item_f(const PassArgs &A, const TargetArg
         else
             pair_chunk<KIND, false, SERIES_WIDE, TB, true>(W, tl, 0, 1, 0, A.Q, tx, ty, A.k, k2, SERIES_WIDE_HI, false,
                                                            far);
+        if constexpr (KIND == KIFMM_KERNEL_LAPLACE) {
+#pragma unroll
+            for (int a = 0; a < TB; a++)
+                if (out_of_reach(tx[a], ty[a])) far[a] = far_apart<false>(lg, den, A.Q, tx[a], ty[a]);
+        }
     }
 #pragma unroll
     for (int a = 0; a < TB; a++)
@@ -373,11 +434,11 @@ __global__ void __launch_bounds__(32 * TF_WARPS, TF_BLOCKS_PER_SM)
 static TargetArgs group_targets(kifmm_plan *P, const PassArgs &A, const double *tx, const double *ty, int64_t n,
                                 int check_self, bool fp32, double *pot) {
     cudaStream_t s = P->stream;
-    // Targets per item: 64 in the FP32 form, which keeps a target on one lane, 32 in
-    // the others; fewer where that leaves the resident warps less than four items
-    // each (a launch of 1.3 rounds of items lasts two), down to 32 and 8.
+    // Targets per item: 64, fewer where that leaves the resident warps less than
+    // four items each (a launch of 1.3 rounds of items lasts two); down to 32 for
+    // the FP32 form, which keeps a target on one lane, and to 8 for the others.
     const int64_t nn = P->n_nodes, want = 4 * (int64_t)P->num_sms * L64_BLOCKS_PER_SM * L64_MAX_WARPS;
-    int per = fp32 ? TI_MAX : 32;
+    int per = TI_MAX;
     while (per > (fp32 ? 32 : 8) && n / per < want) per >>= 1;
     const int64_t max_items = (n + per - 1) / per + std::min(n, nn);
     P->tleaf.alloc(n);
@@ -388,14 +449,17 @@ static TargetArgs group_targets(kifmm_plan *P, const PassArgs &A, const double *
     unsigned *cnt = P->tcount.p + TC_WORDS, *off = cnt + nn;
     KIFMM_CUDA(cudaMemsetAsync(P->tcount.p, 0, (TC_WORDS + nn) * sizeof(unsigned), s));
     k_target_leaf<<<(unsigned)((n + TL_TILE - 1) / TL_TILE), TL_THREADS, 0, s>>>(
-        A, tx, ty, n, std::ldexp(P->W, -KEY_DEPTH), cnt, P->tleaf.p, P->trank.p);
+        A, tx, ty, n, std::ldexp(P->W, -KEY_DEPTH), cnt, P->tleaf.p, P->trank.p, P->tcount.p,
+        P->kern.kind == KIFMM_KERNEL_LAPLACE && !fp32 ? P->tperm.p : nullptr);
     KIFMM_LAUNCHED();
-    k_target_items<<<(unsigned)((nn + 255) / 256), 256, 0, s>>>(A, nn, per, !fp32, cnt, off, (TargetItem *)P->titems.p,
+    k_target_items<<<(unsigned)((nn + 255) / 256), 256, 0, s>>>(A, nn, per, cnt, off, (TargetItem *)P->titems.p,
                                                                 P->tcount.p);
     KIFMM_LAUNCHED();
     k_target_place<<<grid_for(n, 256, P->num_sms * 16), 256, 0, s>>>(n, P->tleaf.p, P->trank.p, off, P->tperm.p);
     KIFMM_LAUNCHED();
     TargetArgs T{};
+    T.n = n;
+    T.leaf = P->tleaf.p;
     T.tx = tx;
     T.ty = ty;
     T.order = P->tperm.p;
