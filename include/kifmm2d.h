@@ -153,7 +153,8 @@ int kifmm_build_tree(kifmm_plan *plan, const double *x, const double *y, int64_t
 int kifmm_precompute(kifmm_plan *plan);
 
 /* FMM.build_expansions(tau) (class_fmm.py:299-352): P2M, M2M, M2L, L2L.
- * Every call starts from zeroed workspaces (a repeated apply is exact). */
+ * A repeated apply is exact: every call writes the same nodes' expansions, the
+ * others stay zero (cleared with the tree). */
 int kifmm_build_expansions(kifmm_plan *plan, const double *tau, int32_t mem);
 
 /* FMM.evaluate_to_points(x, y, check_self) at the plan's own source points
