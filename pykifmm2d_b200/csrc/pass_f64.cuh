@@ -20,7 +20,7 @@ const double *launch_node_density(kifmm_plan *P, const PassArgs &A);
 // (its own points, then its colleagues') are staged in chunks; the L2P is the
 // same loop over the Q equivalent points of the leaf's local expansion, in
 // box-relative coordinates.  Bound by issue: 12 FP64 instructions (two slots
-// each) and about 9 others per Laplace pair.  Warps draw items from a ticket
+// each) and about 10 others per Laplace pair.  Warps draw items from a ticket
 // (the leaves differ in work by more than 10x); each warp draws one ticket past
 // the end, so atomicInc's wrap leaves the counter at zero for the next launch.
 constexpr int L64_CHUNK = 64;  // sources staged per pass, two per lane

@@ -170,7 +170,10 @@ __global__ void k_planned_p2m(PassArgs A, const int32_t *__restrict__ p2m, int64
 constexpr int PL_ROWS = 4;
 constexpr int PL_STAGE = 4096;      // bytes of staged charges
 
-// asks for `bytes` (a multiple of 16, from a 16-byte boundary) to be brought into L2
+// asks for `bytes` (a multiple of 16, from a 16-byte boundary) to be brought into L2;
+// blocks up to L2_AHEAD bytes are asked for whole (a block of several GB, from leaves of
+// 11,000 points, has a size that the instruction's 32 bits do not hold)
+constexpr int64_t L2_AHEAD = 8 << 20;
 __device__ __forceinline__ void l2_prefetch(const void *p, uint32_t bytes) {
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
@@ -195,7 +198,8 @@ __global__ void __launch_bounds__(THREADS) k_planned_near(PassArgs A, const int6
     if (tid < LEAF_REC_WORDS) rec[tid] = A.leaf_rec[i * LEAF_REC_WORDS + tid];
     const int64_t n0 = near_off[i];
     const int64_t sz = near_off[i + 1] - n0;
-    if (sizeof(T) == 4 && tid == 0 && sz > 0) l2_prefetch(near + n0, (uint32_t)(sz * sizeof(T)));
+    if (sizeof(T) == 4 && tid == 0 && sz > 0 && sz * (int64_t)sizeof(T) <= L2_AHEAD)
+        l2_prefetch(near + n0, (uint32_t)(sz * sizeof(T)));
     __syncthreads();
     const int b = rec[LR_BOT], nt = rec[LR_TOP] - b, ns = rec[LR_NSRC];
     const int nsp = (int)pad_row(ns, VW);
