@@ -168,6 +168,7 @@ static int guarded(F &&f) {
         f();
         return KIFMM_OK;
     } catch (const Fail &e) {
+        cudaGetLastError();  // reported here: not to be met again by the next call's launches
         return e.code;
     } catch (const std::bad_alloc &) {
         set_error("host allocation failed");
