@@ -95,6 +95,7 @@ void launch_leaf_eval_d(kifmm_plan *P, const PassArgs &A, int check_self);
 // planned.cu
 void launch_planned_p2m(kifmm_plan *P, const PassArgs &A);
 void launch_planned_near(kifmm_plan *P, cudaStream_t s);
+bool planned_near_fits(const kifmm_plan *P);
 void run_planned_leaf(kifmm_plan *P, const PassArgs &A);
 // passes_complex.cu (complex values: FP64 point passes on double2 densities)
 void launch_gather_tau_c(kifmm_plan *P);

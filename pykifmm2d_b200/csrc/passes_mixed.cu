@@ -847,6 +847,7 @@ static bool near_form(const kifmm_plan *P) {
 }
 bool near_possible(kifmm_plan *P) {
     if (!near_form(P) || P->n_leaf_list <= 0 || (P->opt.planned != 0) != planned_ready(P)) return false;
+    if (P->opt.planned && !planned_near_fits(P)) return false;
     if (callers_capture(P)) return false;  // it may end between the apply and the evaluation that joins
     ensure_aux_streams(P);
     return true;

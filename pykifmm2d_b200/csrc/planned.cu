@@ -349,9 +349,15 @@ void launch_planned_p2m(kifmm_plan *P, const PassArgs &A) { launch_planned_p2m_q
 // while others stage their charges or reduce (500k points, lists of 250: the near
 // pass 157 us, 175 with 128 threads); 256 where there are too few leaves to fill
 // the GPU and a leaf's own time counts (10k points: an apply 55 us, 90 with 64).
+static size_t near_smem(const kifmm_plan *P) {
+    return PL_STAGE + (size_t)P->ppl * sizeof(double);  // leaves hold <= Ncutoff points
+}
+// Whether a leaf's sums fit in shared memory.  Where they do not, the evaluation at
+// the sources fails; an apply must not, since other evaluations need no near matrix.
+bool planned_near_fits(const kifmm_plan *P) { return near_smem(P) + 1024 <= (size_t)(227 << 10); }
 template <typename T, int THREADS>
 static void launch_near(kifmm_plan *P, cudaStream_t s, const T *mat) {
-    const size_t smem = PL_STAGE + (size_t)P->ppl * sizeof(double);  // leaves hold <= Ncutoff points
+    const size_t smem = near_smem(P);
     ensure_dyn_smem(k_planned_near<T, THREADS>, smem);
     launch_pdl(k_planned_near<T, THREADS>, dim3((unsigned)P->n_leaf_list), dim3(THREADS), smem, s, make_pass_args(P),
                (const int64_t *)P->pm_near_off.p, mat);

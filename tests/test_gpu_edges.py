@@ -398,3 +398,26 @@ def test_planned_p2m_of_every_number_of_check_points(nequiv):
     r21 = (4 - np.sqrt(2) - 0.02) / (np.sqrt(2) + 0.01)
     tol = 8 * EPS * nequiv / 2 * r21 ** (nequiv / 2)
     assert np.abs(pots[1] - pots[0]).max() <= max(tol, 64 * EPS) * np.abs(pots[0]).max()
+
+
+def test_planned_leaves_beyond_shared_memory():
+    """A planned near pass keeps a leaf's sums in shared memory.  For an Ncutoff that
+    does not fit, the evaluation at the sources is refused, as it always was; the apply
+    and evaluations elsewhere are not, before or after it."""
+    from pykifmm2d_b200 import _lib as B
+    n, cutoff = 30100, 30000
+    x, y, tau = cloud(n, 1)
+    x[4:], y[4:] = np.abs(x[4:]), np.abs(y[4:])  # one quadrant splits: three levels
+    x[:4], y[:4] = -np.abs(x[:4]), -np.abs(y[:4])
+    tx, ty, _ = cloud(200, 2)
+    f = fmm("laplace", 0.0, x, y, cutoff, precision="mixed", planned=True)
+    g = fmm("laplace", 0.0, x, y, cutoff, precision="mixed")
+    assert f.tree_info().levels == 3
+    for h in (f, g):
+        h.build_expansions(tau)
+    ref = g.evaluate_to_points(tx, ty, False)
+    scale = np.abs(ref).max()
+    assert np.abs(f.evaluate_to_points(tx, ty, False) - ref).max() <= 1e-9 * scale
+    with pytest.raises(B.KifmmError):
+        f.evaluate_to_points(x, y, True)
+    assert np.abs(f.evaluate_to_points(tx, ty, False) - ref).max() <= 1e-9 * scale
